@@ -5,14 +5,14 @@
 // features of a candidate order; the order search (order_search.cpp) sums
 // the predictions into a work estimate and keeps the cheapest order.
 //
-// Training is full-batch or mini-batch Adam on the mean squared error.  One
-// fused kernel runs forward + backward for a slice of samples per block,
-// keeping both hidden activations in shared memory, and accumulates the
-// block's gradient in shared memory before one atomic add per parameter.
-// Sizes are tiny (in <= 32, H = 64), so the kernels are latency-bound FP32
-// CUDA-core work; tensor cores are not worth their setup here.
+// Training is full-batch or mini-batch Adam on the mean squared error: two
+// launches per step (k_mlp_grad, k_mlp_adam).  Sizes are tiny (in <= 32,
+// H = 64), so a step is a few microseconds of FP32 CUDA-core work bound by
+// shared-memory latency and launches; tensor cores would mean TF32 or BF16
+// operands, less precision than the FP32 the model is kept in.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -33,8 +33,9 @@ namespace {
 
 constexpr int kH = MLP_HIDDEN;
 constexpr int kMaxIn = MLP_MAX_IN;
-constexpr int kThreads = 256;          // 4 samples in flight per block, 64 threads each
-constexpr int kPerBlock = kThreads / kH;
+constexpr int kThreads = 256;
+constexpr int kRows = 32;              // samples per tile
+constexpr int kS = kH + 4;             // row stride of the 64-wide tiles in shared memory
 
 // parameter layout: W1[H][in] b1[H] W2[H][H] b2[H] W3[H] b3
 __host__ __device__ inline int n_params(int in) { return kH * in + kH + kH * kH + kH + kH + 1; }
@@ -54,94 +55,237 @@ __host__ __device__ inline Layout layout(int in) {
     return L;
 }
 
-// Forward (and, when grad != nullptr, backward) over samples [0, n).
-// loss_acc += sum (y - t)^2; grad += d(mean loss)/d(params).
-__global__ void __launch_bounds__(kThreads)
-k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X,
-      const float *__restrict__ T, int n, float *__restrict__ Y, float *__restrict__ grad,
-      float *__restrict__ loss_acc) {
-    extern __shared__ float sm[];
+// Forward (and, with GRAD, backward) over samples [0, n) in tiles of kRows,
+// grid-strided.  A block keeps the weights and one tile's activations in
+// shared memory and computes 2 rows x 4 units per thread; the gradient is
+// accumulated over the block's tiles in registers (a 4 x 4 tile of dW2, 4 x 2
+// of dW1, one bias or W3 entry per thread) and written once per block to
+// part[block][param], which k_mlp_adam / k_mlp_reduce sum in a fixed order in
+// FP64.  lossp[block] = the block's sum of squared errors.  No atomics: the
+// form with one shared-memory atomic per sample and weight took 260 us for
+// 4,096 rows of 16 features (forward and backward), this one 18 us (both ncu,
+// cold caches); a fit of 48 such steps and a prediction of 6,000 rows, copies
+// included, 13.33 -> 1.39 ms.  Rows of the tiles are
+// padded to 68 words, so 16-byte reads of 8 consecutive rows (W2 by unit) hit
+// 8 different bank groups.
+template <bool GRAD>
+__global__ void __launch_bounds__(kThreads, 2)
+k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, const float *__restrict__ T, int n,
+      float *__restrict__ Y, float *__restrict__ part, double *__restrict__ lossp) {
+    extern __shared__ __align__(16) float sm[];
     const Layout L = layout(in);
-    float *P = sm;                        // params
-    float *G = P + L.total;               // block gradient (only when training)
-    float *x = G + (grad ? L.total : 0);  // [kPerBlock][kMaxIn]
-    float *h1 = x + kPerBlock * kMaxIn;   // [kPerBlock][H]
-    float *h2 = h1 + kPerBlock * kH;      // [kPerBlock][H]
-    float *dh2 = h2 + kPerBlock * kH;     // [kPerBlock][H]
-    float *red = dh2 + kPerBlock * kH;    // [kPerBlock][2]
-    for (int i = threadIdx.x; i < L.total; i += blockDim.x) {
-        P[i] = params[i];
-        if (grad) G[i] = 0.f;
+    const int s1 = in | 1;                 // odd row stride of W1: units on different banks
+    float *W2 = sm;                        // [H][kS]
+    float *h1 = W2 + kH * kS;              // [kRows][kS]
+    float *h2 = h1 + kRows * kS;           // [kRows][kS]: layer 2, then dL/d(layer 2)
+    float *d1 = h2 + kRows * kS;           // [kRows][kS]: dL/d(layer 1)
+    float *B1 = d1 + kRows * kS;           // [H]
+    float *B2 = B1 + kH, *W3 = B2 + kH;
+    float *dy = W3 + kH;                   // [kRows]
+    float *x = dy + kRows;                 // [kRows][in]
+    float *W1 = x + kRows * kMaxIn;        // [H][s1]
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int i = tid; i < kH * kH; i += kThreads) W2[(i / kH) * kS + i % kH] = params[L.w2 + i];
+    for (int i = tid; i < kH * in; i += kThreads) W1[(i / in) * s1 + i % in] = params[L.w1 + i];
+    if (tid < kH) {
+        B1[tid] = params[L.b1 + tid];
+        B2[tid] = params[L.b2 + tid];
+        W3[tid] = params[L.w3 + tid];
     }
-    __syncthreads();
-    const int s = threadIdx.x / kH;   // sample slot in the block
-    const int j = threadIdx.x % kH;   // hidden unit
-    const int lane = threadIdx.x & 31;
-    float lsum = 0.f;
+    const float b3 = params[L.b3];
     const float inv_n = 1.f / float(max(n, 1));
-    for (int base = blockIdx.x * kPerBlock; base < n; base += gridDim.x * kPerBlock) {
-        const int r = base + s;
-        const bool valid = r < n;
-        if (j < in) x[s * kMaxIn + j] = valid ? X[size_t(r) * in + j] : 0.f;
+    float g2[4][4] = {}, g1[4][2] = {}, gv = 0.f;
+    double lsum = 0.0;
+    for (int base = blockIdx.x * kRows; base < n; base += gridDim.x * kRows) {
+        const int rows = min(kRows, n - base);
+        __syncthreads();  // the weights are in; the previous tile is done with
+        for (int i = tid; i < kRows * in; i += kThreads) x[i] = i < rows * in ? X[size_t(base) * in + i] : 0.f;
         __syncthreads();
-        // layer 1
-        float a = P[L.b1 + j];
-        for (int f = 0; f < in; ++f) a += P[L.w1 + j * in + f] * x[s * kMaxIn + f];
-        const float z1 = fmaxf(a, 0.f);
-        h1[s * kH + j] = z1;
+        float acc[2][4], z2[2][4];
+        // layer 1: units tx + 16 q of rows ty, ty + 16
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) acc[0][q] = acc[1][q] = B1[tx + 16 * q];
+        for (int f = 0; f < in; ++f) {
+            const float xa = x[ty * in + f], xb = x[(ty + 16) * in + f];
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float w = W1[(tx + 16 * q) * s1 + f];
+                acc[0][q] += w * xa;
+                acc[1][q] += w * xb;
+            }
+        }
+        #pragma unroll
+        for (int r = 0; r < 2; ++r)
+            #pragma unroll
+            for (int q = 0; q < 4; ++q)
+                h1[(ty + 16 * r) * kS + tx + 16 * q] = ty + 16 * r < rows ? fmaxf(acc[r][q], 0.f) : 0.f;
         __syncthreads();
         // layer 2
-        float b = P[L.b2 + j];
-        for (int i = 0; i < kH; ++i) b += P[L.w2 + j * kH + i] * h1[s * kH + i];
-        const float z2 = fmaxf(b, 0.f);
-        h2[s * kH + j] = z2;
-        // output: two warps per sample slot reduce w3 . h2
-        float o = P[L.w3 + j] * z2;
         #pragma unroll
-        for (int d = 16; d; d >>= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
-        if (lane == 0) red[s * 2 + (j >> 5)] = o;
-        __syncthreads();
-        const float y = red[s * 2] + red[s * 2 + 1] + P[L.b3];
-        if (valid && j == 0 && Y) Y[r] = y;
-        float dy = 0.f;
-        if (valid && T) {
-            const float e = y - T[r];
-            if (j == 0) lsum += e * e;
-            dy = 2.f * e * inv_n;
+        for (int q = 0; q < 4; ++q) acc[0][q] = acc[1][q] = B2[tx + 16 * q];
+        #pragma unroll 4
+        for (int i = 0; i < kH; i += 4) {
+            const float4 a = *reinterpret_cast<const float4 *>(h1 + ty * kS + i);
+            const float4 b = *reinterpret_cast<const float4 *>(h1 + (ty + 16) * kS + i);
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 w = *reinterpret_cast<const float4 *>(W2 + (tx + 16 * q) * kS + i);
+                acc[0][q] += w.x * a.x; acc[0][q] += w.y * a.y; acc[0][q] += w.z * a.z; acc[0][q] += w.w * a.w;
+                acc[1][q] += w.x * b.x; acc[1][q] += w.y * b.y; acc[1][q] += w.z * b.z; acc[1][q] += w.w * b.w;
+            }
         }
-        if (grad && valid) {
-            // output layer
-            atomicAdd(&G[L.w3 + j], dy * z2);
-            if (j == 0) atomicAdd(&G[L.b3], dy);
-            const float d2 = z2 > 0.f ? dy * P[L.w3 + j] : 0.f;
-            dh2[s * kH + j] = d2;
-            atomicAdd(&G[L.b2 + j], d2);
-            for (int i = 0; i < kH; ++i) atomicAdd(&G[L.w2 + j * kH + i], d2 * h1[s * kH + i]);
+        // output: the 16 threads of a row reduce w3 . h2
+        #pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float o = 0.f;
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                z2[r][q] = fmaxf(acc[r][q], 0.f);
+                o += W3[tx + 16 * q] * z2[r][q];
+            }
+            #pragma unroll
+            for (int d = 8; d; d >>= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
+            const int row = ty + 16 * r;
+            const bool valid = row < rows;
+            const float y = o + b3;
+            float e = 0.f;
+            if (valid && T) e = y - T[base + row];
+            const float de = 2.f * e * inv_n;
+            if (tx == 0) {
+                if (valid && Y) Y[base + row] = y;
+                if (valid) lsum += double(e) * double(e);
+                if (GRAD) dy[row] = de;
+            }
+            if (GRAD)
+                #pragma unroll
+                for (int q = 0; q < 4; ++q) h2[row * kS + tx + 16 * q] = valid ? z2[r][q] : 0.f;
         }
-        __syncthreads();
-        if (grad && valid) {
-            // hidden unit j of layer 1
-            float d1 = 0.f;
-            for (int i = 0; i < kH; ++i) d1 += P[L.w2 + i * kH + j] * dh2[s * kH + i];
-            d1 = z1 > 0.f ? d1 : 0.f;
-            atomicAdd(&G[L.b1 + j], d1);
-            for (int f = 0; f < in; ++f) atomicAdd(&G[L.w1 + j * in + f], d1 * x[s * kMaxIn + f]);
+        if constexpr (GRAD) {
+            __syncthreads();
+            // dW3 and db3, before layer 2's values make room for its gradient
+            if (tid >= 128 && tid < 192) {
+                for (int r = 0; r < kRows; ++r) gv += dy[r] * h2[r * kS + tid - 128];
+            } else if (tid == 192) {
+                for (int r = 0; r < kRows; ++r) gv += dy[r];
+            }
+            __syncthreads();
+            #pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int row = ty + 16 * r;
+                const float de = dy[row];
+                #pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    h2[row * kS + tx + 16 * q] = row < rows && z2[r][q] > 0.f ? de * W3[tx + 16 * q] : 0.f;
+            }
+            __syncthreads();
+            // dL/d(layer 1): units 4 tx .. 4 tx + 3 of rows ty, ty + 16
+            float e1[2][4] = {};
+            #pragma unroll 4
+            for (int j = 0; j < kH; ++j) {
+                const float4 w = *reinterpret_cast<const float4 *>(W2 + j * kS + 4 * tx);
+                const float a = h2[ty * kS + j], b = h2[(ty + 16) * kS + j];
+                e1[0][0] += w.x * a; e1[0][1] += w.y * a; e1[0][2] += w.z * a; e1[0][3] += w.w * a;
+                e1[1][0] += w.x * b; e1[1][1] += w.y * b; e1[1][2] += w.z * b; e1[1][3] += w.w * b;
+            }
+            #pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int row = ty + 16 * r;
+                const float4 z = *reinterpret_cast<const float4 *>(h1 + row * kS + 4 * tx);
+                *reinterpret_cast<float4 *>(d1 + row * kS + 4 * tx) =
+                    make_float4(z.x > 0.f ? e1[r][0] : 0.f, z.y > 0.f ? e1[r][1] : 0.f, z.z > 0.f ? e1[r][2] : 0.f,
+                                z.w > 0.f ? e1[r][3] : 0.f);
+            }
+            // dW2[4 ty + a][4 tx + b] over the tile's rows
+            #pragma unroll 4
+            for (int r = 0; r < kRows; ++r) {
+                const float4 d = *reinterpret_cast<const float4 *>(h2 + r * kS + 4 * ty);
+                const float4 h = *reinterpret_cast<const float4 *>(h1 + r * kS + 4 * tx);
+                const float dd[4] = {d.x, d.y, d.z, d.w}, hh[4] = {h.x, h.y, h.z, h.w};
+                #pragma unroll
+                for (int a = 0; a < 4; ++a)
+                    #pragma unroll
+                    for (int b = 0; b < 4; ++b) g2[a][b] += dd[a] * hh[b];
+            }
+            __syncthreads();
+            // dW1[4 ty + a][tx + 16 c], and the two bias gradients
+            for (int r = 0; r < kRows; ++r) {
+                const float4 d = *reinterpret_cast<const float4 *>(d1 + r * kS + 4 * ty);
+                #pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int f = tx + 16 * c;
+                    if (f < in) {
+                        const float v = x[r * in + f];
+                        g1[0][c] += d.x * v; g1[1][c] += d.y * v; g1[2][c] += d.z * v; g1[3][c] += d.w * v;
+                    }
+                }
+            }
+            if (tid < 128) {
+                const float *src = tid < 64 ? d1 + tid : h2 + tid - 64;
+                for (int r = 0; r < kRows; ++r) gv += src[r * kS];
+            }
         }
-        __syncthreads();
     }
-    if (grad) {
-        for (int i = threadIdx.x; i < L.total; i += blockDim.x)
-            if (G[i] != 0.f) atomicAdd(&grad[i], G[i]);
+    if constexpr (GRAD) {
+        float *out = part + size_t(blockIdx.x) * L.total;
+        #pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            #pragma unroll
+            for (int b = 0; b < 4; ++b) out[L.w2 + (4 * ty + a) * kH + 4 * tx + b] = g2[a][b];
+            #pragma unroll
+            for (int c = 0; c < 2; ++c)
+                if (tx + 16 * c < in) out[L.w1 + (4 * ty + a) * in + tx + 16 * c] = g1[a][c];
+        }
+        if (tid < 64) out[L.b1 + tid] = gv;
+        else if (tid < 128) out[L.b2 + tid - 64] = gv;
+        else if (tid < 192) out[L.w3 + tid - 128] = gv;
+        else if (tid == 192) out[L.b3] = gv;
     }
-    if (loss_acc && j == 0 && lsum != 0.f) atomicAdd(loss_acc, lsum);
+    if (lossp) {
+        // tx == 0 threads (lanes 0 and 16 of each warp) hold the sums
+        __shared__ double lred[kThreads / 16];
+        if (tx == 0) lred[ty] = lsum;
+        __syncthreads();
+        if (tid == 0) {
+            double s = 0.0;
+            for (int i = 0; i < kThreads / 16; ++i) s += lred[i];
+            lossp[blockIdx.x] = s;
+        }
+    }
 }
 
-// Adam (Kingma & Ba 2015) with bias correction.
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                       float *__restrict__ v, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
+// Sum of the blocks' partial gradients, 32 parameters x 8 groups of blocks
+// per thread block, in FP64 and in a fixed order; the group-0 threads return
+// it.  Each thread reads nparts / 8 values, independent loads in flight.
+__device__ __forceinline__ float partial_sum(const float *__restrict__ part, int nparts, int total, int i) {
+    __shared__ double red[8][33];
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+    double s = 0.0;
+    if (i < total) {
+        #pragma unroll 8
+        for (int b = grp; b < nparts; b += 8) s += double(part[size_t(b) * total + i]);
+    }
+    red[grp][lane] = s;
+    __syncthreads();
+    s = 0.0;
+    if (grp == 0)
+        for (int q = 0; q < 8; ++q) s += red[q][lane];
+    return float(s);
+}
+
+__global__ void __launch_bounds__(256)
+k_mlp_reduce(const float *__restrict__ part, int nparts, int total, float *__restrict__ g) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float v = partial_sum(part, nparts, total, i);
+    if (threadIdx.x < 32 && i < total) g[i] = v;
+}
+
+// Adam (Kingma & Ba 2015) with bias correction, on the summed partials.
+__global__ void __launch_bounds__(256)
+k_mlp_adam(float *__restrict__ p, const float *__restrict__ part, int nparts, float *__restrict__ m,
+           float *__restrict__ v, int total, float lr, float b1, float b2, float eps, float c1, float c2) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float gi = partial_sum(part, nparts, total, i);
+    if (threadIdx.x < 32 && i < total) {
         const float mi = b1 * m[i] + (1.f - b1) * gi;
         const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
         m[i] = mi;
@@ -150,10 +294,9 @@ __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float
     }
 }
 
-size_t smem_bytes(int in, bool train) {
-    const int total = layout(in).total;
-    return sizeof(float) * (size_t(total) * (train ? 2 : 1) + kPerBlock * kMaxIn + 3 * kPerBlock * kH +
-                            2 * kPerBlock);
+size_t smem_bytes(int in) {
+    return sizeof(float) * (size_t(kH) * kS + 3 * size_t(kRows) * kS + 3 * kH + kRows + kRows * kMaxIn +
+                            size_t(kH) * (in | 1));
 }
 
 }  // namespace
@@ -166,12 +309,15 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
     device = dev;
     MCK(cudaSetDevice(device));
     const int np = n_params(in);
+    // blocks of the training kernel, at most: one per SM
+    MCK(cudaDeviceGetAttribute(&max_blocks, cudaDevAttrMultiProcessorCount, device));
     MCK(cudaMalloc(&d_params, sizeof(float) * np * 4));  // params, grad, adam m, adam v
     d_grad = d_params + np;
     d_m = d_grad + np;
     d_v = d_m + np;
     MCK(cudaMemset(d_params, 0, sizeof(float) * np * 4));
-    MCK(cudaMalloc(&d_scalar, sizeof(float) * 4));
+    MCK(cudaMalloc(&d_loss, sizeof(double) * max_blocks));
+    MCK(cudaMalloc(&d_part, sizeof(float) * size_t(np) * max_blocks));
     // He-uniform initialisation from a splitmix64 stream
     std::vector<float> h(np, 0.f);
     const Layout L = layout(in);
@@ -181,8 +327,8 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
     for (int i = 0; i < kH * kH; ++i) h[L.w2 + i] = uni(std::sqrt(6.f / kH));
     for (int i = 0; i < kH; ++i) h[L.w3 + i] = uni(std::sqrt(6.f / kH));
     MCK(cudaMemcpy(d_params, h.data(), sizeof(float) * np, cudaMemcpyHostToDevice));
-    MCK(cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(smem_bytes(kMaxIn, true))));
+    MCK(cudaFuncSetAttribute(k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes(kMaxIn))));
+    MCK(cudaFuncSetAttribute(k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes(kMaxIn))));
     step = 0;
     return CUTS_OK;
 }
@@ -191,10 +337,12 @@ void Mlp::destroy() {
     if (d_params) {
         cudaSetDevice(device);
         cudaFree(d_params);
-        cudaFree(d_scalar);
+        cudaFree(d_loss);
+        cudaFree(d_part);
         cudaFree(d_X);
     }
-    d_params = d_grad = d_m = d_v = d_scalar = d_X = nullptr;
+    d_params = d_grad = d_m = d_v = d_part = d_X = nullptr;
+    d_loss = nullptr;
 }
 
 int Mlp::upload(const float *X, const float *T, int n) {
@@ -210,26 +358,30 @@ int Mlp::upload(const float *X, const float *T, int n) {
     return CUTS_OK;
 }
 
-static int grid_for(int n) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return std::max(1, std::min((n + kPerBlock - 1) / kPerBlock, sms * 2));
+int Mlp::grid_for(int n) const { return std::max(1, std::min((n + kRows - 1) / kRows, max_blocks)); }
+
+// Mean of the blocks' sums of squared errors.
+int Mlp::read_loss(int blocks, int n, float *loss) {
+    std::vector<double> h(static_cast<size_t>(blocks));
+    MCK(cudaMemcpy(h.data(), d_loss, sizeof(double) * size_t(blocks), cudaMemcpyDeviceToHost));
+    double l = 0;
+    for (double v : h) l += v;
+    *loss = float(l / double(std::max(n, 1)));
+    return CUTS_OK;
 }
 
 int Mlp::loss_grad(const float *X, const float *T, int n, float *loss, float *grad_out) {
     MCK(cudaSetDevice(device));
     int rc = upload(X, T, n);
     if (rc) return rc;
-    const int np = n_params(in);
-    MCK(cudaMemset(d_grad, 0, sizeof(float) * np));
-    MCK(cudaMemset(d_scalar, 0, sizeof(float)));
-    k_mlp<<<grid_for(n), kThreads, smem_bytes(in, true)>>>(d_params, in, d_X, d_X + size_t(cap_rows) * in,
-                                                         n, nullptr, d_grad, d_scalar);
+    const int np = n_params(in), blocks = grid_for(n);
+    k_mlp<true><<<blocks, kThreads, smem_bytes(in)>>>(d_params, in, d_X, d_X + size_t(cap_rows) * in, n, nullptr,
+                                                     d_part, d_loss);
+    k_mlp_reduce<<<(np + 31) / 32, 256>>>(d_part, blocks, np, d_grad);
     MCK(cudaGetLastError());
     float l = 0;
-    MCK(cudaMemcpy(&l, d_scalar, sizeof(float), cudaMemcpyDeviceToHost));
-    if (loss) *loss = l / float(std::max(n, 1));
+    if ((rc = read_loss(blocks, n, &l))) return rc;
+    if (loss) *loss = l;
     if (grad_out) MCK(cudaMemcpy(grad_out, d_grad, sizeof(float) * np, cudaMemcpyDeviceToHost));
     return CUTS_OK;
 }
@@ -245,23 +397,20 @@ int Mlp::train(const float *X, const float *T, int n, int epochs, int batch, flo
     const float *dT = d_X + size_t(cap_rows) * in;
     for (int e = 0; e < epochs; ++e) {
         for (int s0 = 0; s0 < n; s0 += batch) {
-            const int nb = std::min(batch, n - s0);
-            MCK(cudaMemsetAsync(d_grad, 0, sizeof(float) * np));
-            k_mlp<<<grid_for(nb), kThreads, smem_bytes(in, true)>>>(d_params, in, d_X + size_t(s0) * in,
-                                                                  dT + s0, nb, nullptr, d_grad, nullptr);
+            const int nb = std::min(batch, n - s0), blocks = grid_for(nb);
+            k_mlp<true><<<blocks, kThreads, smem_bytes(in)>>>(d_params, in, d_X + size_t(s0) * in, dT + s0, nb, nullptr,
+                                                             d_part, nullptr);
             ++step;
             const float c1 = 1.f - std::pow(b1, float(step)), c2 = 1.f - std::pow(b2, float(step));
-            k_adam<<<(np + 255) / 256, 256>>>(d_params, d_grad, d_m, d_v, np, lr, b1, b2, eps, c1, c2);
+            k_mlp_adam<<<(np + 31) / 32, 256>>>(d_params, d_part, blocks, d_m, d_v, np, lr, b1, b2, eps, c1, c2);
         }
     }
     MCK(cudaGetLastError());
     if (final_loss) {
-        MCK(cudaMemset(d_scalar, 0, sizeof(float)));
-        k_mlp<<<grid_for(n), kThreads, smem_bytes(in, false)>>>(d_params, in, d_X, dT, n, nullptr, nullptr,
-                                                              d_scalar);
-        float l = 0;
-        MCK(cudaMemcpy(&l, d_scalar, sizeof(float), cudaMemcpyDeviceToHost));
-        *final_loss = l / float(std::max(n, 1));
+        const int blocks = grid_for(n);
+        k_mlp<false><<<blocks, kThreads, smem_bytes(in)>>>(d_params, in, d_X, dT, n, nullptr, nullptr, d_loss);
+        MCK(cudaGetLastError());
+        if ((rc = read_loss(blocks, n, final_loss))) return rc;
     }
     MCK(cudaDeviceSynchronize());
     return CUTS_OK;
@@ -272,8 +421,7 @@ int Mlp::predict(const float *X, int n, float *Y) {
     int rc = upload(X, nullptr, n);
     if (rc) return rc;
     float *dY = d_X + size_t(cap_rows) * in;  // reuse the target slot
-    k_mlp<<<grid_for(n), kThreads, smem_bytes(in, false)>>>(d_params, in, d_X, nullptr, n, dY, nullptr,
-                                                          nullptr);
+    k_mlp<false><<<grid_for(n), kThreads, smem_bytes(in)>>>(d_params, in, d_X, nullptr, n, dY, nullptr, nullptr);
     MCK(cudaGetLastError());
     MCK(cudaMemcpy(Y, dY, sizeof(float) * n, cudaMemcpyDeviceToHost));
     return CUTS_OK;

@@ -16,7 +16,9 @@ struct Mlp {
     int in = 0;
     int device = 0;
     float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr;
-    float *d_scalar = nullptr;
+    float *d_part = nullptr;    // [max_blocks][params]: partial gradients of one step
+    double *d_loss = nullptr;   // [max_blocks]: partial sums of squared errors
+    int max_blocks = 1;
     float *d_X = nullptr;  // staged samples: X rows, then targets / outputs
     int cap_rows = 0;
     int64_t step = 0;
@@ -34,6 +36,8 @@ struct Mlp {
 
   private:
     int upload(const float *X, const float *T, int n);
+    int grid_for(int n) const;
+    int read_loss(int blocks, int n, float *loss);
 };
 
 }  // namespace cuts
