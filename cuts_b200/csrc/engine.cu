@@ -101,10 +101,9 @@ __device__ __forceinline__ uint32_t orbit_base(const DevView &g, const LevelPlan
     for (uint32_t xm = F.ofold & ((1u << upto) - 1); xm; xm &= xm - 1) {
         const uint32_t x = __ffs(xm) - 1;
         const uint2 inf = F.jdir[0] ? g.in_info[m(x)] : g.out_info[m(x)];
-        const uint32_t *l = g.adj + inf.x;
         uint32_t sub = 0;
         for (uint32_t j = 0; j < upto; ++j)
-            if (((F.oguar[x] >> j) & 1u) || contains(l, inf.y, m(j))) ++sub;
+            if (((F.oguar[x] >> j) & 1u) || in_list(g, inf.x, inf.y, m(j))) ++sub;
         base += inf.y - sub;
     }
     return base;
@@ -119,7 +118,7 @@ __device__ __forceinline__ uint32_t orbit_weight(const DevView &g, const LevelPl
     if ((F.ofold >> c) & 1u) {
         const uint2 ti = F.jdir[0] ? g.in_info[t] : g.out_info[t];
         w += ti.y - c;
-        if (loops && contains(g.adj + ti.x, ti.y, t)) --w;
+        if (loops && in_list(g, ti.x, ti.y, t)) --w;
     }
     return w;
 }
@@ -154,7 +153,7 @@ __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const Le
         uint32_t sub = 0;
         for (uint32_t j = 0; j <= lvl; ++j) {
             const uint32_t mj = m(j);
-            if (mj >= lo[r] && mj < hi[r] && (((guar >> j) & 1u) || contains(l, len[r], mj))) ++sub;
+            if (mj >= lo[r] && mj < hi[r] && (((guar >> j) & 1u) || in_list(g, off[r], len[r], mj))) ++sub;
         }
         cnt[r] = e0[r] - s0[r] - sub;
     }
@@ -171,8 +170,8 @@ __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const Le
         for (uint32_t j = 0; j <= lvl; ++j) {
             const uint32_t mj = m(j);
             if (mj < wlo || mj >= whi) continue;
-            const bool in0 = ((A.guar1 >> j) & 1u) || contains(g.adj + off[0], len[0], mj);
-            const bool in1 = ((B.guar_mask >> j) & 1u) || contains(g.adj + off[1], len[1], mj);
+            const bool in0 = ((A.guar1 >> j) & 1u) || in_list(g, off[0], len[0], mj);
+            const bool in1 = ((B.guar_mask >> j) & 1u) || in_list(g, off[1], len[1], mj);
             if (in0 && in1) --both;
         }
     }
@@ -394,6 +393,7 @@ k_level(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t pa, 
                 const uint32_t x = x0 + lane;
                 bool ok = x < e0;
                 const uint32_t c = ok ? __ldg(mlist + x) : 0;
+                ok = ok && c >= sL.sig_lo;
                 if (ok)
                     for (uint32_t j = 0; j < lvl; ++j)
                         if (c == my_m[j]) { ok = false; break; }
@@ -440,23 +440,41 @@ k_level(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t pa, 
 }
 
 // ---- levels 1..k-1, flattened form ------------------------------------
-// A warp takes 32 consecutive parents, one per lane.  Each lane rebuilds its
-// parent's partial match (32 pointer chases in flight at once), gathers its
-// joined lists and picks the shortest.  The candidate lists of the 32
-// parents are then treated as one concatenated sequence: an inclusive warp
-// scan of their lengths gives every lane, at every step, the parent that
-// owns candidate f = step*32 + lane (a 5-step binary search over the scan
-// with shuffles), so all 32 lanes stay busy whether the lists hold 2 or
-// 20,000 entries.  Per-parent state lives in the owner lane's registers
-// (read with shuffles) and in shared memory laid out [join][lane], so lanes
-// reading different owners hit different banks.  Last-level parents with a
-// single joined list and no signature are counted by the closed form, one
-// parent per lane.
+// A warp takes up to 32 consecutive parents, one per lane.  Each lane
+// rebuilds its parent's partial match (pointer chases of all lanes in flight
+// at once), gathers its joined lists and picks the shortest.  The candidate
+// lists of the parents are then one concatenated sequence, walked 64
+// candidates a step, so all lanes stay busy whether the lists hold 2 or
+// 20,000 entries.  The non-empty parents are compacted to ranks and what a
+// candidate needs of its owner (where its window lies in the adjacency array,
+// the first other list to test, the owner's lane) is one 16-byte record in
+// shared memory; the owner of candidate f is the number of windows starting
+// at or before f, from one warp-wide OR of the start bits of the step and a
+// population count (a binary search over the scan took 5 dependent shuffles,
+// and 6 more fetched the record).  Membership in the other lists is a
+// one-load table test (in_list) and injectivity is checked after it, on the
+// few that pass; a signature on a degree-ranked symmetric graph is a compare
+// of ids (sig_lo).  What bounds it: instruction issue where the lists are
+// L1/L2 resident, L2 latency otherwise.  Measured against the form with
+// galloping searches, a shuffle search for the owner and 32 parents per warp
+// always (whole counts): house, 100,000 vertices / 500,000 edges, plain
+// 75.5 -> 23.5 ms; 5-cycle, 200,003 / 1M, symmetry breaking 649 -> 347 ms;
+// 4-cycle, 10,000 / 40,000 0.252 -> 0.176 ms; a directed four-vertex query,
+// 150,001 / 1.5M arcs 6.98 -> 3.43 ms.
 constexpr int kFW = 4;    // warps per block
 constexpr int kFJ = 8;    // joined lists per level in this form (more: warp-per-parent kernel)
 
-template <int MODE>
-__global__ void __launch_bounds__(kFW * 32)
+// Words of dynamic shared memory per warp: the parents' matches, their joined
+// lists, the owners' records and start offsets, and the staged output.
+__host__ __device__ inline uint32_t flat_words(uint32_t lvl, uint32_t nj, bool expand) {
+    return 32 * lvl + 64 * nj + 128 + 32 + (expand ? 3 * kOutBuf : 0);
+}
+
+// MODE kExpand writes L_lvl, kCountMode counts, kBytesMode adds the bytes the
+// count reads.  FOLD: the level also counts the one or two after it (plain or
+// orbit fold, pendant pair).
+template <int MODE, bool FOLD>
+__global__ void __launch_bounds__(kFW * 32, FOLD ? 8 : 10)
 k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t pa, uint32_t pb,
              uint32_t *__restrict__ cursor, uint32_t *__restrict__ out_n, uint32_t out_cap,
              uint32_t *__restrict__ err, unsigned long long *__restrict__ acc,
@@ -464,40 +482,40 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     __shared__ LevelPlan sL, sN, sN2;
     __shared__ uint32_t *s_vert[kMaxK];
     __shared__ uint32_t *s_par[kMaxK];
-    __shared__ uint32_t s_k, s_sym, s_stored;
-    __shared__ uint32_t sm_m[kFW][kMaxK][33];   // [position][lane]
-    __shared__ uint32_t sm_off[kFW][kFJ][32], sm_deg[kFW][kFJ][32];
-    __shared__ uint32_t ob_v[MODE == kExpand ? kFW : 1][kOutBuf];
-    __shared__ uint32_t ob_p[MODE == kExpand ? kFW : 1][kOutBuf];
-    __shared__ uint32_t ob_u[MODE == kExpand ? kFW : 1][kOutBuf];
+    extern __shared__ __align__(16) uint32_t dyn[];
     {
         const uint32_t words = sizeof(LevelPlan) / 4;
-        const uint32_t *srcL = reinterpret_cast<const uint32_t *>(&rp->plan.lv[lvl]);
-        uint32_t *dL = reinterpret_cast<uint32_t *>(&sL);
-        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dL[i] = srcL[i];
         const uint32_t nl = lvl + 1 < rp->plan.k ? lvl + 1 : lvl;
-        const uint32_t *srcN = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl]);
-        uint32_t *dN = reinterpret_cast<uint32_t *>(&sN);
-        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dN[i] = srcN[i];
         const uint32_t nl2 = lvl + 2 < rp->plan.k ? lvl + 2 : nl;
-        const uint32_t *srcN2 = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl2]);
-        uint32_t *dN2 = reinterpret_cast<uint32_t *>(&sN2);
-        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dN2[i] = srcN2[i];
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
+            reinterpret_cast<uint32_t *>(&sL)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[lvl])[i];
+            reinterpret_cast<uint32_t *>(&sN)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl])[i];
+            if (FOLD) reinterpret_cast<uint32_t *>(&sN2)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl2])[i];
+        }
         if (threadIdx.x < kMaxK) {
             s_vert[threadIdx.x] = rp->vert[threadIdx.x];
             s_par[threadIdx.x] = rp->par[threadIdx.x];
         }
-        if (threadIdx.x == 0) { s_k = rp->plan.k; s_sym = rp->plan.symmetric; s_stored = rp->stored; }
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t lanemask_lt = (1u << lane) - 1;
-    const bool sym = s_sym != 0;
+    const uint32_t lanemask_lt = (1u << lane) - 1, lanemask_le = lanemask_lt | (1u << lane);
+    const bool sym = rp->plan.symmetric != 0;
+    const uint32_t nj = sL.nj;
+    uint32_t *const wbase = dyn + warp * flat_words(lvl, nj, MODE == kExpand);
+    uint4 *const rec = reinterpret_cast<uint4 *>(wbase);      // [rank]: {window base - start, lane | source join << 8,
+                                                              //          first other list's offset, its length}
+    uint32_t *const starts = wbase + 128;                     // [rank]
+    uint32_t *const sm_off = starts + 32;                     // [join][lane]
+    uint32_t *const sm_deg = sm_off + 32 * nj;                // [join][lane]
+    uint32_t *const sm_m = sm_deg + 32 * nj;                  // [position][lane]
+    uint32_t *const ob_v = sm_m + 32 * lvl;                   // staged output (expand)
+    uint32_t *const ob_p = ob_v + kOutBuf, *const ob_u = ob_p + kOutBuf;
     // pendant pair: this level (k-3) also counts levels k-2 and k-1
-    const uint32_t fold2 = MODE != kExpand ? sL.fold2 : 0u;
+    const uint32_t fold2 = FOLD && MODE != kExpand ? sL.fold2 : 0u;
     unsigned long long local3 = 0;
     const bool store_pos = MODE == kExpand && lvl == rp->pos_lvl;
-    const bool need_ub = (MODE == kExpand && lvl + 1 < s_stored) || store_pos;
+    const bool need_ub = (MODE == kExpand && lvl + 1 < rp->stored) || store_pos;
     uint32_t *out_v = MODE == kExpand ? rp->vert[lvl] : nullptr;
     uint32_t *out_p = MODE == kExpand ? rp->par[lvl] : nullptr;
     uint32_t *out_u = MODE == kExpand ? rp->ub[lvl] : nullptr;
@@ -505,17 +523,20 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     if (need_ub && !store_pos)
         for (uint32_t t = 0; t < sN.nj; ++t)
             if (sN.jpos[t] == lvl) (sN.jdir[t] ? ub_in : ub_out) = true;
-    const uint32_t nj = sL.nj;
     const bool check_sig = sL.check_sig != 0;
-    const bool load_info = check_sig || ub_out || ub_in;
+    const uint32_t sig_lo = sL.sig_lo;
     const bool closed = MODE == kCountMode && sL.closed_form;
     // level k-2 counting level k-1 too: each candidate c adds the last
     // level's closed form, |window of L| - matched vertices in it, where L
     // is an earlier vertex's list and c itself is one of the matched
-    const bool fold = MODE != kExpand && sL.fold;
+    const bool fold = FOLD && MODE != kExpand && sL.fold;
     const bool fold_guar_c = fold && ((sN.guar_mask >> lvl) & 1u);
     const bool loops = rp->plan.data_loops != 0;
     const uint32_t total = pb - pa;
+    // parents per warp: fewer than 32 when that leaves warps without any (a
+    // level of few parents with long lists)
+    const uint32_t nwarps = gridDim.x * kFW;
+    const uint32_t grab = min(32u, max(1u, (total + nwarps - 1) / nwarps));
     const unsigned long long deadline = run_deadline(rp);
     unsigned long long local = 0, local2 = 0;
     uint32_t obn = 0;
@@ -528,9 +549,9 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
         base = __shfl_sync(kFullMask, base, 0);
         if (base + obn <= out_cap && base + obn >= base) {
             for (uint32_t i = lane; i < obn; i += 32) {
-                out_v[base + i] = ob_v[warp][i];
-                out_p[base + i] = ob_p[warp][i];
-                if (need_ub) out_u[base + i] = ob_u[warp][i];
+                out_v[base + i] = ob_v[i];
+                out_p[base + i] = ob_p[i];
+                if (need_ub) out_u[base + i] = ob_u[i];
             }
         } else if (lane == 0) {
             atomicOr(err, 1u);
@@ -541,39 +562,37 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
 
     while (true) {
         uint32_t start = 0;
-        if (lane == 0) start = past_deadline(rp, deadline) ? total : atomicAdd(cursor, 32u);
+        if (lane == 0) start = past_deadline(rp, deadline) ? total : atomicAdd(cursor, grab);
         start = __shfl_sync(kFullMask, start, 0);
         if (start >= total) break;
         const uint32_t p = pa + start + lane;
-        const bool have = start + lane < total;
+        const bool have = uint32_t(lane) < grab && start + lane < total;
         // this lane's parent: partial match into column `lane`
         if (have) {
             uint32_t e = p;
             for (int j = int(lvl) - 1; j >= 0; --j) {
-                sm_m[warp][j][lane] = s_vert[j][e];
+                sm_m[32 * j + lane] = s_vert[j][e];
                 if (j > 0) e = s_par[j][e];
             }
         }
         // joined lists, shortest first
         uint32_t moff = 0, mdeg = 0, tmin = 0, s0 = 0, e0 = 0, ubp = kFullMask;
         uint32_t f_off = 0, f_deg = 0, f_lo = 0, f_hi = kFullMask, fbase = 0;
-        unsigned long long bytes = 0;
         if (have) {
             mdeg = kFullMask;
             for (uint32_t t = 0; t < nj; ++t) {
-                const uint32_t u = sm_m[warp][sL.jpos[t]][lane];
+                const uint32_t u = sm_m[32 * sL.jpos[t] + lane];
                 const uint2 inf = sL.jdir[t] ? g.in_info[u] : g.out_info[u];
-                sm_off[warp][t][lane] = inf.x;
-                sm_deg[warp][t][lane] = inf.y;
-                if (MODE == kBytesMode) bytes += 4ull * inf.y + 8;
+                sm_off[32 * t + lane] = inf.x;
+                sm_deg[32 * t + lane] = inf.y;
                 if (inf.y < mdeg) { mdeg = inf.y; moff = inf.x; tmin = t; }
             }
             if (nj == 0) mdeg = 0;
             uint32_t lo = 0, hi = kFullMask;
-            for (uint32_t msk = sL.gt_mask; msk; msk &= msk - 1) lo = max(lo, sm_m[warp][__ffs(msk) - 1][lane] + 1);
-            for (uint32_t msk = sL.lt_mask; msk; msk &= msk - 1) hi = min(hi, sm_m[warp][__ffs(msk) - 1][lane]);
+            for (uint32_t msk = sL.gt_mask; msk; msk &= msk - 1) lo = max(lo, sm_m[32 * (__ffs(msk) - 1) + lane] + 1);
+            for (uint32_t msk = sL.lt_mask; msk; msk &= msk - 1) hi = min(hi, sm_m[32 * (__ffs(msk) - 1) + lane]);
             const uint32_t *lst = g.adj + moff;
-            const uint32_t mu = nj ? sm_m[warp][sL.jpos[tmin]][lane] : 0;
+            const uint32_t mu = nj ? sm_m[32 * sL.jpos[tmin] + lane] : 0;
             const bool mdir = nj && sL.jdir[tmin];
             s0 = lo ? lbound_own(g, mdir, mu, lst, mdeg, lo, loops) : 0;
             e0 = hi != kFullMask ? lbound_own(g, mdir, mu, lst, mdeg, hi, loops) : mdeg;
@@ -581,65 +600,64 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
             if (need_ub)
                 for (uint32_t t = 0; t < sN.nj; ++t)
                     if (sN.jpos[t] < lvl) {
-                        const uint32_t u = sm_m[warp][sN.jpos[t]][lane];
+                        const uint32_t u = sm_m[32 * sN.jpos[t] + lane];
                         ubp = min(ubp, (sN.jdir[t] ? g.in_info[u] : g.out_info[u]).y);
                     }
             if (fold && sN.ofold) {
-                fbase = orbit_base(g, sN, lvl, [&](uint32_t j) { return sm_m[warp][j][lane]; });
+                fbase = orbit_base(g, sN, lvl, [&](uint32_t j) { return sm_m[32 * j + lane]; });
             } else if (fold) {
-                const uint32_t u = sm_m[warp][sN.jpos[0]][lane];
+                const uint32_t u = sm_m[32 * sN.jpos[0] + lane];
                 const uint2 inf = sN.jdir[0] ? g.in_info[u] : g.out_info[u];
                 f_off = inf.x;
                 f_deg = inf.y;
-                for (uint32_t msk = sN.gt_mask; msk; msk &= msk - 1) f_lo = max(f_lo, sm_m[warp][__ffs(msk) - 1][lane] + 1);
-                for (uint32_t msk = sN.lt_mask; msk; msk &= msk - 1) f_hi = min(f_hi, sm_m[warp][__ffs(msk) - 1][lane]);
+                for (uint32_t msk = sN.gt_mask; msk; msk &= msk - 1) f_lo = max(f_lo, sm_m[32 * (__ffs(msk) - 1) + lane] + 1);
+                for (uint32_t msk = sN.lt_mask; msk; msk &= msk - 1) f_hi = min(f_hi, sm_m[32 * (__ffs(msk) - 1) + lane]);
                 const uint32_t *fl = g.adj + f_off;
                 const uint32_t ws = f_lo ? lbound(fl, f_deg, f_lo) : 0;
                 const uint32_t we = f_hi != kFullMask ? lbound(fl, f_deg, f_hi) : f_deg;
                 uint32_t sub = 0;
                 for (uint32_t j = 0; j < lvl; ++j) {
-                    const uint32_t mj = sm_m[warp][j][lane];
-                    if (mj >= f_lo && mj < f_hi && (((sN.guar_mask >> j) & 1u) || contains(fl, f_deg, mj))) ++sub;
+                    const uint32_t mj = sm_m[32 * j + lane];
+                    if (mj >= f_lo && mj < f_hi && (((sN.guar_mask >> j) & 1u) || in_list(g, f_off, f_deg, mj))) ++sub;
                 }
                 fbase = (we > ws ? we - ws : 0) - sub;
             }
             if (MODE == kBytesMode) {
                 // what this kernel's algorithm reads for the parent: its own
                 // and its ancestors' (vertex, parent) entries, the joined
-                // vertices' info, then either the closed form's probes or the
+                // vertices' info, then either the closed form's tests or the
                 // streamed candidate window plus, per candidate, the signature
-                // gather and one lower-bound probe sequence per other list
-                (void)bytes;
-                auto probes = [](uint32_t len) { return 32u - __clz(len | 1u); };
+                // gather and one membership test per other list
+                auto test = [&](uint32_t l) { return g.tab ? 32u : 4u * (32u - __clz(l | 1u)); };
                 unsigned long long b = 8ull * lvl + 8ull * nj;
                 const uint32_t len = e0 - s0;
                 if (sL.closed_form) {  // the count kernel's closed form
-                    b += 4ull * lvl * probes(mdeg);
+                    b += uint64_t(lvl) * test(mdeg);
                 } else {
                     uint32_t per = check_sig ? 8 : 0;
                     for (uint32_t t = 0; t < nj; ++t)
-                        if (t != tmin) per += 4 * probes(sm_deg[warp][t][lane]);
+                        if (t != tmin) per += test(sm_deg[32 * t + lane]);
                     if (fold) {
-                        b += 8 + 4ull * lvl * probes(f_deg);
-                        if (!fold_guar_c) per += 4 * probes(f_deg);
+                        b += 8 + uint64_t(lvl) * test(f_deg);
+                        if (!fold_guar_c) per += test(f_deg);
                     }
                     b += 4ull * len + uint64_t(len) * per;
                 }
                 local += b;
             }
-            if (closed && MODE == kCountMode) {
+            if (closed) {
                 // one list, no signature: the window minus the matched vertices in it
                 uint32_t sub = 0;
                 for (uint32_t j = 0; j < lvl; ++j) {
-                    const uint32_t mj = sm_m[warp][j][lane];
-                    if (mj >= lo && mj < hi && (((sL.guar_mask >> j) & 1u) || contains(lst, mdeg, mj))) ++sub;
+                    const uint32_t mj = sm_m[32 * j + lane];
+                    if (mj >= lo && mj < hi && (((sL.guar_mask >> j) & 1u) || in_list(g, moff, mdeg, mj))) ++sub;
                 }
                 local += (e0 - s0) - sub;
             }
         }
         if (MODE == kBytesMode || closed) continue;
-        __syncwarp();
-        // concatenated candidate sequence of the 32 parents
+        // concatenated candidate sequence of the parents; the non-empty ones
+        // by rank
         const uint32_t len = e0 - s0;
         uint32_t incl = len;
         #pragma unroll
@@ -648,96 +666,117 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
             if (lane >= o) incl += y;
         }
         const uint32_t ftotal = __shfl_sync(kFullMask, incl, 31);
-        uint32_t gal_owner = kFullMask, gal_pos0 = 0, gal_pos1 = 0;
-        for (uint32_t fstep = 0; fstep < ftotal; fstep += 32) {
-            const uint32_t f = fstep + lane;
-            // owner = number of lanes whose inclusive end is <= f
-            uint32_t owner = 0;
+        if (!ftotal) { __syncwarp(); continue; }
+        const unsigned live = __ballot_sync(kFullMask, len != 0);
+        if (len) {
+            const uint32_t r = __popc(live & lanemask_lt), excl = incl - len, to = tmin ? 0u : 1u;
+            const uint32_t oo = nj > 1 ? sm_off[32 * to + lane] : 0u, od = nj > 1 ? sm_deg[32 * to + lane] : 0u;
+            rec[r] = make_uint4(moff + s0 - excl, uint32_t(lane) | (tmin << 8), oo, od);
+            starts[r] = excl;
+        }
+        __syncwarp();
+        const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? starts[lane] : kFullMask;
+        uint32_t started = 0;  // windows that start before this step
+        for (uint32_t fstep = 0; fstep < ftotal; fstep += 64) {
+            // two candidates per lane, their loads in flight together
+            uint4 rc[2];
+            uint32_t cv[2];
+            bool okv[2];
             #pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const uint32_t probe = __shfl_sync(kFullMask, incl, int(owner + step - 1));
-                if (probe <= f) owner += step;
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t rel = my_start - (fstep + 32 * h);
+                const uint32_t bits = __reduce_or_sync(kFullMask, rel < 32u ? 1u << rel : 0u);
+                const uint32_t own = started + __popc(bits & lanemask_le) - 1;
+                started += __popc(bits);
+                const uint32_t f = fstep + 32 * h + lane;
+                okv[h] = f < ftotal;
+                rc[h] = rec[own];
+                cv[h] = __ldg(g.adj + (rc[h].x + min(f, ftotal - 1)));  // the base may lie below zero: 32-bit sum
             }
-            owner = min(owner, 31u);
-            const uint32_t o_incl = __shfl_sync(kFullMask, incl, int(owner));
-            const uint32_t o_len = __shfl_sync(kFullMask, len, int(owner));
-            const uint32_t o_s0 = __shfl_sync(kFullMask, s0, int(owner));
-            const uint32_t o_moff = __shfl_sync(kFullMask, moff, int(owner));
-            const uint32_t o_tmin = __shfl_sync(kFullMask, tmin, int(owner));
-            const uint32_t o_ubp = __shfl_sync(kFullMask, ubp, int(owner));
-            bool ok = f < ftotal;
-            const uint32_t idx = o_s0 + (f - (o_incl - o_len));
-            const uint32_t c = ok ? __ldg(g.adj + o_moff + idx) : 0;
-            if (ok)
-                for (uint32_t j = 0; j < lvl; ++j)
-                    if (c == sm_m[warp][j][owner]) { ok = false; break; }
-            uint2 co = make_uint2(0, 0), ci = make_uint2(0, 0);
-            if (ok && load_info) {
-                co = g.out_info[c];
-                ci = sym ? co : g.in_info[c];
-            }
-            if (ok && check_sig) ok = ci.y >= sL.qin && co.y >= sL.qout;
-            if (owner != gal_owner) {  // new parent for this lane: restart the searches
-                gal_owner = owner;
-                gal_pos0 = gal_pos1 = 0;
-            }
-            if (ok) {
-                uint32_t r = 0;
-                for (uint32_t t = 0; t < nj; ++t) {
-                    if (t == o_tmin) continue;
-                    const uint32_t *lst = g.adj + sm_off[warp][t][owner];
-                    const uint32_t len2 = sm_deg[warp][t][owner];
-                    // this lane's candidates for one parent rise, so its lower
-                    // bounds in each other list rise too: gallop from the last
-                    const uint32_t from = r == 0 ? gal_pos0 : (r == 1 ? gal_pos1 : 0);
-                    const uint32_t pos = lbound_from(lst, len2, from, c);
-                    if (r == 0) gal_pos0 = pos;
-                    else if (r == 1) gal_pos1 = pos;
-                    ++r;
-                    if (pos >= len2 || __ldg(lst + pos) != c) { ok = false; break; }
+            if (nj > 1) {
+                if (g.tab) {
+                    uint32_t nb[2], b[2];
+                    Bucket bk[2];
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        nb[h] = (rc[h].w + 3) >> 2;
+                        b[h] = tab_bucket(nb[h], cv[h]);
+                        bk[h] = load_bucket(g.tab, rc[h].z, b[h]);
+                    }
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (okv[h] && !bucket_has(bk[h], cv[h]))
+                            okv[h] = tab_continue(g.tab, rc[h].z, nb[h], b[h], bk[h], cv[h]);
+                } else {
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (okv[h]) okv[h] = contains(g.adj + rc[h].z, rc[h].w, cv[h]);
                 }
             }
-            if constexpr (MODE == kCountMode) {
-                if (fold2) {
-                    if (ok) {
-                        const uint64_t p2 = pendant_pairs(g, sN, sN2, fold2, lvl, loops,
-                            [&](uint32_t j) { return j == lvl ? c : sm_m[warp][j][owner]; }, local3);
-                        local += p2;
-                        ++local2;
-                    }
-                } else if (fold) {
-                    const uint32_t o_fbase = __shfl_sync(kFullMask, fbase, int(owner));
-                    const uint32_t o_foff = __shfl_sync(kFullMask, f_off, int(owner));
-                    const uint32_t o_fdeg = __shfl_sync(kFullMask, f_deg, int(owner));
-                    const uint32_t o_flo = __shfl_sync(kFullMask, f_lo, int(owner));
-                    const uint32_t o_fhi = __shfl_sync(kFullMask, f_hi, int(owner));
-                    if (ok && sN.ofold) {
-                        local += orbit_weight(g, sN, lvl, o_fbase, c, loops);
-                        ++local2;
-                    } else if (ok) {
-                        const bool hit = c >= o_flo && c < o_fhi &&
-                                         (fold_guar_c || contains(g.adj + o_foff, o_fdeg, c));
-                        local += o_fbase - (hit ? 1u : 0u);
-                        ++local2;
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (fstep + 32 * h >= ftotal) break;
+                bool ok = okv[h];
+                const uint32_t c = cv[h], owner = rc[h].y & 255u, o_tmin = rc[h].y >> 8;
+                if (ok && nj > 2)
+                    for (uint32_t t = (o_tmin < 2 ? 2u : 1u); t < nj; ++t)
+                        if (t != o_tmin && !in_list(g, sm_off[32 * t + owner], sm_deg[32 * t + owner], c)) {
+                            ok = false;
+                            break;
+                        }
+                ok = ok && c >= sig_lo;
+                if (ok)
+                    for (uint32_t j = 0; j < lvl; ++j)
+                        if (c == sm_m[32 * j + owner]) { ok = false; break; }
+                uint2 co = make_uint2(0, 0), ci = make_uint2(0, 0);
+                if (ok && (check_sig || ub_out || ub_in)) {
+                    co = g.out_info[c];
+                    ci = sym ? co : g.in_info[c];
+                    if (check_sig) ok = ci.y >= sL.qin && co.y >= sL.qout;
+                }
+                if constexpr (MODE == kCountMode) {
+                    if (fold2) {
+                        if (ok) {
+                            const uint64_t p2 = pendant_pairs(g, sN, sN2, fold2, lvl, loops,
+                                [&](uint32_t j) { return j == lvl ? c : sm_m[32 * j + owner]; }, local3);
+                            local += p2;
+                            ++local2;
+                        }
+                    } else if (fold) {
+                        const uint32_t o_fbase = __shfl_sync(kFullMask, fbase, int(owner));
+                        const uint32_t o_foff = __shfl_sync(kFullMask, f_off, int(owner));
+                        const uint32_t o_fdeg = __shfl_sync(kFullMask, f_deg, int(owner));
+                        const uint32_t o_flo = __shfl_sync(kFullMask, f_lo, int(owner));
+                        const uint32_t o_fhi = __shfl_sync(kFullMask, f_hi, int(owner));
+                        if (ok && sN.ofold) {
+                            local += orbit_weight(g, sN, lvl, o_fbase, c, loops);
+                            ++local2;
+                        } else if (ok) {
+                            const bool hit = c >= o_flo && c < o_fhi &&
+                                             (fold_guar_c || in_list(g, o_foff, o_fdeg, c));
+                            local += o_fbase - (hit ? 1u : 0u);
+                            ++local2;
+                        }
+                    } else {
+                        local += ok;
                     }
                 } else {
-                    local += ok;
+                    uint32_t ub = need_ub ? __shfl_sync(kFullMask, ubp, int(owner)) : 0u;
+                    if (ub_out) ub = min(ub, co.y);
+                    if (ub_in) ub = min(ub, ci.y);
+                    // where c sits in the list it came from
+                    if (store_pos) ub = rc[h].x + fstep + 32 * h + lane;
+                    const unsigned m = __ballot_sync(kFullMask, ok);
+                    const uint32_t nn = __popc(m);
+                    if (obn + nn > uint32_t(kOutBuf)) flush();
+                    if (ok) {
+                        const uint32_t r = obn + __popc(m & lanemask_lt);
+                        ob_v[r] = c;
+                        ob_p[r] = pa + start + owner;
+                        ob_u[r] = ub;
+                    }
+                    obn += nn;
                 }
-            } else {
-                uint32_t ub = o_ubp;
-                if (ub_out) ub = min(ub, co.y);
-                if (ub_in) ub = min(ub, ci.y);
-                if (store_pos) ub = o_moff + idx;  // where c sits in the list it came from
-                const unsigned m = __ballot_sync(kFullMask, ok);
-                const uint32_t nn = __popc(m);
-                if (obn + nn > uint32_t(kOutBuf)) flush();
-                if (ok) {
-                    const uint32_t r = obn + __popc(m & lanemask_lt);
-                    ob_v[warp][r] = c;
-                    ob_p[warp][r] = pa + start + owner;
-                    ob_u[warp][r] = ub;
-                }
-                obn += nn;
             }
         }
         __syncwarp();
@@ -999,6 +1038,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, ui
                     for (uint32_t tt = 0; tt < sC.nj; ++tt)
                         if ((extra >> tt) & 1u)
                             if (!contains(g.adj + xoff[warp][tt], xdeg[warp][tt], t)) { ok = false; break; }
+                ok = ok && t >= sC.sig_lo;
                 if (ok && sig_c) {
                     const uint2 o = g.out_info[t], i2 = g.in_info[t];
                     ok = i2.y >= sC.qin && o.y >= sC.qout;
@@ -1102,6 +1142,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, ui
                     for (uint32_t tt = 0; tt < sC.nj; ++tt)
                         if ((extra >> tt) & 1u)
                             if (!contains(g.adj + xoff[warp][tt], xdeg[warp][tt], t)) { ok = false; break; }
+                ok = ok && t >= sC.sig_lo;
                 if (ok && sig_c) {
                     const uint2 o = g.out_info[t], i2 = g.in_info[t];
                     ok = i2.y >= sC.qin && o.y >= sC.qout;
@@ -1214,6 +1255,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, ui
                     for (uint32_t tt = 0; tt < sC.nj; ++tt)
                         if ((extra >> tt) & 1u)
                             if (!contains(g.adj + xoff[warp][tt], xdeg[warp][tt], v)) { ok = false; break; }
+                ok = ok && v >= sC.sig_lo;
                 if (ok && sig_c) {
                     const uint2 o = g.out_info[v], i2 = g.in_info[v];
                     ok = i2.y >= sC.qin && o.y >= sC.qout;
@@ -1496,7 +1538,8 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, ui
                 if (ok)
                     for (uint32_t j = 0; j < p; ++j)
                         if (v == my_m[j]) { ok = false; break; }
-                if (ok) {
+                ok = ok && v >= sP.sig_lo;
+                if (ok && sP.check_sig) {
                     const uint2 o = g.out_info[v], i = g.in_info[v];
                     ok = i.y >= sP.qin && o.y >= sP.qout;
                 }
@@ -1533,7 +1576,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, ui
                 }
                 ns += __popc(m);
                 if ((MODE == kBytesMode || tally) && lane == 0) {
-                    uint32_t per = 8;
+                    uint32_t per = sP.check_sig ? 8 : 0;
                     for (uint32_t t = 0; t < njp; ++t)
                         if (t != tmin) per += 4 * probes(jdeg[warp][t]);
                     const unsigned long long by = 4ull * min(32u, e0 - x0) + uint64_t(min(32u, e0 - x0)) * per;
@@ -1755,7 +1798,7 @@ k_plan(const uint64_t *__restrict__ tsum, uint32_t ntiles, unsigned long long ca
 
 int g_num_sms = 0;
 int g_level_blocks[3] = {0, 0, 0};
-int g_flat_blocks[3] = {0, 0, 0};
+int g_flat_blocks[3][2] = {};  // blocks of k_level_flat<mode, fold> per SM by registers and threads
 int g_fused_blocks[3] = {0, 0, 0};
 int g_fused_walk_blocks = 0;
 // CUTS_LEVEL_KERNEL=warp selects the warp-per-parent form (A/B comparisons)
@@ -1773,12 +1816,14 @@ int launch_geometry() {
     g_level_blocks[kCountMode] = std::max(1, b) * g_num_sms;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level<kBytesMode>, kWarps * 32, 0));
     g_level_blocks[kBytesMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kExpand>, kFW * 32, 0));
-    g_flat_blocks[kExpand] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kCountMode>, kFW * 32, 0));
-    g_flat_blocks[kCountMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kBytesMode>, kFW * 32, 0));
-    g_flat_blocks[kBytesMode] = std::max(1, b) * g_num_sms;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kExpand, false>, kFW * 32, 0));
+    g_flat_blocks[kExpand][0] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kCountMode, false>, kFW * 32, 0));
+    g_flat_blocks[kCountMode][0] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kCountMode, true>, kFW * 32, 0));
+    g_flat_blocks[kCountMode][1] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kBytesMode, true>, kFW * 32, 0));
+    g_flat_blocks[kBytesMode][1] = std::max(1, b);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kCountMode, false>, kZW * 32, 0));
     g_fused_blocks[kCountMode] = std::max(1, b) * g_num_sms;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kBytesMode, false>, kZW * 32, 0));
@@ -1788,6 +1833,17 @@ int launch_geometry() {
     const char *kv = std::getenv("CUTS_LEVEL_KERNEL");
     g_use_flat = !(kv && std::strcmp(kv, "warp") == 0);
     return CUTS_OK;
+}
+
+// Dynamic shared memory of one k_level_flat block, and the blocks that fill
+// the GPU at that size (227 KB per SM, 1 KB of it per block for the system).
+uint32_t flat_smem(int mode, uint32_t lvl, uint32_t nj) {
+    return 4 * kFW * flat_words(lvl, nj, mode == kExpand);
+}
+uint32_t flat_grid(int mode, bool fold, uint32_t smem) {
+    const uint32_t fixed = 3 * uint32_t(sizeof(LevelPlan)) + 16 * kMaxK + 1024;
+    const uint32_t by_smem = 227u * 1024u / (smem + fixed);
+    return std::max(1u, std::min(uint32_t(g_flat_blocks[mode][fold]), by_smem)) * uint32_t(g_num_sms);
 }
 
 // u32 scratch slots
@@ -1849,6 +1905,7 @@ static int device_graph_build(uint32_t n, const uint64_t *out_off, const uint32_
     want = std::min(want, 0.6 * double(freeb));
     g->arena_bytes = size_t(want);
     g->arena_default = g->arena_bytes;
+    g->tab_limit = (freeb - std::min(freeb, g->arena_bytes)) / 2;
     *out = g;
     return CUTS_OK;
 }
@@ -1873,7 +1930,7 @@ void device_graph_free(DeviceGraph *g) {
         if (g->in_info && g->in_info != g->out_info) cudaFreeAsync(g->in_info, g->stream);
         for (void *p : {static_cast<void *>(g->arena), static_cast<void *>(g->out_info),
                         static_cast<void *>(g->adj), static_cast<void *>(g->bwd_out),
-                        static_cast<void *>(g->core_bits)})
+                        static_cast<void *>(g->core_bits), static_cast<void *>(g->tab)})
             if (p) cudaFreeAsync(p, g->stream);
         cudaStreamSynchronize(g->stream);
     }
@@ -1975,11 +2032,14 @@ struct Run {
         uint32_t *out_n = g.d_u32 + kSlotOut + lvl;
         if (mode == kExpand) CK(cudaMemsetAsync(out_n, 0, sizeof(uint32_t), g.stream));
         const uint32_t work = pb - pa;
-        const bool flat = g_use_flat && hp->plan.lv[lvl].nj <= uint32_t(kFJ);
-        const uint32_t per_warp = flat ? 32 : grain;
+        const LevelPlan &L = hp->plan.lv[lvl];
+        const bool flat = g_use_flat && L.nj <= uint32_t(kFJ);
+        const bool fold = mode == kBytesMode || (mode == kCountMode && (L.fold || L.fold2));
+        const uint32_t smem = flat ? flat_smem(mode, lvl, L.nj) : 0;
+        // the flattened form deals out single parents when there are few
+        const uint32_t warps_needed = flat ? work : (work + grain - 1) / grain;
         const uint32_t wpb = flat ? kFW : kWarps;
-        const uint32_t warps_needed = (work + per_warp - 1) / per_warp;
-        uint32_t blocks = std::min<uint32_t>(uint32_t(flat ? g_flat_blocks[mode] : g_level_blocks[mode]),
+        uint32_t blocks = std::min<uint32_t>(flat ? flat_grid(mode, fold, smem) : uint32_t(g_level_blocks[mode]),
                                              (warps_needed + wpb - 1) / wpb);
         blocks = std::max<uint32_t>(blocks, 1);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1989,16 +2049,19 @@ struct Run {
             CK(cudaEventRecord(e0, g.stream));
         }
         if (flat) {
-            unsigned long long *acc = mode == kBytesMode ? g.d_u64 + 2 : g.d_u64;
+            auto go = [&](auto *kernel, uint32_t ocap, unsigned long long *a1, unsigned long long *a2,
+                          unsigned long long *a3) {
+                kernel<<<blocks, kFW * 32, smem, g.stream>>>(view, dp, lvl, pa, pb, g.d_u32 + kSlotCursor, out_n, ocap,
+                                                           g.d_u32 + kSlotErr, a1, a2, a3);
+            };
             if (mode == kExpand)
-                k_level_flat<kExpand><<<blocks, kFW * 32, 0, g.stream>>>(view, dp, lvl, pa, pb,
-                    g.d_u32 + kSlotCursor, out_n, uint32_t(cap), g.d_u32 + kSlotErr, acc, nullptr, nullptr);
+                go(k_level_flat<kExpand, false>, uint32_t(cap), g.d_u64, nullptr, nullptr);
+            else if (mode == kCountMode && fold)
+                go(k_level_flat<kCountMode, true>, 0, g.d_u64, g.d_u64 + 3, g.d_u64 + kU64Pair);
             else if (mode == kCountMode)
-                k_level_flat<kCountMode><<<blocks, kFW * 32, 0, g.stream>>>(view, dp, lvl, pa, pb,
-                    g.d_u32 + kSlotCursor, out_n, 0, g.d_u32 + kSlotErr, acc, g.d_u64 + 3, g.d_u64 + kU64Pair);
+                go(k_level_flat<kCountMode, false>, 0, g.d_u64, g.d_u64 + 3, g.d_u64 + kU64Pair);
             else
-                k_level_flat<kBytesMode><<<blocks, kFW * 32, 0, g.stream>>>(view, dp, lvl, pa, pb,
-                    g.d_u32 + kSlotCursor, out_n, 0, g.d_u32 + kSlotErr, acc, nullptr, nullptr);
+                go(k_level_flat<kBytesMode, true>, 0, g.d_u64 + 2, nullptr, nullptr);
         } else if (mode == kExpand)
             k_level<kExpand><<<blocks, kWarps * 32, 0, g.stream>>>(view, dp, lvl, pa, pb, grain,
                 g.d_u32 + kSlotCursor, out_n, uint32_t(cap), g.d_u32 + kSlotErr, g.d_u64);
@@ -2244,6 +2307,26 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         for (uint32_t i = 0; i < k; ++i) hp->plan.lv[i].fuse = 0;
     const bool fuse = counting && k >= 3 && hp->plan.lv[cl].fuse;
     if (fuse) stored = cl - 1;
+    // on a symmetric graph with degree-ranked ids the vertices of degree d or
+    // more are a suffix of the ids: the signature is a compare of ids, not a
+    // gather of the candidate's degree
+    if (g.symmetric && !g.orig.empty())
+        for (uint32_t i = 1; i < k; ++i) {
+            LevelPlan &L = hp->plan.lv[i];
+            if (!L.check_sig) continue;
+            const uint32_t d = std::max(L.qin, L.qout);
+            L.sig_lo = g.n - uint32_t(d < g.stats.out_ge.size() ? g.stats.out_ge[d] : 0);
+            L.check_sig = 0;
+        }
+    // membership tables, for the levels that test candidates in other lists
+    // or matched vertices in a folded one
+    bool tests = false;
+    for (uint32_t i = 1; i < k && i <= stored; ++i) {
+        const LevelPlan &L = hp->plan.lv[i];
+        if (fuse && i >= stored) break;
+        tests = tests || L.nj >= 2 || (counting && (L.fold || L.fold2 || L.closed_form));
+    }
+    if (tests && (rc = device_tables(g))) return rc;
     hp->stored = stored;
     // before a fused count of levels p = cl - 1 and cl, the entries of
     // level p - 1 record where their vertex sits in its list

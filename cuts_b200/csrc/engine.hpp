@@ -30,6 +30,11 @@ struct DeviceGraph {
     // d - core0, bit u - core0 (kCore x kCore bits)
     uint32_t *core_bits = nullptr;
     uint32_t core0 = 0;
+    // membership tables of the adjacency lists (2 words per padded list
+    // word), built by the first count that tests membership
+    uint32_t *tab = nullptr;
+    bool tab_tried = false;
+    size_t tab_limit = 0;         // bytes the tables may take (from the memory free at upload)
     cudaStream_t stream = nullptr;
 
     // trie-level arena, carved per query
@@ -71,6 +76,9 @@ int device_graph_from_csr(uint32_t n, const uint64_t *out_off, const uint32_t *o
 // (in-lists given), -1 decide; validate checks offsets and list order.
 int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, const uint64_t *in_off,
                   const uint32_t *in_adj, int sym_hint, bool validate, DeviceGraph &g);
+// Builds g.tab on g.stream, once; leaves it null (lists are searched
+// instead) when the device cannot hold it.
+int device_tables(DeviceGraph &g);
 void device_graph_free(DeviceGraph *g);
 
 struct CountResult {

@@ -117,6 +117,9 @@ struct LevelPlan {
                               // window, the second above / below the first)
     uint32_t guar1;           // level k-2 of a pendant pair: positions whose
                               // vertex the query guarantees in its list
+    uint32_t sig_lo;          // signature as a bound on the candidate's id (set by
+                              // the engine on degree-ranked symmetric graphs, where
+                              // check_sig is then 0): candidates below it fail
     uint32_t oguar[kMaxK];    // orbit fold: positions j with m_j guaranteed
                               // in the list of m_x, per orbit position x
     uint8_t jpos[kMaxJ];      // joined position j

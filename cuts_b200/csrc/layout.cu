@@ -214,6 +214,67 @@ __global__ void k_core_bits(uint32_t n, uint32_t core0, const uint2 *__restrict_
     }
 }
 
+// Puts key x into the table of the list {off, len}.
+__device__ __forceinline__ void tab_insert(uint32_t *__restrict__ tab, uint32_t off, uint32_t len, uint32_t x) {
+    const uint32_t nb = (len + 3) >> 2;
+    uint32_t b = tab_bucket(nb, x);
+    uint32_t *const base = tab + 2 * size_t(off);
+    // at most len of the 2 len or more slots are taken, so a free one exists
+    for (uint32_t tries = 0; tries < nb; ++tries) {
+        for (uint32_t i = 0; i < 8; ++i)
+            if (atomicCAS(base + 8 * size_t(b) + i, kTabEmpty, x) == kTabEmpty) return;
+        b = b + 1 == nb ? 0 : b + 1;
+    }
+}
+
+// Membership tables of the lists of vertices [0, h0), one warp per 32
+// vertices, their entries spread over the lanes.
+__global__ void __launch_bounds__(256)
+k_tables(uint32_t h0, const uint2 *__restrict__ info, const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t v0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; v0 < h0; v0 += warps * 32) {
+        const uint32_t v = v0 + lane;
+        const uint2 inf = v < h0 ? info[v] : make_uint2(0, 0);
+        uint32_t incl = inf.y;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+        for (uint32_t f0 = 0; f0 < total; f0 += 32) {
+            const uint32_t f = f0 + lane;
+            uint32_t owner = 0;
+            #pragma unroll
+            for (int step = 16; step; step >>= 1) {
+                const uint32_t probe = __shfl_sync(kFullMask, incl, int(owner + step - 1));
+                if (probe <= f) owner += step;
+            }
+            owner = min(owner, 31u);
+            const uint32_t off = __shfl_sync(kFullMask, inf.x, int(owner));
+            const uint32_t len = __shfl_sync(kFullMask, inf.y, int(owner));
+            const uint32_t end = __shfl_sync(kFullMask, incl, int(owner));
+            if (f < total) tab_insert(tab, off, len, __ldg(adj + off + (f - (end - len))));
+        }
+    }
+}
+
+// The same for the hubs [h0, n): one warp per 512 entries of a list.
+__global__ void __launch_bounds__(256)
+k_tables_hubs(uint32_t h0, uint32_t n, uint32_t chunks, const uint2 *__restrict__ info,
+              const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5, tasks = uint64_t(n - h0) * chunks;
+    for (uint64_t t = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < tasks; t += warps) {
+        const uint2 inf = info[h0 + uint32_t(t / chunks)];
+        const uint32_t a = uint32_t(t % chunks) * 512;
+        if (a >= inf.y) continue;
+        const uint32_t b = min(a + 512, inf.y);
+        for (uint32_t i = a + lane; i < b; i += 32) tab_insert(tab, inf.x, inf.y, __ldg(adj + inf.x + i));
+    }
+}
+
 // Device buffers of one build, stream-ordered from the device's memory pool
 // (reused across builds instead of mapped and unmapped each time), released
 // on every exit.
@@ -478,6 +539,45 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
     }
     g.stats = std::move(st);
     g.orig.swap(orig);
+    return CUTS_OK;
+}
+
+int device_tables(DeviceGraph &g) {
+    if (g.tab_tried) return CUTS_OK;
+    g.tab_tried = true;
+    if (!g.n || !g.arcs) return CUTS_OK;
+    const size_t bytes = sizeof(uint32_t) * 2 * size_t(g.adj_words);
+    if (bytes > g.tab_limit) return CUTS_OK;
+    cudaStream_t s = g.stream;
+    if (cudaMallocAsync(reinterpret_cast<void **>(&g.tab), bytes, s) != cudaSuccess) {
+        cudaGetLastError();
+        g.tab = nullptr;
+        return CUTS_OK;
+    }
+    LCK(cudaMemsetAsync(g.tab, 0xff, bytes, s));
+    const int dirs = g.symmetric ? 1 : 2;
+    auto deg = [&](uint32_t d) {
+        return uint64_t(g.h_out_deg[d]) + (g.symmetric ? 0u : g.h_in_deg[d]);
+    };
+    // ids are degree ranks (unless relabelling is off: then every list goes
+    // to the first kernel): the hubs, more than 512 entries, are a suffix
+    uint32_t h0 = g.n;
+    if (!g.orig.empty()) {
+        uint32_t lo = 0, hi = g.n;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (deg(mid) <= 512) lo = mid + 1; else hi = mid;
+        }
+        h0 = lo;
+    }
+    const uint32_t chunks = (g.max_deg + 511) / 512;
+    for (int dir = 0; dir < dirs; ++dir) {
+        const uint2 *info = dir ? g.in_info : g.out_info;
+        k_tables<<<std::max<uint32_t>(1, std::min<uint32_t>((h0 + 255) / 256, 148u * 8)), 256, 0, s>>>(h0, info, g.adj,
+                                                                                                    g.tab);
+        if (h0 < g.n) k_tables_hubs<<<148 * 8, 256, 0, s>>>(h0, g.n, chunks, info, g.adj, g.tab);
+        LCK(cudaGetLastError());
+    }
     return CUTS_OK;
 }
 
