@@ -180,9 +180,48 @@ __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const Le
 
 enum Mode { kExpand = 0, kCountMode = 1, kBytesMode = 2 };
 
+// The parents [pa, pa + total) of one launch.  Either the host knows them
+// (n null), or the launch was queued behind the one that writes their number:
+// then *n is read here, slice `slice` of `slices` of it is taken (root
+// slices), and an expanding launch whose children may not fit the level
+// (*bound > cap) raises *stop, which every later launch of the chain obeys,
+// so the host can go on from this level in chunks.
+struct Parents {
+    const uint32_t *n;
+    uint32_t a, b;             // host-known range
+    uint32_t slice, slices;
+    const unsigned long long *bound;
+    unsigned long long cap;
+    uint32_t *stop;
+    uint32_t code;             // what *stop says about this launch (never 0)
+};
+
+__device__ __forceinline__ void parents_of(const Parents &P, uint32_t &pa, uint32_t &total) {
+    if (!P.n) {
+        pa = P.a;
+        total = P.b - P.a;
+        return;
+    }
+    pa = total = 0;
+    if (*reinterpret_cast<volatile uint32_t *>(P.stop)) return;
+    if (P.bound && *P.bound > P.cap) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *P.stop = P.code;
+        return;
+    }
+    const uint32_t n = *P.n;
+    if (!n) return;
+    const uint32_t per = (n - 1) / P.slices + 1;
+    const unsigned long long a = (unsigned long long)P.slice * per, end = a + per;
+    if (a >= n) return;
+    pa = uint32_t(a);
+    // (as min(per, n - pa) in 32 bits, nvcc 12.9.86 gave `per` for a short
+    // last slice in k_fused)
+    total = uint32_t((end < n ? end : n) - a);
+}
+
 // ---- level 0: signature scan (device_funcs.cu:267-279) ---------------
 __global__ void k_roots(DevView g, const RunParams *__restrict__ rp, uint32_t shard, uint32_t nshards,
-                        uint32_t *__restrict__ n0) {
+                        uint32_t *__restrict__ n0, unsigned long long *__restrict__ bound) {
     const Plan &P = rp->plan;
     const uint32_t qin = P.lv[0].qin, qout = P.lv[0].qout;
     // L_0 entries carry the child bound for level 1, whose joins all use
@@ -194,6 +233,7 @@ __global__ void k_roots(DevView g, const RunParams *__restrict__ rp, uint32_t sh
     uint32_t *vert0 = rp->vert[0], *ub0 = rp->ub[0];
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0 && rp->budget_ns) *rp->stamp = global_ns();
+    unsigned long long sum = 0;  // of the child bounds
     for (uint32_t base = blockIdx.x * blockDim.x; base < g.n; base += gridDim.x * blockDim.x) {
         const uint32_t u = base + threadIdx.x;
         bool ok = false;
@@ -211,10 +251,16 @@ __global__ void k_roots(DevView g, const RunParams *__restrict__ rp, uint32_t sh
             pos = __shfl_sync(kFull, pos, 0) + __popc(m & ((1u << lane) - 1));
             if (ok) {
                 vert0[pos] = u;
-                if (need_ub) ub0[pos] = ub;
+                if (need_ub) {
+                    ub0[pos] = ub;
+                    sum += ub;
+                }
             }
         }
     }
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+    if (lane == 0 && sum) atomicAdd(bound, sum);
 }
 
 // ---- levels 1..k-1 -----------------------------------------------------
@@ -470,15 +516,19 @@ __host__ __device__ inline uint32_t flat_words(uint32_t lvl, uint32_t nj, bool e
     return 32 * lvl + 64 * nj + 128 + 32 + (expand ? 3 * kOutBuf : 0);
 }
 
-// MODE kExpand writes L_lvl, kCountMode counts, kBytesMode adds the bytes the
+// MODE kExpand writes L_lvl (adding its entries' child bounds to *acc where
+// acc is given), kCountMode counts, kBytesMode adds the bytes the
 // count reads.  FOLD: the level also counts the one or two after it (plain or
 // orbit fold, pendant pair).
 template <int MODE, bool FOLD>
 __global__ void __launch_bounds__(kFW * 32, FOLD ? 8 : 10)
-k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t pa, uint32_t pb,
+k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Parents parents,
              uint32_t *__restrict__ cursor, uint32_t *__restrict__ out_n, uint32_t out_cap,
              uint32_t *__restrict__ err, unsigned long long *__restrict__ acc,
              unsigned long long *__restrict__ acc2, unsigned long long *__restrict__ acc3) {
+    uint32_t pa, total;
+    parents_of(parents, pa, total);
+    if (!total) return;
     __shared__ LevelPlan sL, sN, sN2;
     __shared__ uint32_t *s_vert[kMaxK];
     __shared__ uint32_t *s_par[kMaxK];
@@ -532,7 +582,6 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     const bool fold = FOLD && MODE != kExpand && sL.fold;
     const bool fold_guar_c = fold && ((sN.guar_mask >> lvl) & 1u);
     const bool loops = rp->plan.data_loops != 0;
-    const uint32_t total = pb - pa;
     // parents per warp: fewer than 32 when that leaves warps without any (a
     // level of few parents with long lists)
     const uint32_t nwarps = gridDim.x * kFW;
@@ -774,6 +823,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                         ob_v[r] = c;
                         ob_p[r] = pa + start + owner;
                         ob_u[r] = ub;
+                        local += ub;
                     }
                     obn += nn;
                 }
@@ -783,6 +833,11 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     }
     if constexpr (MODE == kExpand) {
         if (obn) flush();
+        if (acc && need_ub && !store_pos) {
+            #pragma unroll
+            for (int s = 16; s; s >>= 1) local += __shfl_xor_sync(kFullMask, local, s);
+            if (lane == 0 && local) atomicAdd(acc, local);
+        }
     } else {
         #pragma unroll
         for (int s = 16; s; s >>= 1) {
@@ -839,10 +894,13 @@ constexpr uint32_t kHS = 512;  // hash slots of the admissible t, buckets of 4 (
 // loads, and the extra warps outweigh the spills that cap costs.
 template <int MODE, bool WALK, bool TALLY = false>
 __global__ void __launch_bounds__(kZW * 32, WALK ? 8 : 12)
-k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, uint32_t pb, uint32_t phase,
+k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents parents, uint32_t phase,
         uint32_t split, uint32_t *__restrict__ cursor, uint32_t *__restrict__ scratch, uint32_t stride, FusedBig big,
         unsigned long long *__restrict__ acc, unsigned long long *__restrict__ acc_c,
         unsigned long long *__restrict__ acc_p, unsigned long long *__restrict__ acc_bytes) {
+    uint32_t pa, total;
+    parents_of(parents, pa, total);
+    if (!total) return;
     constexpr bool walk_ok = WALK && MODE == kCountMode;
     // TALLY: also add the bytes this count reads from global memory to
     // *acc_bytes (the last level's algorithmic traffic; counts go to scratch)
@@ -902,7 +960,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, uint32_t pa, ui
     unsigned long long local = 0, local_c = 0, local_p = 0;
     uint32_t cached_q = kFullMask;
     const bool phase2 = phase == 2;
-    uint32_t nbig = 0, total = pb - pa;
+    uint32_t nbig = 0;
     if (phase2) {
         const unsigned long long n0 = big.n[0];
         nbig = n0 < big.cap ? uint32_t(n0) : big.cap;
@@ -1847,11 +1905,31 @@ uint32_t flat_grid(int mode, bool fold, uint32_t smem) {
 }
 
 // u32 scratch slots
-enum : int { kSlotN0 = 0, kSlotErr = 1, kSlotNb = 2, kSlotOver = 3, kSlotOut = 8, kSlotCursor = 32, kSlots = 64 };
+enum : int { kSlotN0 = 0, kSlotErr = 1, kSlotNb = 2, kSlotOver = 3, kSlotStop = 4, kSlotOut = 8, kSlotCursor = 32, kSlots = 64 };
 constexpr int kU64Stamp = 5;  // d_u64 slot: device clock at the start of a budgeted run
 constexpr int kU64Scratch = 8;  // d_u64 slots 8..10: counts of the bytes pass (discarded)
 constexpr int kU64Pair = 6;     // d_u64 slot: level k-2 size of a pendant-pair count
+constexpr int kU64Roots = 7;    // d_u64 slot: sum of the roots' child bounds
+constexpr int kU64Big = 11;     // d_u64 slots 11, 12: the fused count's deferred parents
 constexpr int kU64Slots = 16;
+
+// Counters of one root slice of a chain (launches queued without the host
+// reading level sizes in between).
+struct ChainSlice {
+    unsigned long long bound[kMaxK];  // child bounds of L_{lvl-1}, by lvl
+    unsigned long long big[2];        // the fused count's deferred parents
+    uint32_t out_n[kMaxK];
+    uint32_t cursor[kMaxK];
+};
+constexpr uint32_t kChainSlices = 16;  // root slices per chain
+
+// Device scratch and its pinned mirror: the u64 slots, the u32 slots and the
+// chain's slices, cleared and read in one piece.
+constexpr size_t kCtlHead = sizeof(unsigned long long) * kU64Slots + sizeof(uint32_t) * kSlots;
+constexpr size_t kCtlBytes = kCtlHead + sizeof(ChainSlice) * kChainSlices;
+ChainSlice *chain_slices(unsigned long long *u64) {
+    return reinterpret_cast<ChainSlice *>(reinterpret_cast<char *>(u64) + kCtlHead);
+}
 
 }  // namespace
 
@@ -1887,11 +1965,11 @@ static int device_graph_build(uint32_t n, const uint64_t *out_off, const uint32_
         device_graph_free(g);
         return rc;
     }
-    if ((e = cudaMalloc(&g->d_u32, sizeof(uint32_t) * kSlots))) return fail(e, "scratch");
-    if ((e = cudaMalloc(&g->d_u64, sizeof(unsigned long long) * kU64Slots))) return fail(e, "scratch");
+    if ((e = cudaMalloc(&g->d_u64, kCtlBytes))) return fail(e, "scratch");
+    g->d_u32 = reinterpret_cast<uint32_t *>(g->d_u64 + kU64Slots);
     if ((e = cudaMalloc(&g->d_plan, sizeof(RunParams)))) return fail(e, "scratch");
-    if ((e = cudaMallocHost(&g->h_u32, sizeof(uint32_t) * kSlots))) return fail(e, "pinned");
-    if ((e = cudaMallocHost(&g->h_u64, sizeof(unsigned long long) * kU64Slots))) return fail(e, "pinned");
+    if ((e = cudaMallocHost(&g->h_u64, kCtlBytes))) return fail(e, "pinned");
+    g->h_u32 = reinterpret_cast<uint32_t *>(g->h_u64 + kU64Slots);
     if ((e = cudaMallocHost(&g->h_plan, sizeof(RunParams)))) return fail(e, "pinned");
     if ((e = cudaEventCreate(&g->ev0)) || (e = cudaEventCreate(&g->ev1))) return fail(e, "event");
     if ((e = cudaStreamSynchronize(g->stream))) return fail(e, "upload sync");
@@ -1934,14 +2012,12 @@ void device_graph_free(DeviceGraph *g) {
             if (p) cudaFreeAsync(p, g->stream);
         cudaStreamSynchronize(g->stream);
     }
-    cudaFree(g->d_u32);
     cudaFree(g->d_u64);
     cudaFree(g->d_plan);
     cudaFree(g->d_tiles);
     cudaFree(g->d_bounds);
     cudaFree(g->batch_vsorted);
     cudaFree(g->batch_pref);
-    cudaFreeHost(g->h_u32);
     cudaFreeHost(g->h_u64);
     cudaFreeHost(g->h_plan);
     cudaFreeHost(g->h_bounds);
@@ -2027,11 +2103,20 @@ struct Run {
         return CUTS_OK;
     }
 
-    int launch_level(int mode, uint32_t lvl, uint32_t pa, uint32_t pb) {
-        CK(cudaMemsetAsync(g.d_u32 + kSlotCursor, 0, sizeof(uint32_t), g.stream));
-        uint32_t *out_n = g.d_u32 + kSlotOut + lvl;
-        if (mode == kExpand) CK(cudaMemsetAsync(out_n, 0, sizeof(uint32_t), g.stream));
-        const uint32_t work = pb - pa;
+    // A host-known range of parents.
+    static Parents known(uint32_t a, uint32_t b) { return Parents{nullptr, a, b, 0, 1, nullptr, 0, nullptr, 0}; }
+
+    // Level `lvl` over the given parents; `most` bounds their number.  A chain
+    // launch (cs: its slice's counters on the device) uses counters of its own.
+    int launch_level(int mode, uint32_t lvl, const Parents &par, uint32_t most, ChainSlice *cs = nullptr) {
+        uint32_t *out_n = cs ? cs->out_n + lvl : g.d_u32 + kSlotOut + lvl;
+        uint32_t *cursor = cs ? cs->cursor + lvl : g.d_u32 + kSlotCursor;
+        if (!cs) {
+            CK(cudaMemsetAsync(cursor, 0, sizeof(uint32_t), g.stream));
+            if (mode == kExpand) CK(cudaMemsetAsync(out_n, 0, sizeof(uint32_t), g.stream));
+        }
+        const uint32_t work = most;
+        const uint32_t pa = par.a, pb = par.b;  // the warp-per-parent form: host-known ranges only
         const LevelPlan &L = hp->plan.lv[lvl];
         const bool flat = g_use_flat && L.nj <= uint32_t(kFJ);
         const bool fold = mode == kBytesMode || (mode == kCountMode && (L.fold || L.fold2));
@@ -2051,11 +2136,12 @@ struct Run {
         if (flat) {
             auto go = [&](auto *kernel, uint32_t ocap, unsigned long long *a1, unsigned long long *a2,
                           unsigned long long *a3) {
-                kernel<<<blocks, kFW * 32, smem, g.stream>>>(view, dp, lvl, pa, pb, g.d_u32 + kSlotCursor, out_n, ocap,
+                kernel<<<blocks, kFW * 32, smem, g.stream>>>(view, dp, lvl, par, cursor, out_n, ocap,
                                                            g.d_u32 + kSlotErr, a1, a2, a3);
             };
             if (mode == kExpand)
-                go(k_level_flat<kExpand, false>, uint32_t(cap), g.d_u64, nullptr, nullptr);
+                go(k_level_flat<kExpand, false>, uint32_t(cap), cs && lvl + 1 < uint32_t(kMaxK) ? cs->bound + lvl + 1 : nullptr,
+                   nullptr, nullptr);
             else if (mode == kCountMode && fold)
                 go(k_level_flat<kCountMode, true>, 0, g.d_u64, g.d_u64 + 3, g.d_u64 + kU64Pair);
             else if (mode == kCountMode)
@@ -2064,13 +2150,13 @@ struct Run {
                 go(k_level_flat<kBytesMode, true>, 0, g.d_u64 + 2, nullptr, nullptr);
         } else if (mode == kExpand)
             k_level<kExpand><<<blocks, kWarps * 32, 0, g.stream>>>(view, dp, lvl, pa, pb, grain,
-                g.d_u32 + kSlotCursor, out_n, uint32_t(cap), g.d_u32 + kSlotErr, g.d_u64);
+                cursor, out_n, uint32_t(cap), g.d_u32 + kSlotErr, g.d_u64);
         else if (mode == kCountMode)
             k_level<kCountMode><<<blocks, kWarps * 32, 0, g.stream>>>(view, dp, lvl, pa, pb, grain,
-                g.d_u32 + kSlotCursor, out_n, 0, g.d_u32 + kSlotErr, g.d_u64);
+                cursor, out_n, 0, g.d_u32 + kSlotErr, g.d_u64);
         else
             k_level<kBytesMode><<<blocks, kWarps * 32, 0, g.stream>>>(view, dp, lvl, pa, pb, grain,
-                g.d_u32 + kSlotCursor, out_n, 0, g.d_u32 + kSlotErr, g.d_u64 + 2);
+                cursor, out_n, 0, g.d_u32 + kSlotErr, g.d_u64 + 2);
         CK(cudaGetLastError());
         if (profile) {
             CK(cudaEventRecord(e1, g.stream));
@@ -2083,12 +2169,14 @@ struct Run {
     // The fused count of levels p and p+1 over parents [pa, pb) of L_{p-1}:
     // phase 1 over the parents, then (counting) a scan of the parents it
     // deferred and phase 2 over their groups.
-    int launch_fused(int mode, uint32_t p, uint32_t pa, uint32_t pb) {
-        CK(cudaMemsetAsync(g.d_u32 + kSlotCursor, 0, sizeof(uint32_t), g.stream));
+    int launch_fused(int mode, uint32_t p, const Parents &par, uint32_t most, ChainSlice *cs = nullptr) {
+        uint32_t *cur1 = cs ? cs->cursor + p : g.d_u32 + kSlotCursor;
+        uint32_t *cur2 = cs ? cs->cursor + p + 1 : g.d_u32 + kSlotCursor + 1;
+        if (!cs) CK(cudaMemsetAsync(cur1, 0, 2 * sizeof(uint32_t), g.stream));
         uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(g_fused_blocks[mode]),
-                                                                   (pb - pa + kZW - 1) / kZW));
+                                                                   (most + kZW - 1) / kZW));
         FusedBig fb;
-        fb.n = reinterpret_cast<unsigned long long *>(hp->fuse_big);
+        fb.n = cs ? cs->big : g.d_u64 + kU64Big;
         fb.cap = hp->fuse_big_cap;
         fb.gi = hp->fuse_big + 64;
         fb.soff = fb.gi + fb.cap;
@@ -2096,7 +2184,7 @@ struct Run {
         fb.pref = fb.ns + fb.cap;
         fb.pool = fb.pref + fb.cap;
         fb.pool_words = hp->fuse_pool_words;
-        if (mode == kCountMode) CK(cudaMemsetAsync(fb.n, 0, 2 * sizeof(unsigned long long), g.stream));
+        if (!cs) CK(cudaMemsetAsync(fb.n, 0, 2 * sizeof(unsigned long long), g.stream));
         // CUTS_FUSE_SPLIT=<n> sets the deferral threshold (tests use small values)
         uint32_t split = g.fuse_split ? g.fuse_split : kBigS;
         if (const char *e = std::getenv("CUTS_FUSE_SPLIT")) split = uint32_t(std::strtoul(e, nullptr, 10));
@@ -2127,8 +2215,8 @@ struct Run {
             CK(cudaEventRecord(e0, g.stream));
         }
         if (mode == kBytesMode && !walk_ok) {
-            k_fused<kBytesMode, false><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, pa, pb, 1, split,
-                g.d_u32 + kSlotCursor, hp->fuse_scratch, hp->fuse_stride, fb, g.d_u64 + 2, nullptr, nullptr,
+            k_fused<kBytesMode, false><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
+                cur1, hp->fuse_scratch, hp->fuse_stride, fb, g.d_u64 + 2, nullptr, nullptr,
                 nullptr);
             CK(cudaGetLastError());
             res.launches++;
@@ -2140,29 +2228,27 @@ struct Run {
             unsigned long long *acc_c = tal ? g.d_u64 + kU64Scratch + 1 : g.d_u64 + 3;
             unsigned long long *acc_p = tal ? g.d_u64 + kU64Scratch + 2 : g.d_u64 + 4;
             unsigned long long *acc_b = tal ? g.d_u64 + 2 : nullptr;
-            if (tal) CK(cudaMemsetAsync(fb.n, 0, 2 * sizeof(unsigned long long), g.stream));
             const uint32_t wblocks =
-                std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(g_fused_walk_blocks), (pb - pa + kZW - 1) / kZW));
+                std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(g_fused_walk_blocks), (most + kZW - 1) / kZW));
             if (walk_ok && tal)
-                k_fused<kCountMode, true, true><<<wblocks, kZW * 32, 0, g.stream>>>(view, dp, p, pa, pb, 1, split,
-                    g.d_u32 + kSlotCursor, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
+                k_fused<kCountMode, true, true><<<wblocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
+                    cur1, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
             else if (walk_ok)
-                k_fused<kCountMode, true><<<wblocks, kZW * 32, 0, g.stream>>>(view, dp, p, pa, pb, 1, split,
-                    g.d_u32 + kSlotCursor, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
+                k_fused<kCountMode, true><<<wblocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
+                    cur1, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
             else
-                k_fused<kCountMode, false><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, pa, pb, 1, split,
-                    g.d_u32 + kSlotCursor, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
+                k_fused<kCountMode, false><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
+                    cur1, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
             CK(cudaGetLastError());
             k_fused_scan<<<1, 1024, 0, g.stream>>>(fb);
             CK(cudaGetLastError());
-            CK(cudaMemsetAsync(g.d_u32 + kSlotCursor, 0, sizeof(uint32_t), g.stream));
             if (tal)
                 k_fused<kCountMode, false, true><<<uint32_t(g_fused_blocks[kCountMode]), kZW * 32, 0, g.stream>>>(
-                    view, dp, p, pa, pb, 2, split, g.d_u32 + kSlotCursor, hp->fuse_scratch, hp->fuse_stride, fb, acc,
+                    view, dp, p, par, 2, split, cur2, hp->fuse_scratch, hp->fuse_stride, fb, acc,
                     acc_c, acc_p, acc_b);
             else
                 k_fused<kCountMode, false><<<uint32_t(g_fused_blocks[kCountMode]), kZW * 32, 0, g.stream>>>(
-                    view, dp, p, pa, pb, 2, split, g.d_u32 + kSlotCursor, hp->fuse_scratch, hp->fuse_stride, fb, acc,
+                    view, dp, p, par, 2, split, cur2, hp->fuse_scratch, hp->fuse_stride, fb, acc,
                     acc_c, acc_p, acc_b);
             CK(cudaGetLastError());
             res.launches += 3;
@@ -2187,19 +2273,20 @@ struct Run {
         marks.clear();
     }
 
+    uint32_t count_level() const {
+        return (k >= 4 && hp->plan.lv[k - 3].fold2) ? k - 3 : (k >= 3 && hp->plan.lv[k - 2].fold) ? k - 2 : k - 1;
+    }
+
     // Expands parents [pa, pb) of L_{lvl-1}, depth first by chunks.
     int expand(uint32_t lvl, uint32_t pa, uint32_t pb) {
         if (pb <= pa) return CUTS_OK;
         // the last level is counted; with a folded plan, level k-2 counts both;
         // with a fused plan, the counting kernel runs one level earlier
-        const uint32_t count_lvl = (k >= 4 && hp->plan.lv[k - 3].fold2) ? k - 3
-                                   : (k >= 3 && hp->plan.lv[k - 2].fold) ? k - 2 : k - 1;
+        const uint32_t count_lvl = count_level();
         if (!dump && k >= 3 && hp->plan.lv[count_lvl].fuse && lvl == count_lvl - 1)
-            return launch_fused(bytes_mode ? kBytesMode : kCountMode, lvl, pa, pb);
-        if (lvl == count_lvl && !dump) {
-            int rc = launch_level(bytes_mode ? kBytesMode : kCountMode, lvl, pa, pb);
-            return rc;
-        }
+            return launch_fused(bytes_mode ? kBytesMode : kCountMode, lvl, known(pa, pb), pb - pa);
+        if (lvl == count_lvl && !dump)
+            return launch_level(bytes_mode ? kBytesMode : kCountMode, lvl, known(pa, pb), pb - pa);
         std::vector<uint32_t> cuts;
         int rc = plan_chunks(lvl, pa, pb, cuts);
         if (rc) return rc;
@@ -2210,7 +2297,7 @@ struct Run {
                 std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count() >
                     budget_ms)
                 return set_error(CUTS_ERR_BUDGET, "time budget exhausted");
-            rc = launch_level(kExpand, lvl, a, b);
+            rc = launch_level(kExpand, lvl, known(a, b), b - a);
             if (rc) return rc;
             res.chunks++;
             CK(cudaMemcpyAsync(g.h_u32 + kSlotOut + lvl, g.d_u32 + kSlotOut + lvl, sizeof(uint32_t),
@@ -2229,6 +2316,23 @@ struct Run {
         }
         return CUTS_OK;
     }
+
+    // True when every level of the plan runs in kernels that take their
+    // parents' number from the device.
+    bool can_chain() const {
+        if (dump || bytes_mode || !g_use_flat) return false;
+        for (uint32_t i = 1; i <= count_level(); ++i)
+            if (hp->plan.lv[i].nj > uint32_t(kFJ)) return false;
+        return true;
+    }
+
+    // All levels of all root slices queued without waiting: each launch reads
+    // its parents' number on the device, so a count costs one wait instead of
+    // one per level and slice (the GPU is idle between a level's end and the
+    // next launch for a wait and a copy).  4-cycle on 10,000 vertices 174 ->
+    // 119 us, twelve 4-6 vertex queries on 3,000 vertices 2.87 -> 2.10 ms.  A level whose children may not fit is left to
+    // expand(), which cuts it into chunks.
+    int chain(uint32_t chunks);
 
     // Dump: materialise the nout complete matches of L_{k-1} in pieces and
     // write one ans.txt line per match, pairs in matching order
@@ -2390,17 +2494,18 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     return CUTS_OK;
 }
 
-// Level 0 into L_0; returns |L_0|.
-int run_roots(DeviceGraph &g, Run &run, uint32_t shard, uint32_t nshards, uint32_t &n0) {
-    CK(cudaMemsetAsync(g.d_u32, 0, sizeof(uint32_t) * kSlots, g.stream));
-    CK(cudaMemsetAsync(g.d_u64, 0, sizeof(unsigned long long) * kU64Slots, g.stream));
+// Level 0 into L_0; returns |L_0|.  For a chain of `slices` root slices it is
+// only queued (|L_0| stays on the device), the slices' counters cleared.
+int run_roots(DeviceGraph &g, Run &run, uint32_t shard, uint32_t nshards, uint32_t &n0, uint32_t slices = 0) {
+    CK(cudaMemsetAsync(g.d_u64, 0, kCtlHead + sizeof(ChainSlice) * std::min(slices, kChainSlices), g.stream));
     n0 = 0;
     if (!g.n) return CUTS_OK;
     const uint32_t threads = 256;
     const uint32_t blocks = std::min<uint32_t>((g.n + threads - 1) / threads, uint32_t(g_num_sms) * 8);
-    k_roots<<<blocks, threads, 0, g.stream>>>(run.view, run.dp, shard, nshards, g.d_u32 + kSlotN0);
+    k_roots<<<blocks, threads, 0, g.stream>>>(run.view, run.dp, shard, nshards, g.d_u32 + kSlotN0, g.d_u64 + kU64Roots);
     CK(cudaGetLastError());
     run.res.launches++;
+    if (slices) return CUTS_OK;  // a chain reads the number on the device
     CK(cudaMemcpyAsync(g.h_u32 + kSlotN0, g.d_u32 + kSlotN0, sizeof(uint32_t), cudaMemcpyDeviceToHost, g.stream));
     int rc = run.sync();
     if (rc) return rc;
@@ -2416,6 +2521,72 @@ int run_slices(Run &run, uint32_t n0, uint32_t chunks) {
         if (a >= n0) break;
         int rc = run.expand(1, uint32_t(a), uint32_t(std::min<uint64_t>(a + slice, n0)));
         if (rc) return rc;
+    }
+    return CUTS_OK;
+}
+
+int Run::chain(uint32_t chunks) {
+    const uint32_t cl = count_level();
+    const bool fused = k >= 3 && hp->plan.lv[cl].fuse;
+    const uint32_t last = fused ? cl - 1 : cl;  // level of the counting launch
+    // bounds on the levels' sizes, for the launches' grids
+    std::vector<uint64_t> most(last + 1, 0);
+    most[0] = g.n;
+    for (uint32_t i = 1; i < last; ++i) most[i] = std::min<uint64_t>(cap, most[i - 1] * std::max<uint32_t>(g.max_deg, 1));
+    ChainSlice *const ds = chain_slices(g.d_u64), *const hs = chain_slices(g.h_u64);
+    int rc = CUTS_OK;
+    for (uint32_t s0 = 0; s0 < chunks;) {
+        const uint32_t ns = std::min(chunks - s0, kChainSlices);
+        if (s0) CK(cudaMemsetAsync(ds, 0, sizeof(ChainSlice) * ns, g.stream));
+        for (uint32_t i = 0; i < ns; ++i) {
+            for (uint32_t lvl = 1; lvl <= last; ++lvl) {
+                const bool exp = lvl < last;
+                Parents par{lvl == 1 ? g.d_u32 + kSlotN0 : ds[i].out_n + lvl - 1, 0, 0, lvl == 1 ? s0 + i : 0,
+                            lvl == 1 ? chunks : 1,
+                            !exp ? nullptr : lvl == 1 ? g.d_u64 + kU64Roots : ds[i].bound + lvl, cap,
+                            g.d_u32 + kSlotStop, ((i + 1) << 8) | lvl};
+                const uint32_t m = uint32_t(std::min<uint64_t>(lvl == 1 ? most[0] / chunks + 1 : most[lvl - 1], UINT32_MAX));
+                if (!exp && fused) rc = launch_fused(kCountMode, lvl, par, m, ds + i);
+                else rc = launch_level(exp ? kExpand : kCountMode, lvl, par, m, ds + i);
+                if (rc) return rc;
+            }
+        }
+        CK(cudaEventRecord(g.ev1, g.stream));
+        CK(cudaMemcpyAsync(g.h_u64, g.d_u64, kCtlHead + sizeof(ChainSlice) * ns, cudaMemcpyDeviceToHost, g.stream));
+        if ((rc = sync())) return rc;
+        const uint32_t n0 = g.h_u32[kSlotN0], stop = g.h_u32[kSlotStop];
+        res.level_sizes[0] = n0;
+        const uint32_t done = stop ? (stop >> 8) - 1 : ns;  // slices before the one that stopped
+        for (uint32_t i = 0; i < std::min(done + 1, ns); ++i)
+            for (uint32_t lvl = 1; lvl < (i < done ? last : (stop & 255u)); ++lvl) {
+                res.level_sizes[lvl] += hs[i].out_n[lvl];
+                res.chunks++;
+            }
+        if (g.h_u32[kSlotOver]) return set_error(CUTS_ERR_BUDGET, "time budget exhausted");
+        if (g.h_u32[kSlotErr]) return set_error(CUTS_ERR_CAPACITY, "a level overflowed its capacity");
+        if (!n0) break;
+        if (!stop) {
+            s0 += ns;
+            if (uint64_t(s0) * ((n0 - 1) / chunks + 1) >= n0) break;  // the remaining slices are empty
+            continue;
+        }
+        // slice s0 + done from level `lvl` on, in chunks
+        const uint32_t lvl = stop & 255u;
+        uint32_t a = 0, b = lvl > 1 ? hs[done].out_n[lvl - 1] : 0;
+        if (lvl == 1) {
+            const uint32_t per = (n0 - 1) / chunks + 1;
+            const uint64_t a64 = uint64_t(s0 + done) * per;
+            a = uint32_t(std::min<uint64_t>(a64, n0));
+            b = uint32_t(std::min<uint64_t>(a64 + per, n0));
+        }
+        CK(cudaMemsetAsync(g.d_u32 + kSlotStop, 0, sizeof(uint32_t), g.stream));
+        if ((rc = expand(lvl, a, b))) return rc;
+        s0 += done + 1;
+        if (s0 >= chunks) {
+            CK(cudaEventRecord(g.ev1, g.stream));
+            CK(cudaMemcpyAsync(g.h_u64, g.d_u64, kCtlHead, cudaMemcpyDeviceToHost, g.stream));
+            if ((rc = sync())) return rc;
+        }
     }
     return CUTS_OK;
 }
@@ -2503,37 +2674,40 @@ int device_count(DeviceGraph &g, const Query &q, const CountOptions &opt, CountR
     }
     CK(cudaEventRecord(g.ev0, g.stream));
     uint32_t n0 = 0;
-    rc = run_roots(g, run, opt.shard, opt.nshards, n0);
-    if (rc) return rc;
-    res.level_sizes[0] = n0;
-    if (k >= 2 && n0 > 0) {
-        rc = run_slices(run, n0, opt.chunks);
+    if (k >= 2 && g.n && run.can_chain()) {
+        rc = run_roots(g, run, opt.shard, opt.nshards, n0, opt.chunks);
+        if (rc) return rc;
+        rc = run.chain(opt.chunks);
+        if (rc) return rc;
+        n0 = g.h_u32[kSlotN0];
+    } else {
+        rc = run_roots(g, run, opt.shard, opt.nshards, n0);
+        if (rc) return rc;
+        res.level_sizes[0] = n0;
+        if (k >= 2 && n0 > 0) {
+            rc = run_slices(run, n0, opt.chunks);
+            if (rc) return rc;
+        }
+        CK(cudaEventRecord(g.ev1, g.stream));
+        CK(cudaMemcpyAsync(g.h_u64, g.d_u64, kCtlHead, cudaMemcpyDeviceToHost, g.stream));
+        rc = run.sync();
         if (rc) return rc;
     }
-    CK(cudaEventRecord(g.ev1, g.stream));
-    CK(cudaMemcpyAsync(g.h_u64, g.d_u64, sizeof(unsigned long long), cudaMemcpyDeviceToHost, g.stream));
-    CK(cudaMemcpyAsync(g.h_u32 + kSlotOver, g.d_u32 + kSlotOver, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                       g.stream));
-    rc = run.sync();
-    if (rc) return rc;
     run.collect_profile();
     CK(cudaEventElapsedTime(&res.ms, g.ev0, g.ev1));
     if (g.h_u32[kSlotOver]) return set_error(CUTS_ERR_BUDGET, "time budget exhausted");
     const uint64_t raw = k >= 2 ? uint64_t(g.h_u64[0]) : 0;
     res.level_sizes[k - 1] = k >= 2 ? raw : n0;
     if (k >= 4 && hp->plan.lv[k - 3].fold2) {  // level k-3 counted both pendant levels
-        CK(cudaMemcpy(g.h_u64 + 3, g.d_u64 + 3, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost));
         res.level_sizes[k - 3] = g.h_u64[3];
         res.level_sizes[k - 2] = g.h_u64[kU64Pair];
     }
     if (k >= 3 && hp->plan.lv[k - 2].fold) {
-        CK(cudaMemcpy(g.h_u64 + 3, g.d_u64 + 3, sizeof(unsigned long long), cudaMemcpyDeviceToHost));
         res.level_sizes[k - 2] = g.h_u64[3];
     }
     if (k >= 3) {
         const uint32_t cl = hp->plan.lv[k - 2].fold ? k - 2 : k - 1;
         if (hp->plan.lv[cl].fuse) {  // the fused level before the counted one
-            CK(cudaMemcpy(g.h_u64 + 4, g.d_u64 + 4, sizeof(unsigned long long), cudaMemcpyDeviceToHost));
             res.level_sizes[cl - 1] = g.h_u64[4];
         }
     }
