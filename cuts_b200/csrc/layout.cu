@@ -28,27 +28,73 @@ constexpr uint32_t kPad = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t padded(uint32_t len) { return (len + 3u) & ~3u; }
 
-// Offsets monotone and within the arc count; every list strictly increasing
-// with ids below n.  flag |= 1 (offsets) or 2 (lists).  One warp per vertex,
-// its lanes across the list (coalesced; a hub's list no longer serialises
-// one thread).
-__global__ void k_validate(uint32_t n, uint64_t m, const uint64_t *__restrict__ off,
-                           const uint32_t *__restrict__ adj, uint32_t *__restrict__ flag) {
+// Walks every vertex's list: body(v, thread, threads) by one warp per vertex,
+// or, for lists of more than kLongList entries, by the whole block after its
+// warps are through with theirs.  One warp per vertex alone leaves a
+// 20,000-entry hub's 625 dependent steps as the launch's tail: the symmetry
+// check of 1M vertices / 20M arcs took 4.06 ms that way, 0.77 ms this way.
+// len(v) gives the list's length.
+constexpr uint32_t kLongList = 512;
+constexpr uint32_t kLongQueue = 512;
+
+template <class Len, class Body>
+__device__ __forceinline__ void per_list(uint32_t n, Len len, Body body) {
+    __shared__ uint32_t q[kLongQueue];
+    __shared__ uint32_t qn;
+    if (threadIdx.x == 0) qn = 0;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
-        const uint64_t a = off[v], b = off[v + 1];
-        if (b < a || b > m) {
-            if (lane == 0) atomicOr(flag, 1u);
-            continue;
+        uint32_t slot = kLongQueue;
+        if (len(v) > kLongList) {
+            if (lane == 0) slot = atomicAdd(&qn, 1u);
+            slot = __shfl_sync(kFullMask, slot, 0);
+            if (slot < kLongQueue && lane == 0) q[slot] = v;
         }
-        bool bad = false;
-        for (uint64_t x = a + lane; x < b; x += 32) {
-            const uint32_t id = adj[x];
-            if (id >= n || (x > a && id <= adj[x - 1])) bad = true;
-        }
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(flag, 2u);
+        if (slot >= kLongQueue) body(v, lane, 32u);
     }
+    __syncthreads();
+    const uint32_t nq = min(qn, kLongQueue);
+    for (uint32_t i = 0; i < nq; ++i) body(q[i], threadIdx.x, blockDim.x);
+}
+
+// The lane whose part of a warp's concatenated sequence holds element w
+// (incl: inclusive scan of the lanes' lengths).
+__device__ __forceinline__ uint32_t run_owner(uint32_t incl, uint32_t w) {
+    uint32_t owner = 0;
+    #pragma unroll
+    for (int step = 16; step; step >>= 1) {
+        const uint32_t probe = __shfl_sync(kFullMask, incl, int(owner + step - 1));
+        if (probe <= w) owner += step;
+    }
+    return min(owner, 31u);
+}
+
+// Offsets monotone and within the arc count; every list strictly increasing
+// with ids below n.  flag |= 1 (offsets) or 2 (lists).
+__global__ void k_validate(uint32_t n, uint64_t m, const uint64_t *__restrict__ off,
+                           const uint32_t *__restrict__ adj, uint32_t *__restrict__ flag) {
+    bool bad = false;
+    per_list(
+        n,
+        [&](uint32_t v) {
+            const uint64_t a = off[v], b = off[v + 1];
+            if (b < a || b > m) return 0u;
+            return uint32_t(min(b - a, uint64_t(0xffffffffu)));
+        },
+        [&](uint32_t v, uint32_t t, uint32_t nt) {
+            const uint64_t a = off[v], b = off[v + 1];
+            if (b < a || b > m) {
+                if (t == 0) atomicOr(flag, 1u);
+                return;
+            }
+            for (uint64_t x = a + t; x < b; x += nt) {
+                const uint32_t id = adj[x];
+                if (id >= n || (x > a && id <= adj[x - 1])) bad = true;
+            }
+        });
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flag, 2u);
 }
 
 // flag |= 1 where the two arrays differ.
@@ -66,17 +112,16 @@ __global__ void k_differ(uint64_t cnt, const T *__restrict__ a, const T *__restr
 // have equal sizes exactly when every up arc's reverse exists too.  So only
 // a down arc u -> v is searched for, as u in v's list -- the shorter of the
 // two: a hub's list is never searched -- and the arcs going up and down are
-// counted into updown[0] / updown[1] (a self-loop is its own reverse).  One
-// warp per vertex u.
+// counted into updown[0] / updown[1] (a self-loop is its own reverse).
 __global__ void k_symmetric(uint32_t n, const uint64_t *__restrict__ off, const uint32_t *__restrict__ adj,
                             uint32_t *__restrict__ flag, unsigned long long *__restrict__ updown) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     unsigned long long up = 0, down = 0;
-    for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
+    auto len = [&](uint32_t u) { return uint32_t(off[u + 1] - off[u]); };
+    per_list(n, len, [&](uint32_t u, uint32_t t, uint32_t nt) {
         const uint64_t a = off[u], b = off[u + 1];
         const uint64_t du = b - a;
-        for (uint64_t x = a + lane; x < b; x += 32) {
+        for (uint64_t x = a + t; x < b; x += nt) {
             const uint32_t v = adj[x];
             if (v == u) continue;
             const uint64_t lo0 = off[v], hi0 = off[v + 1], dv = hi0 - lo0;
@@ -92,7 +137,7 @@ __global__ void k_symmetric(uint32_t n, const uint64_t *__restrict__ off, const 
             }
             if (lo == hi0 || adj[lo] != u) atomicOr(flag, 1u);
         }
-    }
+    });
     for (int sh = 16; sh; sh >>= 1) {
         up += __shfl_xor_sync(0xffffffffu, up, sh);
         down += __shfl_xor_sync(0xffffffffu, down, sh);
@@ -149,18 +194,67 @@ __global__ void k_info(uint32_t n, const uint32_t *__restrict__ orig, const uint
     }
 }
 
-// One warp per device vertex: its list, ids mapped through rank (when
-// given), and the padding.
-__global__ void k_fill(uint32_t n, const uint32_t *__restrict__ orig, const uint32_t *__restrict__ rank,
-                       const uint64_t *__restrict__ off, const uint32_t *__restrict__ src,
-                       const uint2 *__restrict__ info, uint32_t *__restrict__ dst) {
-    const uint32_t lane = threadIdx.x & 31;
+// Device vertices' lists, ids mapped through rank (when given), and the
+// padding: a warp takes 32 consecutive vertices and spreads their words over
+// its lanes, four chains of reads (list entry, rank) in flight per lane; lists
+// of more than kLongList entries are queued for k_fill_long.  20M arcs: 0.56
+// ms with one warp per vertex, 0.28 ms this way.
+__global__ void __launch_bounds__(256)
+k_fill(uint32_t n, const uint32_t *__restrict__ orig, const uint32_t *__restrict__ rank,
+       const uint64_t *__restrict__ off, const uint32_t *__restrict__ src, const uint2 *__restrict__ info,
+       uint32_t *__restrict__ dst, uint32_t *__restrict__ queue, uint32_t *__restrict__ queued) {
+    const int lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; d < n; d += warps) {
-        const uint32_t v = orig ? orig[d] : d;
-        const uint64_t a = off[v];
+    for (uint32_t d0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; d0 < n; d0 += warps * 32) {
+        const uint32_t d = d0 + lane;
+        const uint2 inf = d < n ? info[d] : make_uint2(0, 0);
+        const unsigned long long a = d < n ? off[orig ? orig[d] : d] : 0ull;
+        const bool longl = inf.y > kLongList;
+        if (longl) queue[atomicAdd(queued, 1u)] = d;
+        const uint32_t words = longl ? 0u : padded(inf.y);
+        uint32_t incl = words;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+        for (uint32_t w0 = 0; w0 < total; w0 += 128) {
+            uint32_t x[4], to[4];
+            #pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const uint32_t w = w0 + 32 * h + lane, owner = run_owner(incl, w);
+                const uint32_t ow = __shfl_sync(kFullMask, words, int(owner)), oi = __shfl_sync(kFullMask, incl, int(owner));
+                const uint32_t at = w - (oi - ow);  // place in its list
+                to[h] = __shfl_sync(kFullMask, inf.x, int(owner)) + at;
+                const uint32_t len = __shfl_sync(kFullMask, inf.y, int(owner));
+                const unsigned long long oa = __shfl_sync(kFullMask, a, int(owner));
+                x[h] = w < total && at < len ? src[oa + at] : kPad;
+            }
+            if (rank) {
+                #pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    if (x[h] != kPad) x[h] = rank[x[h]];
+            }
+            #pragma unroll
+            for (int h = 0; h < 4; ++h)
+                if (w0 + 32 * h + lane < total) dst[to[h]] = x[h];
+        }
+    }
+}
+
+// The queued lists, one block each.
+__global__ void __launch_bounds__(512)
+k_fill_long(const uint32_t *__restrict__ orig, const uint32_t *__restrict__ rank, const uint64_t *__restrict__ off,
+            const uint32_t *__restrict__ src, const uint2 *__restrict__ info, uint32_t *__restrict__ dst,
+            const uint32_t *__restrict__ queue, const uint32_t *__restrict__ queued) {
+    const uint32_t nq = *queued;
+    for (uint32_t i = blockIdx.x; i < nq; i += gridDim.x) {
+        const uint32_t d = queue[i];
+        const uint64_t a = off[orig ? orig[d] : d];
         const uint2 inf = info[d];
-        for (uint32_t j = lane; j < padded(inf.y); j += 32) {
+        #pragma unroll 2
+        for (uint32_t j = threadIdx.x; j < padded(inf.y); j += blockDim.x) {
             uint32_t x = kPad;
             if (j < inf.y) {
                 x = src[a + j];
@@ -214,12 +308,12 @@ __global__ void k_core_bits(uint32_t n, uint32_t core0, const uint2 *__restrict_
     }
 }
 
-// Puts key x into the table of the list {off, len}.
-__device__ __forceinline__ void tab_insert(uint32_t *__restrict__ tab, uint32_t off, uint32_t len, uint32_t x) {
+// Puts key x into the table of a list of len entries at `base` (global or
+// shared memory).  At most len of the 2 len or more slots are taken, so a free
+// one exists.
+__device__ __forceinline__ void tab_insert(uint32_t *base, uint32_t len, uint32_t x) {
     const uint32_t nb = (len + 3) >> 2;
     uint32_t b = tab_bucket(nb, x);
-    uint32_t *const base = tab + 2 * size_t(off);
-    // at most len of the 2 len or more slots are taken, so a free one exists
     for (uint32_t tries = 0; tries < nb; ++tries) {
         for (uint32_t i = 0; i < 8; ++i)
             if (atomicCAS(base + 8 * size_t(b) + i, kTabEmpty, x) == kTabEmpty) return;
@@ -227,42 +321,102 @@ __device__ __forceinline__ void tab_insert(uint32_t *__restrict__ tab, uint32_t 
     }
 }
 
-// Membership tables of the lists of vertices [0, h0), one warp per 32
-// vertices, their entries spread over the lanes.
-__global__ void __launch_bounds__(256)
+// Membership tables of the lists of vertices [0, h0): consecutive vertices'
+// lists, and so their tables, lie one after the other, so a warp builds the
+// tables of up to kTabWords list words at a time in shared memory and writes
+// them out whole -- 4 B read and 8 B written per entry, the atomics in shared
+// memory (built by compare-and-swap in global memory they took 2.3 ms for 20M
+// entries, 0.72 ms this way).  A list longer than that (ids not degree-ranked)
+// is built in place.
+constexpr uint32_t kTabWords = 1024;
+constexpr int kTabWarps = 4;
+
+__global__ void __launch_bounds__(kTabWarps * 32)
 k_tables(uint32_t h0, const uint2 *__restrict__ info, const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t v0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; v0 < h0; v0 += warps * 32) {
+    __shared__ uint4 sh[kTabWarps][kTabWords / 2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4 *const t4 = sh[warp];
+    uint32_t *const t = reinterpret_cast<uint32_t *>(t4);
+    const uint32_t warps = gridDim.x * kTabWarps;
+    for (uint32_t v0 = (blockIdx.x * kTabWarps + warp) * 32; v0 < h0; v0 += warps * 32) {
         const uint32_t v = v0 + lane;
         const uint2 inf = v < h0 ? info[v] : make_uint2(0, 0);
-        uint32_t incl = inf.y;
-        #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-        for (uint32_t f0 = 0; f0 < total; f0 += 32) {
-            const uint32_t f = f0 + lane;
-            uint32_t owner = 0;
+        uint32_t left = padded(inf.y);  // words of this lane's list not built yet
+        while (true) {
+            // the lanes whose lists fit together, from the first one left on
+            uint32_t incl = left;
             #pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const uint32_t probe = __shfl_sync(kFullMask, incl, int(owner + step - 1));
-                if (probe <= f) owner += step;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= o) incl += y;
             }
-            owner = min(owner, 31u);
-            const uint32_t off = __shfl_sync(kFullMask, inf.x, int(owner));
-            const uint32_t len = __shfl_sync(kFullMask, inf.y, int(owner));
-            const uint32_t end = __shfl_sync(kFullMask, incl, int(owner));
-            if (f < total) tab_insert(tab, off, len, __ldg(adj + off + (f - (end - len))));
+            const unsigned todo = __ballot_sync(kFullMask, left != 0);
+            if (!todo) break;
+            const int first = __ffs(todo) - 1;
+            const uint32_t off0 = __shfl_sync(kFullMask, inf.x, first);
+            const unsigned sel = __ballot_sync(kFullMask, left != 0 && incl <= kTabWords);
+            if (!sel) {  // the first one alone is too long
+                const uint32_t len = __shfl_sync(kFullMask, inf.y, first);
+                uint32_t *const base = tab + 2 * size_t(off0);
+                for (uint32_t i = lane; i < 2 * padded(len); i += 32) base[i] = kTabEmpty;
+                __syncwarp();
+                for (uint32_t i = lane; i < len; i += 32) tab_insert(base, len, __ldg(adj + off0 + i));
+                __syncwarp();
+                if (lane == first) left = 0;
+                continue;
+            }
+            const bool mine = (sel >> lane) & 1u;
+            const uint32_t words = __shfl_sync(kFullMask, incl, 31 - __clz(sel));
+            for (uint32_t i = lane; i < words / 2; i += 32) t4[i] = make_uint4(kTabEmpty, kTabEmpty, kTabEmpty, kTabEmpty);
+            __syncwarp();
+            // word w of the run belongs to the last selected list that starts
+            // at or before it; the padding is skipped
+            for (uint32_t w0 = 0; w0 < words; w0 += 128) {
+                uint32_t x[4];  // four reads in flight per lane
+                #pragma unroll
+                for (int h = 0; h < 4; ++h) x[h] = w0 + 32 * h + lane < words ? __ldg(adj + off0 + w0 + 32 * h + lane) : kPad;
+                #pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const uint32_t w = w0 + 32 * h + lane, owner = run_owner(incl, w);
+                    const uint32_t off = __shfl_sync(kFullMask, inf.x, int(owner));
+                    const uint32_t len = __shfl_sync(kFullMask, inf.y, int(owner));
+                    if (x[h] != kPad) tab_insert(t + 2 * (off - off0), len, x[h]);
+                }
+            }
+            __syncwarp();
+            uint4 *const out = reinterpret_cast<uint4 *>(tab + 2 * size_t(off0));
+            for (uint32_t i = lane; i < words / 2; i += 32) out[i] = t4[i];
+            __syncwarp();
+            if (mine) left = 0;
         }
     }
 }
 
-// The same for the hubs [h0, n): one warp per 512 entries of a list.
+// The same for hubs, one block per list of [h0, h1) with its table of 8 B per
+// entry in dynamic shared memory.
+__global__ void __launch_bounds__(1024)
+k_tables_hub(uint32_t h0, uint32_t h1, const uint2 *__restrict__ info, const uint32_t *__restrict__ adj,
+             uint32_t *__restrict__ tab) {
+    extern __shared__ __align__(16) uint32_t t[];
+    uint4 *const t4 = reinterpret_cast<uint4 *>(t);
+    for (uint32_t v = h0 + blockIdx.x; v < h1; v += gridDim.x) {
+        const uint2 inf = info[v];
+        const uint32_t quads = padded(inf.y) / 2;
+        for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x)
+            t4[i] = make_uint4(kTabEmpty, kTabEmpty, kTabEmpty, kTabEmpty);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < inf.y; i += blockDim.x) tab_insert(t, inf.y, __ldg(adj + inf.x + i));
+        __syncthreads();
+        uint4 *const out = reinterpret_cast<uint4 *>(tab + 2 * size_t(inf.x));
+        for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x) out[i] = t4[i];
+        __syncthreads();
+    }
+}
+
+// Hubs whose table does not fit shared memory: in global memory (cleared
+// before), one warp per 512 entries of a list.
 __global__ void __launch_bounds__(256)
-k_tables_hubs(uint32_t h0, uint32_t n, uint32_t chunks, const uint2 *__restrict__ info,
+k_tables_long(uint32_t h0, uint32_t n, uint32_t chunks, const uint2 *__restrict__ info,
               const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5, tasks = uint64_t(n - h0) * chunks;
@@ -271,7 +425,7 @@ k_tables_hubs(uint32_t h0, uint32_t n, uint32_t chunks, const uint2 *__restrict_
         const uint32_t a = uint32_t(t % chunks) * 512;
         if (a >= inf.y) continue;
         const uint32_t b = min(a + 512, inf.y);
-        for (uint32_t i = a + lane; i < b; i += 32) tab_insert(tab, inf.x, inf.y, __ldg(adj + inf.x + i));
+        for (uint32_t i = a + lane; i < b; i += 32) tab_insert(tab + 2 * size_t(inf.x), inf.y, __ldg(adj + inf.x + i));
     }
 }
 
@@ -439,7 +593,8 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
         LCK(sc.get(&seg_e, size_t(n) * dirs));
         LCK(sc.get(&fill, total));
     }
-    const uint32_t wgrid = std::max<uint32_t>(1, std::min<uint32_t>((n + 7) / 8, 148u * 16));
+    uint32_t *d_queue = nullptr;
+    LCK(sc.get(&d_queue, n));
     for (int dir = 0; dir < dirs; ++dir) {
         const uint64_t *off = dir ? d_ioff : d_ooff;
         const uint32_t *src = dir ? d_iadj : d_oadj;
@@ -448,7 +603,12 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
         k_info<<<grid, 256, 0, s>>>(n, d_orig, off, starts[dir], base, info,
                                     seg_b ? seg_b + size_t(dir) * n : nullptr,
                                     seg_e ? seg_e + size_t(dir) * n : nullptr);
-        if (n) k_fill<<<wgrid, 256, 0, s>>>(n, d_orig, d_rank, off, src, info, fill);
+        if (n) {
+            LCK(cudaMemsetAsync(d_flag, 0, sizeof(uint32_t), s));  // here: lists queued
+            k_fill<<<std::max<uint32_t>(1, std::min<uint32_t>((n + 255) / 256, 148u * 8)), 256, 0, s>>>(
+                n, d_orig, d_rank, off, src, info, fill, d_queue, d_flag);
+            k_fill_long<<<148 * 4, 512, 0, s>>>(d_orig, d_rank, off, src, info, fill, d_queue, d_flag);
+        }
         LCK(cudaGetLastError());
     }
     if (relabel && m) {
@@ -554,28 +714,40 @@ int device_tables(DeviceGraph &g) {
         g.tab = nullptr;
         return CUTS_OK;
     }
-    LCK(cudaMemsetAsync(g.tab, 0xff, bytes, s));
     const int dirs = g.symmetric ? 1 : 2;
     auto deg = [&](uint32_t d) {
         return uint64_t(g.h_out_deg[d]) + (g.symmetric ? 0u : g.h_in_deg[d]);
     };
     // ids are degree ranks (unless relabelling is off: then every list goes
-    // to the first kernel): the hubs, more than 512 entries, are a suffix
-    uint32_t h0 = g.n;
-    if (!g.orig.empty()) {
+    // to the first kernel), so the lists of more than L entries are a suffix
+    auto longer = [&](uint64_t L) {
         uint32_t lo = 0, hi = g.n;
+        if (g.orig.empty()) return g.n;
         while (lo < hi) {
             const uint32_t mid = lo + (hi - lo) / 2;
-            if (deg(mid) <= 512) lo = mid + 1; else hi = mid;
+            if (deg(mid) <= L) lo = mid + 1; else hi = mid;
         }
-        h0 = lo;
-    }
-    const uint32_t chunks = (g.max_deg + 511) / 512;
+        return lo;
+    };
+    constexpr uint32_t kMid = 4096, kBig = 24576;  // 32 KB and 192 KB of shared memory
+    const uint32_t h0 = longer(kTabWords), h1 = longer(kMid), h2 = longer(kBig);
+    LCK(cudaFuncSetAttribute(k_tables_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBig * 8)));
     for (int dir = 0; dir < dirs; ++dir) {
         const uint2 *info = dir ? g.in_info : g.out_info;
-        k_tables<<<std::max<uint32_t>(1, std::min<uint32_t>((h0 + 255) / 256, 148u * 8)), 256, 0, s>>>(h0, info, g.adj,
-                                                                                                    g.tab);
-        if (h0 < g.n) k_tables_hubs<<<148 * 8, 256, 0, s>>>(h0, g.n, chunks, info, g.adj, g.tab);
+        k_tables<<<std::max<uint32_t>(1, std::min<uint32_t>((h0 + 127) / 128, 148u * 7)), kTabWarps * 32, 0, s>>>(
+            h0, info, g.adj, g.tab);
+        if (h1 > h0) k_tables_hub<<<std::min<uint32_t>(h1 - h0, 148u * 6), 256, kMid * 8, s>>>(h0, h1, info, g.adj, g.tab);
+        if (h2 > h1) k_tables_hub<<<std::min<uint32_t>(h2 - h1, 148u), 1024, kBig * 8, s>>>(h1, h2, info, g.adj, g.tab);
+        if (h2 < g.n) {
+            // their words are the last ones of this direction's lists
+            uint2 first = make_uint2(0, 0);
+            LCK(cudaMemcpyAsync(&first, info + h2, sizeof(first), cudaMemcpyDeviceToHost, s));
+            LCK(cudaStreamSynchronize(s));
+            uint64_t words = 0;
+            for (uint32_t d = h2; d < g.n; ++d) words += (uint64_t(dir ? g.h_in_deg[d] : g.h_out_deg[d]) + 3) & ~uint64_t(3);
+            LCK(cudaMemsetAsync(g.tab + 2 * size_t(first.x), 0xff, 8 * words, s));
+            k_tables_long<<<148 * 8, 256, 0, s>>>(h2, g.n, (g.max_deg + 511) / 512, info, g.adj, g.tab);
+        }
         LCK(cudaGetLastError());
     }
     return CUTS_OK;

@@ -67,3 +67,42 @@ def test_tables_match_oracle(directed, ranked, monkeypatch):
             assert (r.count, r.level_sizes) == (cnt, lv), (name, flags)
         assert g.count(q, flags=cb.FLAG_SYMMETRY_BREAK).count == cnt, name
     g.close()
+
+
+@pytest.mark.parametrize("ranked", [True, False])
+@pytest.mark.parametrize("directed", [False, True])
+def test_hub_tables(directed, ranked, monkeypatch):
+    """Lists at the lengths where the tables' build changes kernel (one run in
+    shared memory, one block, one large block, in place): hubs over a ring, so
+    every triangle tests a hub's table."""
+    if not ranked:
+        monkeypatch.setenv("CUTS_NO_RELABEL", "1")
+    degs = [1020, 1023, 1024, 1025, 4095, 4096, 4097, 24574, 24576, 24577, 26000]
+    h, ring = len(degs), 26100
+    n = h + ring
+    rng = np.random.default_rng(3)
+    src, dst = [np.arange(ring) + h], [(np.arange(ring) + 1) % ring + h]
+    for i, d in enumerate(degs):  # d ring vertices each, so d or d + 10 entries
+        to = rng.choice(ring, d, replace=False) + h
+        src.append(np.full(d, i))
+        dst.append(to)
+    a, b = np.triu_indices(h, 1)
+    if not directed:
+        src.append(a)
+        dst.append(b)
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    if not directed:
+        src, dst = np.concatenate([src, dst]), np.concatenate([dst, src])
+    oo, oa, io, ia, s, d = csr_from_arcs(n, src.astype(np.uint32), dst.astype(np.uint32))
+    g = cb.Graph.from_csr(n, oo, oa, io, ia)
+    od = O.Graph.from_arrays(n, s, d)
+    k, arcs = (3, [(0, 1), (1, 2), (0, 2)]) if directed else cb.named_query_arcs("triangle")
+    q = cb.Query.from_arcs(k, arcs)
+    cnt, lv, _ = O.count(od, O.Graph.from_arcs(k, arcs), q.order)
+    assert cnt > 0
+    for flags in (0, cb.FLAG_NO_FUSE, cb.FLAG_NO_FUSE | cb.FLAG_SYMMETRY_BREAK):
+        r = g.count(q, flags=flags, stats=True)
+        assert r.count == cnt, flags
+        if not flags & cb.FLAG_SYMMETRY_BREAK:
+            assert r.level_sizes == lv, flags
+    g.close()
