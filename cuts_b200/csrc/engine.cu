@@ -65,7 +65,8 @@ struct RunParams {
     uint32_t pos_lvl;
     uint32_t fuse_stride;  // words per warp row of the fused kernel's scratch
     uint32_t *fuse_scratch;
-    uint32_t *fuse_big;    // the fused kernel's deferred parents (counters, arrays, pool)
+    uint32_t pairs;        // the fused count runs in k_pairs (else k_fused)
+    uint32_t *fuse_big;    // the fused kernel's deferred parents (arrays, pool or bitmaps)
     uint32_t fuse_big_cap;
     uint32_t fuse_pool_words;
     uint32_t *vert[kMaxK];
@@ -881,45 +882,23 @@ struct FusedBig {
     unsigned long long pool_words;
 };
 
-// Phase 1 keeps a parent's candidate set S in shared memory when it holds at
-// most kTS vertices; every pair (s, t) of S is then tested by a lane-balanced
-// walk (see pair_walk below).
-constexpr uint32_t kTS = 256;
-constexpr uint32_t kHS = 512;  // hash slots of the admissible t, buckets of 4 (load at most 1/2)
-
-// WALK instances (phase 1 of plans the pair walk covers): 8 resident blocks
-// (32 warps) per SM at up to 64 registers -- the walk keeps its row state
-// in registers and ~25 KB of tables in shared memory.  The others: 12
-// resident blocks (48 warps) at 40 registers -- they wait on dependent L2
-// loads, and the extra warps outweigh the spills that cap costs.
-template <int MODE, bool WALK, bool TALLY = false>
-__global__ void __launch_bounds__(kZW * 32, WALK ? 8 : 12)
+// 12 resident blocks (48 warps) per SM at 40 registers: the kernel waits on
+// dependent L2 loads, and the extra warps outweigh the spills that cap costs.
+template <int MODE>
+__global__ void __launch_bounds__(kZW * 32, 12)
 k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents parents, uint32_t phase,
         uint32_t split, uint32_t *__restrict__ cursor, uint32_t *__restrict__ scratch, uint32_t stride, FusedBig big,
         unsigned long long *__restrict__ acc, unsigned long long *__restrict__ acc_c,
-        unsigned long long *__restrict__ acc_p, unsigned long long *__restrict__ acc_bytes) {
+        unsigned long long *__restrict__ acc_p) {
     uint32_t pa, total;
     parents_of(parents, pa, total);
     if (!total) return;
-    constexpr bool walk_ok = WALK && MODE == kCountMode;
-    // TALLY: also add the bytes this count reads from global memory to
-    // *acc_bytes (the last level's algorithmic traffic; counts go to scratch)
-    constexpr bool tally = TALLY && MODE == kCountMode;
-    unsigned long long tb = 0;
     __shared__ LevelPlan sP, sC, sF;
     __shared__ uint32_t *s_vert[kMaxK];
     __shared__ uint32_t *s_par[kMaxK];
     __shared__ uint32_t wm[kZW][kMaxK];
     __shared__ uint32_t joff[kZW][kMaxJ], jdeg[kZW][kMaxJ], jver[kZW][kMaxJ];
     __shared__ uint32_t xoff[kZW][kMaxJ], xdeg[kZW][kMaxJ];
-    // the pair walk's per-parent tables: S, and a hash table of the vertices
-    // admissible as t (keys in buckets of 4, their index in S and term B)
-    __shared__ uint32_t tS[walk_ok ? kZW : 1][kTS];
-    __shared__ uint4 tHK[walk_ok ? kZW : 1][kHS / 4];
-    // dense core: the admissible t of S as bits of the core (per warp)
-    __shared__ uint32_t tSV[walk_ok ? kZW : 1][kCore / 32];
-    __shared__ uint8_t tHI[walk_ok ? kZW : 1][kHS];
-    __shared__ int32_t tHB[walk_ok ? kZW : 1][kHS];
     {
         const uint32_t words = sizeof(LevelPlan) / 4;
         const uint32_t c = p + 1;
@@ -1027,12 +1006,11 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                     }
                     fbase = (we > ws ? we - ws : 0) - sub;
                 }
-                if (MODE == kBytesMode || tally) {
+                if (MODE == kBytesMode) {
                     const unsigned long long by = 12 + 4ull * nit + uint64_t(nit) * 4 * probes(iters ? ds : nS) +
                                                   (sig_c ? 8ull * nit : 0) +
                                                   (cfold ? 8 + 4ull * (p + 1) * probes(fdeg) : 0);
-                    if (MODE == kBytesMode) local += by;
-                    else tb += by;
+                    local += by;
                 }
             }
             if (MODE == kBytesMode) return;
@@ -1168,14 +1146,11 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             const uint32_t nS = te - ts, nL = ls1 > ls0 ? ls1 - ls0 : 0;
             const bool iterS = nS <= nL;
             const uint32_t nit = iterS ? nS : nL;
-            if (MODE == kBytesMode || tally) {
+            if (MODE == kBytesMode) {
                 const unsigned long long by = 12 + 4ull * nit + uint64_t(nit) * 4 * probes(iterS ? ds : nS) +
                                               (sig_c ? 8ull * nit : 0) + (cfold ? 8 + 4ull * (p + 1) * probes(fdeg) : 0);
-                if (lane == 0) {
-                    if (MODE == kBytesMode) local += by;
-                    else tb += by;
-                }
-                if (MODE == kBytesMode) continue;
+                if (lane == 0) local += by;
+                continue;
             }
             uint32_t gal = iterS ? ls0 : ts;
             for (uint32_t y0 = 0; y0 < nit; y0 += 32) {
@@ -1219,297 +1194,6 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             }
         }
         __syncwarp();
-    };
-
-    // Level c over all pairs of a parent whose S fits tS (phase 1).  A pair
-    // (s, t) of S counts when t lies in s's list, inside s's window (t > s
-    // or t < s when the plan orders them; t != s otherwise), and passes the
-    // tests that depend on t alone (window of the positions below p, the
-    // extra lists, the signature); its weight splits as A(s) + B(t):
-    //   no fold:     1 + 0;
-    //   orbit fold:  (orbit base with s at p) - #orbit positions below c,
-    //                plus, when c is in the orbit, |L(t)| - c - [t loops];
-    //   plain fold:  f_base(s) - [t in the fold's window and list], the fold's
-    //                list and window fixed by the positions below p
-    //                (walk_ok is set only then).
-    // The admissible t go into a hash table in shared memory (buckets of
-    // four keys read with one 128-bit load; each slot keeps B(t) and t's
-    // index in S).  Each s's list window is then streamed with 128-bit
-    // loads: the windows of 32 vertices s (one per lane, each lane also
-    // holding its A(s)) form one sequence of 16-byte quads spread over the
-    // lanes, two quads per lane per step (owner found by a binary search
-    // over the lanes' inclusive scan), and each of the four list entries of
-    // a quad is looked up in the table -- coalesced global reads and
-    // shared-memory probes instead of a search in a list and a gather of
-    // the pendant's weight per pair.
-    auto pair_walk = [&](uint32_t ns, uint32_t lo_c, uint32_t hi_c) {
-        uint32_t *const S = tS[warp];
-        const long long akc = (cfold && sF.ofold) ? __popc(sF.ofold & ((1u << c) - 1)) : 0;
-        const bool c_in_orbit = cfold && sF.ofold && ((sF.ofold >> c) & 1u);
-        const bool p_in_orbit = cfold && sF.ofold && ((sF.ofold >> p) & 1u);
-        // plain fold: the fold's list and window, fixed for this parent
-        uint32_t f_off = 0, f_deg = 0, f_lo = 0, f_hi = kFullMask, f_ws = 0, f_we = 0, f_sub = 0;
-        if (cfold && !sF.ofold) {
-            const uint32_t u = my_m[sF.jpos[0]];
-            const uint2 inf = sF.jdir[0] ? g.in_info[u] : g.out_info[u];
-            f_off = inf.x;
-            f_deg = inf.y;
-            for (uint32_t msk = sF.gt_mask & below; msk; msk &= msk - 1) f_lo = max(f_lo, my_m[__ffs(msk) - 1] + 1);
-            for (uint32_t msk = sF.lt_mask & below; msk; msk &= msk - 1) f_hi = min(f_hi, my_m[__ffs(msk) - 1]);
-            const uint32_t *fl = g.adj + f_off;
-            f_ws = f_lo ? lbound(fl, f_deg, f_lo) : 0;
-            f_we = f_hi != kFullMask ? lbound(fl, f_deg, f_hi) : f_deg;
-            for (uint32_t j = 0; j < p; ++j) {
-                const uint32_t mj = my_m[j];
-                if (mj >= f_lo && mj < f_hi && (((sF.guar_mask >> j) & 1u) || contains(fl, f_deg, mj))) ++f_sub;
-            }
-        }
-        // orbit fold: the part of the orbit base fixed by the positions below
-        // p (the lists of the orbit positions x < p, minus the members the
-        // positions below p put there)
-        uint32_t ob_par = 0;
-        const uint32_t ob_low = (cfold && sF.ofold) ? (sF.ofold & below) : 0;
-        for (uint32_t xm = ob_low; xm; xm &= xm - 1) {
-            const uint32_t x = __ffs(xm) - 1;
-            const uint2 inf = sF.jdir[0] ? g.in_info[my_m[x]] : g.out_info[my_m[x]];
-            uint32_t sub = 0;
-            for (uint32_t j = 0; j < p; ++j)
-                if (((sF.oguar[x] >> j) & 1u) || contains(g.adj + inf.x, inf.y, my_m[j])) ++sub;
-            ob_par += inf.y - sub;
-        }
-        // the table: buckets of 4 slots (one 128-bit shared load), a power of
-        // two of at least one bucket per two vertices of S, 8..kHS/4; a full
-        // bucket continues in the next one
-        uint32_t lg = 3;
-        while ((1u << lg) * 2 < ns && (1u << lg) < kHS / 4) ++lg;
-        const uint32_t bmask = (1u << lg) - 1;
-        const uint32_t hshift = 32 - lg;
-        uint4 *const HK4 = tHK[warp];
-        uint32_t *const HK = reinterpret_cast<uint32_t *>(tHK[warp]);
-        uint8_t *const HI = tHI[warp];
-        int32_t *const HB = tHB[warp];
-        const bool need_idx = !c_gt_s && !c_lt_s && loops;
-        // dense core path for rows s in the core: every t > s is then in the
-        // core too, and s's pairs are popcounts of its bitmap row against
-        // the admissible t (needs t > s, no extra lists, and B(t) from t's
-        // degree alone)
-        const bool core_rows = g.core_bits && c_gt_s && !extra && (!cfold || (sF.ofold && !loops));
-        // the table serves rows below the core only
-        const bool table = !core_rows || S[0] < g.core0;
-        uint32_t *const SV = tSV[warp];
-        if (core_rows) SV[lane] = 0;
-        if (table)
-            for (uint32_t x = lane; x <= bmask; x += 32) HK4[x] = make_uint4(kFullMask, kFullMask, kFullMask, kFullMask);
-        __syncwarp();
-        // the admissible t, with B(t), into the table
-        uint32_t nv = 0;
-        for (uint32_t i0 = 0; i0 < ns; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            bool ok = i < ns;
-            const uint32_t v = ok ? S[i] : 0;
-            if (ok) {
-                ok = v >= lo_c && v < hi_c;
-                if (ok && extra)
-                    for (uint32_t tt = 0; tt < sC.nj; ++tt)
-                        if ((extra >> tt) & 1u)
-                            if (!contains(g.adj + xoff[warp][tt], xdeg[warp][tt], v)) { ok = false; break; }
-                ok = ok && v >= sC.sig_lo;
-                if (ok && sig_c) {
-                    const uint2 o = g.out_info[v], i2 = g.in_info[v];
-                    ok = i2.y >= sC.qin && o.y >= sC.qout;
-                }
-            }
-            if (ok && core_rows && v >= g.core0) {
-                const uint32_t u = v - g.core0;
-                atomicOr(&SV[u >> 5], 1u << (u & 31));
-            }
-            if (ok && table) {
-                int32_t b = 0;
-                if (c_in_orbit) {
-                    if (tally) tb += 8;
-                    const uint2 vi = sF.jdir[0] ? g.in_info[v] : g.out_info[v];
-                    b = int32_t(vi.y) - int32_t(c) - ((loops && contains(g.adj + vi.x, vi.y, v)) ? 1 : 0);
-                } else if (cfold && !sF.ofold) {
-                    const bool h = v >= f_lo && v < f_hi && (fguar_t || contains(g.adj + f_off, f_deg, v));
-                    b = h ? -1 : 0;
-                }
-                uint32_t bk = (v * 2654435769u) >> hshift;
-                while (true) {
-                    uint32_t slot = kFullMask;
-                    #pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        if (slot == kFullMask && atomicCAS(&HK[bk * 4 + q], kFullMask, v) == kFullMask) slot = bk * 4 + q;
-                    if (slot != kFullMask) {
-                        HI[slot] = uint8_t(i);
-                        HB[slot] = b;
-                        break;
-                    }
-                    bk = (bk + 1) & bmask;
-                }
-            }
-            nv += __popc(__ballot_sync(kFullMask, ok));
-        }
-        if (nv == 0) return;
-        __syncwarp();
-        long long sum = 0;
-        unsigned long long hits = 0;
-        const uint4 *const adj4 = reinterpret_cast<const uint4 *>(g.adj);
-        for (uint32_t r0 = 0; r0 < ns; r0 += 32) {
-            // this lane's row: s = S[r0 + lane], its list window as quads and
-            // its term A(s)
-            const uint32_t i = r0 + lane;
-            uint32_t ea = 0, eb = 0, nq = 0, arow = 1;
-            if (i < ns) {
-                const uint32_t sv = S[i];
-                {
-                    // A(s): the orbit base with s at p (orbit_base's sum, the
-                    // parent's part computed once), or the plain fold's base
-                    if (cfold && sF.ofold) {
-                        arow = ob_par;
-                        for (uint32_t xm = ob_low; xm; xm &= xm - 1) {
-                            const uint32_t x = __ffs(xm) - 1;
-                            if ((sF.oguar[x] >> p) & 1u) {
-                                --arow;
-                            } else {
-                                const uint2 xi = sF.jdir[0] ? g.in_info[my_m[x]] : g.out_info[my_m[x]];
-                                if (contains(g.adj + xi.x, xi.y, sv)) --arow;
-                            }
-                        }
-                        if (p_in_orbit) {
-                            const uint2 vi = sF.jdir[0] ? g.in_info[sv] : g.out_info[sv];
-                            uint32_t sub = (((sF.oguar[p] >> p) & 1u) || (loops && contains(g.adj + vi.x, vi.y, sv)))
-                                               ? 1u : 0u;
-                            for (uint32_t j = 0; j < p; ++j)
-                                if (((sF.oguar[p] >> j) & 1u) || contains(g.adj + vi.x, vi.y, my_m[j])) ++sub;
-                            arow += vi.y - sub;
-                        }
-                    } else if (cfold) {
-                        const bool in = sv >= f_lo && sv < f_hi &&
-                                        (((sF.guar_mask >> p) & 1u) || contains(g.adj + f_off, f_deg, sv));
-                        arow = (f_we > f_ws ? f_we - f_ws : 0) - f_sub - (in ? 1u : 0u);
-                    }
-                }
-                if (core_rows && sv >= g.core0) {
-                    // a core row: t ranges over the admissible core bits
-                    // above s in s's bitmap row
-                    const uint32_t si = sv - g.core0;
-                    const uint4 *rowp = reinterpret_cast<const uint4 *>(g.core_bits + size_t(si) * (kCore / 32));
-                    const uint32_t w0 = si >> 5;
-                    uint32_t cnt = 0;
-                    long long dsum = 0;
-                    for (uint32_t q = w0 >> 2; q < kCore / 128; ++q) {
-                        const uint4 r4 = __ldg(rowp + q);
-                        const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
-                        #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) {
-                            const uint32_t j = 4 * q + k;
-                            if (j < w0) continue;
-                            uint32_t w = rw[k] & SV[j];
-                            if (j == w0) w &= ~((2u << (si & 31)) - 1u);
-                            cnt += __popc(w);
-                            if (c_in_orbit)
-                                for (; w; w &= w - 1) dsum += g.out_info[g.core0 + 32 * j + __ffs(w) - 1].y;
-                        }
-                    }
-                    // the row's bitmap words from s's own word on, and t's
-                    // degree per hit (orbit fold)
-                    if (tally) tb += 8 + 16ull * (kCore / 128 - (w0 >> 2)) + (c_in_orbit ? 8ull * cnt : 0);
-                    if (cnt) {
-                        hits += cnt;
-                        // B(t) = |L(t)| - c for the orbit fold's pendant (no self-loops here)
-                        sum += (long long)cnt * ((long long)arow - akc) + (c_in_orbit ? dsum - (long long)cnt * c : 0);
-                    }
-                } else {
-                    const uint2 is = sC.jdir[tp] ? g.in_info[sv] : g.out_info[sv];
-                    const uint32_t *Ls = g.adj + is.x;
-                    uint32_t lo_v = lo_c, hi_v = hi_c;
-                    if (c_gt_s) lo_v = max(lo_v, sv + 1);
-                    if (c_lt_s) hi_v = min(hi_v, sv);
-                    const bool sdir = sC.jdir[tp] != 0;
-                    const uint32_t p0 = lo_v ? lbound_own(g, sdir, sv, Ls, is.y, lo_v, loops) : 0;
-                    const uint32_t p1 = hi_v != kFullMask ? lbound_own(g, sdir, sv, Ls, is.y, hi_v, loops) : is.y;
-                    if (p1 > p0) {
-                        ea = is.x + p0;
-                        eb = is.x + p1;
-                        nq = ((eb + 3) >> 2) - (ea >> 2);
-                    }
-                    // s's info, its window bound, the window's quads
-                    if (tally) tb += 12 + 16ull * nq;
-                }
-            }
-            uint32_t incl = nq;
-            #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const uint32_t qtotal = __shfl_sync(kFullMask, incl, 31);
-            const uint32_t excl = incl - nq;
-            // two quads per lane per step (more loads in flight)
-            for (uint32_t fstep = 0; fstep < qtotal; fstep += 64) {
-                uint32_t quad[2], qea[2], qeb[2], qoi[2], qa[2];
-                bool have[2];
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint32_t f = fstep + 32 * h + lane;
-                    uint32_t owner = 0;
-                    #pragma unroll
-                    for (int step = 16; step; step >>= 1) {
-                        const uint32_t probe = __shfl_sync(kFullMask, incl, int(owner + step - 1));
-                        if (probe <= f) owner += step;
-                    }
-                    owner = min(owner, 31u);
-                    const int ow = int(owner);
-                    const uint32_t o_excl = __shfl_sync(kFullMask, excl, ow);
-                    qea[h] = __shfl_sync(kFullMask, ea, ow);
-                    qeb[h] = __shfl_sync(kFullMask, eb, ow);
-                    qa[h] = __shfl_sync(kFullMask, arow, ow);
-                    have[h] = f < qtotal;
-                    qoi[h] = r0 + owner;
-                    quad[h] = (qea[h] >> 2) + (f - o_excl);
-                }
-                uint4 xq[2];
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) xq[h] = have[h] ? __ldg(adj4 + quad[h]) : make_uint4(0, 0, 0, 0);
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (!have[h]) continue;
-                    const uint32_t e0 = quad[h] << 2;
-                    const uint32_t vals[4] = {xq[h].x, xq[h].y, xq[h].z, xq[h].w};
-                    uint32_t cnt = 0;
-                    long long bs = 0;
-                    #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint32_t e = e0 + uint32_t(k);
-                        if (e < qea[h] || e >= qeb[h]) continue;
-                        const uint32_t v = vals[k];
-                        uint32_t bk = (v * 2654435769u) >> hshift;
-                        while (true) {
-                            const uint4 kk = HK4[bk];
-                            const uint32_t eq = (kk.x == v ? 1u : 0u) | (kk.y == v ? 2u : 0u) |
-                                                (kk.z == v ? 4u : 0u) | (kk.w == v ? 8u : 0u);
-                            if (eq) {
-                                const uint32_t slot = bk * 4 + __ffs(eq) - 1;
-                                // t == s only when s lists itself (a data self-loop)
-                                if (!need_idx || HI[slot] != qoi[h]) {
-                                    ++cnt;
-                                    bs += HB[slot];
-                                }
-                                break;
-                            }
-                            if (kk.w == kFullMask) break;  // slots fill in order: an empty slot ends the chain
-                            bk = (bk + 1) & bmask;
-                        }
-                    }
-                    if (cnt) {
-                        hits += cnt;
-                        sum += (long long)cnt * ((long long)qa[h] - akc) + bs;
-                    }
-                }
-            }
-        }
-        local += (unsigned long long)sum;
-        local_c += hits;
     };
 
     while (true) {
@@ -1586,9 +1270,6 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             // this lane's candidates rise, so its lower bounds in the first
             // two other lists rise too: gallop from the last
             uint32_t gp0 = 0, gp1 = 0;
-            // S goes to shared memory when the pair walk will read it (the
-            // other paths search S with global-memory loads)
-            uint32_t *const small = walk_ok ? tS[warp] : row;
             for (uint32_t x0 = s0; x0 < e0; x0 += 32) {
                 const uint32_t x = x0 + lane;
                 bool ok = x < e0;
@@ -1629,21 +1310,18 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                 const unsigned m = __ballot_sync(kFullMask, ok);
                 if (ok) {
                     const uint32_t idx = ns + __popc(m & lanemask_lt);
-                    if (idx < kTS) small[idx] = v;
-                    else row[idx] = v;
+                    row[idx] = v;
                 }
                 ns += __popc(m);
-                if ((MODE == kBytesMode || tally) && lane == 0) {
+                if (MODE == kBytesMode && lane == 0) {
                     uint32_t per = sP.check_sig ? 8 : 0;
                     for (uint32_t t = 0; t < njp; ++t)
                         if (t != tmin) per += 4 * probes(jdeg[warp][t]);
                     const unsigned long long by = 4ull * min(32u, e0 - x0) + uint64_t(min(32u, e0 - x0)) * per;
-                    if (MODE == kBytesMode) local += by;
-                    else tb += by;
+                    local += by;
                 }
             }
             __syncwarp();
-            if (tally && lane == 0) tb += 8ull * p + 8ull * njp + 4ull * ns;
             if (MODE == kCountMode && ns > split) {
                 // defer: save S in the pool for phase 2 (or keep it here when full)
                 unsigned long long off = 0;
@@ -1658,7 +1336,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                 e = __shfl_sync(kFullMask, e, 0);
                 off = __shfl_sync(kFullMask, off, 0);
                 if (e != kFullMask) {
-                    for (uint32_t i = lane; i < ns; i += 32) big.pool[off + i] = i < kTS ? small[i] : row[i];
+                    for (uint32_t i = lane; i < ns; i += 32) big.pool[off + i] = row[i];
                     if (lane == 0) {
                         big.gi[e] = q0;
                         big.soff[e] = uint32_t(off);
@@ -1671,11 +1349,6 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             if (lane == 0) {
                 local_p += ns;
                 if (MODE == kBytesMode) local += 8ull * p + 8ull * njp + 4ull * ns;
-            }
-            if (walk_ok && ns > kTS) {
-                // the first kTS entries join the rest in the scratch row
-                for (uint32_t i = lane; i < kTS; i += 32) row[i] = small[i];
-                __syncwarp();
             }
         } else {
             S = big.pool + big.soff[b];
@@ -1695,11 +1368,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
         for (uint32_t msk = sC.gt_mask & below; msk; msk &= msk - 1) lo_c = max(lo_c, my_m[__ffs(msk) - 1] + 1);
         for (uint32_t msk = sC.lt_mask & below; msk; msk &= msk - 1) hi_c = min(hi_c, my_m[__ffs(msk) - 1]);
         if (!phase2) {
-            if (walk_ok && ns <= kTS) {
-                if constexpr (walk_ok) pair_walk(ns, lo_c, hi_c);
-                __syncwarp();
-            } else
-                for (uint32_t i0 = 0; i0 < ns; i0 += 32) group(S, ns, i0, lo_c, hi_c);
+            for (uint32_t i0 = 0; i0 < ns; i0 += 32) group(S, ns, i0, lo_c, hi_c);
         } else {
             group(S, ns, grp * 32, lo_c, hi_c);
         }
@@ -1716,25 +1385,23 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             if (local_p) atomicAdd(acc_p, local_p);
         }
     }
-    if (tally) {
-        #pragma unroll
-        for (int o = 16; o; o >>= 1) tb += __shfl_xor_sync(kFullMask, tb, o);
-        if (lane == 0 && tb) atomicAdd(acc_bytes, tb);
-    }
 }
 
-// Inclusive prefix sum of the deferred parents' group counts (one block).
-__global__ void __launch_bounds__(1024) k_fused_scan(FusedBig big) {
+// Inclusive prefix sum of the deferred parents' work items, ceil(len / per)
+// each (one block).
+__global__ void __launch_bounds__(1024)
+k_fused_scan(const unsigned long long *__restrict__ nb, uint32_t cap, const uint32_t *__restrict__ len, uint32_t per,
+             uint32_t *__restrict__ pref) {
     __shared__ uint32_t wsum[32];
     __shared__ uint32_t carry;
-    const unsigned long long n0 = big.n[0];
-    const uint32_t n = n0 < big.cap ? uint32_t(n0) : big.cap;
+    const unsigned long long n0 = nb[0];
+    const uint32_t n = n0 < cap ? uint32_t(n0) : cap;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (uint32_t base = 0; base < n; base += blockDim.x) {
         const uint32_t i = base + threadIdx.x;
-        uint32_t v = i < n ? (big.ns[i] + 31) / 32 : 0, x = v;
+        uint32_t v = i < n ? (len[i] + per - 1) / per : 0, x = v;
         #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(kFullMask, x, o);
@@ -1753,10 +1420,709 @@ __global__ void __launch_bounds__(1024) k_fused_scan(FusedBig big) {
         }
         __syncthreads();
         const uint32_t pre = carry + (w ? wsum[w - 1] : 0) + x;
-        if (i < n) big.pref[i] = pre;
+        if (i < n) pref[i] = pre;
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) carry = pre;
         __syncthreads();
+    }
+}
+
+// ---- fused count on symmetric graphs: pairs of a candidate set ----------
+// With p and c = p + 1 fused, level c is every pair (s, t) of one parent's
+// candidate set S (level p) with t in s's list.  On a symmetric graph without
+// self-loops the pairs are unordered: each {a < b} of S with b in a's list is
+// found once and counted for s = a, t = b and for s = b, t = a, as far as the
+// plan's order between p and c and t's own tests (window, extra lists,
+// signature: `adm`) allow.  A pair's weight is A(s) + B(t) (1 + 0 without a
+// fold; see pair_a / pair_b).
+//
+// A warp takes up to 32 parents, one per lane, so the fixed chain per parent
+// (trie path, lists' info, window) runs for all of them at once, and builds
+// their sets, up to kPS vertices a round, into one shared-memory buffer by the
+// candidate walk of k_level_flat.  Then every vertex a of the buffer is an
+// item whose partners are walked the same way, 64 pairs a step: the rest of
+// its set, tested in a's table, or a's neighbours above it, tested for
+// membership in the set through the tables of the parent's lists, whichever
+// are fewer -- one 32-byte load per pair either way.  Vertices of a set with
+// kPC or more in the dense core are rows of the core bitmap instead: per row
+// the admissible members above and below it are 32 popcounts, and the sums
+// over t of B(t) come from the rows of t, so no pair is visited at all.
+// Parents with more than kPS candidates are left to a second launch that
+// deals them out in pieces of kPK candidates (their core members as bitmaps
+// from k_pair_bits); a piece pairs its vertices with neighbours above only.
+//
+// Bound: L2 latency and instruction issue (46 % of issue slots in the 4-clique
+// + pendant's hub slice).  Whole counts against the form with one parent per
+// warp, a hash table of S in shared memory and a degree gather per pair (and,
+// without an order between p and c, galloping intersections): 4-clique +
+// pendant, 1M vertices / 10M edges, symmetry breaking 33.4 -> 8.2 ms; triangle
+// there, plain 75.5 -> 7.0 ms; triangle, 4M / 40M, symmetry breaking 20.2 ->
+// 9.5 ms.
+constexpr int kPW = 4;            // warps per block
+constexpr uint32_t kPS = 512;     // candidates of one round, shared memory words per warp
+constexpr uint32_t kPC = 32;      // core members from which a set's core part is counted by rows
+constexpr uint32_t kPK = 64;      // candidates per piece of a deferred parent
+constexpr uint32_t kPG = 1024;    // candidates a warp keeps of the root parents it took
+
+struct PairBig {
+    unsigned long long *n;  // [0] deferred parents
+    uint32_t *q;            // parent index in L_{p-1}
+    uint32_t *len;          // candidates in its window
+    uint32_t *pref;         // inclusive prefix sum of pieces
+    uint32_t *bits;         // per parent: core members of S, then of T (kCore / 32 words each)
+    uint32_t cap;
+};
+
+// Per-lane columns in shared memory, [row][lane].
+enum PairRow : int { kRowLo = 0, kRowHi, kRowLoC, kRowHiC, kRowBase, kRowFOff, kRowFDeg, kRowFLo, kRowFHi, kPairRows };
+
+__host__ __device__ inline uint32_t pair_words(uint32_t p, uint32_t njp) {
+    return kPS + kPS / 4 + 128 + 4 * 32 + 2 * (kCore / 32) + 32 * (kPairRows + p + 2 * njp);
+}
+
+// What the level-p and level-c tests of one warp's parents need.
+struct PairCtx {
+    const DevView &g;
+    const LevelPlan &P, &C, &F;
+    uint32_t p, extra;
+    bool cfold, ts;             // ts: every member of S is admissible as t
+    const uint32_t *m;          // [position][lane]
+    const uint32_t *off, *deg;  // [join of p][lane]
+    const uint32_t *row;        // [PairRow][lane]
+};
+
+// in_list for the tests off the hot path (weights, t's own tests, third and
+// later lists): one load site, the tables known to be there.
+__device__ __forceinline__ uint32_t pair_list_has(const uint32_t *tab, uint32_t off, uint32_t len, uint32_t v) {
+    if (!len) return 0;
+    const uint32_t nb = (len + 3) >> 2;
+    uint32_t b = tab_bucket(nb, v);
+    while (true) {
+        const Bucket bk = load_bucket(tab, off, b);
+        if (bucket_has(bk, v)) return 1;
+        if (bk.k[7] == kTabEmpty) return 0;
+        b = b + 1 == nb ? 0 : b + 1;
+    }
+}
+
+__device__ __forceinline__ bool pair_sig(const DevView &g, const LevelPlan &L, uint32_t v) {
+    if (v < L.sig_lo) return false;
+    if (!L.check_sig) return true;
+    const uint32_t d = g.out_info[v].y;  // symmetric: both degrees
+    return d >= L.qin && d >= L.qout;
+}
+
+// v, known to lie in join t0 of the parent in column l, is in its S.
+__device__ __forceinline__ bool pair_in_set(const PairCtx &x, uint32_t l, uint32_t t0, uint32_t v) {
+    if (v < x.row[32 * kRowLo + l] || v >= x.row[32 * kRowHi + l]) return false;
+    for (uint32_t t = 0; t < x.P.nj; ++t)
+        if (t != t0 && !pair_list_has(x.g.tab, x.off[32 * t + l], x.deg[32 * t + l], v)) return false;
+    for (uint32_t j = 0; j < x.p; ++j)
+        if (x.m[32 * j + l] == v) return false;
+    return pair_sig(x.g, x.P, v);
+}
+
+// The member v of S is admissible as t.
+__device__ __forceinline__ bool pair_adm(const PairCtx &x, uint32_t l, uint32_t v) {
+    if (x.ts) return true;
+    if (v < x.row[32 * kRowLoC + l] || v >= x.row[32 * kRowHiC + l]) return false;
+    for (uint32_t t = 0; t < x.C.nj; ++t)
+        if ((x.extra >> t) & 1u) {
+            const uint2 inf = x.g.out_info[x.m[32 * x.C.jpos[t] + l]];
+            if (!pair_list_has(x.g.tab, inf.x, inf.y, v)) return false;
+        }
+    return pair_sig(x.g, x.C, v);
+}
+
+// A(v): the weight of v at position p, without what t adds -- the orbit base
+// with v at p minus the orbit positions below c (each of their lists holds
+// t), or the plain fold's base minus v's own membership.
+__device__ __forceinline__ uint32_t pair_a(const PairCtx &x, uint32_t l, uint32_t v) {
+    if (!x.cfold) return 1;
+    const LevelPlan &F = x.F;
+    uint32_t a = x.row[32 * kRowBase + l];
+    if (F.ofold) {
+        for (uint32_t xm = F.ofold & ((1u << x.p) - 1); xm; xm &= xm - 1) {
+            const uint32_t o = __ffs(xm) - 1;
+            bool in = (F.oguar[o] >> x.p) & 1u;
+            if (!in) {
+                const uint2 inf = x.g.out_info[x.m[32 * o + l]];
+                in = pair_list_has(x.g.tab, inf.x, inf.y, v);
+            }
+            a -= in;
+        }
+        if ((F.ofold >> x.p) & 1u) {
+            const uint2 inf = x.g.out_info[v];
+            a += inf.y;
+            for (uint32_t j = 0; j < x.p; ++j)
+                if (((F.oguar[x.p] >> j) & 1u) || pair_list_has(x.g.tab, inf.x, inf.y, x.m[32 * j + l])) --a;
+        }
+        return a - __popc(F.ofold & ((1u << (x.p + 1)) - 1));
+    }
+    const bool in = v >= x.row[32 * kRowFLo + l] && v < x.row[32 * kRowFHi + l] &&
+                    (((F.guar_mask >> x.p) & 1u) || pair_list_has(x.g.tab, x.row[32 * kRowFOff + l], x.row[32 * kRowFDeg + l], v));
+    return a - in;
+}
+
+// B(v): what v at position c adds (an orbit vertex its own list outside the
+// core; the plain fold loses v itself).  Sums wrap in 32 bits, totals do not.
+__device__ __forceinline__ uint32_t pair_b(const PairCtx &x, uint32_t l, uint32_t v) {
+    if (!x.cfold) return 0;
+    const LevelPlan &F = x.F;
+    const uint32_t c = x.p + 1;
+    if (F.ofold) return ((F.ofold >> c) & 1u) ? x.g.out_info[v].y - c : 0u;
+    const bool in = v >= x.row[32 * kRowFLo + l] && v < x.row[32 * kRowFHi + l] &&
+                    (((F.guar_mask >> c) & 1u) || pair_list_has(x.g.tab, x.row[32 * kRowFOff + l], x.row[32 * kRowFDeg + l], v));
+    return in ? 0xffffffffu : 0u;
+}
+
+// One lane's parent q0 at level p - 1: matched vertices, joined lists, windows
+// and fold data into its columns; the shortest list and its window out.
+struct PairParent {
+    uint32_t moff, s0, e0, tmin;
+};
+
+__device__ __forceinline__ PairParent pair_parent(const DevView &g, const RunParams *rp, const LevelPlan &P,
+                                                  const LevelPlan &C, const LevelPlan &F, bool cfold, uint32_t p,
+                                                  uint32_t *const *s_vert, uint32_t *const *s_par, uint32_t q0,
+                                                  uint32_t lane, uint32_t *m, uint32_t *off, uint32_t *deg,
+                                                  uint32_t *row) {
+    uint32_t e = q0;
+    for (int j = int(p) - 1; j >= 0; --j) {
+        m[32 * j + lane] = s_vert[j][e];
+        if (j > 0) e = s_par[j][e];
+    }
+    PairParent r{0, 0, 0, 0};
+    uint32_t mdeg = kFullMask;
+    for (uint32_t t = 0; t < P.nj; ++t) {
+        const uint2 inf = g.out_info[m[32 * P.jpos[t] + lane]];
+        off[32 * t + lane] = inf.x;
+        deg[32 * t + lane] = inf.y;
+        if (inf.y < mdeg) { mdeg = inf.y; r.moff = inf.x; r.tmin = t; }
+    }
+    uint32_t lo = 0, hi = kFullMask, loc = 0, hic = kFullMask;
+    const uint32_t below = (1u << p) - 1;
+    for (uint32_t k = P.gt_mask; k; k &= k - 1) lo = max(lo, m[32 * (__ffs(k) - 1) + lane] + 1);
+    for (uint32_t k = P.lt_mask; k; k &= k - 1) hi = min(hi, m[32 * (__ffs(k) - 1) + lane]);
+    for (uint32_t k = C.gt_mask & below; k; k &= k - 1) loc = max(loc, m[32 * (__ffs(k) - 1) + lane] + 1);
+    for (uint32_t k = C.lt_mask & below; k; k &= k - 1) hic = min(hic, m[32 * (__ffs(k) - 1) + lane]);
+    row[32 * kRowLo + lane] = lo;
+    row[32 * kRowHi + lane] = hi;
+    row[32 * kRowLoC + lane] = loc;
+    row[32 * kRowHiC + lane] = hic;
+    const uint32_t mu = m[32 * P.jpos[r.tmin] + lane];
+    const uint32_t *lst = g.adj + r.moff;
+    r.s0 = kFullMask;
+    if (lo && p >= 2 && rp->pos_lvl == p - 1 && lo == m[32 * (p - 1) + lane] + 1) {
+        // the window starts right after the parent's own vertex: when that
+        // vertex was drawn from this very list, its offset is known
+        const uint32_t apos = rp->ub[p - 1][q0];
+        if (apos >= r.moff && apos - r.moff < mdeg) r.s0 = apos - r.moff + 1;
+    }
+    if (r.s0 == kFullMask) r.s0 = lo ? lbound_own(g, false, mu, lst, mdeg, lo, false) : 0;
+    r.e0 = hi != kFullMask ? lbound_own(g, false, mu, lst, mdeg, hi, false) : mdeg;
+    if (r.e0 < r.s0) r.e0 = r.s0;
+    if (cfold && F.ofold) {
+        // the orbit base of the positions below p
+        uint32_t base = 0;
+        for (uint32_t xm = F.ofold & below; xm; xm &= xm - 1) {
+            const uint32_t o = __ffs(xm) - 1;
+            const uint2 inf = g.out_info[m[32 * o + lane]];
+            base += inf.y;
+            for (uint32_t j = 0; j < p; ++j)
+                if (((F.oguar[o] >> j) & 1u) || pair_list_has(g.tab, inf.x, inf.y, m[32 * j + lane])) --base;
+        }
+        row[32 * kRowBase + lane] = base;
+    } else if (cfold) {
+        // the plain fold's list and window, fixed by the positions below p
+        const uint2 inf = g.out_info[m[32 * F.jpos[0] + lane]];
+        uint32_t flo = 0, fhi = kFullMask;
+        for (uint32_t k = F.gt_mask & below; k; k &= k - 1) flo = max(flo, m[32 * (__ffs(k) - 1) + lane] + 1);
+        for (uint32_t k = F.lt_mask & below; k; k &= k - 1) fhi = min(fhi, m[32 * (__ffs(k) - 1) + lane]);
+        const uint32_t *fl = g.adj + inf.x;
+        const uint32_t ws = flo ? lbound(fl, inf.y, flo) : 0, we = fhi != kFullMask ? lbound(fl, inf.y, fhi) : inf.y;
+        uint32_t sub = 0;
+        for (uint32_t j = 0; j < p; ++j) {
+            const uint32_t mj = m[32 * j + lane];
+            if (mj >= flo && mj < fhi && (((F.guar_mask >> j) & 1u) || pair_list_has(g.tab, inf.x, inf.y, mj))) ++sub;
+        }
+        row[32 * kRowBase + lane] = (we > ws ? we - ws : 0) - sub;
+        row[32 * kRowFOff + lane] = inf.x;
+        row[32 * kRowFDeg + lane] = inf.y;
+        row[32 * kRowFLo + lane] = flo;
+        row[32 * kRowFHi + lane] = fhi;
+    }
+    return r;
+}
+
+// The plan's pieces and the shared layout, the same in both pair kernels.
+#define PAIR_PROLOGUE()                                                                                       \
+    __shared__ LevelPlan sP, sC, sF;                                                                          \
+    __shared__ uint32_t *s_vert[kMaxK];                                                                       \
+    __shared__ uint32_t *s_par[kMaxK];                                                                        \
+    extern __shared__ __align__(16) uint32_t dyn[];                                                           \
+    {                                                                                                         \
+        const uint32_t words = sizeof(LevelPlan) / 4, f = p + 2 < rp->plan.k ? p + 2 : p + 1;                 \
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {                                          \
+            reinterpret_cast<uint32_t *>(&sP)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[p])[i];    \
+            reinterpret_cast<uint32_t *>(&sC)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[p + 1])[i]; \
+            reinterpret_cast<uint32_t *>(&sF)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[f])[i];    \
+        }                                                                                                     \
+        if (threadIdx.x < kMaxK) {                                                                            \
+            s_vert[threadIdx.x] = rp->vert[threadIdx.x];                                                      \
+            s_par[threadIdx.x] = rp->par[threadIdx.x];                                                        \
+        }                                                                                                     \
+    }                                                                                                         \
+    __syncthreads();                                                                                          \
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;                                               \
+    const uint32_t njp = sP.nj;                                                                               \
+    uint32_t *const wbase = dyn + warp * pair_words(p, njp);                                                  \
+    uint4 *const rec = reinterpret_cast<uint4 *>(wbase);                                                      \
+    uint32_t *const starts = wbase + 128;                                                                     \
+    uint32_t *const segs = starts + 32;   /* [lane]: first entry of its segment that is a row */              \
+    uint32_t *const sege = segs + 32;     /* [lane]: its segment's end, or kFullMask for a piece */           \
+    uint32_t *const itemA = sege + 32;    /* [rank]: A of the item's vertex */                                \
+    uint32_t *const Sb = itemA + 32;      /* core members of S, then of T */                                  \
+    uint32_t *const Tb = Sb + kCore / 32;                                                                     \
+    uint32_t *const S = Tb + kCore / 32;                                                                      \
+    uint8_t *const So = reinterpret_cast<uint8_t *>(S + kPS);  /* the member's column */                      \
+    uint32_t *const row = S + kPS + kPS / 4;                                                                  \
+    uint32_t *const col_off = row + 32 * kPairRows, *const col_deg = col_off + 32 * njp;                      \
+    uint32_t *const col_m = col_deg + 32 * njp;                                                               \
+    const uint32_t below = (1u << p) - 1;                                                                     \
+    const bool cfold = FOLD && sC.fold != 0;                                                                  \
+    const uint32_t extra = sC.fuse_extra;                                                                     \
+    const bool sig_same = sC.sig_lo <= sP.sig_lo && (!sC.check_sig || (sP.check_sig && sC.qin <= sP.qin &&    \
+                                                                       sC.qout <= sP.qout));                  \
+    const bool ts = !extra && sig_same && (sC.gt_mask & below) == (sP.gt_mask & below) &&                     \
+                    (sC.lt_mask & below) == (sP.lt_mask & below);                                             \
+    const PairCtx x{g, sP, sC, sF, p, extra, cfold, ts, col_m, col_off, col_deg, row};
+
+template <bool FOLD, bool TALLY>
+__global__ void __launch_bounds__(kPW * 32, 8)
+k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents parents, uint32_t phase, uint32_t split,
+        uint32_t *__restrict__ cursor, PairBig big, unsigned long long *__restrict__ acc,
+        unsigned long long *__restrict__ acc_c, unsigned long long *__restrict__ acc_p,
+        unsigned long long *__restrict__ acc_bytes) {
+    uint32_t pa, total;
+    parents_of(parents, pa, total);
+    if (!total) return;
+    PAIR_PROLOGUE()
+    const uint32_t lanemask_lt = (1u << lane) - 1, lanemask_le = lanemask_lt | (1u << lane);
+    // t above s only, below s only, or both
+    const bool o1 = !((sC.lt_mask >> p) & 1u), o2 = !((sC.gt_mask >> p) & 1u);
+    const bool phase2 = phase == 2;
+    uint32_t nbig = 0;
+    if (phase2) {
+        const unsigned long long n0 = big.n[0];
+        nbig = n0 < big.cap ? uint32_t(n0) : big.cap;
+        total = nbig ? big.pref[nbig - 1] : 0;
+    }
+    const uint32_t nwarps = gridDim.x * kPW;
+    // a few grabs per warp at least: parents differ in work
+    const uint32_t grab = min(phase2 ? 1u : 32u, max(1u, total / (4 * nwarps)));
+    const unsigned long long deadline = run_deadline(rp);
+    unsigned long long local = 0, local_c = 0, local_p = 0, tb = 0;
+    // A(v) - B(v) is the same for every v of one parent: both or neither of p
+    // and c in the orbit and every membership given by the query's arcs, or a
+    // plain fold that treats both alike
+    bool kconst = !cfold;
+    if (cfold && sF.ofold) {
+        kconst = ((sF.ofold >> p) & 1u) == ((sF.ofold >> (p + 1)) & 1u);
+        for (uint32_t xm = sF.ofold & below; xm; xm &= xm - 1) kconst = kconst && ((sF.oguar[__ffs(xm) - 1] >> p) & 1u);
+        if ((sF.ofold >> p) & 1u) kconst = kconst && (sF.oguar[p] & below) == below;
+    } else if (cfold) {
+        kconst = ((sF.guar_mask >> p) & 1u) == ((sF.guar_mask >> (p + 1)) & 1u);
+    }
+    const uint32_t orders = (o1 ? 1u : 0u) + (o2 ? 1u : 0u);
+
+    while (true) {
+        uint32_t start = 0;
+        if (lane == 0) start = past_deadline(rp, deadline) ? total : atomicAdd(cursor, grab);
+        start = __shfl_sync(kFullMask, start, 0);
+        if (start >= total) break;
+        // this lane's parent and the candidates [pos, end) of its window left
+        uint32_t pos = 0, end = 0, b = kFullMask;
+        bool piece = false;  // part of a window only: pairs with neighbours above
+        PairParent pp{0, 0, 0, 0};
+        if (uint32_t(lane) < grab && start + lane < total) {
+            uint32_t q0 = pa + start + lane, ch = 0;
+            if (phase2) {
+                const uint32_t gi = start + lane;
+                uint32_t lo = 0, hi = nbig - 1;  // first b with pref[b] > gi
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (big.pref[mid] > gi) hi = mid; else lo = mid + 1;
+                }
+                b = lo;
+                ch = gi - (b ? big.pref[b - 1] : 0);
+                q0 = big.q[b];
+            }
+            pp = pair_parent(g, rp, sP, sC, sF, cfold, p, s_vert, s_par, q0, lane, col_m, col_off, col_deg, row);
+            pos = pp.s0;
+            end = pp.e0;
+            if (TALLY) tb += 8ull * p + 8ull * njp;
+            if (phase2) {
+                piece = true;
+                pos = min(pp.s0 + ch * kPK, end);
+                end = min(pos + kPK, end);
+            }
+        }
+        if (!phase2) {
+            // long windows, and of root parents (whose sets need no tests, so
+            // pieces repeat none) all beyond kPG candidates of this warp, are
+            // dealt out in pieces: neighbouring hubs would be the launch's tail
+            uint32_t before = 0;
+            if (p == 1) {
+                before = end - pos;
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFullMask, before, o);
+                    if (lane >= o) before += y;
+                }
+            }
+            if (end - pos > split || (before > kPG && end != pos && end - pos >= kPK / 4)) {
+                piece = true;
+                const unsigned long long slot = atomicAdd(&big.n[0], 1ull);
+                if (slot < big.cap) {
+                    big.q[slot] = pa + start + lane;
+                    big.len[slot] = end - pos;
+                    end = pos;
+                }  // else: the list is full, this warp counts it piece by piece
+            }
+        }
+        while (true) {
+            // ---- the next round: whole windows (pieces of kPS) while they fit
+            const uint32_t take = min(end - pos, kPS);
+            uint32_t incl = take;
+            #pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const uint32_t len = incl <= kPS ? take : 0u;  // a prefix of the lanes
+            const unsigned live = __ballot_sync(kFullMask, len != 0);
+            if (!live) break;
+            const uint32_t ftotal = __shfl_sync(kFullMask, incl, 31 - __clz(live));
+            if (len) {
+                const uint32_t r = __popc(live & lanemask_lt), excl = incl - len, to = pp.tmin ? 0u : 1u;
+                rec[r] = make_uint4(pp.moff + pos - excl, uint32_t(lane) | (pp.tmin << 8),
+                                    njp > 1 ? col_off[32 * to + lane] : 0u, njp > 1 ? col_deg[32 * to + lane] : 0u);
+                starts[r] = excl;
+                pos += len;
+            }
+            __syncwarp();
+            // ---- the sets, in order of the lanes
+            uint32_t ns = 0;
+            {
+                const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? starts[lane] : kFullMask;
+                uint32_t started = 0;
+                for (uint32_t fstep = 0; fstep < ftotal; fstep += 32) {
+                    const uint32_t rel = my_start - fstep;
+                    const uint32_t bits = __reduce_or_sync(kFullMask, rel < 32u ? 1u << rel : 0u);
+                    const uint4 rc = rec[started + __popc(bits & lanemask_le) - 1];
+                    started += __popc(bits);
+                    const uint32_t f = fstep + lane, owner = rc.y & 255u, tmin = rc.y >> 8;
+                    bool ok = f < ftotal;
+                    const uint32_t v = __ldg(g.adj + (rc.x + min(f, ftotal - 1)));
+                    ok = ok && v >= sP.sig_lo;
+                    if (ok && njp > 1) ok = in_list(g, rc.z, rc.w, v);
+                    if (ok && njp > 2)
+                        for (uint32_t t = (tmin < 2 ? 2u : 1u); t < njp; ++t)
+                            if (t != tmin && !pair_list_has(g.tab, col_off[32 * t + owner], col_deg[32 * t + owner], v)) {
+                                ok = false;
+                                break;
+                            }
+                    if (ok)
+                        for (uint32_t j = 0; j < p; ++j)
+                            if (v == col_m[32 * j + owner]) { ok = false; break; }
+                    if (ok && sP.check_sig) ok = pair_sig(g, sP, v);
+                    const unsigned m = __ballot_sync(kFullMask, ok);
+                    if (ok) {
+                        const uint32_t i = ns + __popc(m & lanemask_lt);
+                        S[i] = v;
+                        So[i] = uint8_t(owner);
+                    }
+                    ns += __popc(m);
+                    if (TALLY && f < ftotal) tb += 4 + 32ull * (njp - 1) + (sP.check_sig ? 8 : 0);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) local_p += ns;
+            // ---- segments: [lo, hi) of the lane, its core members from cut on
+            uint32_t lo = 0;
+            for (uint32_t n = ns; n;) {  // first member whose column is >= lane
+                const uint32_t half = n >> 1;
+                if (So[lo + half] < lane) { lo += half + 1; n -= half + 1; }
+                else n = half;
+            }
+            uint32_t hi = __shfl_down_sync(kFullMask, lo, 1);
+            if (lane == 31) hi = ns;
+            uint32_t cut = hi;
+            if (g.core_bits && (piece ? b != kFullMask && hi > lo : hi - lo >= kPC)) {
+                uint32_t c0 = lo;
+                for (uint32_t n = hi - lo; n;) {
+                    const uint32_t half = n >> 1;
+                    if (S[c0 + half] < g.core0) { c0 += half + 1; n -= half + 1; }
+                    else n = half;
+                }
+                if (piece || hi - c0 >= kPC) cut = c0;
+            }
+            segs[lane] = cut;
+            sege[lane] = piece ? kFullMask : hi;
+            __syncwarp();
+            // ---- items: each member that is no row, with its partners above
+            for (uint32_t i0 = 0; i0 < ns; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                uint32_t ilen = 0, ibase = 0, ioff = 0, ideg = 0, ow = 0, mode = 0, a = 0;
+                if (i < ns) {
+                    ow = So[i];
+                    a = S[i];
+                    if (i < segs[ow]) {
+                        const uint32_t se = sege[ow];
+                        const uint32_t lenS = se == kFullMask ? kFullMask : se - i - 1;
+                        if (lenS) {
+                            const uint2 inf = g.out_info[a];
+                            const uint32_t bw = __ldg(g.bwd_out + a), lenN = inf.y - bw;
+                            if (TALLY) tb += 12;
+                            mode = lenN < lenS ? 1u : 0u;
+                            ilen = min(lenN, lenS);
+                            ibase = mode ? inf.x + bw : i + 1;
+                            ioff = mode ? col_off[ow] : inf.x;
+                            ideg = mode ? col_deg[ow] : inf.y;
+                        }
+                    }
+                }
+                uint32_t iincl = ilen;
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFullMask, iincl, o);
+                    if (lane >= o) iincl += y;
+                }
+                const uint32_t itotal = __shfl_sync(kFullMask, iincl, 31);
+                if (!itotal) continue;
+                const unsigned ilive = __ballot_sync(kFullMask, ilen != 0);
+                if (ilen) {
+                    const uint32_t r = __popc(ilive & lanemask_lt), excl = iincl - ilen;
+                    rec[r] = make_uint4(ibase - excl, ow | (mode << 8) | (i << 16), ioff, ideg);
+                    starts[r] = excl;
+                    if (FOLD) itemA[r] = o1 ? pair_a(x, ow, a) : 0u;
+                }
+                __syncwarp();
+                const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(ilive)) ? starts[lane] : kFullMask;
+                uint32_t started = 0;
+                for (uint32_t fstep = 0; fstep < itotal; fstep += 64) {
+                    uint4 rc[2];
+                    uint32_t tv[2], rk[2];
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t rel = my_start - (fstep + 32 * h);
+                        const uint32_t bits = __reduce_or_sync(kFullMask, rel < 32u ? 1u << rel : 0u);
+                        rk[h] = started + __popc(bits & lanemask_le) - 1;
+                        started += __popc(bits);
+                        rc[h] = rec[rk[h]];
+                        const uint32_t at = rc[h].x + min(fstep + 32 * h + lane, itotal - 1);
+                        tv[h] = (rc[h].y & 256u) ? __ldg(g.adj + at) : S[at];
+                    }
+                    uint32_t nb[2], bu[2];
+                    Bucket bk[2];
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        nb[h] = (rc[h].w + 3) >> 2;
+                        bu[h] = tab_bucket(nb[h], tv[h]);
+                        bk[h] = load_bucket(g.tab, rc[h].z, bu[h]);
+                    }
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        bool ok = fstep + 32 * h + lane < itotal;
+                        const uint32_t t = tv[h];
+                        if (TALLY && ok) tb += 32 + ((rc[h].y & 256u) ? 4 : 0);
+                        if (ok && !bucket_has(bk[h], t)) ok = tab_continue(g.tab, rc[h].z, nb[h], bu[h], bk[h], t);
+                        if (ok) {
+                            const uint32_t l = rc[h].y & 255u;
+                            if (rc[h].y & 256u) ok = pair_in_set(x, l, 0, t);
+                            if (ok) {
+                                const uint32_t av = S[rc[h].y >> 16];
+                                if (o1 && pair_adm(x, l, t)) {
+                                    ++local_c;
+                                    local += FOLD ? uint32_t(itemA[rk[h]] + pair_b(x, l, t)) : 1u;
+                                }
+                                if (o2 && pair_adm(x, l, av)) {
+                                    ++local_c;
+                                    local += FOLD ? uint32_t(pair_a(x, l, t) + pair_b(x, l, av)) : 1u;
+                                }
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            // ---- rows: the core members of the larger sets
+            for (unsigned todo = __ballot_sync(kFullMask, cut < hi); todo; todo &= todo - 1) {
+                const int l = __ffs(todo) - 1;
+                const uint32_t c0 = __shfl_sync(kFullMask, cut, l), ce = __shfl_sync(kFullMask, hi, l);
+                const uint32_t lb = __shfl_sync(kFullMask, b, l);
+                __syncwarp();
+                if (lb != kFullMask) {
+                    Sb[lane] = big.bits[size_t(lb) * (kCore / 16) + lane];
+                    Tb[lane] = big.bits[size_t(lb) * (kCore / 16) + kCore / 32 + lane];
+                    __syncwarp();
+                } else {
+                    Sb[lane] = 0;
+                    Tb[lane] = 0;
+                    __syncwarp();
+                    for (uint32_t i = c0 + lane; i < ce; i += 32) {
+                        const uint32_t u = S[i] - g.core0;
+                        atomicOr(&Sb[u >> 5], 1u << (u & 31));
+                        if (!ts && pair_adm(x, uint32_t(l), S[i])) atomicOr(&Tb[u >> 5], 1u << (u & 31));
+                    }
+                    __syncwarp();
+                    if (ts) Tb[lane] = Sb[lane];
+                    __syncwarp();
+                }
+                if (lb == kFullMask && ts && kconst) {
+                    // a whole set, every member admissible: with n(v) the
+                    // members of S in v's row, the pairs' weights add up to
+                    // sum B(v) n(v) + (A - B) * pairs, pairs = sum n(v) / 2
+                    uint32_t n2 = 0, kap = 0;
+                    unsigned long long wsum = 0;
+                    const uint32_t q0 = (S[c0] - g.core0) >> 7;  // words below the lowest member are empty
+                    for (uint32_t i = c0 + lane; i < ce; i += 32) {
+                        const uint32_t v = S[i];
+                        const uint4 *rp4 = reinterpret_cast<const uint4 *>(g.core_bits + size_t(v - g.core0) * (kCore / 32));
+                        uint32_t n = 0;
+                        #pragma unroll 4
+                        for (uint32_t q = q0; q < kCore / 128; ++q) {
+                            const uint4 r4 = __ldg(rp4 + q), s4 = reinterpret_cast<const uint4 *>(Sb)[q];
+                            n += __popc(r4.x & s4.x) + __popc(r4.y & s4.y) + __popc(r4.z & s4.z) + __popc(r4.w & s4.w);
+                        }
+                        n2 += n;
+                        if (TALLY) tb += 8 + 16ull * (kCore / 128 - q0);
+                        if (FOLD) {
+                            const uint32_t B = pair_b(x, uint32_t(l), v);
+                            wsum += (unsigned long long)((long long)int32_t(B) * n);
+                            if (i == c0) kap = pair_a(x, uint32_t(l), v) - B;
+                        }
+                    }
+                    #pragma unroll
+                    for (int o = 16; o; o >>= 1) n2 += __shfl_xor_sync(kFullMask, n2, o);
+                    const uint32_t pairs = n2 >> 1;
+                    if (FOLD) local += orders * wsum;
+                    if (lane == 0) {
+                        local += (unsigned long long)(orders * pairs) * (FOLD ? kap : 1u);  // A - B >= 0 where there is a pair
+                        local_c += orders * pairs;
+                    }
+                    continue;
+                }
+                for (uint32_t i = c0 + lane; i < ce; i += 32) {
+                    const uint32_t v = S[i], u = v - g.core0, w0 = u >> 5;
+                    const uint32_t above = ~((2u << (u & 31)) - 1u), under = (1u << (u & 31)) - 1u;
+                    const uint4 *rp4 = reinterpret_cast<const uint4 *>(g.core_bits + size_t(u) * (kCore / 32));
+                    uint32_t upS = 0, dnS = 0, upT = 0, dnT = 0;
+                    #pragma unroll 2
+                    for (uint32_t q = 0; q < kCore / 128; ++q) {
+                        const uint4 r4 = __ldg(rp4 + q);
+                        const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
+                        #pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) {
+                            const uint32_t j = 4 * q + k;
+                            const uint32_t ma = j > w0 ? kFullMask : (j == w0 ? above : 0u);
+                            const uint32_t mb = j < w0 ? kFullMask : (j == w0 ? under : 0u);
+                            const uint32_t ws = rw[k] & Sb[j];
+                            upS += __popc(ws & ma);
+                            if (FOLD || !ts || !o1) dnS += __popc(ws & mb);
+                            if (!ts) {
+                                const uint32_t wt = rw[k] & Tb[j];
+                                upT += __popc(wt & ma);
+                                dnT += __popc(wt & mb);
+                            }
+                        }
+                    }
+                    if (ts) {
+                        upT = upS;
+                        dnT = dnS;
+                    }
+                    if (TALLY) tb += 8 + kCore / 8;
+                    if (!FOLD && ts && o1) {
+                        // every pair once, from its lower row
+                        const uint32_t n = o2 ? 2 * upS : upS;
+                        local += n;
+                        local_c += n;
+                    } else {
+                        const bool adm = ts || pair_adm(x, uint32_t(l), v);
+                        const uint32_t A = pair_a(x, uint32_t(l), v), B = pair_b(x, uint32_t(l), v);
+                        // A of a vertex with a pair fits 32 bits; B is below
+                        // 2^31 or, in a plain fold, -1
+                        long long s = 0;
+                        if (o1) {
+                            s += (long long)A * upT + (adm ? (long long)int32_t(B) * dnS : 0);
+                            local_c += upT;
+                        }
+                        if (o2) {
+                            s += (long long)A * dnT + (adm ? (long long)int32_t(B) * upS : 0);
+                            local_c += dnT;
+                        }
+                        local += (unsigned long long)s;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+    }
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        local += __shfl_xor_sync(kFullMask, local, o);
+        local_c += __shfl_xor_sync(kFullMask, local_c, o);
+        if (TALLY) tb += __shfl_xor_sync(kFullMask, tb, o);
+    }
+    if (lane == 0) {
+        if (local) atomicAdd(acc, local);
+        if (local_c) atomicAdd(acc_c, local_c);
+        if (local_p) atomicAdd(acc_p, local_p);
+        if (TALLY && tb) atomicAdd(acc_bytes, tb);
+    }
+}
+
+// Core members of the deferred parents' sets, one warp per parent.
+template <bool FOLD>
+__global__ void __launch_bounds__(kPW * 32)
+k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big) {
+    const unsigned long long n0 = big.n[0];
+    const uint32_t nbig = n0 < big.cap ? uint32_t(n0) : big.cap;
+    if (!nbig || !g.core_bits) return;
+    PAIR_PROLOGUE()
+    (void)rec; (void)starts; (void)segs; (void)sege; (void)itemA; (void)S; (void)So;
+    for (uint32_t b = blockIdx.x * kPW + warp; b < nbig; b += gridDim.x * kPW) {
+        uint32_t moff = 0, s0 = 0, e0 = 0, tmin = 0;
+        if (lane == 0) {
+            const PairParent pp = pair_parent(g, rp, sP, sC, sF, false, p, s_vert, s_par, big.q[b], 0, col_m, col_off,
+                                              col_deg, row);
+            moff = pp.moff;
+            s0 = pp.s0;
+            e0 = pp.e0;
+            tmin = pp.tmin;
+            const uint32_t c0 = lbound(g.adj + moff, e0, g.core0);
+            s0 = max(s0, c0);
+        }
+        moff = __shfl_sync(kFullMask, moff, 0);
+        s0 = __shfl_sync(kFullMask, s0, 0);
+        e0 = __shfl_sync(kFullMask, e0, 0);
+        tmin = __shfl_sync(kFullMask, tmin, 0);
+        Sb[lane] = 0;
+        Tb[lane] = 0;
+        __syncwarp();
+        for (uint32_t i = s0 + lane; i < e0; i += 32) {
+            const uint32_t v = __ldg(g.adj + moff + i), u = v - g.core0;
+            if (pair_in_set(x, 0, tmin, v)) {
+                atomicOr(&Sb[u >> 5], 1u << (u & 31));
+                if (pair_adm(x, 0, v)) atomicOr(&Tb[u >> 5], 1u << (u & 31));
+            }
+        }
+        __syncwarp();
+        big.bits[size_t(b) * (kCore / 16) + lane] = Sb[lane];
+        big.bits[size_t(b) * (kCore / 16) + kCore / 32 + lane] = Tb[lane];
+        __syncwarp();
     }
 }
 
@@ -1858,7 +2224,7 @@ int g_num_sms = 0;
 int g_level_blocks[3] = {0, 0, 0};
 int g_flat_blocks[3][2] = {};  // blocks of k_level_flat<mode, fold> per SM by registers and threads
 int g_fused_blocks[3] = {0, 0, 0};
-int g_fused_walk_blocks = 0;
+int g_pair_blocks[2] = {0, 0};  // blocks of k_pairs<fold> per SM by registers and threads
 // CUTS_LEVEL_KERNEL=warp selects the warp-per-parent form (A/B comparisons)
 bool g_use_flat = true;
 
@@ -1882,12 +2248,14 @@ int launch_geometry() {
     g_flat_blocks[kCountMode][1] = std::max(1, b);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kBytesMode, true>, kFW * 32, 0));
     g_flat_blocks[kBytesMode][1] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kCountMode, false>, kZW * 32, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kCountMode>, kZW * 32, 0));
     g_fused_blocks[kCountMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kBytesMode, false>, kZW * 32, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kBytesMode>, kZW * 32, 0));
     g_fused_blocks[kBytesMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kCountMode, true>, kZW * 32, 0));
-    g_fused_walk_blocks = std::max(1, b) * g_num_sms;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<false, false>, kPW * 32, 0));
+    g_pair_blocks[0] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<true, false>, kPW * 32, 0));
+    g_pair_blocks[1] = std::max(1, b);
     const char *kv = std::getenv("CUTS_LEVEL_KERNEL");
     g_use_flat = !(kv && std::strcmp(kv, "warp") == 0);
     return CUTS_OK;
@@ -2166,92 +2534,100 @@ struct Run {
         return CUTS_OK;
     }
 
-    // The fused count of levels p and p+1 over parents [pa, pb) of L_{p-1}:
-    // phase 1 over the parents, then (counting) a scan of the parents it
-    // deferred and phase 2 over their groups.
+    // The fused count of levels p and p+1 over the given parents of L_{p-1}:
+    // phase 1 over the parents, then a scan of the parents it deferred and
+    // phase 2 over their pieces (k_pairs) or groups (k_fused).
     int launch_fused(int mode, uint32_t p, const Parents &par, uint32_t most, ChainSlice *cs = nullptr) {
         uint32_t *cur1 = cs ? cs->cursor + p : g.d_u32 + kSlotCursor;
         uint32_t *cur2 = cs ? cs->cursor + p + 1 : g.d_u32 + kSlotCursor + 1;
-        if (!cs) CK(cudaMemsetAsync(cur1, 0, 2 * sizeof(uint32_t), g.stream));
-        uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(g_fused_blocks[mode]),
-                                                                   (most + kZW - 1) / kZW));
-        FusedBig fb;
-        fb.n = cs ? cs->big : g.d_u64 + kU64Big;
-        fb.cap = hp->fuse_big_cap;
-        fb.gi = hp->fuse_big + 64;
-        fb.soff = fb.gi + fb.cap;
-        fb.ns = fb.soff + fb.cap;
-        fb.pref = fb.ns + fb.cap;
-        fb.pool = fb.pref + fb.cap;
-        fb.pool_words = hp->fuse_pool_words;
-        if (!cs) CK(cudaMemsetAsync(fb.n, 0, 2 * sizeof(unsigned long long), g.stream));
-        // CUTS_FUSE_SPLIT=<n> sets the deferral threshold (tests use small values)
-        uint32_t split = g.fuse_split ? g.fuse_split : kBigS;
-        if (const char *e = std::getenv("CUTS_FUSE_SPLIT")) split = uint32_t(std::strtoul(e, nullptr, 10));
-        // the phase-1 pair walk covers the fused plans that order the
-        // vertices at p and c (symmetry breaking: each pair of S once, and a
-        // row's list window starts or ends at s), except an extra list of c
-        // on p itself and a plain fold whose list or window moves with the
-        // vertex at p; a plan without that order (every ordered pair, so a
-        // row's window is s's whole list) keeps the per-pair intersection,
-        // which iterates the shorter side.  CUTS_FUSE_WALK=0 turns the walk
-        // off (A/B comparisons)
-        uint32_t walk_ok = 1;
-        {
-            const LevelPlan &Lc = hp->plan.lv[p + 1];
-            const LevelPlan &Lf = hp->plan.lv[p + 2 < k ? p + 2 : p + 1];
-            if (!(((Lc.gt_mask | Lc.lt_mask) >> p) & 1u)) walk_ok = 0;
-            for (uint32_t t = 0; t < Lc.nj; ++t)
-                if (((Lc.fuse_extra >> t) & 1u) && Lc.jpos[t] == p) walk_ok = 0;
-            if (Lc.fold && !Lf.ofold && (Lf.jpos[0] == p || (((Lf.gt_mask | Lf.lt_mask) >> p) & 1u))) walk_ok = 0;
-            if (g.max_deg >= (1u << 31)) walk_ok = 0;
-            const char *w = std::getenv("CUTS_FUSE_WALK");
-            if (w && w[0] == '0') walk_ok = 0;
+        unsigned long long *bn = cs ? cs->big : g.d_u64 + kU64Big;
+        if (!cs) {
+            CK(cudaMemsetAsync(cur1, 0, 2 * sizeof(uint32_t), g.stream));
+            CK(cudaMemsetAsync(bn, 0, 2 * sizeof(unsigned long long), g.stream));
         }
+        // CUTS_FUSE_SPLIT=<n> sets the deferral threshold (tests use small values)
+        uint32_t split = g.fuse_split;
+        const char *es = std::getenv("CUTS_FUSE_SPLIT");
+        if (es) split = uint32_t(std::strtoul(es, nullptr, 10));
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (profile) {
             CK(cudaEventCreate(&e0));
             CK(cudaEventCreate(&e1));
             CK(cudaEventRecord(e0, g.stream));
         }
-        if (mode == kBytesMode && !walk_ok) {
-            k_fused<kBytesMode, false><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
-                cur1, hp->fuse_scratch, hp->fuse_stride, fb, g.d_u64 + 2, nullptr, nullptr,
-                nullptr);
+        // counting; the bytes pass of a pair plan runs the same launches with
+        // their byte tally on and the counts sent to scratch slots
+        const bool tal = mode == kBytesMode;
+        unsigned long long *acc = tal ? g.d_u64 + kU64Scratch : g.d_u64;
+        unsigned long long *acc_c = tal ? g.d_u64 + kU64Scratch + 1 : g.d_u64 + 3;
+        unsigned long long *acc_p = tal ? g.d_u64 + kU64Scratch + 2 : g.d_u64 + 4;
+        if (hp->pairs) {
+            PairBig pb;
+            pb.n = bn;
+            pb.cap = hp->fuse_big_cap;
+            pb.q = hp->fuse_big;
+            pb.len = pb.q + pb.cap;
+            pb.pref = pb.len + pb.cap;
+            pb.bits = pb.pref + pb.cap;
+            split = es || g.fuse_split ? std::min(split, kPS) : kPS;
+            // parents that are roots (p = 1) have their own list's window for S,
+            // so dealing them out in pieces repeats no test, and it keeps a
+            // hub's pairs from one warp: 64 there (triangle, 4M / 40M: 512 14.6 ms,
+            // 128 12.7 ms, 64 9.5 ms)
+            if (p == 1) split = std::min(split, kPK);
+            const bool fold = hp->plan.lv[p + 1].fold != 0;
+            const uint32_t smem = 4 * kPW * pair_words(p, hp->plan.lv[p].nj);
+            const uint32_t fixed = 3 * uint32_t(sizeof(LevelPlan)) + 16 * kMaxK + 1024;
+            const uint32_t full = std::max(1u, std::min(uint32_t(g_pair_blocks[fold]), 227u * 1024u / (smem + fixed))) *
+                                  uint32_t(g_num_sms);
+            const uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(full, (most + kPW - 1) / kPW));
+            auto go = [&](auto *kernel, uint32_t grid, uint32_t phase, uint32_t *cur) {
+                kernel<<<grid, kPW * 32, smem, g.stream>>>(view, dp, p, par, phase, split, cur, pb, acc, acc_c, acc_p,
+                                                          tal ? g.d_u64 + 2 : nullptr);
+            };
+            auto phase = [&](uint32_t grid, uint32_t ph, uint32_t *cur) {
+                if (fold) tal ? go(k_pairs<true, true>, grid, ph, cur) : go(k_pairs<true, false>, grid, ph, cur);
+                else tal ? go(k_pairs<false, true>, grid, ph, cur) : go(k_pairs<false, false>, grid, ph, cur);
+            };
+            phase(blocks, 1, cur1);
             CK(cudaGetLastError());
             res.launches++;
+            // no parent can be deferred where no list is longer than the split
+            if (g.max_deg > split) {
+                k_fused_scan<<<1, 1024, 0, g.stream>>>(pb.n, pb.cap, pb.len, kPK, pb.pref);
+                k_pair_bits<false><<<full, kPW * 32, smem, g.stream>>>(view, dp, p, pb);
+                phase(full, 2, cur2);
+                CK(cudaGetLastError());
+                res.launches += 3;
+            }
         } else {
-            // counting; the bytes pass of a walk plan runs the same launches
-            // with their byte tally on and the counts sent to scratch slots
-            const bool tal = mode == kBytesMode;
-            unsigned long long *acc = tal ? g.d_u64 + kU64Scratch : g.d_u64;
-            unsigned long long *acc_c = tal ? g.d_u64 + kU64Scratch + 1 : g.d_u64 + 3;
-            unsigned long long *acc_p = tal ? g.d_u64 + kU64Scratch + 2 : g.d_u64 + 4;
-            unsigned long long *acc_b = tal ? g.d_u64 + 2 : nullptr;
-            const uint32_t wblocks =
-                std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(g_fused_walk_blocks), (most + kZW - 1) / kZW));
-            if (walk_ok && tal)
-                k_fused<kCountMode, true, true><<<wblocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
-                    cur1, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
-            else if (walk_ok)
-                k_fused<kCountMode, true><<<wblocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
-                    cur1, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
-            else
-                k_fused<kCountMode, false><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split,
-                    cur1, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p, acc_b);
-            CK(cudaGetLastError());
-            k_fused_scan<<<1, 1024, 0, g.stream>>>(fb);
-            CK(cudaGetLastError());
-            if (tal)
-                k_fused<kCountMode, false, true><<<uint32_t(g_fused_blocks[kCountMode]), kZW * 32, 0, g.stream>>>(
-                    view, dp, p, par, 2, split, cur2, hp->fuse_scratch, hp->fuse_stride, fb, acc,
-                    acc_c, acc_p, acc_b);
-            else
-                k_fused<kCountMode, false><<<uint32_t(g_fused_blocks[kCountMode]), kZW * 32, 0, g.stream>>>(
-                    view, dp, p, par, 2, split, cur2, hp->fuse_scratch, hp->fuse_stride, fb, acc,
-                    acc_c, acc_p, acc_b);
-            CK(cudaGetLastError());
-            res.launches += 3;
+            const uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(g_fused_blocks[mode]),
+                                                                             (most + kZW - 1) / kZW));
+            if (!es && !split) split = kBigS;
+            FusedBig fb;
+            fb.n = bn;
+            fb.cap = hp->fuse_big_cap;
+            fb.gi = hp->fuse_big;
+            fb.soff = fb.gi + fb.cap;
+            fb.ns = fb.soff + fb.cap;
+            fb.pref = fb.ns + fb.cap;
+            fb.pool = fb.pref + fb.cap;
+            fb.pool_words = hp->fuse_pool_words;
+            if (tal) {
+                k_fused<kBytesMode><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split, cur1,
+                    hp->fuse_scratch, hp->fuse_stride, fb, g.d_u64 + 2, nullptr, nullptr);
+                CK(cudaGetLastError());
+                res.launches++;
+            } else {
+                k_fused<kCountMode><<<blocks, kZW * 32, 0, g.stream>>>(view, dp, p, par, 1, split, cur1,
+                    hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p);
+                CK(cudaGetLastError());
+                k_fused_scan<<<1, 1024, 0, g.stream>>>(fb.n, fb.cap, fb.ns, 32, fb.pref);
+                k_fused<kCountMode><<<uint32_t(g_fused_blocks[kCountMode]), kZW * 32, 0, g.stream>>>(
+                    view, dp, p, par, 2, split, cur2, hp->fuse_scratch, hp->fuse_stride, fb, acc, acc_c, acc_p);
+                CK(cudaGetLastError());
+                res.launches += 3;
+            }
         }
         if (profile) {
             CK(cudaEventRecord(e1, g.stream));
@@ -2361,6 +2737,22 @@ __global__ void k_materialize(const RunParams *__restrict__ rp, uint32_t first, 
 
 constexpr uint32_t kDumpRows = 1u << 22;  // rows materialised per piece
 
+// True when the fused count of levels p and p + 1 runs in k_pairs: a symmetric
+// graph without self-loops (its pairs are unordered) with membership tables,
+// no list of level p + 1 on p itself beyond the pair's, and no plain fold
+// whose list or window moves with the vertex at p.  Everything else keeps
+// k_fused.  CUTS_FUSE_WALK=0 keeps k_fused always (A/B comparisons).
+bool pairs_plan(const DeviceGraph &g, const Plan &plan, uint32_t p) {
+    if (!g.symmetric || g.loops || !g.tab || g.max_deg >= (1u << 31)) return false;
+    const LevelPlan &Lc = plan.lv[p + 1];
+    const LevelPlan &Lf = plan.lv[p + 2 < plan.k ? p + 2 : p + 1];
+    for (uint32_t t = 0; t < Lc.nj; ++t)
+        if (((Lc.fuse_extra >> t) & 1u) && Lc.jpos[t] == p) return false;
+    if (Lc.fold && !Lf.ofold && (Lf.jpos[0] == p || (((Lf.gt_mask | Lf.lt_mask) >> p) & 1u))) return false;
+    const char *w = std::getenv("CUTS_FUSE_WALK");
+    return !(w && w[0] == '0');
+}
+
 // Carves the arena for `stored` levels and uploads the run parameters.
 int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, RunParams *&hp,
             RunParams *&dp, uint64_t &cap) {
@@ -2430,7 +2822,8 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         if (fuse && i >= stored) break;
         tests = tests || L.nj >= 2 || (counting && (L.fold || L.fold2 || L.closed_form));
     }
-    if (tests && (rc = device_tables(g))) return rc;
+    if ((tests || (fuse && g.symmetric && !g.loops)) && (rc = device_tables(g))) return rc;
+    hp->pairs = fuse && pairs_plan(g, hp->plan, cl - 1);
     hp->stored = stored;
     // before a fused count of levels p = cl - 1 and cl, the entries of
     // level p - 1 record where their vertex sits in its list
@@ -2447,13 +2840,20 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     const uint64_t l0_bytes = ((8 * n + 255) / 256) * 256 + 256;
     // fused kernel: one scratch row per resident warp, as long as the longest list
     uint64_t fuse_bytes = 0, big_bytes = 0;
-    if (fuse) {
+    if (fuse && hp->pairs) {
+        // deferred parents: index, length and prefix sum, and two core bitmaps
+        // each; a parent beyond the list's capacity is counted where it is found
+        const uint64_t per = 3 + kCore / 16;
+        hp->fuse_big_cap = uint32_t(std::max<uint64_t>(64, std::min<uint64_t>(1u << 17, g.arena_bytes / 64 / (4 * per))));
+        big_bytes = (4 * per * hp->fuse_big_cap + 255) / 256 * 256;
+        fuse_bytes = big_bytes;
+    } else if (fuse) {
         hp->fuse_stride = ((std::max<uint32_t>(g.max_deg, 1) + 31) / 32) * 32;
         fuse_bytes = uint64_t(g_fused_blocks[kCountMode] > g_fused_blocks[kBytesMode] ? g_fused_blocks[kCountMode]
                                                                                       : g_fused_blocks[kBytesMode]) *
                      kZW * hp->fuse_stride * 4;
-        // deferred parents: 256 B of counters, four arrays of cap words and a
-        // pool of saved candidate sets (1/32 of the arena, 1M..16M words)
+        // deferred parents: four arrays of cap words and a pool of saved
+        // candidate sets (1/32 of the arena, 1M..16M words)
         hp->fuse_big_cap = 1u << 17;
         const uint64_t pool = std::min<uint64_t>(16ull << 20, std::max<uint64_t>(1ull << 20, g.arena_bytes / 128));
         hp->fuse_pool_words = uint32_t(std::max<uint64_t>(pool, 2ull * hp->fuse_stride));
@@ -2465,8 +2865,9 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     if (g.arena_bytes < l0_bytes + fuse_bytes)
         return set_error(CUTS_ERR_NOMEM, "arena smaller than the root level and scratch");
     if (fuse) {
-        hp->fuse_scratch = reinterpret_cast<uint32_t *>(static_cast<char *>(g.arena) + g.arena_bytes - fuse_bytes);
-        hp->fuse_big = reinterpret_cast<uint32_t *>(static_cast<char *>(g.arena) + g.arena_bytes - big_bytes);
+        char *const end = static_cast<char *>(g.arena) + (g.arena_bytes & ~uint64_t(255));
+        hp->fuse_scratch = reinterpret_cast<uint32_t *>(end - fuse_bytes);
+        hp->fuse_big = reinterpret_cast<uint32_t *>(end - big_bytes);
     }
     if (stored >= 2) {
         cap = (g.arena_bytes - l0_bytes - fuse_bytes) / (12ull * (stored - 1));
