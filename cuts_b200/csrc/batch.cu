@@ -47,6 +47,10 @@ struct BWarp {  // per-warp depth-first state, shared memory
     uint32_t nb[kBatchMaxK], bi[kBatchMaxK], tmin[kBatchMaxK], nj[kBatchMaxK];
     uint32_t joff[kBatchMaxK][kBatchMaxJ], jdeg[kBatchMaxK][kBatchMaxJ];
     uint32_t buf[kBatchMaxK][32];
+    // the counted frontier's records, by rank of the lane (count_frontier)
+    uint4 rec[32];
+    uint2 rec2[32];
+    uint32_t starts[32];
 };
 
 struct Ctx {
@@ -105,6 +109,7 @@ __device__ __forceinline__ bool test_candidate(const Ctx &c, uint32_t d, uint32_
     if (ok)
         for (uint32_t j = 0; j < d; ++j)
             if (v == c.S->m[j]) { ok = false; break; }
+    ok = ok && v >= L.sig_lo;
     if (ok && L.check_sig) {
         const uint2 o = c.g.out_info[v], i = c.g.in_info[v];
         ok = i.y >= L.qin && o.y >= L.qout;
@@ -113,7 +118,7 @@ __device__ __forceinline__ bool test_candidate(const Ctx &c, uint32_t d, uint32_
         const uint32_t nj = c.S->nj[d], tm = c.S->tmin[d];
         for (uint32_t t = 0; t < nj; ++t) {
             if (t == tm) continue;
-            if (!contains(c.g.adj + c.S->joff[d][t], c.S->jdeg[d][t], v)) { ok = false; break; }
+            if (!in_list(c.g, c.S->joff[d][t], c.S->jdeg[d][t], v)) { ok = false; break; }
         }
     }
     cand = v;
@@ -190,6 +195,165 @@ __device__ unsigned long long count_level_fold(const Ctx &c, uint32_t d) {
     return n;
 }
 
+// Level e = d + 1 counted for the whole frontier of level d (buf[d], nb[d]
+// vertices, at most 32), one vertex per lane: each lane finds its own shortest
+// list and window -- lists of positions below d are the warp's, the list of
+// position d the lane's -- and the lanes' candidate windows are one sequence
+// walked 64 candidates a step, as in k_level_flat (engine.cu).  Counting one
+// frontier vertex after another left most lanes idle on short lists: 64 mixed
+// queries of 3 and 4 vertices on 200,000 vertices / 1.6M edges took 480 ms,
+// BATCH_NEW this way.  With a fold at e, each candidate adds the closed form
+// of level e + 1.  Returns the lane's part of the count.
+__device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
+    const uint32_t e = d + 1, nj = c.Q->lv[e].nj;
+    const BLevel &L = c.Q->lv[e];
+    const BLevel &F = c.Q->lv[e + 1 < c.Q->k ? e + 1 : e];
+    const bool fold = L.fold && e + 2 == c.Q->k;
+    const DevView &g = c.g;
+    BWarp *const S = c.S;
+    const int lane = c.lane;
+    if (uint32_t(lane) < nj && L.jpos[lane] != d) {
+        const uint32_t u = S->m[L.jpos[lane]];
+        const uint2 inf = L.jdir[lane] ? g.in_info[u] : g.out_info[u];
+        S->joff[e][lane] = inf.x;
+        S->jdeg[e][lane] = inf.y;
+    }
+    __syncwarp();
+    const bool have = uint32_t(lane) < S->nb[d];
+    const uint32_t v = have ? S->buf[d][lane] : 0u;
+    auto m = [&](uint32_t j) { return j == d ? v : S->m[j]; };
+    uint32_t moff = 0, mdeg = 0, tmin = 0, s0 = 0, e0 = 0;
+    uint2 own[2] = {make_uint2(0, 0), make_uint2(0, 0)};  // v's out- and in-list
+    uint32_t f_off = 0, f_deg = 0, f_lo = 0, f_hi = kFullMask, fbase = 0;
+    unsigned long long n = 0;
+    if (have) {
+        mdeg = kFullMask;
+        for (uint32_t t = 0; t < nj; ++t) {
+            uint2 inf;
+            if (L.jpos[t] == d) {
+                inf = L.jdir[t] ? g.in_info[v] : g.out_info[v];
+                own[L.jdir[t] ? 1 : 0] = inf;
+            } else {
+                inf = make_uint2(S->joff[e][t], S->jdeg[e][t]);
+            }
+            if (inf.y < mdeg) { mdeg = inf.y; moff = inf.x; tmin = t; }
+        }
+        if (nj == 0) mdeg = 0;
+        uint32_t lo = 0, hi = kFullMask;
+        for (uint32_t k = L.gt_mask; k; k &= k - 1) lo = max(lo, m(__ffs(k) - 1) + 1);
+        for (uint32_t k = L.lt_mask; k; k &= k - 1) hi = min(hi, m(__ffs(k) - 1));
+        const uint32_t *lst = g.adj + moff;
+        const uint32_t mu = nj ? m(L.jpos[tmin]) : 0u;
+        const bool mdir = nj && L.jdir[tmin];
+        s0 = (lo && nj) ? lbound_own(g, mdir, mu, lst, mdeg, lo, true) : 0;
+        e0 = hi != kFullMask ? lbound_own(g, mdir, mu, lst, mdeg, hi, true) : mdeg;
+        if (e0 < s0) e0 = s0;
+        if (L.closed_form && nj == 1) {
+            // one list, no signature: the window minus the matched vertices in it
+            uint32_t sub = 0;
+            for (uint32_t j = 0; j <= d; ++j) {
+                const uint32_t mj = m(j);
+                if (mj >= lo && mj < hi && (((L.guar_mask >> j) & 1u) || in_list(g, moff, mdeg, mj))) ++sub;
+            }
+            n = (e0 - s0) - sub;
+        } else if (fold) {
+            const uint32_t u = m(F.jpos[0]);
+            const uint2 inf = F.jdir[0] ? g.in_info[u] : g.out_info[u];
+            f_off = inf.x;
+            f_deg = inf.y;
+            for (uint32_t k = F.gt_mask; k; k &= k - 1) f_lo = max(f_lo, m(__ffs(k) - 1) + 1);
+            for (uint32_t k = F.lt_mask; k; k &= k - 1) f_hi = min(f_hi, m(__ffs(k) - 1));
+            const uint32_t *fl = g.adj + f_off;
+            const uint32_t ws = f_lo ? lbound(fl, f_deg, f_lo) : 0, we = f_hi != kFullMask ? lbound(fl, f_deg, f_hi) : f_deg;
+            uint32_t sub = 0;
+            for (uint32_t j = 0; j <= d; ++j) {
+                const uint32_t mj = m(j);
+                if (mj >= f_lo && mj < f_hi && (((F.guar_mask >> j) & 1u) || in_list(g, f_off, f_deg, mj))) ++sub;
+            }
+            fbase = (we > ws ? we - ws : 0) - sub;
+        }
+    }
+    if (L.closed_form && nj == 1) return n;
+    const bool fold_guar = (F.guar_mask >> e) & 1u;
+    const uint32_t len = e0 - s0;
+    uint32_t incl = len;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+    if (!total) return 0;
+    const uint32_t lt = (1u << lane) - 1, le = lt | (1u << lane);
+    const unsigned live = __ballot_sync(kFullMask, len != 0);
+    if (len) {
+        const uint32_t r = __popc(live & lt), excl = incl - len;
+        S->rec[r] = make_uint4(moff + s0 - excl, uint32_t(lane) | (tmin << 8), own[0].x, own[0].y);
+        S->rec2[r] = own[1];
+        S->starts[r] = excl;
+    }
+    __syncwarp();
+    const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? S->starts[lane] : kFullMask;
+    uint32_t started = 0;
+    for (uint32_t f0 = 0; f0 < total; f0 += 64) {
+        uint4 rc[2];
+        uint32_t cv[2], rk[2];
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t rel = my_start - (f0 + 32 * h);
+            const uint32_t bits = __reduce_or_sync(kFullMask, rel < 32u ? 1u << rel : 0u);
+            rk[h] = started + __popc(bits & le) - 1;
+            started += __popc(bits);
+            rc[h] = S->rec[rk[h]];
+            cv[h] = __ldg(g.adj + (rc[h].x + min(f0 + 32 * h + lane, total - 1)));
+        }
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t w = cv[h], owner = rc[h].y & 255u, o_tmin = rc[h].y >> 8;
+            bool ok = f0 + 32 * h + lane < total && w >= L.sig_lo;
+            if (ok)
+                for (uint32_t t = 0; t < nj; ++t) {
+                    if (t == o_tmin) continue;
+                    uint32_t off, deg;
+                    if (L.jpos[t] != d) {
+                        off = S->joff[e][t];
+                        deg = S->jdeg[e][t];
+                    } else if (L.jdir[t]) {
+                        off = S->rec2[rk[h]].x;
+                        deg = S->rec2[rk[h]].y;
+                    } else {
+                        off = rc[h].z;
+                        deg = rc[h].w;
+                    }
+                    if (!in_list(g, off, deg, w)) { ok = false; break; }
+                }
+            if (ok)
+                for (uint32_t j = 0; j < d; ++j)
+                    if (w == S->m[j]) { ok = false; break; }
+            if (ok) ok = w != S->buf[d][owner];
+            if (ok && L.check_sig) {
+                const uint2 o = g.out_info[w], i = g.in_info[w];
+                ok = i.y >= L.qin && o.y >= L.qout;
+            }
+            if (fold) {
+                const uint32_t o_base = __shfl_sync(kFullMask, fbase, int(owner));
+                const uint32_t o_off = __shfl_sync(kFullMask, f_off, int(owner));
+                const uint32_t o_deg = __shfl_sync(kFullMask, f_deg, int(owner));
+                const uint32_t o_lo = __shfl_sync(kFullMask, f_lo, int(owner));
+                const uint32_t o_hi = __shfl_sync(kFullMask, f_hi, int(owner));
+                if (ok) {
+                    const bool hit = w >= o_lo && w < o_hi && (fold_guar || in_list(g, o_off, o_deg, w));
+                    n += o_base - (hit ? 1u : 0u);
+                }
+            } else {
+                n += ok;
+            }
+        }
+    }
+    __syncwarp();
+    return n;
+}
+
 // Next up-to-32 candidates of level d into its frontier buffer.
 __device__ void refill(const Ctx &c, uint32_t d) {
     uint32_t v;
@@ -203,6 +367,31 @@ __device__ void refill(const Ctx &c, uint32_t d) {
         c.S->bi[d] = 0;
     }
     __syncwarp();
+}
+
+// Adds the lanes' parts of one query's count to its counter.
+__device__ __forceinline__ void add_count(unsigned long long *__restrict__ to, unsigned long long part, int lane) {
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(kFullMask, part, o);
+    if (lane == 0 && part) atomicAdd(to, part);
+}
+
+// Level d's whole frontier is counted at once (its children are the last
+// level stored, or the one folded with it).
+__device__ __forceinline__ bool counts_next(const BQuery &Q, uint32_t d) {
+    return d + 2 == Q.k || (d + 3 == Q.k && Q.lv[d + 1].fold);
+}
+
+// One vertex of level d's frontier becomes matched; its children are next.
+__device__ __forceinline__ void descend(const Ctx &c, uint32_t d) {
+    const uint32_t v = c.S->buf[d][c.S->bi[d]];
+    __syncwarp();
+    if (c.lane == 0) {
+        c.S->bi[d]++;
+        c.S->m[d] = v;
+    }
+    __syncwarp();
+    enter_level(c, d + 1);
 }
 
 __global__ void __launch_bounds__(kBW * 32)
@@ -234,7 +423,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
         for (unsigned long long cc = c0; cc < c1; ++cc) {
             const unsigned long long t = cc * nshards + shard;
             if (cur == kFullMask || t < qbase[cur] || t >= qbase[cur + 1]) {
-                if (cur != kFullMask && lane == 0 && qcount) atomicAdd(&counts[cur], qcount);
+                if (cur != kFullMask) add_count(&counts[cur], qcount, lane);
                 qcount = 0;
                 uint32_t lo = 0, hi = nq - 1;  // last q with qbase[q] <= t
                 while (lo < hi) {
@@ -306,12 +495,9 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
                 }
                 __syncwarp();
             }
-            if (Q.k == 2) {
-                qcount += count_level(c, 1);
-                continue;
-            }
-            if (Q.k == 3 && Q.lv[1].fold) {
-                qcount += count_level_fold(c, 1);
+            if (Q.k == 2 || (Q.k == 3 && Q.lv[1].fold)) {
+                const unsigned long long r1 = Q.k == 2 ? count_level(c, 1) : count_level_fold(c, 1);
+                if (lane == 0) qcount += r1;  // the warp's
                 continue;
             }
             // depth-first over levels 1..k-2, counting level k-1
@@ -319,17 +505,15 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
             bool abandoned = false, dropped = false;
             while (d >= 1) {
                 if (c.S->bi[d] < c.S->nb[d]) {
-                    const uint32_t v = c.S->buf[d][c.S->bi[d]];
-                    __syncwarp();
-                    if (lane == 0) {
-                        c.S->bi[d]++;
-                        c.S->m[d] = v;
+                    if (counts_next(Q, d)) {
+                        qcount += count_frontier(c, d);
+                        __syncwarp();
+                        if (lane == 0) c.S->bi[d] = c.S->nb[d];
+                        __syncwarp();
+                    } else {
+                        descend(c, d);
+                        ++d;
                     }
-                    __syncwarp();
-                    enter_level(c, d + 1);
-                    if (d + 2 == Q.k) qcount += count_level(c, d + 1);
-                    else if (d + 3 == Q.k && Q.lv[d + 1].fold) qcount += count_level_fold(c, d + 1);
-                    else ++d;
                 } else if (c.S->x[d] < c.S->xend[d]) {
                     const unsigned long long now = global_ns();
                     if (*vstop || now > deadline) { abandoned = true; break; }
@@ -353,7 +537,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
             }
         }
     }
-    if (cur != kFullMask && lane == 0 && qcount) atomicAdd(&counts[cur], qcount);
+    if (cur != kFullMask) add_count(&counts[cur], qcount, lane);
 }
 
 }  // namespace
@@ -452,6 +636,7 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
     aut.assign(nq, 1);
     eligible.assign(nq, 0);
     const uint32_t n = g->n;
+    if ((rc = device_tables(*g))) return rc;
     for (uint32_t i = 0; i < nq; ++i) {
         const Query &q = *qs[i];
         Plan plan;
@@ -474,6 +659,13 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
             B.closed_form = L.closed_form;
             B.fold = L.fold;
             B.guar_mask = L.guar_mask;
+            B.sig_lo = 0;
+            if (d && B.check_sig && g->symmetric && !g->orig.empty()) {
+                // degree-ranked ids: the signature is a compare of ids
+                const uint32_t deg = std::max(B.qin, B.qout);
+                B.sig_lo = n - uint32_t(deg < g->stats.out_ge.size() ? g->stats.out_ge[deg] : 0);
+                B.check_sig = 0;
+            }
             for (uint32_t t = 0; t < L.nj; ++t) {
                 B.jpos[t] = L.jpos[t];
                 B.jdir[t] = L.jdir[t];
@@ -665,16 +857,27 @@ __global__ void k_noalloc_plans(const NoAllocPlans plans, uint32_t first, uint32
     }
 }
 
-// Tasks are (query, root vertex) pairs in vertex-id order, query-major; each
-// runs the root's whole level-1 list depth first with the same level steps as
-// k_batch.  No budget: every query runs to completion.
+// Tasks are (slice, query, block of 32 roots): the lanes look at the block's
+// roots at once, and of each root that passes the level-0 signature the warp
+// runs the slice's part of its level-1 list depth first, with the same level
+// steps as k_batch.  Slice r of kSlices holds the blocks b of kSliceLen
+// level-1 candidates with b % kSlices == r, so a hub's work is spread over
+// kSlices warps; the slices above 0, empty for most roots, come first.  With
+// the whole list of a root as one task, hubs were the launch's tail: 16
+// queries of 2-4 vertices on 50,001 vertices / 300,000 edges took 67.5 ms,
+// NOALLOC_NEW this way (frontiers counted at once included).  No budget: every
+// query runs to completion.
+constexpr uint32_t kSlices = 16;
+constexpr uint32_t kSliceLen = 32;
+
 __global__ void __launch_bounds__(kBW * 32)
 k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq,
                 unsigned long long *__restrict__ counts) {
     __shared__ BWarp ws[kBW];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Ctx c{g, nullptr, &ws[warp], lane};
-    const unsigned long long total = (unsigned long long)nq * g.n;
+    const uint32_t nblk = (g.n + 31) / 32;
+    const unsigned long long per = (unsigned long long)nq * nblk, total = per * kSlices;
     uint32_t cur = kFullMask;
     unsigned long long qcount = 0;
     while (true) {
@@ -682,44 +885,67 @@ k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq,
         if (lane == 0) t = atomicAdd(&sc->task_ctr, 1ull);
         t = __shfl_sync(kFullMask, t, 0);
         if (t >= total) break;
-        const uint32_t q = uint32_t(t / g.n), u = uint32_t(t % g.n);
+        const uint32_t slice = kSlices - 1 - uint32_t(t / per);
+        const unsigned long long in = t % per;
+        const uint32_t q = uint32_t(in / nblk), u0 = uint32_t(in % nblk) * 32;
         if (q != cur) {
-            if (cur != kFullMask && lane == 0 && qcount) atomicAdd(&counts[cur], qcount);
+            if (cur != kFullMask) add_count(&counts[cur], qcount, lane);
             qcount = 0;
             cur = q;
             c.Q = sc->queries + q;
         }
         const BQuery &Q = *c.Q;
         if (Q.k < 2) continue;
-        const uint2 uo = g.out_info[u], ui = g.in_info[u];
-        if (ui.y < Q.lv[0].qin || uo.y < Q.lv[0].qout) continue;  // level-0 signature
-        if (lane == 0) c.S->m[0] = u;
-        __syncwarp();
-        enter_level(c, 1);  // the whole shortest level-1 list, symmetry window applied
-        if (Q.k == 2) { qcount += count_level(c, 1); continue; }
-        if (Q.k == 3 && Q.lv[1].fold) { qcount += count_level_fold(c, 1); continue; }
-        uint32_t d = 1;
-        while (d >= 1) {
-            if (c.S->bi[d] < c.S->nb[d]) {
-                const uint32_t v = c.S->buf[d][c.S->bi[d]];
+        // the block's roots with level-1 candidates in this slice
+        bool pass = false;
+        if (u0 + lane < g.n) {
+            const uint2 uo = g.out_info[u0 + lane], ui = g.in_info[u0 + lane];
+            uint32_t len = kFullMask;
+            for (uint32_t j = 0; j < Q.lv[1].nj; ++j) len = min(len, Q.lv[1].jdir[j] ? ui.y : uo.y);
+            pass = ui.y >= Q.lv[0].qin && uo.y >= Q.lv[0].qout && len != kFullMask && len > slice * kSliceLen;
+        }
+        for (unsigned todo = __ballot_sync(kFullMask, pass); todo; todo &= todo - 1) {
+            if (lane == 0) c.S->m[0] = u0 + __ffs(todo) - 1;
+            __syncwarp();
+            enter_level(c, 1);  // the whole shortest level-1 list
+            const uint32_t xend = c.S->xend[1];
+            for (uint32_t x0 = slice * kSliceLen; x0 < xend; x0 += kSlices * kSliceLen) {
                 __syncwarp();
                 if (lane == 0) {
-                    c.S->bi[d]++;
-                    c.S->m[d] = v;
+                    c.S->x[1] = x0;
+                    c.S->xend[1] = min(x0 + kSliceLen, xend);
+                    c.S->nb[1] = 0;
+                    c.S->bi[1] = 0;
                 }
                 __syncwarp();
-                enter_level(c, d + 1);
-                if (d + 2 == Q.k) qcount += count_level(c, d + 1);
-                else if (d + 3 == Q.k && Q.lv[d + 1].fold) qcount += count_level_fold(c, d + 1);
-                else ++d;
-            } else if (c.S->x[d] < c.S->xend[d]) {
-                refill(c, d);
-            } else {
-                --d;
+                if (Q.k == 2 || (Q.k == 3 && Q.lv[1].fold)) {
+                    const unsigned long long r1 = Q.k == 2 ? count_level(c, 1) : count_level_fold(c, 1);
+                    if (lane == 0) qcount += r1;  // the warp's
+                    continue;
+                }
+                uint32_t d = 1;
+                while (d >= 1) {
+                    if (c.S->bi[d] < c.S->nb[d]) {
+                        if (counts_next(Q, d)) {
+                            qcount += count_frontier(c, d);
+                            __syncwarp();
+                            if (lane == 0) c.S->bi[d] = c.S->nb[d];
+                            __syncwarp();
+                        } else {
+                            descend(c, d);
+                            ++d;
+                        }
+                    } else if (c.S->x[d] < c.S->xend[d]) {
+                        refill(c, d);
+                    } else {
+                        --d;
+                    }
+                }
             }
+            __syncwarp();
         }
     }
-    if (cur != kFullMask && lane == 0 && qcount) atomicAdd(&counts[cur], qcount);
+    if (cur != kFullMask) add_count(&counts[cur], qcount, lane);
 }
 
 }  // namespace
@@ -761,6 +987,7 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
             B.closed_form = L.closed_form;
             B.fold = L.fold;
             B.guar_mask = L.guar_mask;
+            B.sig_lo = 0;
             for (uint32_t t = 0; t < L.nj; ++t) {
                 B.jpos[t] = L.jpos[t];
                 B.jdir[t] = L.jdir[t];
@@ -805,7 +1032,7 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
     const DevView view{reinterpret_cast<const uint2 *>(info_out),
                        reinterpret_cast<const uint2 *>(sym ? info_out : info_in), adj, n, nullptr, nullptr,
                        nullptr, 0, nullptr};
-    const unsigned long long total = (unsigned long long)nq * n;
+    const unsigned long long total = (unsigned long long)nq * ((n + 31) / 32) * kSlices;
     const uint32_t grid = uint32_t(std::min<unsigned long long>(blocks, (total + kBW - 1) / kBW));
     k_batch_noalloc<<<std::max<uint32_t>(grid, 1), kBW * 32, 0, stream>>>(view, sc, nq, counts);
     if (cudaGetLastError() != cudaSuccess)
