@@ -202,7 +202,7 @@ __device__ unsigned long long count_level_fold(const Ctx &c, uint32_t d) {
 // walked 64 candidates a step, as in k_level_flat (engine.cu).  Counting one
 // frontier vertex after another left most lanes idle on short lists: 64 mixed
 // queries of 3 and 4 vertices on 200,000 vertices / 1.6M edges took 480 ms,
-// BATCH_NEW this way.  With a fold at e, each candidate adds the closed form
+// 207 ms this way.  With a fold at e, each candidate adds the closed form
 // of level e + 1.  Returns the lane's part of the count.
 __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
     const uint32_t e = d + 1, nj = c.Q->lv[e].nj;
@@ -865,7 +865,7 @@ __global__ void k_noalloc_plans(const NoAllocPlans plans, uint32_t first, uint32
 // kSlices warps; the slices above 0, empty for most roots, come first.  With
 // the whole list of a root as one task, hubs were the launch's tail: 16
 // queries of 2-4 vertices on 50,001 vertices / 300,000 edges took 67.5 ms,
-// NOALLOC_NEW this way (frontiers counted at once included).  No budget: every
+// 16.8 ms this way (frontiers counted at once included).  No budget: every
 // query runs to completion.
 constexpr uint32_t kSlices = 16;
 constexpr uint32_t kSliceLen = 32;
