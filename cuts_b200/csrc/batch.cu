@@ -209,6 +209,8 @@ __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
     const BLevel &L = c.Q->lv[e];
     const BLevel &F = c.Q->lv[e + 1 < c.Q->k ? e + 1 : e];
     const bool fold = L.fold && e + 2 == c.Q->k;
+    // twins: level e + 1 has a vertex's other candidates of level e
+    const uint32_t twin = e + 2 == c.Q->k ? L.twin : 0u;
     const DevView &g = c.g;
     BWarp *const S = c.S;
     const int lane = c.lane;
@@ -294,6 +296,11 @@ __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
     }
     __syncwarp();
     const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? S->starts[lane] : kFullMask;
+    if (twin) {
+        __syncwarp();
+        S->starts[lane] = 0;  // from here on: candidates of the lane's vertex
+        __syncwarp();
+    }
     uint32_t started = 0;
     for (uint32_t f0 = 0; f0 < total; f0 += 64) {
         uint4 rc[2];
@@ -335,7 +342,16 @@ __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
                 const uint2 o = g.out_info[w], i = g.in_info[w];
                 ok = i.y >= L.qin && o.y >= L.qout;
             }
-            if (fold) {
+            if (twin) {
+                // lanes of one vertex are neighbours: the first of them adds
+                const unsigned mk = __ballot_sync(kFullMask, ok);
+                const uint32_t up = __shfl_up_sync(kFullMask, owner, 1);
+                const bool head = lane == 0 || up != owner;
+                const unsigned next = __ballot_sync(kFullMask, head) & ~le;
+                const unsigned seg = (next ? (1u << (__ffs(next) - 1)) - 1u : kFullMask) & ~lt;
+                if (head) S->starts[owner] += __popc(mk & seg);
+                __syncwarp();
+            } else if (fold) {
                 const uint32_t o_base = __shfl_sync(kFullMask, fbase, int(owner));
                 const uint32_t o_off = __shfl_sync(kFullMask, f_off, int(owner));
                 const uint32_t o_deg = __shfl_sync(kFullMask, f_deg, int(owner));
@@ -349,6 +365,11 @@ __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
                 n += ok;
             }
         }
+    }
+    __syncwarp();
+    if (twin && len) {
+        const unsigned long long q = S->starts[lane], pr = q ? q * (q - 1) : 0;
+        n = twin == 2 ? pr / 2 : pr;
     }
     __syncwarp();
     return n;
@@ -379,7 +400,7 @@ __device__ __forceinline__ void add_count(unsigned long long *__restrict__ to, u
 // Level d's whole frontier is counted at once (its children are the last
 // level stored, or the one folded with it).
 __device__ __forceinline__ bool counts_next(const BQuery &Q, uint32_t d) {
-    return d + 2 == Q.k || (d + 3 == Q.k && Q.lv[d + 1].fold);
+    return d + 2 == Q.k || (d + 3 == Q.k && (Q.lv[d + 1].fold || Q.lv[d + 1].twin));
 }
 
 // One vertex of level d's frontier becomes matched; its children are next.
@@ -658,6 +679,7 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
             B.lt_mask = L.lt_mask;
             B.closed_form = L.closed_form;
             B.fold = L.fold;
+            B.twin = L.twin;
             B.guar_mask = L.guar_mask;
             B.sig_lo = 0;
             if (d && B.check_sig && g->symmetric && !g->orig.empty()) {
@@ -986,6 +1008,7 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
             B.lt_mask = L.lt_mask;
             B.closed_form = L.closed_form;
             B.fold = L.fold;
+            B.twin = L.twin;
             B.guar_mask = L.guar_mask;
             B.sig_lo = 0;
             for (uint32_t t = 0; t < L.nj; ++t) {

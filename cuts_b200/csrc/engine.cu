@@ -520,7 +520,7 @@ __host__ __device__ inline uint32_t flat_words(uint32_t lvl, uint32_t nj, bool e
 // MODE kExpand writes L_lvl (adding its entries' child bounds to *acc where
 // acc is given), kCountMode counts, kBytesMode adds the bytes the
 // count reads.  FOLD: the level also counts the one or two after it (plain or
-// orbit fold, pendant pair).
+// orbit fold, pendant pair, twins).
 template <int MODE, bool FOLD>
 __global__ void __launch_bounds__(kFW * 32, FOLD ? 8 : 10)
 k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Parents parents,
@@ -564,6 +564,9 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Pa
     uint32_t *const ob_p = ob_v + kOutBuf, *const ob_u = ob_p + kOutBuf;
     // pendant pair: this level (k-3) also counts levels k-2 and k-1
     const uint32_t fold2 = FOLD && MODE != kExpand ? sL.fold2 : 0u;
+    // twins: this level (k-2) also counts level k-1, from each parent's number
+    // of candidates (counted into `starts`' place by the parent's lane)
+    const uint32_t twin = FOLD && MODE != kExpand ? sL.twin : 0u;
     unsigned long long local3 = 0;
     const bool store_pos = MODE == kExpand && lvl == rp->pos_lvl;
     const bool need_ub = (MODE == kExpand && lvl + 1 < rp->stored) || store_pos;
@@ -726,6 +729,11 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Pa
         }
         __syncwarp();
         const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? starts[lane] : kFullMask;
+        if (FOLD && twin) {
+            __syncwarp();
+            starts[lane] = 0;  // from here on: candidates of the lane's parent
+            __syncwarp();
+        }
         uint32_t started = 0;  // windows that start before this step
         for (uint32_t fstep = 0; fstep < ftotal; fstep += 64) {
             // two candidates per lane, their loads in flight together
@@ -785,7 +793,17 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Pa
                     if (check_sig) ok = ci.y >= sL.qin && co.y >= sL.qout;
                 }
                 if constexpr (MODE == kCountMode) {
-                    if (fold2) {
+                    if (twin) {
+                        // lanes of one parent are neighbours: the first of them adds
+                        const unsigned m = __ballot_sync(kFullMask, ok);
+                        const uint32_t up = __shfl_up_sync(kFullMask, owner, 1);
+                        const bool head = lane == 0 || up != owner;
+                        const unsigned heads = __ballot_sync(kFullMask, head);
+                        const unsigned next = heads & ~lanemask_le;
+                        const unsigned seg = (next ? (1u << (__ffs(next) - 1)) - 1u : kFullMask) & ~lanemask_lt;
+                        if (head) starts[owner] += __popc(m & seg);
+                        __syncwarp();
+                    } else if (fold2) {
                         if (ok) {
                             const uint64_t p2 = pendant_pairs(g, sN, sN2, fold2, lvl, loops,
                                 [&](uint32_t j) { return j == lvl ? c : sm_m[32 * j + owner]; }, local3);
@@ -829,6 +847,12 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Pa
                     obn += nn;
                 }
             }
+        }
+        __syncwarp();
+        if (FOLD && twin && have && len) {
+            const unsigned long long n = starts[lane], pr = n ? n * (n - 1) : 0;
+            local2 += n;
+            local += twin == 2 ? pr / 2 : pr;
         }
         __syncwarp();
     }
@@ -2487,7 +2511,7 @@ struct Run {
         const uint32_t pa = par.a, pb = par.b;  // the warp-per-parent form: host-known ranges only
         const LevelPlan &L = hp->plan.lv[lvl];
         const bool flat = g_use_flat && L.nj <= uint32_t(kFJ);
-        const bool fold = mode == kBytesMode || (mode == kCountMode && (L.fold || L.fold2));
+        const bool fold = mode == kBytesMode || (mode == kCountMode && (L.fold || L.fold2 || L.twin));
         const uint32_t smem = flat ? flat_smem(mode, lvl, L.nj) : 0;
         // the flattened form deals out single parents when there are few
         const uint32_t warps_needed = flat ? work : (work + grain - 1) / grain;
@@ -2650,7 +2674,8 @@ struct Run {
     }
 
     uint32_t count_level() const {
-        return (k >= 4 && hp->plan.lv[k - 3].fold2) ? k - 3 : (k >= 3 && hp->plan.lv[k - 2].fold) ? k - 2 : k - 1;
+        if (k >= 4 && hp->plan.lv[k - 3].fold2) return k - 3;
+        return k >= 3 && (hp->plan.lv[k - 2].fold || hp->plan.lv[k - 2].twin) ? k - 2 : k - 1;
     }
 
     // Expands parents [pa, pb) of L_{lvl-1}, depth first by chunks.
@@ -2795,6 +2820,11 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         const bool fused_here = hp->plan.lv[k - 2].fuse != 0;
         if (!fused_here && (!g_use_flat || hp->plan.lv[k - 2].nj > uint32_t(kFJ))) hp->plan.lv[k - 2].fold = 0;
         else if (counting) stored = k - 2;  // level k-2 is counted, not stored
+    }
+    if (k >= 4 && hp->plan.lv[k - 2].twin) {
+        // twins are counted by the flattened kernel at level k-2
+        if (counting && g_use_flat && hp->plan.lv[k - 2].nj <= uint32_t(kFJ)) stored = k - 2;
+        else hp->plan.lv[k - 2].twin = 0;
     }
     // the counted level and, when fused, the one before it are not stored
     const uint32_t cl = (k >= 3 && hp->plan.lv[k - 2].fold) ? k - 2 : k - 1;
@@ -3103,7 +3133,7 @@ int device_count(DeviceGraph &g, const Query &q, const CountOptions &opt, CountR
         res.level_sizes[k - 3] = g.h_u64[3];
         res.level_sizes[k - 2] = g.h_u64[kU64Pair];
     }
-    if (k >= 3 && hp->plan.lv[k - 2].fold) {
+    if (k >= 3 && (hp->plan.lv[k - 2].fold || hp->plan.lv[k - 2].twin)) {
         res.level_sizes[k - 2] = g.h_u64[3];
     }
     if (k >= 3) {

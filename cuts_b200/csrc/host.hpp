@@ -117,6 +117,9 @@ struct LevelPlan {
                               // window, the second above / below the first)
     uint32_t guar1;           // level k-2 of a pendant pair: positions whose
                               // vertex the query guarantees in its list
+    uint32_t twin;            // level k-2: the last level's candidates are this
+                              // level's other ones, so both are counted from the
+                              // number c of candidates: 1 c (c - 1), 2 half of it
     uint32_t sig_lo;          // signature as a bound on the candidate's id (set by
                               // the engine on degree-ranked symmetric graphs, where
                               // check_sig is then 0): candidates below it fail

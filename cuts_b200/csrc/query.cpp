@@ -480,6 +480,27 @@ int build_plan(const Query &q, bool data_symmetric, uint32_t flags, Plan &plan) 
             }
         }
     }
+    // Twins: the last two vertices join the same two or more lists, none of
+    // them each other's, under the same conditions from earlier positions (and
+    // at most an order between the two): with c candidates at level k-2, level
+    // k-1 has the other c - 1 for each, so both levels are counted from c (the
+    // two middle vertices of a diamond).  Their arcs all go to joined
+    // positions, so the joins imply both signatures; with one joined list the
+    // fold and the pendant pair above apply instead.
+    if (k >= 4 && !(flags & CUTS_FLAG_NO_CLOSED_FORM) && q.sig_in.empty()) {
+        LevelPlan &L1 = plan.lv[k - 2];
+        const LevelPlan &L2 = plan.lv[k - 1];
+        const uint32_t pen = 1u << (k - 2);
+        bool ok = L1.nj >= 2 && L1.nj == L2.nj && !q.self_loop(q.order[k - 2]) && !q.self_loop(q.order[k - 1]);
+        for (uint32_t t = 0; ok && t < L1.nj; ++t) {
+            bool found = false;
+            for (uint32_t u = 0; u < L2.nj; ++u) found = found || (L2.jpos[u] == L1.jpos[t] && L2.jdir[u] == L1.jdir[t]);
+            ok = found && L1.jpos[t] < k - 2;
+        }
+        ok = ok && (L2.gt_mask & ~pen) == L1.gt_mask && (L2.lt_mask & ~pen) == L1.lt_mask &&
+             ((L2.gt_mask & pen) == 0 || (L2.lt_mask & pen) == 0);
+        if (ok) L1.twin = ((L2.gt_mask | L2.lt_mask) & pen) ? 2 : 1;
+    }
     // Fuse the counted level c with level p = c-1 when c's candidates are a
     // subset of p's: every list p joins is joined at c too, c also joins p's
     // own vertex, p's signature is no stricter than c's, and p's symmetry
