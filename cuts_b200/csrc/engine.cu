@@ -509,6 +509,14 @@ k_level(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t pa, 
 // 4-cycle, 10,000 / 40,000 0.252 -> 0.176 ms; a directed four-vertex query,
 // 150,001 / 1.5M arcs 6.98 -> 3.43 ms.
 constexpr int kFW = 4;    // warps per block
+// Turns a warp should get: a parent has at most max_deg candidates, 64 a step,
+// so with lists of up to 64 entries all parents cost about the same and one
+// turn of total / warps parents each is best (each turn is an atomic on one
+// address: with 8 turns the 10,000-vertex 4-cycle took 194 us, not 117); with
+// hubs among them one turn each left the 5-cycle's expansions at 19 % of warps
+// active (count 344 ms; 8 turns 274 ms, 16 turns 301 ms; a directed query 3.35,
+// 2.2 and 3.3 ms).
+inline uint32_t flat_turns(uint32_t max_deg) { return std::min(8u, std::max(1u, max_deg / 64)); }
 constexpr int kFJ = 8;    // joined lists per level in this form (more: warp-per-parent kernel)
 
 // Words of dynamic shared memory per warp: the parents' matches, their joined
@@ -523,7 +531,7 @@ __host__ __device__ inline uint32_t flat_words(uint32_t lvl, uint32_t nj, bool e
 // orbit fold, pendant pair, twins).
 template <int MODE, bool FOLD>
 __global__ void __launch_bounds__(kFW * 32, FOLD ? 8 : 10)
-k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Parents parents,
+k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t turns, const Parents parents,
              uint32_t *__restrict__ cursor, uint32_t *__restrict__ out_n, uint32_t out_cap,
              uint32_t *__restrict__ err, unsigned long long *__restrict__ acc,
              unsigned long long *__restrict__ acc2, unsigned long long *__restrict__ acc3) {
@@ -586,10 +594,10 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, const Pa
     const bool fold = FOLD && MODE != kExpand && sL.fold;
     const bool fold_guar_c = fold && ((sN.guar_mask >> lvl) & 1u);
     const bool loops = rp->plan.data_loops != 0;
-    // parents per warp: fewer than 32 when that leaves warps without any (a
-    // level of few parents with long lists)
-    const uint32_t nwarps = gridDim.x * kFW;
-    const uint32_t grab = min(32u, max(1u, (total + nwarps - 1) / nwarps));
+    // parents per warp and turn: fewer than 32 where that would leave a warp
+    // fewer than `turns` turns
+    const uint32_t nturns = turns * gridDim.x * kFW;
+    const uint32_t grab = min(32u, (total + nturns - 1) / nturns);
     const unsigned long long deadline = run_deadline(rp);
     unsigned long long local = 0, local2 = 0;
     uint32_t obn = 0;
@@ -2528,7 +2536,7 @@ struct Run {
         if (flat) {
             auto go = [&](auto *kernel, uint32_t ocap, unsigned long long *a1, unsigned long long *a2,
                           unsigned long long *a3) {
-                kernel<<<blocks, kFW * 32, smem, g.stream>>>(view, dp, lvl, par, cursor, out_n, ocap,
+                kernel<<<blocks, kFW * 32, smem, g.stream>>>(view, dp, lvl, flat_turns(g.max_deg), par, cursor, out_n, ocap,
                                                            g.d_u32 + kSlotErr, a1, a2, a3);
             };
             if (mode == kExpand)
