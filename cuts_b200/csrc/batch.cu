@@ -635,6 +635,14 @@ static bool level_engine_pays(const Query &q, bool symmetric, uint32_t flags) {
     return plan.lv[cl].fuse != 0 && !(flags & CUTS_FLAG_NO_FUSE);
 }
 
+// True when the level engine counts q's last two levels as edges between two
+// candidate sets (k_edges): a 4-cycle on 200,000 vertices / 1.6M edges takes
+// 18 ms in a launch of its own here and 10 ms there.
+static bool level_engine_edges(const Query &q, const DeviceGraph &g, uint32_t flags) {
+    Plan plan;
+    return !g.orig.empty() && g.tab && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
+}
+
 int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_t flags_,
                   const BatchTuning &tune_) {
     g = &dg;
@@ -698,6 +706,8 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
         // count, dense-core rows and hub split have no counterpart in the
         // persistent kernel, which walks one candidate at a time
         if (ok && q.k >= 4 && route_level && (route_all || level_engine_pays(q, g->symmetric, flags))) ok = false;
+        const bool edges = ok && q.k >= 4 && route_level && level_engine_edges(q, *g, flags);
+        if (edges) ok = false;
         unsigned long long tasks = 0;
         if (ok) {
             b.k = q.k;
@@ -715,9 +725,10 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
                 index.push_back(i);
             }
         }
-        eligible[i] = ok ? 1 : (b.root_cnt == 0 && b.k ? 2 : 0);
+        eligible[i] = ok ? 1 : edges ? 3 : (b.root_cnt == 0 && b.k ? 2 : 0);
     }
-    // eligible: 1 = in the launch, 2 = no root (count 0), 0 = counted by the level engine
+    // eligible: 1 = in the launch, 2 = no root (count 0), 0 = counted by the
+    // level engine, 3 = the same, within the launch's budget
     nb = uint32_t(hq.size());
     total_tasks = qbase.back();
     BCK(cudaMalloc(&d_queries, sizeof(BQuery) * std::max<size_t>(hq.size(), 1)));
@@ -807,20 +818,31 @@ int Batch::run(double budget_ms, std::vector<uint64_t> &counts, std::vector<int>
         const bool unfinished = h_aborted[b] || (stopped && qbase_host[b + 1] > stop_at);
         if (unfinished) status[i] = CUTS_ERR_BUDGET;
     }
-    // queries outside the batched kernel's limits: the level engine, one by one
+    // queries outside the batched kernel's limits, and those the level engine
+    // is better at: one by one
+    double left = budget_ms - t;  // of the launch's budget, where there is one
     for (uint32_t i = 0; i < nq; ++i) {
-        if (eligible[i] != 0) continue;
+        if (eligible[i] != 0 && eligible[i] != 3) continue;
         CountResult r;
         CountOptions opt;
         opt.flags = flags;
         opt.budget_ms = query_budget_ms;
+        if (eligible[i] == 3 && budget_ms > 0) {
+            if (left <= 0) {
+                status[i] = CUTS_ERR_BUDGET;
+                continue;
+            }
+            opt.budget_ms = query_budget_ms > 0 ? std::min(query_budget_ms, left) : left;
+        }
         opt.shard = shard;
         opt.nshards = nshards;
         rc = device_count(*g, *queries[i], opt, r);
         if (rc) {
+            if (eligible[i] == 3) left -= opt.budget_ms;
             status[i] = rc;
             continue;
         }
+        if (eligible[i] == 3) left -= r.ms;
         counts[i] = r.count;
         t += r.ms;
     }

@@ -45,7 +45,7 @@ struct Batch {
     uint32_t nq = 0;                 // all queries
     uint32_t nb = 0;                 // queries in the launch
     std::vector<uint32_t> index;     // launch slot -> query
-    std::vector<int> eligible;       // 1 in the launch, 2 no root, 0 level engine
+    std::vector<int> eligible;       // 1 in the launch, 2 no root, 0 level engine, 3 level engine within the budget
     bool route_level = true;         // fused / orbit-folded queries of 4+ vertices to the level engine
     bool route_all = false;          // every query of 4+ vertices to the level engine
     std::vector<uint64_t> aut;       // count multiplier per query

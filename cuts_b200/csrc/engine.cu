@@ -65,6 +65,7 @@ struct RunParams {
     uint32_t pos_lvl;
     uint32_t fuse_stride;  // words per warp row of the fused kernel's scratch
     uint32_t *fuse_scratch;
+    uint32_t edges;        // levels k-2 and k-1 are counted by k_edges
     uint32_t pairs;        // the fused count runs in k_pairs (else k_fused)
     uint32_t *fuse_big;    // the fused kernel's deferred parents (arrays, pool or bitmaps)
     uint32_t fuse_big_cap;
@@ -2158,6 +2159,309 @@ k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big
     }
 }
 
+// ---- edges between two candidate sets ----------------------------------
+// When level d = k-2 joins one list of an earlier vertex and the last level
+// joins the vertex at d and one earlier vertex (cycles, the house, ladders),
+// one parent at level d-1 fixes two sets, C (candidates of d) and T (those of
+// the last level but for d's list), and the two levels' matches are the edges
+// between them.  L_d is neither stored nor walked entry by entry: its size is
+// |C| by list arithmetic, and the edges are found from the smaller set.  A warp takes up
+// to 32 parents, one per lane, puts their smaller sets into shared memory and
+// walks, for every vertex v there, the other set's window (tested in v's
+// table) or v's own neighbours (tested in the other set's list), whichever is
+// shorter, 64 a step as in k_level_flat.  Sets of more than `split` vertices
+// are dealt out in pieces by a second launch.  On a graph whose ids are degree
+// ranks, so that d's signature is a bound on the id.
+// What it saves is the set-up per entry of L_d: the 5-cycle on 200,003
+// vertices / 1M edges has 6.9e9 of them with 1.5 last-level candidates each.
+// Whole counts against expanding L_d and counting its entries: that 5-cycle
+// 273 -> 45 ms, the house on 100,000 / 500,000 22 -> 18.4 ms, the 4-cycle on
+// 10,000 / 40,000 117 -> 101 us.  Bound: instruction issue (55 % of slots) and
+// L2 latency.
+enum EdgeRow : int { kECOff = 0, kECDeg, kETOff, kETDeg, kEOLo, kEOHi, kEOBase, kEOLen, kESide, kEMatched, kEdgeRows };
+
+__host__ __device__ inline uint32_t edge_words(uint32_t d) {
+    return kPS + kPS / 4 + 128 + 32 + 32 * (kEdgeRows + d);
+}
+
+template <bool TALLY>
+__global__ void __launch_bounds__(kPW * 32, 8)
+k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns, const Parents parents, uint32_t phase,
+        uint32_t split, uint32_t *__restrict__ cursor, PairBig big, unsigned long long *__restrict__ acc,
+        unsigned long long *__restrict__ acc_d, unsigned long long *__restrict__ accb) {
+    uint32_t pa, total;
+    parents_of(parents, pa, total);
+    if (!total) return;
+    __shared__ LevelPlan sC, sT;
+    __shared__ uint32_t *s_vert[kMaxK];
+    __shared__ uint32_t *s_par[kMaxK];
+    extern __shared__ __align__(16) uint32_t dyn[];
+    {
+        const uint32_t words = sizeof(LevelPlan) / 4;
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
+            reinterpret_cast<uint32_t *>(&sC)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[d])[i];
+            reinterpret_cast<uint32_t *>(&sT)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[d + 1])[i];
+        }
+        if (threadIdx.x < kMaxK) {
+            s_vert[threadIdx.x] = rp->vert[threadIdx.x];
+            s_par[threadIdx.x] = rp->par[threadIdx.x];
+        }
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1, le = lt | (1u << lane);
+    uint32_t *const wbase = dyn + warp * edge_words(d);
+    uint4 *const rec = reinterpret_cast<uint4 *>(wbase);
+    uint32_t *const starts = wbase + 128;
+    uint32_t *const S = starts + 32;
+    uint8_t *const So = reinterpret_cast<uint8_t *>(S + kPS);  // the member's column
+    uint32_t *const row = S + kPS + kPS / 4;                   // [EdgeRow][lane]
+    uint32_t *const m = row + 32 * kEdgeRows;                  // [position][lane]
+    const uint32_t jt = sT.jpos[0] == d ? sT.jpos[1] : sT.jpos[0];  // T's list
+    const bool t_above = (sT.gt_mask >> d) & 1u, t_below = (sT.lt_mask >> d) & 1u;  // order between d and the last level
+    const uint32_t below = (1u << d) - 1;
+    const bool loops = rp->plan.data_loops != 0;
+    const bool ordered = t_above || t_below || loops;  // a hit is compared with its vertex
+    const bool phase2 = phase == 2;
+    uint32_t nbig = 0;
+    if (phase2) {
+        const unsigned long long n0 = big.n[0];
+        nbig = n0 < big.cap ? uint32_t(n0) : big.cap;
+        total = nbig ? big.pref[nbig - 1] : 0;
+    }
+    const uint32_t nturns = turns * gridDim.x * kPW;
+    const uint32_t grab = phase2 ? 1u : min(32u, (total + nturns - 1) / nturns);
+    const unsigned long long deadline = run_deadline(rp);
+    unsigned long long local = 0, local_d = 0, tb = 0;
+
+    while (true) {
+        uint32_t start = 0;
+        if (lane == 0) start = past_deadline(rp, deadline) ? total : atomicAdd(cursor, grab);
+        start = __shfl_sync(kFullMask, start, 0);
+        if (start >= total) break;
+        uint32_t pos = 0, end = 0;  // the smaller set's candidates left, as adjacency words
+        if (uint32_t(lane) < grab && start + lane < total) {
+            uint32_t q0 = pa + start + lane, ch = 0;
+            if (phase2) {
+                const uint32_t gi = start + lane;
+                uint32_t lo = 0, hi = nbig - 1;  // first b with pref[b] > gi
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (big.pref[mid] > gi) hi = mid; else lo = mid + 1;
+                }
+                ch = gi - (lo ? big.pref[lo - 1] : 0);
+                q0 = big.q[lo];
+            }
+            uint32_t e = q0;
+            for (int j = int(d) - 1; j >= 0; --j) {
+                m[32 * j + lane] = s_vert[j][e];
+                if (j > 0) e = s_par[j][e];
+            }
+            // a set's list, value bounds and window
+            uint32_t off[2], deg[2], lo[2], hi[2], s0[2], e0[2];
+            #pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const LevelPlan &L = r ? sT : sC;
+                const uint32_t u = m[32 * (r ? jt : uint32_t(sC.jpos[0])) + lane];
+                const uint2 inf = g.out_info[u];
+                off[r] = inf.x;
+                deg[r] = inf.y;
+                lo[r] = L.sig_lo;
+                hi[r] = kFullMask;
+                for (uint32_t k = L.gt_mask & below; k; k &= k - 1) lo[r] = max(lo[r], m[32 * (__ffs(k) - 1) + lane] + 1);
+                for (uint32_t k = L.lt_mask & below; k; k &= k - 1) hi[r] = min(hi[r], m[32 * (__ffs(k) - 1) + lane]);
+                const uint32_t *l = g.adj + inf.x;
+                s0[r] = lo[r] && inf.y && __ldg(l) < lo[r] ? lbound_own(g, false, u, l, inf.y, lo[r], loops) : 0;
+                e0[r] = hi[r] != kFullMask ? lbound_own(g, false, u, l, inf.y, hi[r], loops) : inf.y;
+                if (e0[r] < s0[r]) e0[r] = s0[r];
+            }
+            const uint32_t nc = e0[0] - s0[0], nt = e0[1] - s0[1];
+            const uint32_t side = nt < nc ? 1u : 0u;  // whose vertices are gone through
+            // matched vertices in C's window and list, and in T's where T is
+            // the other set
+            uint32_t in_c = 0, in_t = 0;
+            for (uint32_t j = 0; j < d; ++j) {
+                const uint32_t mj = m[32 * j + lane];
+                if (mj >= lo[0] && mj < hi[0] && in_list(g, off[0], deg[0], mj)) in_c |= 1u << j;
+                if (!side && mj >= lo[1] && mj < hi[1] && in_list(g, off[1], deg[1], mj)) in_t |= 1u << j;
+            }
+            if (!phase2) {
+                local_d += nc - __popc(in_c);  // |C|
+                if (TALLY) tb += 8ull * d + 16 + 32ull * d;
+            }
+            row[32 * kEMatched + lane] = side ? in_c : in_t;
+            row[32 * kESide + lane] = side;
+            row[32 * kECOff + lane] = off[0];
+            row[32 * kECDeg + lane] = deg[0];
+            row[32 * kETOff + lane] = off[1];
+            row[32 * kETDeg + lane] = deg[1];
+            row[32 * kEOLo + lane] = side ? lo[0] : lo[1];
+            row[32 * kEOHi + lane] = side ? hi[0] : hi[1];
+            row[32 * kEOBase + lane] = side ? off[0] + s0[0] : off[1] + s0[1];
+            row[32 * kEOLen + lane] = side ? nc : nt;
+            if (nc && nt) {
+                pos = side ? off[1] + s0[1] : off[0] + s0[0];
+                end = side ? off[1] + e0[1] : off[0] + e0[0];
+            }
+            if (phase2) {
+                pos = min(pos + ch * kPK, end);
+                end = min(pos + kPK, end);
+            } else if (end - pos > split) {
+                const unsigned long long slot = atomicAdd(&big.n[0], 1ull);
+                if (slot < big.cap) {  // (a full list: this warp counts it)
+                    big.q[slot] = q0;
+                    big.len[slot] = end - pos;
+                    end = pos;
+                }
+            }
+        }
+        while (true) {
+            // ---- the next round: as many of the sets as fit, a prefix of the lanes
+            const uint32_t take = min(end - pos, kPS);
+            uint32_t incl = take;
+            #pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const uint32_t len = incl <= kPS ? take : 0u;
+            const unsigned live = __ballot_sync(kFullMask, len != 0);
+            if (!live) break;
+            const uint32_t ftotal = __shfl_sync(kFullMask, incl, 31 - __clz(live));
+            if (len) {
+                const uint32_t r = __popc(live & lt), excl = incl - len;
+                rec[r] = make_uint4(pos - excl, uint32_t(lane), 0, 0);
+                starts[r] = excl;
+                pos += len;
+            }
+            __syncwarp();
+            uint32_t ns = 0;
+            {
+                const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? starts[lane] : kFullMask;
+                uint32_t started = 0;
+                for (uint32_t fstep = 0; fstep < ftotal; fstep += 32) {
+                    const uint32_t rel = my_start - fstep;
+                    const uint32_t bits = __reduce_or_sync(kFullMask, rel < 32u ? 1u << rel : 0u);
+                    const uint4 rc = rec[started + __popc(bits & le) - 1];
+                    started += __popc(bits);
+                    const uint32_t f = fstep + lane, owner = rc.y;
+                    bool ok = f < ftotal;
+                    const uint32_t v = __ldg(g.adj + (rc.x + min(f, ftotal - 1)));
+                    for (uint32_t j = 0; j < d; ++j) ok = ok && v != m[32 * j + owner];
+                    const unsigned mk = __ballot_sync(kFullMask, ok);
+                    if (ok) {
+                        const uint32_t i = ns + __popc(mk & lt);
+                        S[i] = v;
+                        So[i] = uint8_t(owner);
+                    }
+                    ns += __popc(mk);
+                    if (TALLY && f < ftotal) tb += 4;
+                }
+            }
+            __syncwarp();
+            // ---- each vertex of the smaller sets with its possible partners
+            for (uint32_t i0 = 0; i0 < ns; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                uint32_t ilen = 0, ibase = 0, ioff = 0, ideg = 0, ow = 0, mode = 0;
+                if (i < ns) {
+                    ow = So[i];
+                    const uint32_t v = S[i];
+                    const uint32_t side = row[32 * kESide + ow];
+                    const uint2 inf = g.out_info[v];
+                    uint32_t a = 0, b = inf.y;  // the part of v's list that the order allows
+                    if (side ? t_below : t_above) a = __ldg(g.bwd_out + v);
+                    if (side ? t_above : t_below) b = __ldg(g.bwd_out + v);
+                    const uint32_t lenO = row[32 * kEOLen + ow], lenV = b - a;
+                    mode = lenV < lenO ? 1u : 0u;
+                    ilen = mode ? lenV : lenO;
+                    ibase = mode ? inf.x + a : row[32 * kEOBase + ow];
+                    ioff = mode ? row[32 * (side ? kECOff : kETOff) + ow] : inf.x;
+                    ideg = mode ? row[32 * (side ? kECDeg : kETDeg) + ow] : inf.y;
+                    mode |= side << 1;
+                    if (TALLY) tb += 8;
+                    // the matched vertices among v's partners, taken off here
+                    // rather than compared with every hit
+                    for (uint32_t k = ilen ? row[32 * kEMatched + ow] : 0u; k; k &= k - 1) {
+                        const uint32_t mj = m[32 * (__ffs(k) - 1) + ow];
+                        if (side ? t_below : t_above) { if (mj < v) continue; }
+                        if (side ? t_above : t_below) { if (mj > v) continue; }
+                        if (in_list(g, inf.x, inf.y, mj)) --local;
+                    }
+                }
+                uint32_t iincl = ilen;
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFullMask, iincl, o);
+                    if (lane >= o) iincl += y;
+                }
+                const uint32_t itotal = __shfl_sync(kFullMask, iincl, 31);
+                if (!itotal) continue;
+                const unsigned ilive = __ballot_sync(kFullMask, ilen != 0);
+                if (ilen) {
+                    const uint32_t r = __popc(ilive & lt), excl = iincl - ilen;
+                    rec[r] = make_uint4(ibase - excl, ow | (mode << 8) | (i << 16), ioff, ideg);
+                    starts[r] = excl;
+                }
+                __syncwarp();
+                const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(ilive)) ? starts[lane] : kFullMask;
+                uint32_t started = 0;
+                for (uint32_t fstep = 0; fstep < itotal; fstep += 64) {
+                    uint4 rc[2];
+                    uint32_t wv[2], nb[2], bu[2];
+                    Bucket bk[2];
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t rel = my_start - (fstep + 32 * h);
+                        const uint32_t bits = __reduce_or_sync(kFullMask, rel < 32u ? 1u << rel : 0u);
+                        rc[h] = rec[started + __popc(bits & le) - 1];
+                        started += __popc(bits);
+                        wv[h] = __ldg(g.adj + (rc[h].x + min(fstep + 32 * h + lane, itotal - 1)));
+                    }
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        nb[h] = (rc[h].w + 3) >> 2;
+                        bu[h] = tab_bucket(nb[h], wv[h]);
+                        bk[h] = load_bucket(g.tab, rc[h].z, bu[h]);
+                    }
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        bool ok = fstep + 32 * h + lane < itotal;
+                        const uint32_t w = wv[h];
+                        if (TALLY && ok) tb += 36;
+                        if (ok && !bucket_has(bk[h], w)) ok = tab_continue(g.tab, rc[h].z, nb[h], bu[h], bk[h], w);
+                        if (ok) {
+                            const uint32_t l = rc[h].y & 255u;
+                            ok = w >= row[32 * kEOLo + l] && w < row[32 * kEOHi + l];
+                            if (ordered) {
+                                const uint32_t v = S[rc[h].y >> 16];
+                                const bool item_t = (rc[h].y >> 9) & 1u;
+                                ok = ok && w != v;  // v lists itself only where there are self-loops
+                                if (item_t ? t_below : t_above) ok = ok && w > v;
+                                if (item_t ? t_above : t_below) ok = ok && w < v;
+                            }
+                            local += ok;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+    }
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        local += __shfl_xor_sync(kFullMask, local, o);
+        local_d += __shfl_xor_sync(kFullMask, local_d, o);
+        if (TALLY) tb += __shfl_xor_sync(kFullMask, tb, o);
+    }
+    if (lane == 0) {
+        if (local) atomicAdd(acc, local);
+        if (local_d) atomicAdd(acc_d, local_d);
+        if (TALLY && tb) atomicAdd(accb, tb);
+    }
+}
+
 // ---- chunk planner ------------------------------------------------------
 // Tile sums of the child bounds of parents [pa, pb).
 __global__ void k_tile_sums(const uint32_t *__restrict__ ub, uint32_t pa, uint32_t pb,
@@ -2256,6 +2560,7 @@ int g_num_sms = 0;
 int g_level_blocks[3] = {0, 0, 0};
 int g_flat_blocks[3][2] = {};  // blocks of k_level_flat<mode, fold> per SM by registers and threads
 int g_fused_blocks[3] = {0, 0, 0};
+int g_edge_blocks = 0;  // blocks of k_edges per SM by registers and threads
 int g_pair_blocks[2] = {0, 0};  // blocks of k_pairs<fold> per SM by registers and threads
 // CUTS_LEVEL_KERNEL=warp selects the warp-per-parent form (A/B comparisons)
 bool g_use_flat = true;
@@ -2288,6 +2593,8 @@ int launch_geometry() {
     g_pair_blocks[0] = std::max(1, b);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<true, false>, kPW * 32, 0));
     g_pair_blocks[1] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edges<false>, kPW * 32, 0));
+    g_edge_blocks = std::max(1, b);
     const char *kv = std::getenv("CUTS_LEVEL_KERNEL");
     g_use_flat = !(kv && std::strcmp(kv, "warp") == 0);
     return CUTS_OK;
@@ -2668,6 +2975,60 @@ struct Run {
         return CUTS_OK;
     }
 
+    // Levels d = k-2 and k-1 over the given parents of L_{d-1} as edges between
+    // two sets, then the pieces of the sets it listed.
+    int launch_edges(int mode, uint32_t d, const Parents &par, uint32_t most, ChainSlice *cs = nullptr) {
+        uint32_t *cur1 = cs ? cs->cursor + d : g.d_u32 + kSlotCursor;
+        uint32_t *cur2 = cs ? cs->cursor + d + 1 : g.d_u32 + kSlotCursor + 1;
+        PairBig pb;
+        pb.n = cs ? cs->big : g.d_u64 + kU64Big;
+        pb.cap = hp->fuse_big_cap;
+        pb.q = hp->fuse_big;
+        pb.len = pb.q + pb.cap;
+        pb.pref = pb.len + pb.cap;
+        pb.bits = nullptr;
+        if (!cs) {
+            CK(cudaMemsetAsync(cur1, 0, 2 * sizeof(uint32_t), g.stream));
+            CK(cudaMemsetAsync(pb.n, 0, 2 * sizeof(unsigned long long), g.stream));
+        }
+        const bool tal = mode == kBytesMode;
+        unsigned long long *a1 = tal ? g.d_u64 + kU64Scratch : g.d_u64;
+        unsigned long long *ad = tal ? g.d_u64 + kU64Scratch + 1 : g.d_u64 + 4;
+        const uint32_t smem = 4 * kPW * edge_words(d);
+        const uint32_t fixed = 2 * uint32_t(sizeof(LevelPlan)) + 16 * kMaxK + 1024;
+        const uint32_t full = std::max(1u, std::min(uint32_t(g_edge_blocks), 227u * 1024u / (smem + fixed))) *
+                              uint32_t(g_num_sms);
+        const uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(full, (most + kPW - 1) / kPW));
+        const uint32_t split = kPK;
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        if (profile) {
+            CK(cudaEventCreate(&e0));
+            CK(cudaEventCreate(&e1));
+            CK(cudaEventRecord(e0, g.stream));
+        }
+        auto phase = [&](uint32_t grid, uint32_t ph, uint32_t *cur) {
+            auto go = [&](auto *kernel) {
+                kernel<<<grid, kPW * 32, smem, g.stream>>>(view, dp, d, flat_turns(g.max_deg), par, ph, split, cur, pb,
+                                                          a1, ad, g.d_u64 + 2);
+            };
+            tal ? go(k_edges<true>) : go(k_edges<false>);
+        };
+        phase(blocks, 1, cur1);
+        CK(cudaGetLastError());
+        res.launches++;
+        if (g.max_deg > split) {  // else no set can be listed
+            k_fused_scan<<<1, 1024, 0, g.stream>>>(pb.n, pb.cap, pb.len, kPK, pb.pref);
+            phase(full, 2, cur2);
+            CK(cudaGetLastError());
+            res.launches += 2;
+        }
+        if (profile) {
+            CK(cudaEventRecord(e1, g.stream));
+            marks.push_back({kCountMode, {e0, e1}});
+        }
+        return CUTS_OK;
+    }
+
     // Sums the profiled launch times per kernel (after a sync).
     void collect_profile() {
         for (auto &m : marks) {
@@ -2694,6 +3055,8 @@ struct Run {
         const uint32_t count_lvl = count_level();
         if (!dump && k >= 3 && hp->plan.lv[count_lvl].fuse && lvl == count_lvl - 1)
             return launch_fused(bytes_mode ? kBytesMode : kCountMode, lvl, known(pa, pb), pb - pa);
+        if (!dump && hp->edges && lvl == count_lvl - 1)
+            return launch_edges(bytes_mode ? kBytesMode : kCountMode, lvl, known(pa, pb), pb - pa);
         if (lvl == count_lvl && !dump)
             return launch_level(bytes_mode ? kBytesMode : kCountMode, lvl, known(pa, pb), pb - pa);
         std::vector<uint32_t> cuts;
@@ -2841,6 +3204,16 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         for (uint32_t i = 0; i < k; ++i) hp->plan.lv[i].fuse = 0;
     const bool fuse = counting && k >= 3 && hp->plan.lv[cl].fuse;
     if (fuse) stored = cl - 1;
+    // levels k-2 and k-1 as edges between two candidate sets, where the id
+    // bounds stand for k-2's signature (degree-ranked ids) and the lists have
+    // tables
+    bool edges = counting && !fuse && g_use_flat && !g.orig.empty() && edges_shape(hp->plan);
+    if (edges) {
+        if ((rc = device_tables(g))) return rc;
+        edges = g.tab != nullptr;
+    }
+    hp->edges = edges ? 1u : 0u;
+    if (edges) stored = k - 2;
     // on a symmetric graph with degree-ranked ids the vertices of degree d or
     // more are a suffix of the ids: the signature is a compare of ids, not a
     // gather of the candidate's degree
@@ -2885,6 +3258,12 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         hp->fuse_big_cap = uint32_t(std::max<uint64_t>(64, std::min<uint64_t>(1u << 17, g.arena_bytes / 64 / (4 * per))));
         big_bytes = (4 * per * hp->fuse_big_cap + 255) / 256 * 256;
         fuse_bytes = big_bytes;
+    } else if (edges) {
+        // listed sets: parent, length and prefix sum each (beyond the list's
+        // capacity a set is counted where it is found)
+        hp->fuse_big_cap = uint32_t(std::max<uint64_t>(64, std::min<uint64_t>(1u << 18, g.arena_bytes / 64 / 12)));
+        big_bytes = (12ull * hp->fuse_big_cap + 255) / 256 * 256;
+        fuse_bytes = big_bytes;
     } else if (fuse) {
         hp->fuse_stride = ((std::max<uint32_t>(g.max_deg, 1) + 31) / 32) * 32;
         fuse_bytes = uint64_t(g_fused_blocks[kCountMode] > g_fused_blocks[kBytesMode] ? g_fused_blocks[kCountMode]
@@ -2902,7 +3281,7 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     cap = 0;
     if (g.arena_bytes < l0_bytes + fuse_bytes)
         return set_error(CUTS_ERR_NOMEM, "arena smaller than the root level and scratch");
-    if (fuse) {
+    if (fuse || edges) {
         char *const end = static_cast<char *>(g.arena) + (g.arena_bytes & ~uint64_t(255));
         hp->fuse_scratch = reinterpret_cast<uint32_t *>(end - fuse_bytes);
         hp->fuse_big = reinterpret_cast<uint32_t *>(end - big_bytes);
@@ -2967,7 +3346,7 @@ int run_slices(Run &run, uint32_t n0, uint32_t chunks) {
 int Run::chain(uint32_t chunks) {
     const uint32_t cl = count_level();
     const bool fused = k >= 3 && hp->plan.lv[cl].fuse;
-    const uint32_t last = fused ? cl - 1 : cl;  // level of the counting launch
+    const uint32_t last = fused || hp->edges ? cl - 1 : cl;  // level of the counting launch
     // bounds on the levels' sizes, for the launches' grids
     std::vector<uint64_t> most(last + 1, 0);
     most[0] = g.n;
@@ -2986,6 +3365,7 @@ int Run::chain(uint32_t chunks) {
                             g.d_u32 + kSlotStop, ((i + 1) << 8) | lvl};
                 const uint32_t m = uint32_t(std::min<uint64_t>(lvl == 1 ? most[0] / chunks + 1 : most[lvl - 1], UINT32_MAX));
                 if (!exp && fused) rc = launch_fused(kCountMode, lvl, par, m, ds + i);
+                else if (!exp && hp->edges) rc = launch_edges(kCountMode, lvl, par, m, ds + i);
                 else rc = launch_level(exp ? kExpand : kCountMode, lvl, par, m, ds + i);
                 if (rc) return rc;
             }
@@ -3146,9 +3526,8 @@ int device_count(DeviceGraph &g, const Query &q, const CountOptions &opt, CountR
     }
     if (k >= 3) {
         const uint32_t cl = hp->plan.lv[k - 2].fold ? k - 2 : k - 1;
-        if (hp->plan.lv[cl].fuse) {  // the fused level before the counted one
+        if (hp->plan.lv[cl].fuse || hp->edges)  // the level before the counted one, counted with it
             res.level_sizes[cl - 1] = g.h_u64[4];
-        }
     }
     res.count = raw * hp->plan.aut;
     if (opt.want_bytes && k >= 2 && n0 > 0) {

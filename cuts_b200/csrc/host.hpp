@@ -137,6 +137,18 @@ struct Plan {
     LevelPlan lv[kMaxK];
 };
 
+// True when the plan's last two levels are the edges between two candidate
+// sets on a symmetric graph: level k-2 joins one list, the last one the vertex
+// at k-2 and one earlier vertex, nothing is folded into either and the last
+// level needs no signature (see k_edges in engine.cu).
+inline bool edges_shape(const Plan &plan) {
+    const uint32_t k = plan.k;
+    if (!plan.symmetric || k < 3) return false;
+    const LevelPlan &C = plan.lv[k - 2], &T = plan.lv[k - 1];
+    if (C.nj != 1 || T.nj != 2 || T.check_sig || C.fold || C.twin || (k >= 4 && plan.lv[k - 3].fold2)) return false;
+    return (T.jpos[0] == k - 2) != (T.jpos[1] == k - 2);
+}
+
 // Builds the plan for q.order on a graph with the given symmetry.
 int build_plan(const Query &q, bool data_symmetric, uint32_t flags, Plan &plan);
 
