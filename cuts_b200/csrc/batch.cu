@@ -2,7 +2,10 @@
 // launch, captured in a CUDA graph.
 //
 // Work is a flat space of tasks, query-major: a task is (query q, root u,
-// range r of u's level-1 candidate list).  Roots are the data vertices in
+// range r of u's level-1 candidate list), or, for the roots whose list is one
+// range, 8 or 32 roots -- finding a task's root is two binary searches of ~20
+// dependent loads, which with one task per root was most of a small query's
+// time (a triangle on 200,000 vertices alone 0.92 ms, 0.45 ms this way).  Roots are the data vertices in
 // out-degree order, so every query's root level is a prefix of one sorted
 // array, and a per-graph prefix sum of ceil(len / grain) turns a task index
 // into (u, r) with two binary searches -- nothing per query is materialised.
@@ -403,6 +406,12 @@ __device__ __forceinline__ bool counts_next(const BQuery &Q, uint32_t d) {
     return d + 2 == Q.k || (d + 3 == Q.k && (Q.lv[d + 1].fold || Q.lv[d + 1].twin));
 }
 
+// Single-range roots of one task: 32 where they are counted at once, fewer
+// where the warp goes through them one after another (a tail of 32 subtrees).
+__host__ __device__ inline uint32_t roots_per_task(const BQuery &Q) {
+    return Q.k == 2 || (Q.k == 3 && Q.lv[1].fold) ? 32u : 8u;
+}
+
 // One vertex of level d's frontier becomes matched; its children are next.
 __device__ __forceinline__ void descend(const Ctx &c, uint32_t d) {
     const uint32_t v = c.S->buf[d][c.S->bi[d]];
@@ -477,20 +486,86 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
             const BQuery &Q = *c.Q;
             const unsigned long long local = t - qbase[cur];
             const unsigned long long *pref = Q.type == 0 ? pref0 : (Q.type == 1 ? pref1 : pref2);
-            uint32_t lo = 0, hi = Q.root_cnt - 1;  // root: last j with pref[j] <= local
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1) >> 1;
-                if (pref[mid] <= local) lo = mid; else hi = mid - 1;
-            }
-            const uint32_t u = vsorted[lo];
-            const uint32_t r = uint32_t(local - pref[lo]);
-            const uint2 uo = g.out_info[u], ui = g.in_info[u];
-            if (ui.y < Q.lv[0].qin || uo.y < Q.lv[0].qout) continue;  // level-0 signature
-            if (lane == 0) c.S->m[0] = u;
-            __syncwarp();
-            // level 1: joins all on position 0; the task fixes the list and range
-            enter_level(c, 1);
-            {
+            bool abandoned = false, dropped = false;
+            // the subtree of the root m[0] from the level-1 candidates
+            // [x[1], xend[1]) on: depth-first over levels 1..k-2, counting k-1
+            auto subtree = [&]() {
+                if (Q.k == 2 || (Q.k == 3 && Q.lv[1].fold)) {
+                    const unsigned long long r1 = Q.k == 2 ? count_level(c, 1) : count_level_fold(c, 1);
+                    if (lane == 0) qcount += r1;  // the warp's
+                    return;
+                }
+                uint32_t d = 1;
+                while (d >= 1) {
+                    if (c.S->bi[d] < c.S->nb[d]) {
+                        if (counts_next(Q, d)) {
+                            qcount += count_frontier(c, d);
+                            __syncwarp();
+                            if (lane == 0) c.S->bi[d] = c.S->nb[d];
+                            __syncwarp();
+                        } else {
+                            descend(c, d);
+                            ++d;
+                        }
+                    } else if (c.S->x[d] < c.S->xend[d]) {
+                        const unsigned long long now = global_ns();
+                        if (*vstop || now > deadline) { abandoned = true; return; }
+                        if (qlimit && reinterpret_cast<volatile unsigned long long *>(qtime)[cur] +
+                                              (now - task_start) > qlimit) {
+                            dropped = true;
+                            return;
+                        }
+                        refill(c, d);
+                    } else {
+                        --d;
+                    }
+                }
+            };
+            const unsigned long long heavy = pref[Q.heavy_roots];
+            if (local >= heavy) {
+                // roots of one range each: looked at together, and counted
+                // together where level 1 is the last one walked
+                const uint32_t per = roots_per_task(Q);
+                const uint32_t ri = Q.heavy_roots + uint32_t(local - heavy) * per + lane;
+                uint32_t u = 0;
+                bool pass = uint32_t(lane) < per && ri < Q.root_cnt;
+                if (pass) {
+                    u = vsorted[ri];
+                    const uint2 uo = g.out_info[u], ui = g.in_info[u];
+                    pass = ui.y >= Q.lv[0].qin && uo.y >= Q.lv[0].qout;
+                }
+                const unsigned m = __ballot_sync(kFullMask, pass);
+                __syncwarp();
+                if (pass) c.S->buf[0][__popc(m & ((1u << lane) - 1))] = u;
+                if (lane == 0) c.S->nb[0] = __popc(m);
+                __syncwarp();
+                if (m && counts_next(Q, 0)) {
+                    qcount += count_frontier(c, 0);
+                } else {
+                    const uint32_t nr = __popc(m);
+                    for (uint32_t i = 0; i < nr && !abandoned && !dropped; ++i) {
+                        __syncwarp();
+                        if (lane == 0) c.S->m[0] = c.S->buf[0][i];
+                        __syncwarp();
+                        enter_level(c, 1);
+                        subtree();
+                    }
+                }
+                __syncwarp();
+            } else {
+                uint32_t lo = 0, hi = Q.heavy_roots - 1;  // root: last j with pref[j] <= local
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi + 1) >> 1;
+                    if (pref[mid] <= local) lo = mid; else hi = mid - 1;
+                }
+                const uint32_t u = vsorted[lo];
+                const uint32_t r = uint32_t(local - pref[lo]);
+                const uint2 uo = g.out_info[u], ui = g.in_info[u];
+                if (ui.y < Q.lv[0].qin || uo.y < Q.lv[0].qout) continue;  // level-0 signature
+                if (lane == 0) c.S->m[0] = u;
+                __syncwarp();
+                // level 1: joins all on position 0; the task fixes the list and range
+                enter_level(c, 1);
                 // the task space was cut on the type's list (out, in or the
                 // shorter): make that list the candidate source
                 const bool use_in = Q.type == 1 || (Q.type == 2 && ui.y < uo.y);
@@ -515,38 +590,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
                     c.S->xend[1] = max(xs, xe);
                 }
                 __syncwarp();
-            }
-            if (Q.k == 2 || (Q.k == 3 && Q.lv[1].fold)) {
-                const unsigned long long r1 = Q.k == 2 ? count_level(c, 1) : count_level_fold(c, 1);
-                if (lane == 0) qcount += r1;  // the warp's
-                continue;
-            }
-            // depth-first over levels 1..k-2, counting level k-1
-            uint32_t d = 1;
-            bool abandoned = false, dropped = false;
-            while (d >= 1) {
-                if (c.S->bi[d] < c.S->nb[d]) {
-                    if (counts_next(Q, d)) {
-                        qcount += count_frontier(c, d);
-                        __syncwarp();
-                        if (lane == 0) c.S->bi[d] = c.S->nb[d];
-                        __syncwarp();
-                    } else {
-                        descend(c, d);
-                        ++d;
-                    }
-                } else if (c.S->x[d] < c.S->xend[d]) {
-                    const unsigned long long now = global_ns();
-                    if (*vstop || now > deadline) { abandoned = true; break; }
-                    if (qlimit && reinterpret_cast<volatile unsigned long long *>(qtime)[cur] +
-                                          (now - task_start) > qlimit) {
-                        dropped = true;
-                        break;
-                    }
-                    refill(c, d);
-                } else {
-                    --d;
-                }
+                subtree();
             }
             if (abandoned && lane == 0) {
                 atomicOr(stop, 1u);
@@ -719,7 +763,15 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
             if (b.root_cnt == 0) {
                 ok = false;  // no root passes: the count is 0 without a launch
             } else {
-                tasks = g->batch_pref_host[size_t(b.type) * (n + 1) + b.root_cnt];
+                const unsigned long long *pref = g->batch_pref_host.data() + size_t(b.type) * (n + 1);
+                // the roots with several tasks each, in out-degree order (where
+                // tasks are cut on another list: all of them)
+                const size_t over = size_t(tune.grain) + 1;
+                const uint64_t longer = over < g->stats.out_ge.size() ? g->stats.out_ge[over] : 0;
+                b.heavy_roots = b.type == 0 ? uint32_t(std::min<uint64_t>(b.root_cnt, longer)) : b.root_cnt;
+                info_tasks += pref[b.root_cnt];
+                const uint32_t rpt = roots_per_task(b);
+                tasks = pref[b.heavy_roots] + (b.root_cnt - b.heavy_roots + rpt - 1) / rpt;
                 hq.push_back(b);
                 qbase.push_back(qbase.back() + tasks);
                 index.push_back(i);

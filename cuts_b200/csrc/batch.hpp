@@ -23,7 +23,7 @@ struct BQuery {
     uint32_t k;
     uint32_t type;      // level-1 candidate list: 0 out, 1 in, 2 the shorter
     uint32_t root_cnt;  // roots = the first root_cnt vertices in out-degree order
-    uint32_t pad;
+    uint32_t heavy_roots;  // those with more than one level-1 range, a prefix
 };
 
 // Launch shape picked by the autotuner (0 = default).
@@ -50,7 +50,8 @@ struct Batch {
     bool route_all = false;          // every query of 4+ vertices to the level engine
     std::vector<uint64_t> aut;       // count multiplier per query
     std::vector<unsigned long long> qbase_host;
-    unsigned long long total_tasks = 0;
+    unsigned long long total_tasks = 0;  // of the launch (32 single-range roots are one)
+    unsigned long long info_tasks = 0;   // (query, root, range) triples, as reported
     BQuery *d_queries = nullptr;
     unsigned long long *d_qbase = nullptr, *d_counts = nullptr, *d_ctr = nullptr;
     uint32_t *d_aborted = nullptr;

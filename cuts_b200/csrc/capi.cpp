@@ -638,7 +638,7 @@ int cuts_batch_set_shard(cuts_batch b, uint32_t shard, uint32_t nshards) {
 
 int cuts_batch_info(cuts_batch b, uint64_t *tasks, uint32_t *blocks) {
     if (!b) return set_error(CUTS_ERR_ARG, "null batch");
-    if (tasks) *tasks = b->b.total_tasks;
+    if (tasks) *tasks = b->b.info_tasks;
     if (blocks) *blocks = b->b.launch_blocks;
     return CUTS_OK;
 }
