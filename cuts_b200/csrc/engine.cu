@@ -2169,7 +2169,9 @@ k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big
 // to 32 parents, one per lane, puts their smaller sets into shared memory and
 // walks, for every vertex v there, the other set's window (tested in v's
 // table) or v's own neighbours (tested in the other set's list), whichever is
-// shorter, 64 a step as in k_level_flat.  Sets of more than `split` vertices
+// shorter, 64 a step as in k_level_flat.  Where both sets have kECore or more
+// vertices in the dense core, the edges there are popcounts of its bitmap rows
+// against the other set's core members.  Sets of more than `split` vertices
 // are dealt out in pieces by a second launch.  On a graph whose ids are degree
 // ranks, so that d's signature is a bound on the id.
 // What it saves is the set-up per entry of L_d: the 5-cycle on 200,003
@@ -2178,13 +2180,14 @@ k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big
 // 273 -> 45 ms, the house on 100,000 / 500,000 22 -> 18.4 ms, the 4-cycle on
 // 10,000 / 40,000 117 -> 101 us.  Bound: instruction issue (55 % of slots) and
 // L2 latency.
-enum EdgeRow : int { kECOff = 0, kECDeg, kETOff, kETDeg, kEOLo, kEOHi, kEOBase, kEOLen, kESide, kEMatched, kEdgeRows };
+constexpr uint32_t kECore = 8;    // core members of each set from which they are counted by rows
+enum EdgeRow : int { kECOff = 0, kECDeg, kETOff, kETDeg, kEOLo, kEOHi, kEOBase, kEOLen, kESide, kEMatched, kEONear, kECut, kEdgeRows };
 
 __host__ __device__ inline uint32_t edge_words(uint32_t d) {
-    return kPS + kPS / 4 + 128 + 32 + 32 * (kEdgeRows + d);
+    return kPS + kPS / 4 + 128 + 32 + kCore / 32 + 32 * (kEdgeRows + d);
 }
 
-template <bool TALLY>
+template <bool ROWS, bool TALLY>
 __global__ void __launch_bounds__(kPW * 32, 8)
 k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns, const Parents parents, uint32_t phase,
         uint32_t split, uint32_t *__restrict__ cursor, PairBig big, unsigned long long *__restrict__ acc,
@@ -2213,7 +2216,8 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
     uint32_t *const wbase = dyn + warp * edge_words(d);
     uint4 *const rec = reinterpret_cast<uint4 *>(wbase);
     uint32_t *const starts = wbase + 128;
-    uint32_t *const S = starts + 32;
+    uint32_t *const Ob = starts + 32;                          // core members of one other set
+    uint32_t *const S = Ob + kCore / 32;
     uint8_t *const So = reinterpret_cast<uint8_t *>(S + kPS);  // the member's column
     uint32_t *const row = S + kPS + kPS / 4;                   // [EdgeRow][lane]
     uint32_t *const m = row + 32 * kEdgeRows;                  // [position][lane]
@@ -2240,6 +2244,7 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
         start = __shfl_sync(kFullMask, start, 0);
         if (start >= total) break;
         uint32_t pos = 0, end = 0;  // the smaller set's candidates left, as adjacency words
+        uint32_t far = 0;           // the other set's core members
         if (uint32_t(lane) < grab && start + lane < total) {
             uint32_t q0 = pa + start + lane, ch = 0;
             if (phase2) {
@@ -2299,6 +2304,12 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
             row[32 * kEOHi + lane] = side ? hi[0] : hi[1];
             row[32 * kEOBase + lane] = side ? off[0] + s0[0] : off[1] + s0[1];
             row[32 * kEOLen + lane] = side ? nc : nt;
+            // the other set's entries below the core
+            const uint32_t ob = side ? off[0] + s0[0] : off[1] + s0[1], on = side ? nc : nt;
+            far = 0;
+            if (ROWS && g.core_bits && on >= kECore && nc && nt && __ldg(g.adj + ob + on - kECore) >= g.core0)
+                far = on - lbound(g.adj + ob, on, g.core0);
+            if (ROWS) row[32 * kEONear + lane] = on - far;
             if (nc && nt) {
                 pos = side ? off[1] + s0[1] : off[0] + s0[0];
                 end = side ? off[1] + e0[1] : off[0] + e0[0];
@@ -2359,6 +2370,33 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
                 }
             }
             __syncwarp();
+            // ---- the lanes' segments of S; from `cut` on (when short of the
+            // end) the members are rows of the core
+            uint32_t cut = ns, hi = ns;
+            if (ROWS && __any_sync(kFullMask, far >= kECore)) {
+                uint32_t lo = 0;
+                for (uint32_t n = ns; n;) {  // first member whose column is >= lane
+                    const uint32_t half = n >> 1;
+                    if (So[lo + half] < lane) { lo += half + 1; n -= half + 1; }
+                    else n = half;
+                }
+                hi = __shfl_down_sync(kFullMask, lo, 1);
+                if (lane == 31) hi = ns;
+                cut = hi;
+                if (far >= kECore && hi - lo >= kECore) {
+                    uint32_t c0 = lo;
+                    for (uint32_t n = hi - lo; n;) {
+                        const uint32_t half = n >> 1;
+                        if (S[c0 + half] < g.core0) { c0 += half + 1; n -= half + 1; }
+                        else n = half;
+                    }
+                    if (hi - c0 >= kECore) cut = c0;
+                }
+            }
+            if (ROWS) {
+                row[32 * kECut + lane] = cut;
+                __syncwarp();
+            }
             // ---- each vertex of the smaller sets with its possible partners
             for (uint32_t i0 = 0; i0 < ns; i0 += 32) {
                 const uint32_t i = i0 + lane;
@@ -2371,7 +2409,12 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
                     uint32_t a = 0, b = inf.y;  // the part of v's list that the order allows
                     if (side ? t_below : t_above) a = __ldg(g.bwd_out + v);
                     if (side ? t_above : t_below) b = __ldg(g.bwd_out + v);
-                    const uint32_t lenO = row[32 * kEOLen + ow], lenV = b - a;
+                    // a core row's partners here are those below the core,
+                    // where they are fewer than v's own neighbours
+                    const uint32_t lenV = b - a, near = ROWS ? row[32 * kEONear + ow] : 0u;
+                    const bool rowv = ROWS && i >= row[32 * kECut + ow] && near < lenV;
+                    if (rowv) So[i] = uint8_t(ow | 128u);
+                    const uint32_t lenO = rowv ? near : row[32 * kEOLen + ow];
                     mode = lenV < lenO ? 1u : 0u;
                     ilen = mode ? lenV : lenO;
                     ibase = mode ? inf.x + a : row[32 * kEOBase + ow];
@@ -2381,7 +2424,7 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
                     if (TALLY) tb += 8;
                     // the matched vertices among v's partners, taken off here
                     // rather than compared with every hit
-                    for (uint32_t k = ilen ? row[32 * kEMatched + ow] : 0u; k; k &= k - 1) {
+                    for (uint32_t k = ilen || rowv ? row[32 * kEMatched + ow] : 0u; k; k &= k - 1) {
                         const uint32_t mj = m[32 * (__ffs(k) - 1) + ow];
                         if (side ? t_below : t_above) { if (mj < v) continue; }
                         if (side ? t_above : t_below) { if (mj > v) continue; }
@@ -2444,6 +2487,46 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
                     }
                 }
                 __syncwarp();
+            }
+            // ---- rows: the core members of both sets
+            for (unsigned todo = ROWS ? __ballot_sync(kFullMask, cut < hi) : 0u; todo; todo &= todo - 1) {
+                const int l = __ffs(todo) - 1;
+                const uint32_t c0 = __shfl_sync(kFullMask, cut, l), ce = __shfl_sync(kFullMask, hi, l);
+                const uint32_t nf = __shfl_sync(kFullMask, far, l), ob = row[32 * kEOBase + l] + row[32 * kEONear + l];
+                const bool item_t = row[32 * kESide + l] != 0;
+                const bool up = item_t ? t_below : t_above, down = item_t ? t_above : t_below;
+                __syncwarp();
+                Ob[lane] = 0;
+                __syncwarp();
+                for (uint32_t i = lane; i < nf; i += 32) {
+                    const uint32_t u = __ldg(g.adj + ob + i) - g.core0;
+                    atomicOr(&Ob[u >> 5], 1u << (u & 31));
+                }
+                __syncwarp();
+                const uint32_t q0 = (__ldg(g.adj + ob) - g.core0) >> 7;  // words below the lowest member are empty
+                for (uint32_t i = c0 + lane; i < ce; i += 32) {
+                    if (!(So[i] & 128u)) continue;  // its own neighbours were walked
+                    const uint32_t u = S[i] - g.core0, w0 = u >> 5;
+                    const uint4 *rp4 = reinterpret_cast<const uint4 *>(g.core_bits + size_t(u) * (kCore / 32));
+                    uint32_t n = 0;
+                    if (!ordered) {
+                        #pragma unroll 4
+                        for (uint32_t q = q0; q < kCore / 128; ++q) {
+                            const uint4 r4 = __ldg(rp4 + q), o4 = reinterpret_cast<const uint4 *>(Ob)[q];
+                            n += __popc(r4.x & o4.x) + __popc(r4.y & o4.y) + __popc(r4.z & o4.z) + __popc(r4.w & o4.w);
+                        }
+                    } else {
+                        // partners above v, below it, or all but v itself
+                        const uint32_t own = 1u << (u & 31), ma = down ? 0u : ~(2 * own - 1), mb = up ? 0u : own - 1;
+                        const uint32_t *rw = reinterpret_cast<const uint32_t *>(rp4);
+                        for (uint32_t j = 4 * q0; j < kCore / 32; ++j) {
+                            const uint32_t msk = j == w0 ? (ma | mb) : (j > w0 ? (down ? 0u : kFullMask) : (up ? 0u : kFullMask));
+                            n += __popc(__ldg(rw + j) & Ob[j] & msk);
+                        }
+                    }
+                    local += n;
+                    if (TALLY) tb += 4 + kCore / 8;
+                }
             }
             __syncwarp();
         }
@@ -2593,7 +2676,7 @@ int launch_geometry() {
     g_pair_blocks[0] = std::max(1, b);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<true, false>, kPW * 32, 0));
     g_pair_blocks[1] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edges<false>, kPW * 32, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edges<true, false>, kPW * 32, 0));
     g_edge_blocks = std::max(1, b);
     const char *kv = std::getenv("CUTS_LEVEL_KERNEL");
     g_use_flat = !(kv && std::strcmp(kv, "warp") == 0);
@@ -3011,7 +3094,12 @@ struct Run {
                 kernel<<<grid, kPW * 32, smem, g.stream>>>(view, dp, d, flat_turns(g.max_deg), par, ph, split, cur, pb,
                                                           a1, ad, g.d_u64 + 2);
             };
-            tal ? go(k_edges<true>) : go(k_edges<false>);
+            // core rows pay where lists are longer than the core: 64 mixed
+            // queries on 200,000 vertices of up to ~1,500 neighbours 79 -> 61
+            // ms (sets of 8 core members on; 24: 69 ms), but the 5-cycle of at
+            // most 619 neighbours 48 -> 52 ms for the larger kernel
+            if (g.max_deg >= kCore) tal ? go(k_edges<true, true>) : go(k_edges<true, false>);
+            else tal ? go(k_edges<false, true>) : go(k_edges<false, false>);
         };
         phase(blocks, 1, cur1);
         CK(cudaGetLastError());
