@@ -311,13 +311,14 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
     const int np = n_params(in);
     // blocks of the training kernel, at most: one per SM
     MCK(cudaDeviceGetAttribute(&max_blocks, cudaDevAttrMultiProcessorCount, device));
-    MCK(cudaMalloc(&d_params, sizeof(float) * np * 4));  // params, grad, adam m, adam v
+    // params, grad, adam m, adam v, then (8-byte aligned) the loss partials
+    const size_t pw = (size_t(np) * 4 + 1) & ~size_t(1);
+    MCK(cudaMalloc(&d_params, sizeof(float) * pw + sizeof(double) * max_blocks));
+    d_loss = reinterpret_cast<double *>(d_params + pw);
     d_grad = d_params + np;
     d_m = d_grad + np;
     d_v = d_m + np;
     MCK(cudaMemset(d_params, 0, sizeof(float) * np * 4));
-    MCK(cudaMalloc(&d_loss, sizeof(double) * max_blocks));
-    MCK(cudaMalloc(&d_part, sizeof(float) * size_t(np) * max_blocks));
     // He-uniform initialisation from a splitmix64 stream
     std::vector<float> h(np, 0.f);
     const Layout L = layout(in);
@@ -334,10 +335,10 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
 }
 
 void Mlp::destroy() {
+    part_blocks = 0;
     if (d_params) {
         cudaSetDevice(device);
         cudaFree(d_params);
-        cudaFree(d_loss);
         cudaFree(d_part);
         cudaFree(d_X);
     }
@@ -358,6 +359,17 @@ int Mlp::upload(const float *X, const float *T, int n) {
     return CUTS_OK;
 }
 
+// Room for the partial gradients of `blocks` blocks, kept for later steps.
+int Mlp::reserve(int blocks) {
+    if (blocks <= part_blocks) return CUTS_OK;
+    cudaFree(d_part);
+    d_part = nullptr;
+    part_blocks = 0;
+    MCK(cudaMalloc(&d_part, sizeof(float) * size_t(n_params(in)) * size_t(blocks)));
+    part_blocks = blocks;
+    return CUTS_OK;
+}
+
 int Mlp::grid_for(int n) const { return std::max(1, std::min((n + kRows - 1) / kRows, max_blocks)); }
 
 // Mean of the blocks' sums of squared errors.
@@ -375,6 +387,7 @@ int Mlp::loss_grad(const float *X, const float *T, int n, float *loss, float *gr
     int rc = upload(X, T, n);
     if (rc) return rc;
     const int np = n_params(in), blocks = grid_for(n);
+    if ((rc = reserve(blocks))) return rc;
     k_mlp<true><<<blocks, kThreads, smem_bytes(in)>>>(d_params, in, d_X, d_X + size_t(cap_rows) * in, n, nullptr,
                                                      d_part, d_loss);
     k_mlp_reduce<<<(np + 31) / 32, 256>>>(d_part, blocks, np, d_grad);
@@ -394,6 +407,7 @@ int Mlp::train(const float *X, const float *T, int n, int epochs, int batch, flo
     const int np = n_params(in);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     if (batch <= 0 || batch > n) batch = n;
+    if ((rc = reserve(grid_for(batch)))) return rc;
     const float *dT = d_X + size_t(cap_rows) * in;
     for (int e = 0; e < epochs; ++e) {
         for (int s0 = 0; s0 < n; s0 += batch) {

@@ -16,7 +16,8 @@ struct Mlp {
     int in = 0;
     int device = 0;
     float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr;
-    float *d_part = nullptr;    // [max_blocks][params]: partial gradients of one step
+    float *d_part = nullptr;    // [part_blocks][params]: partial gradients of one step
+    int part_blocks = 0;
     double *d_loss = nullptr;   // [max_blocks]: partial sums of squared errors
     int max_blocks = 1;
     float *d_X = nullptr;  // staged samples: X rows, then targets / outputs
@@ -37,6 +38,7 @@ struct Mlp {
   private:
     int upload(const float *X, const float *T, int n);
     int grid_for(int n) const;
+    int reserve(int blocks);
     int read_loss(int blocks, int n, float *loss);
 };
 
