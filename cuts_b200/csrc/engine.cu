@@ -1490,7 +1490,7 @@ k_fused_scan(const unsigned long long *__restrict__ nb, uint32_t cap, const uint
 // without an order between p and c, galloping intersections): 4-clique +
 // pendant, 1M vertices / 10M edges, symmetry breaking 33.4 -> 8.2 ms; triangle
 // there, plain 75.5 -> 7.0 ms; triangle, 4M / 40M, symmetry breaking 20.2 ->
-// 9.5 ms.
+// 9.2 ms.
 constexpr int kPW = 4;            // warps per block
 constexpr uint32_t kPS = 512;     // candidates of one round, shared memory words per warp
 constexpr uint32_t kPC = 32;      // core members from which a set's core part is counted by rows
@@ -1543,6 +1543,19 @@ __device__ __forceinline__ bool pair_sig(const DevView &g, const LevelPlan &L, u
     if (!L.check_sig) return true;
     const uint32_t d = g.out_info[v].y;  // symmetric: both degrees
     return d >= L.qin && d >= L.qout;
+}
+
+// v, above a member of S of the parent in column l and in the list of its
+// join 0, is in S too.  Being above a member, v passes the lower bounds; being
+// in a list of m_j it is not m_j (no self-loops here), so only the positions
+// that P does not join (`free_pos`) are compared.
+__device__ __forceinline__ bool pair_above_in_set(const PairCtx &x, uint32_t l, uint32_t free_pos, uint32_t v) {
+    if (x.P.lt_mask && v >= x.row[32 * kRowHi + l]) return false;
+    for (uint32_t t = 1; t < x.P.nj; ++t)
+        if (!pair_list_has(x.g.tab, x.off[32 * t + l], x.deg[32 * t + l], v)) return false;
+    for (uint32_t k = free_pos; k; k &= k - 1)
+        if (x.m[32 * (__ffs(k) - 1) + l] == v) return false;
+    return !x.P.check_sig || pair_sig(x.g, x.P, v);
 }
 
 // v, known to lie in join t0 of the parent in column l, is in its S.
@@ -1768,6 +1781,8 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
         kconst = ((sF.guar_mask >> p) & 1u) == ((sF.guar_mask >> (p + 1)) & 1u);
     }
     const uint32_t orders = (o1 ? 1u : 0u) + (o2 ? 1u : 0u);
+    uint32_t free_pos = below;  // positions below p whose lists P does not join
+    for (uint32_t t = 0; t < njp; ++t) free_pos &= ~(1u << sP.jpos[t]);
 
     while (true) {
         uint32_t start = 0;
@@ -1943,7 +1958,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                 }
                 __syncwarp();
                 const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(ilive)) ? starts[lane] : kFullMask;
-                uint32_t started = 0;
+                uint32_t started = 0, hits = 0;  // hits: of a batch without weights
                 for (uint32_t fstep = 0; fstep < itotal; fstep += 64) {
                     uint4 rc[2];
                     uint32_t tv[2], rk[2];
@@ -1971,10 +1986,14 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         const uint32_t t = tv[h];
                         if (TALLY && ok) tb += 32 + ((rc[h].y & 256u) ? 4 : 0);
                         if (ok && !bucket_has(bk[h], t)) ok = tab_continue(g.tab, rc[h].z, nb[h], bu[h], bk[h], t);
-                        if (ok) {
+                        if (ok && (rc[h].y & 256u))
+                            ok = FOLD ? pair_in_set(x, rc[h].y & 255u, 0, t)
+                                      : pair_above_in_set(x, rc[h].y & 255u, free_pos, t);
+                        if (!FOLD && ts) {
+                            hits += ok;
+                        } else if (ok) {
                             const uint32_t l = rc[h].y & 255u;
-                            if (rc[h].y & 256u) ok = pair_in_set(x, l, 0, t);
-                            if (ok) {
+                            {
                                 const uint32_t av = S[rc[h].y >> 16];
                                 if (o1 && pair_adm(x, l, t)) {
                                     ++local_c;
@@ -1988,6 +2007,8 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         }
                     }
                 }
+                local += uint64_t(hits) * orders;
+                local_c += uint64_t(hits) * orders;
                 __syncwarp();
             }
             // ---- rows: the core members of the larger sets
