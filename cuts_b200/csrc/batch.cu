@@ -612,6 +612,8 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
 int batch_prepare_graph(DeviceGraph &g, uint32_t grain) {
     if (g.batch_vsorted && g.batch_grain == grain) return CUTS_OK;
     const uint32_t n = g.n;
+    const int rc = host_degrees(g);
+    if (rc) return rc;
     std::vector<uint32_t> vs(n);
     std::iota(vs.begin(), vs.end(), 0u);
     std::stable_sort(vs.begin(), vs.end(),
@@ -684,7 +686,7 @@ static bool level_engine_pays(const Query &q, bool symmetric, uint32_t flags) {
 // 18 ms in a launch of its own here and 10 ms there.
 static bool level_engine_edges(const Query &q, const DeviceGraph &g, uint32_t flags) {
     Plan plan;
-    return !g.orig.empty() && g.tab && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
+    return g.ranked && g.tab && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
 }
 
 int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_t flags_,
@@ -734,7 +736,7 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
             B.twin = L.twin;
             B.guar_mask = L.guar_mask;
             B.sig_lo = 0;
-            if (d && B.check_sig && g->symmetric && !g->orig.empty()) {
+            if (d && B.check_sig && g->symmetric && g->ranked) {
                 // degree-ranked ids: the signature is a compare of ids
                 const uint32_t deg = std::max(B.qin, B.qout);
                 B.sig_lo = n - uint32_t(deg < g->stats.out_ge.size() ? g->stats.out_ge[deg] : 0);

@@ -2819,7 +2819,8 @@ void device_graph_free(DeviceGraph *g) {
         if (g->in_info && g->in_info != g->out_info) cudaFreeAsync(g->in_info, g->stream);
         for (void *p : {static_cast<void *>(g->arena), static_cast<void *>(g->out_info),
                         static_cast<void *>(g->adj), static_cast<void *>(g->bwd_out),
-                        static_cast<void *>(g->core_bits), static_cast<void *>(g->tab)})
+                        static_cast<void *>(g->core_bits), static_cast<void *>(g->tab),
+                        static_cast<void *>(g->d_orig)})
             if (p) cudaFreeAsync(p, g->stream);
         cudaStreamSynchronize(g->stream);
     }
@@ -3316,7 +3317,7 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     // levels k-2 and k-1 as edges between two candidate sets, where the id
     // bounds stand for k-2's signature (degree-ranked ids) and the lists have
     // tables
-    bool edges = counting && !fuse && g_use_flat && !g.orig.empty() && edges_shape(hp->plan);
+    bool edges = counting && !fuse && g_use_flat && g.ranked && edges_shape(hp->plan);
     if (edges) {
         if ((rc = device_tables(g))) return rc;
         edges = g.tab != nullptr;
@@ -3326,7 +3327,7 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     // on a symmetric graph with degree-ranked ids the vertices of degree d or
     // more are a suffix of the ids: the signature is a compare of ids, not a
     // gather of the candidate's degree
-    if (g.symmetric && !g.orig.empty())
+    if (g.symmetric && g.ranked)
         for (uint32_t i = 1; i < k; ++i) {
             LevelPlan &L = hp->plan.lv[i];
             if (!L.check_sig) continue;
@@ -3674,6 +3675,7 @@ int device_dump(DeviceGraph &g, const Query &q, const char *path, uint64_t *line
     uint64_t cap = 0;
     rc = prepare(g, q, CUTS_FLAG_NO_CLOSED_FORM, k, hp, dp, cap);
     if (rc) return rc;
+    if ((rc = host_orig(g))) return rc;
     CountResult res;
     Run run{g, graph_view(g), hp, dp, k, cap, 4, false, res};
     run.dump = true;

@@ -57,8 +57,11 @@ struct DeviceGraph {
     uint32_t *h_bounds = nullptr;          // pinned
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     DegreeStats stats;                     // degree tails, for order features
-    std::vector<uint32_t> h_out_deg, h_in_deg;  // by device id
-    std::vector<uint32_t> orig;            // device id -> host vertex (empty: the same)
+    bool ranked = false;                   // device ids are degree ranks (else the host's ids)
+    uint32_t *d_orig = nullptr;            // device id -> host vertex, when ranked
+    // host copies, fetched by the first caller that needs them
+    std::vector<uint32_t> h_out_deg, h_in_deg;  // by device id (host_degrees)
+    std::vector<uint32_t> orig;            // (host_orig; empty when ids are the host's)
 
     // batched engine: vertices in out-degree order and task prefix sums
     uint32_t *batch_vsorted = nullptr;
@@ -79,6 +82,8 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
 // Builds g.tab on g.stream, once; leaves it null (lists are searched
 // instead) when the device cannot hold it.
 int device_tables(DeviceGraph &g);
+int host_degrees(DeviceGraph &g);
+int host_orig(DeviceGraph &g);
 void device_graph_free(DeviceGraph *g);
 
 struct CountResult {

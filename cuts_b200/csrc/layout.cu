@@ -483,6 +483,47 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
         LCK(cudaMemcpyAsync(d_ioff, in_off, sizeof(uint64_t) * (size_t(n) + 1), cudaMemcpyHostToDevice, s));
         if (m) LCK(cudaMemcpyAsync(d_iadj, in_adj, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, s));
     }
+    // host-side tables, while the copies and the first kernels run: the
+    // largest degree, degree tails, padded words.  An offset pair that the
+    // validation below will refuse counts as an empty list.
+    auto host_deg = [&](const uint64_t *off, uint32_t v) {
+        return off[v + 1] >= off[v] && off[v + 1] <= m ? uint32_t(off[v + 1] - off[v]) : 0u;
+    };
+    const uint64_t *const ioff_host = in_off ? in_off : out_off;  // without in-lists: symmetric, or refused below
+    uint32_t maxd = 0;
+    uint64_t w0 = 0, w1 = 0;
+    #pragma omp parallel for reduction(max : maxd) reduction(+ : w0, w1) schedule(static)
+    for (int64_t v = 0; v < int64_t(n); ++v) {
+        const uint32_t o = host_deg(out_off, uint32_t(v)), i = in_off ? host_deg(in_off, uint32_t(v)) : o;
+        maxd = std::max(maxd, std::max(o, i));
+        w0 += (uint64_t(o) + 3) & ~uint64_t(3);
+        w1 += (uint64_t(i) + 3) & ~uint64_t(3);
+    }
+    const uint64_t words_of[2] = {w0, w1};
+    DegreeStats st;
+    st.n = n;
+    st.out_ge.assign(size_t(maxd) + 2, 0);
+    st.in_ge.assign(size_t(maxd) + 2, 0);
+    // per-thread histograms while they are small (two of 8 B x (maxd + 2)
+    // per thread: 1 MB at the bound); one pass otherwise
+    #pragma omp parallel if (maxd < (1u << 16))
+    {
+        std::vector<uint64_t> lo(size_t(maxd) + 2, 0), li(size_t(maxd) + 2, 0);
+        #pragma omp for schedule(static) nowait
+        for (int64_t v = 0; v < int64_t(n); ++v) {
+            lo[host_deg(out_off, uint32_t(v))]++;
+            li[host_deg(ioff_host, uint32_t(v))]++;
+        }
+        #pragma omp critical
+        for (size_t d = 0; d < lo.size(); ++d) {
+            st.out_ge[d] += lo[d];
+            st.in_ge[d] += li[d];
+        }
+    }
+    for (int64_t d = int64_t(maxd); d >= 0; --d) {
+        st.out_ge[d] += st.out_ge[d + 1];
+        st.in_ge[d] += st.in_ge[d + 1];
+    }
     uint32_t h_flag = 0;
     auto read_flag = [&]() -> int {
         LCK(cudaMemcpyAsync(&h_flag, d_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -527,12 +568,7 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
 
     // degree ranks (CUTS_NO_RELABEL=1 keeps host ids); the per-list sort
     // indexes words with int, so a layout of 2^31 words or more keeps them too
-    uint64_t pre_words = 0;
-    for (int dir = 0; dir < (symmetric ? 1 : 2); ++dir) {
-        const uint64_t *off = dir ? in_off : out_off;
-        #pragma omp parallel for reduction(+ : pre_words) schedule(static)
-        for (int64_t v = 0; v < int64_t(n); ++v) pre_words += (off[v + 1] - off[v] + 3) & ~uint64_t(3);
-    }
+    uint64_t pre_words = words_of[0] + (symmetric ? 0 : words_of[1]);
     const char *nr = std::getenv("CUTS_NO_RELABEL");
     const bool relabel = !(nr && nr[0] == '1') && n > 1 && pre_words < (uint64_t(1) << 31);
     uint32_t *d_orig = nullptr, *d_rank = nullptr;
@@ -540,7 +576,8 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
         unsigned long long *k0 = nullptr, *k1 = nullptr;
         LCK(sc.get(&k0, n));
         LCK(sc.get(&k1, n));
-        LCK(sc.get(&d_orig, n));
+        LCK(cudaMallocAsync(reinterpret_cast<void **>(&g.d_orig), sizeof(uint32_t) * n, s));
+        d_orig = g.d_orig;
         LCK(sc.get(&d_rank, n));
         k_keys<<<grid, 256, 0, s>>>(n, d_ooff, ioff_used, k0);
         LCK(cudaGetLastError());
@@ -607,7 +644,7 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
             LCK(cudaMemsetAsync(d_flag, 0, sizeof(uint32_t), s));  // here: lists queued
             k_fill<<<std::max<uint32_t>(1, std::min<uint32_t>((n + 255) / 256, 148u * 8)), 256, 0, s>>>(
                 n, d_orig, d_rank, off, src, info, fill, d_queue, d_flag);
-            k_fill_long<<<148 * 4, 512, 0, s>>>(d_orig, d_rank, off, src, info, fill, d_queue, d_flag);
+            if (maxd > kLongList) k_fill_long<<<148 * 4, 512, 0, s>>>(d_orig, d_rank, off, src, info, fill, d_queue, d_flag);
         }
         LCK(cudaGetLastError());
     }
@@ -652,53 +689,38 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
     g.n = n;
     g.arcs = m;
 
-    // host-side tables: the id map, degrees by device id, degree tails
-    std::vector<uint32_t> orig;
-    if (relabel) {
-        orig.resize(n);
-        LCK(cudaMemcpyAsync(orig.data(), d_orig, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
-        LCK(cudaStreamSynchronize(s));
-    }
-    auto odeg = [&](uint32_t v) { return uint32_t(out_off[v + 1] - out_off[v]); };
-    auto ideg = [&](uint32_t v) { return symmetric ? odeg(v) : uint32_t(in_off[v + 1] - in_off[v]); };
-    uint32_t maxd = 0;
-    #pragma omp parallel for reduction(max : maxd) schedule(static)
-    for (int64_t v = 0; v < int64_t(n); ++v) maxd = std::max(maxd, std::max(odeg(uint32_t(v)), ideg(uint32_t(v))));
     g.max_deg = maxd;
-    g.h_out_deg.resize(n);
-    g.h_in_deg.resize(n);
-    #pragma omp parallel for schedule(static)
-    for (int64_t d = 0; d < int64_t(n); ++d) {
-        const uint32_t v = relabel ? orig[size_t(d)] : uint32_t(d);
-        g.h_out_deg[size_t(d)] = odeg(v);
-        g.h_in_deg[size_t(d)] = ideg(v);
-    }
-    DegreeStats st;
-    st.n = n;
-    st.out_ge.assign(size_t(maxd) + 2, 0);
-    st.in_ge.assign(size_t(maxd) + 2, 0);
-    // per-thread histograms while they are small (two of 8 B x (maxd + 2)
-    // per thread: 1 MB at the bound); one pass otherwise
-    #pragma omp parallel if (maxd < (1u << 16))
-    {
-        std::vector<uint64_t> lo(size_t(maxd) + 2, 0), li(size_t(maxd) + 2, 0);
-        #pragma omp for schedule(static) nowait
-        for (int64_t v = 0; v < int64_t(n); ++v) {
-            lo[odeg(uint32_t(v))]++;
-            li[ideg(uint32_t(v))]++;
-        }
-        #pragma omp critical
-        for (size_t d = 0; d < lo.size(); ++d) {
-            st.out_ge[d] += lo[d];
-            st.in_ge[d] += li[d];
-        }
-    }
-    for (int64_t d = int64_t(maxd); d >= 0; --d) {
-        st.out_ge[d] += st.out_ge[d + 1];
-        st.in_ge[d] += st.in_ge[d + 1];
-    }
     g.stats = std::move(st);
+    g.ranked = relabel;
+    return CUTS_OK;
+}
+
+// The id map on the host (dumps), fetched once.
+int host_orig(DeviceGraph &g) {
+    if (!g.ranked || !g.orig.empty()) return CUTS_OK;
+    std::vector<uint32_t> orig(g.n);
+    LCK(cudaMemcpyAsync(orig.data(), g.d_orig, sizeof(uint32_t) * g.n, cudaMemcpyDeviceToHost, g.stream));
+    LCK(cudaStreamSynchronize(g.stream));
     g.orig.swap(orig);
+    return CUTS_OK;
+}
+
+// Degrees by device id on the host (the batched engine's task table, a
+// directed graph's membership tables), fetched once.
+int host_degrees(DeviceGraph &g) {
+    if (!g.h_out_deg.empty() || !g.n) return CUTS_OK;
+    std::vector<uint2> info(g.n);
+    std::vector<uint32_t> deg[2];
+    for (int dir = 0; dir < (g.symmetric ? 1 : 2); ++dir) {
+        LCK(cudaMemcpyAsync(info.data(), dir ? g.in_info : g.out_info, sizeof(uint2) * g.n, cudaMemcpyDeviceToHost,
+                            g.stream));
+        LCK(cudaStreamSynchronize(g.stream));
+        deg[dir].resize(g.n);
+        #pragma omp parallel for schedule(static)
+        for (int64_t d = 0; d < int64_t(g.n); ++d) deg[dir][size_t(d)] = info[size_t(d)].y;
+    }
+    g.h_in_deg = g.symmetric ? deg[0] : std::move(deg[1]);
+    g.h_out_deg = std::move(deg[0]);
     return CUTS_OK;
 }
 
@@ -715,14 +737,17 @@ int device_tables(DeviceGraph &g) {
         return CUTS_OK;
     }
     const int dirs = g.symmetric ? 1 : 2;
-    auto deg = [&](uint32_t d) {
-        return uint64_t(g.h_out_deg[d]) + (g.symmetric ? 0u : g.h_in_deg[d]);
-    };
+    if (!g.symmetric) {
+        const int rc = host_degrees(g);
+        if (rc) return rc;
+    }
+    auto deg = [&](uint32_t d) { return uint64_t(g.h_out_deg[d]) + g.h_in_deg[d]; };
     // ids are degree ranks (unless relabelling is off: then every list goes
     // to the first kernel), so the lists of more than L entries are a suffix
     auto longer = [&](uint64_t L) {
         uint32_t lo = 0, hi = g.n;
-        if (g.orig.empty()) return g.n;
+        if (!g.ranked) return g.n;
+        if (g.symmetric) return g.n - uint32_t(L + 1 < g.stats.out_ge.size() ? g.stats.out_ge[L + 1] : 0);
         while (lo < hi) {
             const uint32_t mid = lo + (hi - lo) / 2;
             if (deg(mid) <= L) lo = mid + 1; else hi = mid;
@@ -740,11 +765,12 @@ int device_tables(DeviceGraph &g) {
         if (h2 > h1) k_tables_hub<<<std::min<uint32_t>(h2 - h1, 148u), 1024, kBig * 8, s>>>(h1, h2, info, g.adj, g.tab);
         if (h2 < g.n) {
             // their words are the last ones of this direction's lists
-            uint2 first = make_uint2(0, 0);
-            LCK(cudaMemcpyAsync(&first, info + h2, sizeof(first), cudaMemcpyDeviceToHost, s));
+            std::vector<uint2> hubs(g.n - h2);
+            LCK(cudaMemcpyAsync(hubs.data(), info + h2, sizeof(uint2) * hubs.size(), cudaMemcpyDeviceToHost, s));
             LCK(cudaStreamSynchronize(s));
+            const uint2 first = hubs[0];
             uint64_t words = 0;
-            for (uint32_t d = h2; d < g.n; ++d) words += (uint64_t(dir ? g.h_in_deg[d] : g.h_out_deg[d]) + 3) & ~uint64_t(3);
+            for (const uint2 &h : hubs) words += (uint64_t(h.y) + 3) & ~uint64_t(3);
             LCK(cudaMemsetAsync(g.tab + 2 * size_t(first.x), 0xff, 8 * words, s));
             k_tables_long<<<148 * 8, 256, 0, s>>>(h2, g.n, (g.max_deg + 511) / 512, info, g.adj, g.tab);
         }
