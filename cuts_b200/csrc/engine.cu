@@ -1489,7 +1489,7 @@ k_fused_scan(const unsigned long long *__restrict__ nb, uint32_t cap, const uint
 // warp, a hash table of S in shared memory and a degree gather per pair (and,
 // without an order between p and c, galloping intersections): 4-clique +
 // pendant, 1M vertices / 10M edges, symmetry breaking 33.4 -> 8.2 ms; triangle
-// there, plain 75.5 -> 7.0 ms; triangle, 4M / 40M, symmetry breaking 20.2 ->
+// there, plain 75.5 -> 6.2 ms; triangle, 4M / 40M, symmetry breaking 20.2 ->
 // 9.2 ms.
 constexpr int kPW = 4;            // warps per block
 constexpr uint32_t kPS = 512;     // candidates of one round, shared memory words per warp
@@ -3267,6 +3267,14 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     std::memset(hp, 0, sizeof(RunParams));
     int rc = build_plan(q, g.symmetric, flags, hp->plan);
     if (rc) return rc;
+    // the arena before the membership tables: these do without memory
+    if (!g.arena) {
+        cudaError_t e = cudaMallocAsync(&g.arena, g.arena_bytes, g.stream);
+        if (e != cudaSuccess) {
+            g.arena = nullptr;
+            return set_error(CUTS_ERR_NOMEM, "arena allocation failed: " + std::string(cudaGetErrorString(e)));
+        }
+    }
     const bool counting = stored == k - 1;
     const char *nf = std::getenv("CUTS_NO_FUSE");  // 1 = fusion off process-wide (A/B comparisons)
     const bool env_nofuse = nf && nf[0] == '1';
@@ -3349,13 +3357,6 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     // before a fused count of levels p = cl - 1 and cl, the entries of
     // level p - 1 record where their vertex sits in its list
     hp->pos_lvl = (fuse && cl >= 3) ? cl - 2 : 0xffffffffu;
-    if (!g.arena) {
-        cudaError_t e = cudaMallocAsync(&g.arena, g.arena_bytes, g.stream);
-        if (e != cudaSuccess) {
-            g.arena = nullptr;
-            return set_error(CUTS_ERR_NOMEM, "arena allocation failed: " + std::string(cudaGetErrorString(e)));
-        }
-    }
     // L_0: vert + ub (n entries each); L_1..L_{stored-1}: vert + par + ub
     const uint64_t n = g.n;
     const uint64_t l0_bytes = ((8 * n + 255) / 256) * 256 + 256;

@@ -6,10 +6,13 @@
 // the predictions into a work estimate and keeps the cheapest order.
 //
 // Training is full-batch or mini-batch Adam on the mean squared error: two
-// launches per step (k_mlp_grad, k_mlp_adam).  Sizes are tiny (in <= 32,
-// H = 64), so a step is a few microseconds of FP32 CUDA-core work bound by
-// shared-memory latency and launches; tensor cores would mean TF32 or BF16
-// operands, less precision than the FP32 the model is kept in.
+// launches per step (k_mlp, k_mlp_adam).  Callers give and get FP32; the
+// weights, the optimiser's state and all sums are kept in FP64, so a training
+// run follows the exact one (a ReLU that flips on a rounding error changes the
+// steps after it: with FP32 sums runs of 48 steps ended up to 8e-6 from it,
+// with FP64 3e-8, for 1.73 ms instead of 1.38 for such a fit).  Sizes are tiny (in <= 32, H = 64), so a
+// step is a few microseconds of CUDA-core work bound by shared-memory latency
+// and launches; tensor cores would mean less precision.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,7 +38,7 @@ constexpr int kH = MLP_HIDDEN;
 constexpr int kMaxIn = MLP_MAX_IN;
 constexpr int kThreads = 256;
 constexpr int kRows = 32;              // samples per tile
-constexpr int kS = kH + 4;             // row stride of the 64-wide tiles in shared memory
+constexpr int kS = kH + 2;             // row stride of the 64-wide tiles in shared memory
 
 // parameter layout: W1[H][in] b1[H] W2[H][H] b2[H] W3[H] b3
 __host__ __device__ inline int n_params(int in) { return kH * in + kH + kH * kH + kH + kH + 1; }
@@ -65,25 +68,25 @@ __host__ __device__ inline Layout layout(int in) {
 // form with one shared-memory atomic per sample and weight took 260 us for
 // 4,096 rows of 16 features (forward and backward), this one 18 us (both ncu,
 // cold caches); a fit of 48 such steps and a prediction of 6,000 rows, copies
-// included, 13.33 -> 1.39 ms.  Rows of the tiles are
-// padded to 68 words, so 16-byte reads of 8 consecutive rows (W2 by unit) hit
-// 8 different bank groups.
+// included, 13.33 -> 1.39 ms in FP32 and 1.73 ms in FP64.  Rows of the tiles
+// are padded to 66 values, so 16-byte reads of 8 consecutive rows (W2 by unit)
+// hit 8 different bank groups.
 template <bool GRAD>
-__global__ void __launch_bounds__(kThreads, 2)
-k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, const float *__restrict__ T, int n,
-      float *__restrict__ Y, float *__restrict__ part, double *__restrict__ lossp) {
-    extern __shared__ __align__(16) float sm[];
+__global__ void __launch_bounds__(kThreads, 1)
+k_mlp(const double *__restrict__ params, int in, const float *__restrict__ X, const float *__restrict__ T, int n,
+      float *__restrict__ Y, double *__restrict__ part, double *__restrict__ lossp) {
+    extern __shared__ __align__(16) double sm[];
     const Layout L = layout(in);
     const int s1 = in | 1;                 // odd row stride of W1: units on different banks
-    float *W2 = sm;                        // [H][kS]
-    float *h1 = W2 + kH * kS;              // [kRows][kS]
-    float *h2 = h1 + kRows * kS;           // [kRows][kS]: layer 2, then dL/d(layer 2)
-    float *d1 = h2 + kRows * kS;           // [kRows][kS]: dL/d(layer 1)
-    float *B1 = d1 + kRows * kS;           // [H]
-    float *B2 = B1 + kH, *W3 = B2 + kH;
-    float *dy = W3 + kH;                   // [kRows]
-    float *x = dy + kRows;                 // [kRows][in]
-    float *W1 = x + kRows * kMaxIn;        // [H][s1]
+    double *W2 = sm;                        // [H][kS]
+    double *h1 = W2 + kH * kS;              // [kRows][kS]
+    double *h2 = h1 + kRows * kS;           // [kRows][kS]: layer 2, then dL/d(layer 2)
+    double *d1 = h2 + kRows * kS;           // [kRows][kS]: dL/d(layer 1)
+    double *B1 = d1 + kRows * kS;           // [H]
+    double *B2 = B1 + kH, *W3 = B2 + kH;
+    double *dy = W3 + kH;                   // [kRows]
+    double *x = dy + kRows;                 // [kRows][in]
+    double *W1 = x + kRows * kMaxIn;        // [H][s1]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     for (int i = tid; i < kH * kH; i += kThreads) W2[(i / kH) * kS + i % kH] = params[L.w2 + i];
     for (int i = tid; i < kH * in; i += kThreads) W1[(i / in) * s1 + i % in] = params[L.w1 + i];
@@ -92,24 +95,24 @@ k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, con
         B2[tid] = params[L.b2 + tid];
         W3[tid] = params[L.w3 + tid];
     }
-    const float b3 = params[L.b3];
-    const float inv_n = 1.f / float(max(n, 1));
-    float g2[4][4] = {}, g1[4][2] = {}, gv = 0.f;
+    const double b3 = params[L.b3];
+    const double inv_n = 1.0 / double(max(n, 1));
+    double g2[4][4] = {}, g1[4][2] = {}, gv = 0.0;
     double lsum = 0.0;
     for (int base = blockIdx.x * kRows; base < n; base += gridDim.x * kRows) {
         const int rows = min(kRows, n - base);
         __syncthreads();  // the weights are in; the previous tile is done with
-        for (int i = tid; i < kRows * in; i += kThreads) x[i] = i < rows * in ? X[size_t(base) * in + i] : 0.f;
+        for (int i = tid; i < kRows * in; i += kThreads) x[i] = i < rows * in ? double(X[size_t(base) * in + i]) : 0.0;
         __syncthreads();
-        float acc[2][4], z2[2][4];
+        double acc[2][4], z2[2][4];
         // layer 1: units tx + 16 q of rows ty, ty + 16
         #pragma unroll
         for (int q = 0; q < 4; ++q) acc[0][q] = acc[1][q] = B1[tx + 16 * q];
         for (int f = 0; f < in; ++f) {
-            const float xa = x[ty * in + f], xb = x[(ty + 16) * in + f];
+            const double xa = x[ty * in + f], xb = x[(ty + 16) * in + f];
             #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float w = W1[(tx + 16 * q) * s1 + f];
+                const double w = W1[(tx + 16 * q) * s1 + f];
                 acc[0][q] += w * xa;
                 acc[1][q] += w * xb;
             }
@@ -118,47 +121,49 @@ k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, con
         for (int r = 0; r < 2; ++r)
             #pragma unroll
             for (int q = 0; q < 4; ++q)
-                h1[(ty + 16 * r) * kS + tx + 16 * q] = ty + 16 * r < rows ? fmaxf(acc[r][q], 0.f) : 0.f;
+                h1[(ty + 16 * r) * kS + tx + 16 * q] = ty + 16 * r < rows ? fmax(acc[r][q], 0.0) : 0.0;
         __syncthreads();
         // layer 2
         #pragma unroll
         for (int q = 0; q < 4; ++q) acc[0][q] = acc[1][q] = B2[tx + 16 * q];
         #pragma unroll 4
-        for (int i = 0; i < kH; i += 4) {
-            const float4 a = *reinterpret_cast<const float4 *>(h1 + ty * kS + i);
-            const float4 b = *reinterpret_cast<const float4 *>(h1 + (ty + 16) * kS + i);
+        for (int i = 0; i < kH; i += 2) {
+            const double2 a = *reinterpret_cast<const double2 *>(h1 + ty * kS + i);
+            const double2 b = *reinterpret_cast<const double2 *>(h1 + (ty + 16) * kS + i);
             #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float4 w = *reinterpret_cast<const float4 *>(W2 + (tx + 16 * q) * kS + i);
-                acc[0][q] += w.x * a.x; acc[0][q] += w.y * a.y; acc[0][q] += w.z * a.z; acc[0][q] += w.w * a.w;
-                acc[1][q] += w.x * b.x; acc[1][q] += w.y * b.y; acc[1][q] += w.z * b.z; acc[1][q] += w.w * b.w;
+                const double2 w = *reinterpret_cast<const double2 *>(W2 + (tx + 16 * q) * kS + i);
+                acc[0][q] += w.x * a.x;
+                acc[0][q] += w.y * a.y;
+                acc[1][q] += w.x * b.x;
+                acc[1][q] += w.y * b.y;
             }
         }
         // output: the 16 threads of a row reduce w3 . h2
         #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            float o = 0.f;
+            double o = 0.0;
             #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                z2[r][q] = fmaxf(acc[r][q], 0.f);
+                z2[r][q] = fmax(acc[r][q], 0.0);
                 o += W3[tx + 16 * q] * z2[r][q];
             }
             #pragma unroll
             for (int d = 8; d; d >>= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
             const int row = ty + 16 * r;
             const bool valid = row < rows;
-            const float y = o + b3;
-            float e = 0.f;
-            if (valid && T) e = y - T[base + row];
-            const float de = 2.f * e * inv_n;
+            const double y = o + b3;
+            double e = 0.0;
+            if (valid && T) e = y - double(T[base + row]);
+            const double de = 2.0 * e * inv_n;
             if (tx == 0) {
-                if (valid && Y) Y[base + row] = y;
-                if (valid) lsum += double(e) * double(e);
+                if (valid && Y) Y[base + row] = float(y);
+                if (valid) lsum += e * e;
                 if (GRAD) dy[row] = de;
             }
             if (GRAD)
                 #pragma unroll
-                for (int q = 0; q < 4; ++q) h2[row * kS + tx + 16 * q] = valid ? z2[r][q] : 0.f;
+                for (int q = 0; q < 4; ++q) h2[row * kS + tx + 16 * q] = valid ? z2[r][q] : 0.0;
         }
         if constexpr (GRAD) {
             __syncthreads();
@@ -172,35 +177,37 @@ k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, con
             #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int row = ty + 16 * r;
-                const float de = dy[row];
+                const double de = dy[row];
                 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    h2[row * kS + tx + 16 * q] = row < rows && z2[r][q] > 0.f ? de * W3[tx + 16 * q] : 0.f;
+                    h2[row * kS + tx + 16 * q] = row < rows && z2[r][q] > 0.0 ? de * W3[tx + 16 * q] : 0.0;
             }
             __syncthreads();
             // dL/d(layer 1): units 4 tx .. 4 tx + 3 of rows ty, ty + 16
-            float e1[2][4] = {};
+            double e1[2][4] = {};
             #pragma unroll 4
             for (int j = 0; j < kH; ++j) {
-                const float4 w = *reinterpret_cast<const float4 *>(W2 + j * kS + 4 * tx);
-                const float a = h2[ty * kS + j], b = h2[(ty + 16) * kS + j];
-                e1[0][0] += w.x * a; e1[0][1] += w.y * a; e1[0][2] += w.z * a; e1[0][3] += w.w * a;
-                e1[1][0] += w.x * b; e1[1][1] += w.y * b; e1[1][2] += w.z * b; e1[1][3] += w.w * b;
+                const double2 w0 = *reinterpret_cast<const double2 *>(W2 + j * kS + 4 * tx);
+                const double2 w1 = *reinterpret_cast<const double2 *>(W2 + j * kS + 4 * tx + 2);
+                const double a = h2[ty * kS + j], b = h2[(ty + 16) * kS + j];
+                e1[0][0] += w0.x * a; e1[0][1] += w0.y * a; e1[0][2] += w1.x * a; e1[0][3] += w1.y * a;
+                e1[1][0] += w0.x * b; e1[1][1] += w0.y * b; e1[1][2] += w1.x * b; e1[1][3] += w1.y * b;
             }
             #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int row = ty + 16 * r;
-                const float4 z = *reinterpret_cast<const float4 *>(h1 + row * kS + 4 * tx);
-                *reinterpret_cast<float4 *>(d1 + row * kS + 4 * tx) =
-                    make_float4(z.x > 0.f ? e1[r][0] : 0.f, z.y > 0.f ? e1[r][1] : 0.f, z.z > 0.f ? e1[r][2] : 0.f,
-                                z.w > 0.f ? e1[r][3] : 0.f);
-            }
+            for (int r = 0; r < 2; ++r)
+                #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int at = (ty + 16 * r) * kS + 4 * tx + q;
+                    d1[at] = h1[at] > 0.0 ? e1[r][q] : 0.0;
+                }
             // dW2[4 ty + a][4 tx + b] over the tile's rows
-            #pragma unroll 4
+            #pragma unroll 2
             for (int r = 0; r < kRows; ++r) {
-                const float4 d = *reinterpret_cast<const float4 *>(h2 + r * kS + 4 * ty);
-                const float4 h = *reinterpret_cast<const float4 *>(h1 + r * kS + 4 * tx);
-                const float dd[4] = {d.x, d.y, d.z, d.w}, hh[4] = {h.x, h.y, h.z, h.w};
+                const double2 d0 = *reinterpret_cast<const double2 *>(h2 + r * kS + 4 * ty);
+                const double2 dd1 = *reinterpret_cast<const double2 *>(h2 + r * kS + 4 * ty + 2);
+                const double2 hh0 = *reinterpret_cast<const double2 *>(h1 + r * kS + 4 * tx);
+                const double2 hh1 = *reinterpret_cast<const double2 *>(h1 + r * kS + 4 * tx + 2);
+                const double dd[4] = {d0.x, d0.y, dd1.x, dd1.y}, hh[4] = {hh0.x, hh0.y, hh1.x, hh1.y};
                 #pragma unroll
                 for (int a = 0; a < 4; ++a)
                     #pragma unroll
@@ -209,24 +216,25 @@ k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, con
             __syncthreads();
             // dW1[4 ty + a][tx + 16 c], and the two bias gradients
             for (int r = 0; r < kRows; ++r) {
-                const float4 d = *reinterpret_cast<const float4 *>(d1 + r * kS + 4 * ty);
+                const double2 d0 = *reinterpret_cast<const double2 *>(d1 + r * kS + 4 * ty);
+                const double2 dd1 = *reinterpret_cast<const double2 *>(d1 + r * kS + 4 * ty + 2);
                 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     const int f = tx + 16 * c;
                     if (f < in) {
-                        const float v = x[r * in + f];
-                        g1[0][c] += d.x * v; g1[1][c] += d.y * v; g1[2][c] += d.z * v; g1[3][c] += d.w * v;
+                        const double v = x[r * in + f];
+                        g1[0][c] += d0.x * v; g1[1][c] += d0.y * v; g1[2][c] += dd1.x * v; g1[3][c] += dd1.y * v;
                     }
                 }
             }
             if (tid < 128) {
-                const float *src = tid < 64 ? d1 + tid : h2 + tid - 64;
+                const double *src = tid < 64 ? d1 + tid : h2 + tid - 64;
                 for (int r = 0; r < kRows; ++r) gv += src[r * kS];
             }
         }
     }
     if constexpr (GRAD) {
-        float *out = part + size_t(blockIdx.x) * L.total;
+        double *out = part + size_t(blockIdx.x) * L.total;
         #pragma unroll
         for (int a = 0; a < 4; ++a) {
             #pragma unroll
@@ -256,46 +264,46 @@ k_mlp(const float *__restrict__ params, int in, const float *__restrict__ X, con
 // Sum of the blocks' partial gradients, 32 parameters x 8 groups of blocks
 // per thread block, in FP64 and in a fixed order; the group-0 threads return
 // it.  Each thread reads nparts / 8 values, independent loads in flight.
-__device__ __forceinline__ float partial_sum(const float *__restrict__ part, int nparts, int total, int i) {
+__device__ __forceinline__ double partial_sum(const double *__restrict__ part, int nparts, int total, int i) {
     __shared__ double red[8][33];
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     double s = 0.0;
     if (i < total) {
         #pragma unroll 8
-        for (int b = grp; b < nparts; b += 8) s += double(part[size_t(b) * total + i]);
+        for (int b = grp; b < nparts; b += 8) s += part[size_t(b) * total + i];
     }
     red[grp][lane] = s;
     __syncthreads();
     s = 0.0;
     if (grp == 0)
         for (int q = 0; q < 8; ++q) s += red[q][lane];
-    return float(s);
+    return s;
 }
 
 __global__ void __launch_bounds__(256)
-k_mlp_reduce(const float *__restrict__ part, int nparts, int total, float *__restrict__ g) {
+k_mlp_reduce(const double *__restrict__ part, int nparts, int total, float *__restrict__ g) {
     const int i = blockIdx.x * 32 + (threadIdx.x & 31);
-    const float v = partial_sum(part, nparts, total, i);
-    if (threadIdx.x < 32 && i < total) g[i] = v;
+    const double v = partial_sum(part, nparts, total, i);
+    if (threadIdx.x < 32 && i < total) g[i] = float(v);
 }
 
 // Adam (Kingma & Ba 2015) with bias correction, on the summed partials.
 __global__ void __launch_bounds__(256)
-k_mlp_adam(float *__restrict__ p, const float *__restrict__ part, int nparts, float *__restrict__ m,
-           float *__restrict__ v, int total, float lr, float b1, float b2, float eps, float c1, float c2) {
+k_mlp_adam(double *__restrict__ p, const double *__restrict__ part, int nparts, double *__restrict__ m,
+           double *__restrict__ v, int total, double lr, double b1, double b2, double eps, double c1, double c2) {
     const int i = blockIdx.x * 32 + (threadIdx.x & 31);
-    const float gi = partial_sum(part, nparts, total, i);
+    const double gi = partial_sum(part, nparts, total, i);
     if (threadIdx.x < 32 && i < total) {
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+        const double mi = b1 * m[i] + (1.0 - b1) * gi;
+        const double vi = b2 * v[i] + (1.0 - b2) * gi * gi;
         m[i] = mi;
         v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        p[i] -= lr * (mi / c1) / (sqrt(vi / c2) + eps);
     }
 }
 
 size_t smem_bytes(int in) {
-    return sizeof(float) * (size_t(kH) * kS + 3 * size_t(kRows) * kS + 3 * kH + kRows + kRows * kMaxIn +
+    return sizeof(double) * (size_t(kH) * kS + 3 * size_t(kRows) * kS + 3 * kH + kRows + kRows * kMaxIn +
                             size_t(kH) * (in | 1));
 }
 
@@ -311,14 +319,12 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
     const int np = n_params(in);
     // blocks of the training kernel, at most: one per SM
     MCK(cudaDeviceGetAttribute(&max_blocks, cudaDevAttrMultiProcessorCount, device));
-    // params, grad, adam m, adam v, then (8-byte aligned) the loss partials
-    const size_t pw = (size_t(np) * 4 + 1) & ~size_t(1);
-    MCK(cudaMalloc(&d_params, sizeof(float) * pw + sizeof(double) * max_blocks));
-    d_loss = reinterpret_cast<double *>(d_params + pw);
-    d_grad = d_params + np;
-    d_m = d_grad + np;
+    // params, adam m, adam v, the loss partials, and the gradient as callers see it
+    MCK(cudaMalloc(&d_params, sizeof(double) * (size_t(np) * 3 + max_blocks) + sizeof(float) * np));
+    d_m = d_params + np;
     d_v = d_m + np;
-    MCK(cudaMemset(d_params, 0, sizeof(float) * np * 4));
+    d_loss = d_v + np;
+    d_grad = reinterpret_cast<float *>(d_loss + max_blocks);
     // He-uniform initialisation from a splitmix64 stream
     std::vector<float> h(np, 0.f);
     const Layout L = layout(in);
@@ -327,7 +333,8 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
     for (int i = 0; i < kH * in; ++i) h[L.w1 + i] = uni(std::sqrt(6.f / in));
     for (int i = 0; i < kH * kH; ++i) h[L.w2 + i] = uni(std::sqrt(6.f / kH));
     for (int i = 0; i < kH; ++i) h[L.w3 + i] = uni(std::sqrt(6.f / kH));
-    MCK(cudaMemcpy(d_params, h.data(), sizeof(float) * np, cudaMemcpyHostToDevice));
+    const int rc = set_params(h.data());
+    if (rc) return rc;
     MCK(cudaFuncSetAttribute(k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes(kMaxIn))));
     MCK(cudaFuncSetAttribute(k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes(kMaxIn))));
     step = 0;
@@ -342,8 +349,8 @@ void Mlp::destroy() {
         cudaFree(d_part);
         cudaFree(d_X);
     }
-    d_params = d_grad = d_m = d_v = d_part = d_X = nullptr;
-    d_loss = nullptr;
+    d_params = d_m = d_v = d_loss = d_part = nullptr;
+    d_grad = d_X = nullptr;
 }
 
 int Mlp::upload(const float *X, const float *T, int n) {
@@ -365,7 +372,7 @@ int Mlp::reserve(int blocks) {
     cudaFree(d_part);
     d_part = nullptr;
     part_blocks = 0;
-    MCK(cudaMalloc(&d_part, sizeof(float) * size_t(n_params(in)) * size_t(blocks)));
+    MCK(cudaMalloc(&d_part, sizeof(double) * size_t(n_params(in)) * size_t(blocks)));
     part_blocks = blocks;
     return CUTS_OK;
 }
@@ -405,7 +412,7 @@ int Mlp::train(const float *X, const float *T, int n, int epochs, int batch, flo
     int rc = upload(X, T, n);
     if (rc) return rc;
     const int np = n_params(in);
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const double b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;  // the FP32 values, as lr
     if (batch <= 0 || batch > n) batch = n;
     if ((rc = reserve(grid_for(batch)))) return rc;
     const float *dT = d_X + size_t(cap_rows) * in;
@@ -415,7 +422,7 @@ int Mlp::train(const float *X, const float *T, int n, int epochs, int batch, flo
             k_mlp<true><<<blocks, kThreads, smem_bytes(in)>>>(d_params, in, d_X + size_t(s0) * in, dT + s0, nb, nullptr,
                                                              d_part, nullptr);
             ++step;
-            const float c1 = 1.f - std::pow(b1, float(step)), c2 = 1.f - std::pow(b2, float(step));
+            const double c1 = 1.0 - std::pow(b1, double(step)), c2 = 1.0 - std::pow(b2, double(step));
             k_mlp_adam<<<(np + 31) / 32, 256>>>(d_params, d_part, blocks, d_m, d_v, np, lr, b1, b2, eps, c1, c2);
         }
     }
@@ -443,15 +450,18 @@ int Mlp::predict(const float *X, int n, float *Y) {
 
 int Mlp::get_params(float *out) {
     MCK(cudaSetDevice(device));
-    MCK(cudaMemcpy(out, d_params, sizeof(float) * n_params(in), cudaMemcpyDeviceToHost));
+    std::vector<double> h(size_t(n_params(in)));
+    MCK(cudaMemcpy(h.data(), d_params, sizeof(double) * h.size(), cudaMemcpyDeviceToHost));
+    for (size_t i = 0; i < h.size(); ++i) out[i] = float(h[i]);
     return CUTS_OK;
 }
 
 int Mlp::set_params(const float *p) {
     MCK(cudaSetDevice(device));
-    MCK(cudaMemcpy(d_params, p, sizeof(float) * n_params(in), cudaMemcpyHostToDevice));
-    const int np = n_params(in);
-    MCK(cudaMemset(d_m, 0, sizeof(float) * np * 2));
+    const size_t np = size_t(n_params(in));
+    std::vector<double> h(p, p + np);
+    h.resize(np * 3, 0.0);  // and the optimiser's state
+    MCK(cudaMemcpy(d_params, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
     step = 0;
     return CUTS_OK;
 }

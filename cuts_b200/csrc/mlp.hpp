@@ -15,8 +15,10 @@ int mlp_param_count(int in);
 struct Mlp {
     int in = 0;
     int device = 0;
-    float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr;
-    float *d_part = nullptr;    // [part_blocks][params]: partial gradients of one step
+    // weights and Adam's moments in FP64 (FP32 at the interface)
+    double *d_params = nullptr, *d_m = nullptr, *d_v = nullptr;
+    float *d_grad = nullptr;
+    double *d_part = nullptr;   // [part_blocks][params]: partial gradients of one step
     int part_blocks = 0;
     double *d_loss = nullptr;   // [max_blocks]: partial sums of squared errors
     int max_blocks = 1;
