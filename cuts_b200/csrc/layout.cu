@@ -326,7 +326,7 @@ __device__ __forceinline__ void tab_insert(uint32_t *base, uint32_t len, uint32_
 // tables of up to kTabWords list words at a time in shared memory and writes
 // them out whole -- 4 B read and 8 B written per entry, the atomics in shared
 // memory (built by compare-and-swap in global memory they took 2.3 ms for 20M
-// entries, 0.72 ms this way).  A list longer than that (ids not degree-ranked)
+// entries, 0.28 ms with the hub kernels below).  A list longer than that (ids not degree-ranked)
 // is built in place.
 constexpr uint32_t kTabWords = 1024;
 constexpr int kTabWarps = 4;
@@ -705,8 +705,8 @@ int host_orig(DeviceGraph &g) {
     return CUTS_OK;
 }
 
-// Degrees by device id on the host (the batched engine's task table, a
-// directed graph's membership tables), fetched once.
+// Degrees by device id on the host (the batched engine's task table), fetched
+// once.
 int host_degrees(DeviceGraph &g) {
     if (!g.h_out_deg.empty() || !g.n) return CUTS_OK;
     std::vector<uint2> info(g.n);
@@ -737,31 +737,30 @@ int device_tables(DeviceGraph &g) {
         return CUTS_OK;
     }
     const int dirs = g.symmetric ? 1 : 2;
-    if (!g.symmetric) {
-        const int rc = host_degrees(g);
-        if (rc) return rc;
-    }
-    auto deg = [&](uint32_t d) { return uint64_t(g.h_out_deg[d]) + g.h_in_deg[d]; };
     // ids are degree ranks (unless relabelling is off: then every list goes
-    // to the first kernel), so the lists of more than L entries are a suffix
+    // to the first kernel), so no list of the vertices below n - c has more
+    // than L entries, c being at least the number of vertices of degree above
+    // L; out- plus in-degree above L needs one of them above L / 2
     auto longer = [&](uint64_t L) {
-        uint32_t lo = 0, hi = g.n;
         if (!g.ranked) return g.n;
-        if (g.symmetric) return g.n - uint32_t(L + 1 < g.stats.out_ge.size() ? g.stats.out_ge[L + 1] : 0);
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            if (deg(mid) <= L) lo = mid + 1; else hi = mid;
-        }
-        return lo;
+        auto above = [&](const std::vector<uint64_t> &ge, uint64_t d) { return d + 1 < ge.size() ? uint64_t(ge[d + 1]) : 0; };
+        const uint64_t c = g.symmetric ? above(g.stats.out_ge, L) : above(g.stats.out_ge, L / 2) + above(g.stats.in_ge, L / 2);
+        return g.n - uint32_t(std::min<uint64_t>(c, g.n));
     };
-    constexpr uint32_t kMid = 4096, kBig = 24576;  // 32 KB and 192 KB of shared memory
-    const uint32_t h0 = longer(kTabWords), h1 = longer(kMid), h2 = longer(kBig);
+    // classes of list lengths: 32 vertices per warp; one block per list with 8,
+    // 32 and 192 KB of shared memory; in place.  The first ends at 128: with
+    // 1,024, 32 neighbouring lists of 500 were a warp's 16 rounds and the build's
+    // tail (20M arcs: build 0.71 ms, 0.28 this way; the first count on 30,000
+    // vertices / 100,000 edges 315 us, 245 this way)
+    constexpr uint32_t kShort = 128, kMid = 4096, kBig = 24576;
+    const uint32_t h0 = longer(kShort), hm = longer(kTabWords), h1 = longer(kMid), h2 = longer(kBig);
     LCK(cudaFuncSetAttribute(k_tables_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBig * 8)));
     for (int dir = 0; dir < dirs; ++dir) {
         const uint2 *info = dir ? g.in_info : g.out_info;
         k_tables<<<std::max<uint32_t>(1, std::min<uint32_t>((h0 + 127) / 128, 148u * 7)), kTabWarps * 32, 0, s>>>(
             h0, info, g.adj, g.tab);
-        if (h1 > h0) k_tables_hub<<<std::min<uint32_t>(h1 - h0, 148u * 6), 256, kMid * 8, s>>>(h0, h1, info, g.adj, g.tab);
+        if (hm > h0) k_tables_hub<<<std::min<uint32_t>(hm - h0, 148u * 16), 128, kTabWords * 8, s>>>(h0, hm, info, g.adj, g.tab);
+        if (h1 > hm) k_tables_hub<<<std::min<uint32_t>(h1 - hm, 148u * 6), 256, kMid * 8, s>>>(hm, h1, info, g.adj, g.tab);
         if (h2 > h1) k_tables_hub<<<std::min<uint32_t>(h2 - h1, 148u), 1024, kBig * 8, s>>>(h1, h2, info, g.adj, g.tab);
         if (h2 < g.n) {
             // their words are the last ones of this direction's lists
