@@ -559,7 +559,7 @@ def main():
                 ex_ms += r.expand_ms
                 lv, _ = q.plan_levels(sym, args.flags)
                 fused = any(x["fuse"] for x in lv) and os.environ.get("CUTS_NO_FUSE") != "1"
-                kinds.append(f"{'k_fused' if fused else 'k_level_flat'}<count> ({name})")
+                kinds.append(f"{'k_pairs' if fused else 'counting kernel'} ({name})")
             achieved = (ll_bytes / max(ll_n, 1)) / ((ll_ms / max(ll_n, 1)) / 1e3) / 1e9 if ll_ms else None
             roofline.update({
                 "kernel": "last counted level: " + ", ".join(kinds),

@@ -508,7 +508,7 @@ class Graph:
 
 
 class Mlp:
-    """FP32 MLP cost model (in -> 64 -> 64 -> 1) resident on one GPU."""
+    """MLP cost model (in -> 64 -> 64 -> 1) resident on one GPU."""
 
     def __init__(self, in_dim: int = FEATURES, seed: int = 0, device: int = 0):
         h = _vp()

@@ -1,4 +1,4 @@
-// mlp.cu -- the learned matching-order cost model: a small FP32 MLP
+// mlp.cu -- the learned matching-order cost model: a small MLP (FP32 at its interface, FP64 inside)
 // (in -> H -> H -> 1, ReLU) trained and evaluated by hand-written kernels.
 //
 // It predicts log(1 + |L_i|), the size of trie level i, from per-step

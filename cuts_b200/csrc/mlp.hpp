@@ -1,4 +1,4 @@
-// mlp.hpp -- FP32 MLP cost model for the learned matching order.
+// mlp.hpp -- MLP cost model for the learned matching order.
 #pragma once
 #include <cstdint>
 

@@ -9,7 +9,7 @@ seeded training queries; on large graphs each run covers a root stripe
 (u % stride == 0) and its level sizes are scaled by the stride, which is
 an unbiased estimate because the stripes partition every level.
 
-The model is trained by the engine's own FP32 kernels (cuts_mlp_train) and
+The model is trained by the engine's own kernels (cuts_mlp_train) and
 used by cuts_plan(..., CUTS_ORDER_LEARNED, ...), which keeps the score order
 whenever the model does not promise enough saving.
 """

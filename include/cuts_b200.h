@@ -258,7 +258,7 @@ int cuts_search(const char *query_file, const char *data_file, int write_to_disk
 
 /* ---- learned matching order ---------------------------------------- */
 
-/* The cost model of the learned order: an FP32 MLP in -> 64 -> 64 -> 1
+/* The cost model of the learned order: an MLP in -> 64 -> 64 -> 1
  * (ReLU) predicting log(1 + |L_i|) from per-step order features, trained and
  * evaluated by this library's own kernels.  No reference counterpart: the
  * reference has only the greedy score order (graph.cpp:62-93). */
