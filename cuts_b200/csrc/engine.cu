@@ -1497,6 +1497,16 @@ constexpr uint32_t kPC = 32;      // core members from which a set's core part i
 constexpr uint32_t kPK = 64;      // candidates per piece of a deferred parent
 constexpr uint32_t kPG = 1024;    // candidates a warp keeps of the root parents it took
 
+// True when phase 1 leaves a parent with a window of `len` candidates to phase
+// 2: one longer than the split, or, of root parents (p = 1: their sets need no
+// tests, so pieces repeat none), one that takes what the warp keeps of a turn,
+// `before` candidates up to and with this one, past kPG -- neighbouring hubs
+// would be the launch's tail.  The host asks with the longest list and a whole
+// turn of them whether phase 2 has to be launched: the rule grows with both.
+__host__ __device__ inline bool pair_defers(uint32_t p, uint32_t split, uint32_t len, uint64_t before) {
+    return len > split || (p == 1 && before > kPG && len >= kPK / 4);
+}
+
 struct PairBig {
     unsigned long long *n;  // [0] deferred parents
     uint32_t *q;            // parent index in L_{p-1}
@@ -1817,9 +1827,6 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             }
         }
         if (!phase2) {
-            // long windows, and of root parents (whose sets need no tests, so
-            // pieces repeat none) all beyond kPG candidates of this warp, are
-            // dealt out in pieces: neighbouring hubs would be the launch's tail
             uint32_t before = 0;
             if (p == 1) {
                 before = end - pos;
@@ -1829,7 +1836,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                     if (lane >= o) before += y;
                 }
             }
-            if (end - pos > split || (before > kPG && end != pos && end - pos >= kPK / 4)) {
+            if (pair_defers(p, split, end - pos, before)) {
                 piece = true;
                 const unsigned long long slot = atomicAdd(&big.n[0], 1ull);
                 if (slot < big.cap) {
@@ -3036,8 +3043,7 @@ struct Run {
             phase(blocks, 1, cur1);
             CK(cudaGetLastError());
             res.launches++;
-            // no parent can be deferred where no list is longer than the split
-            if (g.max_deg > split) {
+            if (pair_defers(p, split, g.max_deg, 32ull * g.max_deg)) {
                 k_fused_scan<<<1, 1024, 0, g.stream>>>(pb.n, pb.cap, pb.len, kPK, pb.pref);
                 k_pair_bits<false><<<full, kPW * 32, smem, g.stream>>>(view, dp, p, pb);
                 phase(full, 2, cur2);
