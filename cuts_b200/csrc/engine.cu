@@ -1508,13 +1508,34 @@ __host__ __device__ inline bool pair_defers(uint32_t p, uint32_t split, uint32_t
 }
 
 struct PairBig {
-    unsigned long long *n;  // [0] deferred parents
+    unsigned long long *n;  // [0] deferred parents, [1] their pieces
     uint32_t *q;            // parent index in L_{p-1}
     uint32_t *len;          // candidates in its window
     uint32_t *pref;         // inclusive prefix sum of pieces
     uint32_t *bits;         // per parent: core members of S, then of T (kCore / 32 words each)
     uint32_t cap;
+    uint32_t max_pieces;    // what the list may hold of pieces
 };
+
+// Pieces a list may hold: their prefix sums and phase 2's work cursor are 32
+// bits wide, and cap parents of up to max_deg candidates need not fit (262,144
+// sets of 2^20 candidates are 2^32 pieces).  CUTS_FUSE_PIECES=<n> lowers it
+// (tests use small values).
+constexpr uint32_t kMaxPieces = 1u << 31;
+
+inline uint32_t list_pieces() {
+    const char *e = std::getenv("CUTS_FUSE_PIECES");
+    return e ? uint32_t(std::min<unsigned long>(std::strtoul(e, nullptr, 10), kMaxPieces)) : kMaxPieces;
+}
+
+// A place in the list for a parent of len candidates, or kFullMask where the
+// list is full: its pieces are reserved first, in 64 bits.
+__device__ __forceinline__ uint32_t list_place(const PairBig &big, uint32_t len) {
+    const unsigned long long pieces = len / kPK + 1;
+    if (atomicAdd(&big.n[1], pieces) + pieces > big.max_pieces) return kFullMask;
+    const unsigned long long slot = atomicAdd(&big.n[0], 1ull);
+    return slot < big.cap ? uint32_t(slot) : kFullMask;
+}
 
 // Per-lane columns in shared memory, [row][lane].
 enum PairRow : int { kRowLo = 0, kRowHi, kRowLoC, kRowHiC, kRowBase, kRowFOff, kRowFDeg, kRowFLo, kRowFHi, kPairRows };
@@ -1838,8 +1859,8 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             }
             if (pair_defers(p, split, end - pos, before)) {
                 piece = true;
-                const unsigned long long slot = atomicAdd(&big.n[0], 1ull);
-                if (slot < big.cap) {
+                const uint32_t slot = list_place(big, end - pos);
+                if (slot != kFullMask) {
                     big.q[slot] = pa + start + lane;
                     big.len[slot] = end - pos;
                     end = pos;
@@ -2346,8 +2367,8 @@ k_edges(DevView g, const RunParams *__restrict__ rp, uint32_t d, uint32_t turns,
                 pos = min(pos + ch * kPK, end);
                 end = min(pos + kPK, end);
             } else if (end - pos > split) {
-                const unsigned long long slot = atomicAdd(&big.n[0], 1ull);
-                if (slot < big.cap) {  // (a full list: this warp counts it)
+                const uint32_t slot = list_place(big, end - pos);
+                if (slot != kFullMask) {  // (a full list: this warp counts it)
                     big.q[slot] = q0;
                     big.len[slot] = end - pos;
                     end = pos;
@@ -3016,6 +3037,7 @@ struct Run {
             PairBig pb;
             pb.n = bn;
             pb.cap = hp->fuse_big_cap;
+            pb.max_pieces = list_pieces();
             pb.q = hp->fuse_big;
             pb.len = pb.q + pb.cap;
             pb.pref = pb.len + pb.cap;
@@ -3094,6 +3116,7 @@ struct Run {
         PairBig pb;
         pb.n = cs ? cs->big : g.d_u64 + kU64Big;
         pb.cap = hp->fuse_big_cap;
+        pb.max_pieces = list_pieces();
         pb.q = hp->fuse_big;
         pb.len = pb.q + pb.cap;
         pb.pref = pb.len + pb.cap;
