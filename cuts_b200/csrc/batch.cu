@@ -432,7 +432,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
         unsigned long long *__restrict__ task_ctr, uint32_t *__restrict__ stop,
         unsigned long long *__restrict__ counts, uint32_t *__restrict__ aborted,
         unsigned long long budget_ns, unsigned long long *__restrict__ qtime,
-        unsigned long long qlimit, uint32_t shard, uint32_t nshards) {
+        unsigned long long qlimit, uint32_t shard, uint32_t nshards, uint32_t rshard, uint32_t nrshards) {
     __shared__ BWarp ws[kBW];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Ctx c{g, nullptr, &ws[warp], lane};
@@ -532,7 +532,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
                 if (pass) {
                     u = vsorted[ri];
                     const uint2 uo = g.out_info[u], ui = g.in_info[u];
-                    pass = ui.y >= Q.lv[0].qin && uo.y >= Q.lv[0].qout;
+                    pass = ui.y >= Q.lv[0].qin && uo.y >= Q.lv[0].qout && (nrshards == 1 || u % nrshards == rshard);
                 }
                 const unsigned m = __ballot_sync(kFullMask, pass);
                 __syncwarp();
@@ -562,6 +562,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
                 const uint32_t r = uint32_t(local - pref[lo]);
                 const uint2 uo = g.out_info[u], ui = g.in_info[u];
                 if (ui.y < Q.lv[0].qin || uo.y < Q.lv[0].qout) continue;  // level-0 signature
+                if (nrshards != 1 && u % nrshards != rshard) continue;
                 if (lane == 0) c.S->m[0] = u;
                 __syncwarp();
                 // level 1: joins all on position 0; the task fixes the list and range
@@ -643,6 +644,8 @@ int batch_prepare_graph(DeviceGraph &g, uint32_t grain) {
 }
 
 void Batch::destroy() {
+    if (spare) spare->destroy();
+    spare.reset();
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     cudaFree(d_queries);
@@ -683,10 +686,12 @@ static bool level_engine_pays(const Query &q, bool symmetric, uint32_t flags) {
 
 // True when the level engine counts q's last two levels as edges between two
 // candidate sets (k_edges): a 4-cycle on 200,000 vertices / 1.6M edges takes
-// 18 ms in a launch of its own here and 10 ms there.
+// 18 ms in a launch of its own here and 10 ms there.  Decided by graph and plan
+// alone, not by the memory that the tables found: the shards of a batch on
+// several GPUs have to take the same parts of a query.
 static bool level_engine_edges(const Query &q, const DeviceGraph &g, uint32_t flags) {
     Plan plan;
-    return g.ranked && g.tab && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
+    return g.ranked && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
 }
 
 int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_t flags_,
@@ -697,8 +702,8 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
     // CUTS_BATCH_ROUTE=0 keeps every query in the persistent launch, =2 sends
     // every query of 4+ vertices to the level engine (A/B comparisons)
     const char *rt = std::getenv("CUTS_BATCH_ROUTE");
-    route_level = !(rt && rt[0] == '0');
-    route_all = rt && rt[0] == '2';
+    route_level = !in_launch && !(rt && rt[0] == '0');
+    route_all = !in_launch && rt && rt[0] == '2';
     if (tune.grain == 0) tune.grain = 64;
     if (tune.tasks_per_grab == 0) tune.tasks_per_grab = 1;
     BCK(cudaSetDevice(g->device));
@@ -804,7 +809,8 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
 
 int Batch::capture(unsigned long long budget_ns) {
     if (exec && budget_ns == captured_budget && query_budget_ms == captured_query_budget &&
-        shard == captured_shard && nshards == captured_nshards)
+        shard == captured_shard && nshards == captured_nshards && rshard == captured_rshard &&
+        nrshards == captured_nrshards)
         return CUTS_OK;
     if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
     if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
@@ -831,7 +837,7 @@ int Batch::capture(unsigned long long budget_ns) {
             graph_view(*g), d_queries, nb, d_qbase, g->batch_vsorted,
             pref, g->symmetric ? pref : pref + stride, g->symmetric ? pref : pref + 2 * stride, tune.grain,
             tune.tasks_per_grab, d_ctr, reinterpret_cast<uint32_t *>(d_ctr + 1), d_counts, d_aborted,
-            budget_ns, d_qtime, qlimit, shard, nshards);
+            budget_ns, d_qtime, qlimit, shard, nshards, rshard, nrshards);
     }
     cudaMemcpyAsync(h_counts, d_counts, sizeof(unsigned long long) * std::max<uint32_t>(nb, 1),
                     cudaMemcpyDeviceToHost, s);
@@ -846,6 +852,8 @@ int Batch::capture(unsigned long long budget_ns) {
     captured_query_budget = query_budget_ms;
     captured_shard = shard;
     captured_nshards = nshards;
+    captured_rshard = rshard;
+    captured_nrshards = nrshards;
     launch_blocks = blocks;
     return CUTS_OK;
 }
@@ -875,6 +883,7 @@ int Batch::run(double budget_ms, std::vector<uint64_t> &counts, std::vector<int>
     // queries outside the batched kernel's limits, and those the level engine
     // is better at: one by one
     double left = budget_ms - t;  // of the launch's budget, where there is one
+    std::vector<uint32_t> again;  // the level engine has no room for these
     for (uint32_t i = 0; i < nq; ++i) {
         if (eligible[i] != 0 && eligible[i] != 3) continue;
         CountResult r;
@@ -891,6 +900,10 @@ int Batch::run(double budget_ms, std::vector<uint64_t> &counts, std::vector<int>
         opt.shard = shard;
         opt.nshards = nshards;
         rc = device_count(*g, *queries[i], opt, r);
+        if (eligible[i] == 3 && (rc == CUTS_ERR_CAPACITY || rc == CUTS_ERR_NOMEM)) {
+            again.push_back(i);
+            continue;
+        }
         if (rc) {
             if (eligible[i] == 3) left -= opt.budget_ms;
             status[i] = rc;
@@ -900,10 +913,48 @@ int Batch::run(double budget_ms, std::vector<uint64_t> &counts, std::vector<int>
         counts[i] = r.count;
         t += r.ms;
     }
+    if (!again.empty() && (rc = run_spare(again, budget_ms > 0 ? left : 0, counts, status, t))) return rc;
     if (ms) *ms = t;
     return CUTS_OK;
 }
 
+int Batch::run_spare(const std::vector<uint32_t> &which, double budget_ms, std::vector<uint64_t> &counts,
+                     std::vector<int> &status, float &ms) {
+    if (budget_ms < 0) {
+        for (uint32_t i : which) status[i] = CUTS_ERR_BUDGET;
+        return CUTS_OK;
+    }
+    if (!spare || spare_of != which) {
+        if (spare) spare->destroy();
+        spare = std::make_unique<Batch>();
+        spare_of.clear();
+        spare->in_launch = true;
+        std::vector<const Query *> qs;
+        for (uint32_t i : which) qs.push_back(queries[i]);
+        const int rc = spare->create(*g, qs, flags, tune);
+        if (rc) {
+            spare->destroy();
+            spare.reset();
+            return rc;
+        }
+        spare_of = which;
+    }
+    spare->set_query_budget(query_budget_ms);
+    // the shard by roots, as the level engine takes it on the other GPUs
+    spare->rshard = shard;
+    spare->nrshards = nshards;
+    std::vector<uint64_t> c;
+    std::vector<int> st;
+    float t = 0;
+    const int rc = spare->run(budget_ms, c, st, &t);
+    if (rc) return rc;
+    for (size_t j = 0; j < which.size(); ++j) {
+        counts[which[j]] = c[j];
+        status[which[j]] = st[j];
+    }
+    ms += t;
+    return CUTS_OK;
+}
 
 // ---- allocation-free entry point ---------------------------------------------
 //

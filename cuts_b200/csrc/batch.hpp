@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
 #include "engine.hpp"
@@ -64,8 +65,14 @@ struct Batch {
     unsigned long long captured_budget = ~0ull;
     double captured_query_budget = -1;
     uint32_t shard = 0, nshards = 1;  // tasks t with t % nshards == shard (one GPU of several)
-    uint32_t captured_shard = 0, captured_nshards = 0;
+    uint32_t captured_shard = 0, captured_nshards = 0, captured_rshard = 0, captured_nrshards = 0;
     uint32_t launch_blocks = 0;
+    bool in_launch = false;           // no query to the level engine that the launch can take
+    uint32_t rshard = 0, nrshards = 1;  // roots u with u % nrshards == rshard only
+    // the queries that the level engine was to count and could not (a level
+    // that fits no capacity, no arena): a launch of their own, which needs none
+    std::unique_ptr<Batch> spare;
+    std::vector<uint32_t> spare_of;
 
     int create(DeviceGraph &g, const std::vector<const Query *> &qs, uint32_t flags,
                const BatchTuning &tune);
@@ -83,6 +90,8 @@ struct Batch {
 
   private:
     int capture(unsigned long long budget_ns);
+    int run_spare(const std::vector<uint32_t> &which, double budget_ms, std::vector<uint64_t> &counts,
+                  std::vector<int> &status, float &ms);
 };
 
 // The allocation-free count (cuts_count_noalloc): graph and counts in the
