@@ -724,18 +724,9 @@ int host_degrees(DeviceGraph &g) {
     return CUTS_OK;
 }
 
-int device_tables(DeviceGraph &g) {
-    if (g.tab_tried) return CUTS_OK;
-    g.tab_tried = true;
-    if (!g.n || !g.arcs) return CUTS_OK;
-    const size_t bytes = sizeof(uint32_t) * 2 * size_t(g.adj_words);
-    if (bytes > g.tab_limit) return CUTS_OK;
+// Builds the tables at `tab`, on g.stream.
+static int build_tables(DeviceGraph &g, uint32_t *tab) {
     cudaStream_t s = g.stream;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&g.tab), bytes, s) != cudaSuccess) {
-        cudaGetLastError();
-        g.tab = nullptr;
-        return CUTS_OK;
-    }
     const int dirs = g.symmetric ? 1 : 2;
     // ids are degree ranks (unless relabelling is off: then every list goes
     // to the first kernel), so no list of the vertices below n - c has more
@@ -758,10 +749,10 @@ int device_tables(DeviceGraph &g) {
     for (int dir = 0; dir < dirs; ++dir) {
         const uint2 *info = dir ? g.in_info : g.out_info;
         k_tables<<<std::max<uint32_t>(1, std::min<uint32_t>((h0 + 127) / 128, 148u * 7)), kTabWarps * 32, 0, s>>>(
-            h0, info, g.adj, g.tab);
-        if (hm > h0) k_tables_hub<<<std::min<uint32_t>(hm - h0, 148u * 16), 128, kTabWords * 8, s>>>(h0, hm, info, g.adj, g.tab);
-        if (h1 > hm) k_tables_hub<<<std::min<uint32_t>(h1 - hm, 148u * 6), 256, kMid * 8, s>>>(hm, h1, info, g.adj, g.tab);
-        if (h2 > h1) k_tables_hub<<<std::min<uint32_t>(h2 - h1, 148u), 1024, kBig * 8, s>>>(h1, h2, info, g.adj, g.tab);
+            h0, info, g.adj, tab);
+        if (hm > h0) k_tables_hub<<<std::min<uint32_t>(hm - h0, 148u * 16), 128, kTabWords * 8, s>>>(h0, hm, info, g.adj, tab);
+        if (h1 > hm) k_tables_hub<<<std::min<uint32_t>(h1 - hm, 148u * 6), 256, kMid * 8, s>>>(hm, h1, info, g.adj, tab);
+        if (h2 > h1) k_tables_hub<<<std::min<uint32_t>(h2 - h1, 148u), 1024, kBig * 8, s>>>(h1, h2, info, g.adj, tab);
         if (h2 < g.n) {
             // their words are the last ones of this direction's lists
             std::vector<uint2> hubs(g.n - h2);
@@ -770,11 +761,38 @@ int device_tables(DeviceGraph &g) {
             const uint2 first = hubs[0];
             uint64_t words = 0;
             for (const uint2 &h : hubs) words += (uint64_t(h.y) + 3) & ~uint64_t(3);
-            LCK(cudaMemsetAsync(g.tab + 2 * size_t(first.x), 0xff, 8 * words, s));
-            k_tables_long<<<148 * 8, 256, 0, s>>>(h2, g.n, (g.max_deg + 511) / 512, info, g.adj, g.tab);
+            LCK(cudaMemsetAsync(tab + 2 * size_t(first.x), 0xff, 8 * words, s));
+            k_tables_long<<<148 * 8, 256, 0, s>>>(h2, g.n, (g.max_deg + 511) / 512, info, g.adj, tab);
         }
         LCK(cudaGetLastError());
     }
+    return CUTS_OK;
+}
+
+int device_tables(DeviceGraph &g) {
+    if (g.tab_tried) return CUTS_OK;
+    g.tab_tried = true;
+    if (!g.n || !g.arcs) return CUTS_OK;
+    const size_t bytes = sizeof(uint32_t) * 2 * size_t(g.adj_words);
+    if (bytes > g.tab_limit) return CUTS_OK;
+    uint32_t *tab = nullptr;
+    if (cudaMallocAsync(reinterpret_cast<void **>(&tab), bytes, g.stream) != cudaSuccess) {
+        cudaGetLastError();
+        return CUTS_OK;
+    }
+    // the graph has them once they are queued whole: a table built in part has
+    // no end to a search's chain of full buckets
+    struct Hold {
+        DeviceGraph &g;
+        uint32_t *tab;
+        ~Hold() {
+            if (tab) cudaFreeAsync(tab, g.stream);
+        }
+    } hold{g, tab};
+    const int rc = build_tables(g, tab);
+    if (rc) return rc;
+    hold.tab = nullptr;
+    g.tab = tab;
     return CUTS_OK;
 }
 
