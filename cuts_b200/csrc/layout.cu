@@ -485,9 +485,11 @@ int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, 
     }
     // host-side tables, while the copies and the first kernels run: the
     // largest degree, degree tails, padded words.  An offset pair that the
-    // validation below will refuse counts as an empty list.
+    // validation below will refuse counts as an empty list, and so does a list
+    // of more than n entries (not strictly sorted below n): the tails have an
+    // entry per degree.
     auto host_deg = [&](const uint64_t *off, uint32_t v) {
-        return off[v + 1] >= off[v] && off[v + 1] <= m ? uint32_t(off[v + 1] - off[v]) : 0u;
+        return off[v + 1] >= off[v] && off[v + 1] <= m && off[v + 1] - off[v] <= n ? uint32_t(off[v + 1] - off[v]) : 0u;
     };
     const uint64_t *const ioff_host = in_off ? in_off : out_off;  // without in-lists: symmetric, or refused below
     uint32_t maxd = 0;
