@@ -342,38 +342,53 @@ int Mlp::create(int in_dim, uint64_t seed, int dev) {
 }
 
 void Mlp::destroy() {
-    part_blocks = 0;
     if (d_params) {
         cudaSetDevice(device);
         cudaFree(d_params);
-        cudaFree(d_part);
-        cudaFree(d_X);
+        release();
     }
-    d_params = d_m = d_v = d_loss = d_part = nullptr;
-    d_grad = d_X = nullptr;
+    d_params = d_m = d_v = d_loss = nullptr;
+    d_grad = nullptr;
 }
 
-int Mlp::upload(const float *X, const float *T, int n) {
-    if (n > cap_rows) {
-        cudaFree(d_X);
-        d_X = nullptr;
-        cap_rows = 0;
-        MCK(cudaMalloc(&d_X, sizeof(float) * size_t(n) * (in + 2)));
-        cap_rows = n;
-    }
-    MCK(cudaMemcpy(d_X, X, sizeof(float) * size_t(n) * in, cudaMemcpyHostToDevice));
-    if (T) MCK(cudaMemcpy(d_X + size_t(cap_rows) * in, T, sizeof(float) * n, cudaMemcpyHostToDevice));
+void Mlp::release() {
+    if (d_part && pooled) cudaFreeAsync(d_part, cudaStreamLegacy);
+    else cudaFree(d_part);
+    d_part = nullptr;
+    d_X = nullptr;
+    cap_rows = part_blocks = 0;
+}
+
+// Room for the partial gradients of `blocks` blocks and for `rows` staged
+// samples, kept for later calls: one allocation for both, for a model's first
+// fit is usually its only one.  Below 2 MB from the runtime's allocator, which
+// has such blocks at hand (first fit of 500 rows x 2 epochs 0.13 ms, from the
+// pool 0.37), larger ones from the device's pool: there a program that has
+// loaded a graph has the memory already (4,096 rows, one step: 0.42 ms from
+// the runtime, 0.32 to 0.35 from the pool, 0.10 after a graph; the form with
+// shared-memory atomics, which had no partials, 0.38).
+int Mlp::reserve(int rows, int blocks) {
+    if (rows <= cap_rows && blocks <= part_blocks) return CUTS_OK;
+    rows = std::max(rows, cap_rows);
+    blocks = std::max(blocks, part_blocks);
+    release();
+    const size_t part = size_t(n_params(in)) * size_t(blocks);
+    const size_t bytes = sizeof(double) * part + sizeof(float) * size_t(rows) * (in + 2);
+    pooled = bytes >= (size_t(2) << 20);
+    if (pooled) MCK(cudaMallocAsync(reinterpret_cast<void **>(&d_part), bytes, cudaStreamLegacy));
+    else MCK(cudaMalloc(&d_part, bytes));
+    d_X = reinterpret_cast<float *>(d_part + part);
+    cap_rows = rows;
+    part_blocks = blocks;
     return CUTS_OK;
 }
 
-// Room for the partial gradients of `blocks` blocks, kept for later steps.
-int Mlp::reserve(int blocks) {
-    if (blocks <= part_blocks) return CUTS_OK;
-    cudaFree(d_part);
-    d_part = nullptr;
-    part_blocks = 0;
-    MCK(cudaMalloc(&d_part, sizeof(double) * size_t(n_params(in)) * size_t(blocks)));
-    part_blocks = blocks;
+// Stages n samples, with room for `blocks` blocks' partial gradients.
+int Mlp::upload(const float *X, const float *T, int n, int blocks) {
+    const int rc = reserve(n, blocks);
+    if (rc) return rc;
+    MCK(cudaMemcpy(d_X, X, sizeof(float) * size_t(n) * in, cudaMemcpyHostToDevice));
+    if (T) MCK(cudaMemcpy(d_X + size_t(cap_rows) * in, T, sizeof(float) * n, cudaMemcpyHostToDevice));
     return CUTS_OK;
 }
 
@@ -391,10 +406,9 @@ int Mlp::read_loss(int blocks, int n, float *loss) {
 
 int Mlp::loss_grad(const float *X, const float *T, int n, float *loss, float *grad_out) {
     MCK(cudaSetDevice(device));
-    int rc = upload(X, T, n);
-    if (rc) return rc;
     const int np = n_params(in), blocks = grid_for(n);
-    if ((rc = reserve(blocks))) return rc;
+    int rc = upload(X, T, n, blocks);
+    if (rc) return rc;
     k_mlp<true><<<blocks, kThreads, smem_bytes(in)>>>(d_params, in, d_X, d_X + size_t(cap_rows) * in, n, nullptr,
                                                      d_part, d_loss);
     k_mlp_reduce<<<(np + 31) / 32, 256>>>(d_part, blocks, np, d_grad);
@@ -409,12 +423,11 @@ int Mlp::loss_grad(const float *X, const float *T, int n, float *loss, float *gr
 int Mlp::train(const float *X, const float *T, int n, int epochs, int batch, float lr,
                float *final_loss) {
     MCK(cudaSetDevice(device));
-    int rc = upload(X, T, n);
+    if (batch <= 0 || batch > n) batch = n;
+    int rc = upload(X, T, n, grid_for(batch));
     if (rc) return rc;
     const int np = n_params(in);
     const double b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;  // the FP32 values, as lr
-    if (batch <= 0 || batch > n) batch = n;
-    if ((rc = reserve(grid_for(batch)))) return rc;
     const float *dT = d_X + size_t(cap_rows) * in;
     for (int e = 0; e < epochs; ++e) {
         for (int s0 = 0; s0 < n; s0 += batch) {
@@ -439,7 +452,7 @@ int Mlp::train(const float *X, const float *T, int n, int epochs, int batch, flo
 
 int Mlp::predict(const float *X, int n, float *Y) {
     MCK(cudaSetDevice(device));
-    int rc = upload(X, nullptr, n);
+    int rc = upload(X, nullptr, n, 0);
     if (rc) return rc;
     float *dY = d_X + size_t(cap_rows) * in;  // reuse the target slot
     k_mlp<false><<<grid_for(n), kThreads, smem_bytes(in)>>>(d_params, in, d_X, nullptr, n, dY, nullptr, nullptr);

@@ -18,8 +18,9 @@ struct Mlp {
     // weights and Adam's moments in FP64 (FP32 at the interface)
     double *d_params = nullptr, *d_m = nullptr, *d_v = nullptr;
     float *d_grad = nullptr;
-    double *d_part = nullptr;   // [part_blocks][params]: partial gradients of one step
+    double *d_part = nullptr;   // [part_blocks][params]: partial gradients of one step; d_X lies behind it
     int part_blocks = 0;
+    bool pooled = false;        // d_part comes from the device's memory pool
     double *d_loss = nullptr;   // [max_blocks]: partial sums of squared errors
     int max_blocks = 1;
     float *d_X = nullptr;  // staged samples: X rows, then targets / outputs
@@ -38,9 +39,10 @@ struct Mlp {
     int set_params(const float *p);
 
   private:
-    int upload(const float *X, const float *T, int n);
+    int upload(const float *X, const float *T, int n, int blocks);
     int grid_for(int n) const;
-    int reserve(int blocks);
+    int reserve(int rows, int blocks);
+    void release();
     int read_loss(int blocks, int n, float *loss);
 };
 
