@@ -691,7 +691,7 @@ static bool level_engine_pays(const Query &q, bool symmetric, uint32_t flags) {
 // several GPUs have to take the same parts of a query.
 static bool level_engine_edges(const Query &q, const DeviceGraph &g, uint32_t flags) {
     Plan plan;
-    return g.ranked && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
+    return g.ranked && edges_counted(flags) && !build_plan(q, g.symmetric, flags, plan) && edges_shape(plan);
 }
 
 int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_t flags_,

@@ -3288,6 +3288,12 @@ bool pairs_plan(const DeviceGraph &g, const Plan &plan, uint32_t p) {
     return !(w && w[0] == '0');
 }
 
+// CUTS_NO_FUSE=1: fusion off process-wide (A/B comparisons)
+bool no_fuse_env() {
+    const char *nf = std::getenv("CUTS_NO_FUSE");
+    return nf && nf[0] == '1';
+}
+
 // Carves the arena for `stored` levels and uploads the run parameters.
 int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, RunParams *&hp,
             RunParams *&dp, uint64_t &cap) {
@@ -3305,8 +3311,7 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         }
     }
     const bool counting = stored == k - 1;
-    const char *nf = std::getenv("CUTS_NO_FUSE");  // 1 = fusion off process-wide (A/B comparisons)
-    const bool env_nofuse = nf && nf[0] == '1';
+    const bool env_nofuse = no_fuse_env();
     if (k >= 3 && hp->plan.lv[k - 1].ofold) {
         // the orbit fold needs its weight evaluated by the flattened or the
         // fused counting kernel, in 32 bits; otherwise break Q's symmetry
@@ -3353,8 +3358,8 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
     if (fuse) stored = cl - 1;
     // levels k-2 and k-1 as edges between two candidate sets, where the id
     // bounds stand for k-2's signature (degree-ranked ids) and the lists have
-    // tables
-    bool edges = counting && !fuse && g_use_flat && g.ranked && edges_shape(hp->plan);
+    // tables; not where the caller wants level k-2 materialised
+    bool edges = counting && !fuse && edges_counted(flags) && g_use_flat && g.ranked && edges_shape(hp->plan);
     if (edges) {
         if ((rc = device_tables(g))) return rc;
         edges = g.tab != nullptr;
@@ -3611,6 +3616,8 @@ int Run::write_rows(uint32_t nout) {
     cudaFreeHost(h_rows);
     return rc;
 }
+
+bool edges_counted(uint32_t flags) { return !(flags & CUTS_FLAG_NO_FUSE) && !no_fuse_env(); }
 
 int device_count(DeviceGraph &g, const Query &q, const CountOptions &opt, CountResult &res) {
     res = CountResult();

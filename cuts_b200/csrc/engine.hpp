@@ -109,6 +109,11 @@ struct CountOptions {
     double budget_ms = 0;     // > 0: stop launching chunks after this much time
 };
 
+// True when the flags (and CUTS_NO_FUSE) let the last two levels be counted as
+// edges between two candidate sets, without materialising the one before the
+// last.
+bool edges_counted(uint32_t flags);
+
 // Counts embeddings of q (order already set) in g.  chunks >= 1 slices the
 // root level like the reference's trunks.  want_bytes adds an untimed pass
 // computing the last-level kernel's algorithmic traffic.
