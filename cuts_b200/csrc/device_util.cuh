@@ -20,7 +20,7 @@ struct DevView {
     const uint32_t *bwd_in;
     // dense core of a symmetric graph: the kCore vertices of highest id
     // (the hubs, ids being degree ranks), from core0 up; row d - core0 of
-    // core_bits (kCore / 32 words) has bit u - core0 set when d lists u.
+    // core_bits (kCore / 32 words) has bit u - core0 set when d lists u, u != d.
     // Null when absent.
     const uint32_t *core_bits;
     uint32_t core0;

@@ -1462,8 +1462,8 @@ k_fused_scan(const unsigned long long *__restrict__ nb, uint32_t cap, const uint
 
 // ---- fused count on symmetric graphs: pairs of a candidate set ----------
 // With p and c = p + 1 fused, level c is every pair (s, t) of one parent's
-// candidate set S (level p) with t in s's list.  On a symmetric graph without
-// self-loops the pairs are unordered: each {a < b} of S with b in a's list is
+// candidate set S (level p) with t in s's list.  On a symmetric graph the pairs
+// are unordered: each {a < b} of S with b in a's list is
 // found once and counted for s = a, t = b and for s = b, t = a, as far as the
 // plan's order between p and c and t's own tests (window, extra lists,
 // signature: `adm`) allow.  A pair's weight is A(s) + B(t) (1 + 0 without a
@@ -1578,8 +1578,8 @@ __device__ __forceinline__ bool pair_sig(const DevView &g, const LevelPlan &L, u
 
 // v, above a member of S of the parent in column l and in the list of its
 // join 0, is in S too.  Being above a member, v passes the lower bounds; being
-// in a list of m_j it is not m_j (no self-loops here), so only the positions
-// that P does not join (`free_pos`) are compared.
+// in a list of m_j it is not m_j unless there are self-loops, so without them
+// only the positions that P does not join (`free_pos`) are compared.
 __device__ __forceinline__ bool pair_above_in_set(const PairCtx &x, uint32_t l, uint32_t free_pos, uint32_t v) {
     if (x.P.lt_mask && v >= x.row[32 * kRowHi + l]) return false;
     for (uint32_t t = 1; t < x.P.nj; ++t)
@@ -1614,6 +1614,7 @@ __device__ __forceinline__ bool pair_adm(const PairCtx &x, uint32_t l, uint32_t 
 // A(v): the weight of v at position p, without what t adds -- the orbit base
 // with v at p minus the orbit positions below c (each of their lists holds
 // t), or the plain fold's base minus v's own membership.
+template <bool LOOPS>
 __device__ __forceinline__ uint32_t pair_a(const PairCtx &x, uint32_t l, uint32_t v) {
     if (!x.cfold) return 1;
     const LevelPlan &F = x.F;
@@ -1633,6 +1634,7 @@ __device__ __forceinline__ uint32_t pair_a(const PairCtx &x, uint32_t l, uint32_
             a += inf.y;
             for (uint32_t j = 0; j < x.p; ++j)
                 if (((F.oguar[x.p] >> j) & 1u) || pair_list_has(x.g.tab, inf.x, inf.y, x.m[32 * j + l])) --a;
+            if (LOOPS) a -= pair_list_has(x.g.tab, inf.x, inf.y, v);
         }
         return a - __popc(F.ofold & ((1u << (x.p + 1)) - 1));
     }
@@ -1643,11 +1645,16 @@ __device__ __forceinline__ uint32_t pair_a(const PairCtx &x, uint32_t l, uint32_
 
 // B(v): what v at position c adds (an orbit vertex its own list outside the
 // core; the plain fold loses v itself).  Sums wrap in 32 bits, totals do not.
+template <bool LOOPS>
 __device__ __forceinline__ uint32_t pair_b(const PairCtx &x, uint32_t l, uint32_t v) {
     if (!x.cfold) return 0;
     const LevelPlan &F = x.F;
     const uint32_t c = x.p + 1;
-    if (F.ofold) return ((F.ofold >> c) & 1u) ? x.g.out_info[v].y - c : 0u;
+    if (F.ofold) {
+        if (!((F.ofold >> c) & 1u)) return 0u;
+        const uint2 inf = x.g.out_info[v];
+        return inf.y - c - (LOOPS ? pair_list_has(x.g.tab, inf.x, inf.y, v) : 0u);
+    }
     const bool in = v >= x.row[32 * kRowFLo + l] && v < x.row[32 * kRowFHi + l] &&
                     (((F.guar_mask >> c) & 1u) || pair_list_has(x.g.tab, x.row[32 * kRowFOff + l], x.row[32 * kRowFDeg + l], v));
     return in ? 0xffffffffu : 0u;
@@ -1660,7 +1667,7 @@ struct PairParent {
 };
 
 __device__ __forceinline__ PairParent pair_parent(const DevView &g, const RunParams *rp, const LevelPlan &P,
-                                                  const LevelPlan &C, const LevelPlan &F, bool cfold, uint32_t p,
+                                                  const LevelPlan &C, const LevelPlan &F, bool cfold, bool loops, uint32_t p,
                                                   uint32_t *const *s_vert, uint32_t *const *s_par, uint32_t q0,
                                                   uint32_t lane, uint32_t *m, uint32_t *off, uint32_t *deg,
                                                   uint32_t *row) {
@@ -1696,8 +1703,8 @@ __device__ __forceinline__ PairParent pair_parent(const DevView &g, const RunPar
         const uint32_t apos = rp->ub[p - 1][q0];
         if (apos >= r.moff && apos - r.moff < mdeg) r.s0 = apos - r.moff + 1;
     }
-    if (r.s0 == kFullMask) r.s0 = lo ? lbound_own(g, false, mu, lst, mdeg, lo, false) : 0;
-    r.e0 = hi != kFullMask ? lbound_own(g, false, mu, lst, mdeg, hi, false) : mdeg;
+    if (r.s0 == kFullMask) r.s0 = lo ? lbound_own(g, false, mu, lst, mdeg, lo, loops) : 0;
+    r.e0 = hi != kFullMask ? lbound_own(g, false, mu, lst, mdeg, hi, loops) : mdeg;
     if (r.e0 < r.s0) r.e0 = r.s0;
     if (cfold && F.ofold) {
         // the orbit base of the positions below p
@@ -1775,7 +1782,8 @@ __device__ __forceinline__ PairParent pair_parent(const DevView &g, const RunPar
                     (sC.lt_mask & below) == (sP.lt_mask & below);                                             \
     const PairCtx x{g, sP, sC, sF, p, extra, cfold, ts, col_m, col_off, col_deg, row};
 
-template <bool FOLD, bool TALLY>
+// LOOPS: the graph has self-loops.
+template <bool FOLD, bool TALLY, bool LOOPS>
 __global__ void __launch_bounds__(kPW * 32, 8)
 k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents parents, uint32_t phase, uint32_t split,
         uint32_t *__restrict__ cursor, PairBig big, unsigned long long *__restrict__ acc,
@@ -1812,8 +1820,9 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
         kconst = ((sF.guar_mask >> p) & 1u) == ((sF.guar_mask >> (p + 1)) & 1u);
     }
     const uint32_t orders = (o1 ? 1u : 0u) + (o2 ? 1u : 0u);
-    uint32_t free_pos = below;  // positions below p whose lists P does not join
-    for (uint32_t t = 0; t < njp; ++t) free_pos &= ~(1u << sP.jpos[t]);
+    uint32_t free_pos = below;  // positions below p whose lists P does not join (all with self-loops)
+    if (!LOOPS)
+        for (uint32_t t = 0; t < njp; ++t) free_pos &= ~(1u << sP.jpos[t]);
 
     while (true) {
         uint32_t start = 0;
@@ -1837,7 +1846,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                 ch = gi - (b ? big.pref[b - 1] : 0);
                 q0 = big.q[b];
             }
-            pp = pair_parent(g, rp, sP, sC, sF, cfold, p, s_vert, s_par, q0, lane, col_m, col_off, col_deg, row);
+            pp = pair_parent(g, rp, sP, sC, sF, cfold, LOOPS, p, s_vert, s_par, q0, lane, col_m, col_off, col_deg, row);
             pos = pp.s0;
             end = pp.e0;
             if (TALLY) tb += 8ull * p + 8ull * njp;
@@ -1959,7 +1968,9 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         const uint32_t lenS = se == kFullMask ? kFullMask : se - i - 1;
                         if (lenS) {
                             const uint2 inf = g.out_info[a];
-                            const uint32_t bw = __ldg(g.bwd_out + a), lenN = inf.y - bw;
+                            uint32_t bw = __ldg(g.bwd_out + a);
+                            if (LOOPS && bw < inf.y && __ldg(g.adj + inf.x + bw) == a) ++bw;
+                            const uint32_t lenN = inf.y - bw;
                             if (TALLY) tb += 12;
                             mode = lenN < lenS ? 1u : 0u;
                             ilen = min(lenN, lenS);
@@ -1982,7 +1993,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                     const uint32_t r = __popc(ilive & lanemask_lt), excl = iincl - ilen;
                     rec[r] = make_uint4(ibase - excl, ow | (mode << 8) | (i << 16), ioff, ideg);
                     starts[r] = excl;
-                    if (FOLD) itemA[r] = o1 ? pair_a(x, ow, a) : 0u;
+                    if (FOLD) itemA[r] = o1 ? pair_a<LOOPS>(x, ow, a) : 0u;
                 }
                 __syncwarp();
                 const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(ilive)) ? starts[lane] : kFullMask;
@@ -2025,11 +2036,11 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                                 const uint32_t av = S[rc[h].y >> 16];
                                 if (o1 && pair_adm(x, l, t)) {
                                     ++local_c;
-                                    local += FOLD ? uint32_t(itemA[rk[h]] + pair_b(x, l, t)) : 1u;
+                                    local += FOLD ? uint32_t(itemA[rk[h]] + pair_b<LOOPS>(x, l, t)) : 1u;
                                 }
                                 if (o2 && pair_adm(x, l, av)) {
                                     ++local_c;
-                                    local += FOLD ? uint32_t(pair_a(x, l, t) + pair_b(x, l, av)) : 1u;
+                                    local += FOLD ? uint32_t(pair_a<LOOPS>(x, l, t) + pair_b<LOOPS>(x, l, av)) : 1u;
                                 }
                             }
                         }
@@ -2081,9 +2092,9 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         n2 += n;
                         if (TALLY) tb += 8 + 16ull * (kCore / 128 - q0);
                         if (FOLD) {
-                            const uint32_t B = pair_b(x, uint32_t(l), v);
+                            const uint32_t B = pair_b<LOOPS>(x, uint32_t(l), v);
                             wsum += (unsigned long long)((long long)int32_t(B) * n);
-                            if (i == c0) kap = pair_a(x, uint32_t(l), v) - B;
+                            if (i == c0) kap = pair_a<LOOPS>(x, uint32_t(l), v) - B;
                         }
                     }
                     #pragma unroll
@@ -2132,7 +2143,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         local_c += n;
                     } else {
                         const bool adm = ts || pair_adm(x, uint32_t(l), v);
-                        const uint32_t A = pair_a(x, uint32_t(l), v), B = pair_b(x, uint32_t(l), v);
+                        const uint32_t A = pair_a<LOOPS>(x, uint32_t(l), v), B = pair_b<LOOPS>(x, uint32_t(l), v);
                         // A of a vertex with a pair fits 32 bits; B is below
                         // 2^31 or, in a plain fold, -1
                         long long s = 0;
@@ -2178,8 +2189,8 @@ k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big
     for (uint32_t b = blockIdx.x * kPW + warp; b < nbig; b += gridDim.x * kPW) {
         uint32_t moff = 0, s0 = 0, e0 = 0, tmin = 0;
         if (lane == 0) {
-            const PairParent pp = pair_parent(g, rp, sP, sC, sF, false, p, s_vert, s_par, big.q[b], 0, col_m, col_off,
-                                              col_deg, row);
+            const PairParent pp = pair_parent(g, rp, sP, sC, sF, false, rp->plan.data_loops != 0, p, s_vert, s_par,
+                                              big.q[b], 0, col_m, col_off, col_deg, row);
             moff = pp.moff;
             s0 = pp.s0;
             e0 = pp.e0;
@@ -2721,9 +2732,9 @@ int launch_geometry() {
     g_fused_blocks[kCountMode] = std::max(1, b) * g_num_sms;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kBytesMode>, kZW * 32, 0));
     g_fused_blocks[kBytesMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<false, false>, kPW * 32, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<false, false, false>, kPW * 32, 0));
     g_pair_blocks[0] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<true, false>, kPW * 32, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<true, false, false>, kPW * 32, 0));
     g_pair_blocks[1] = std::max(1, b);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edges<true, false>, kPW * 32, 0));
     g_edge_blocks = std::max(1, b);
@@ -3059,8 +3070,10 @@ struct Run {
                                                           tal ? g.d_u64 + 2 : nullptr);
             };
             auto phase = [&](uint32_t grid, uint32_t ph, uint32_t *cur) {
-                if (fold) tal ? go(k_pairs<true, true>, grid, ph, cur) : go(k_pairs<true, false>, grid, ph, cur);
-                else tal ? go(k_pairs<false, true>, grid, ph, cur) : go(k_pairs<false, false>, grid, ph, cur);
+                // (the byte tally is not timed: one instance, for graphs with and without loops)
+                if (tal) fold ? go(k_pairs<true, true, true>, grid, ph, cur) : go(k_pairs<false, true, true>, grid, ph, cur);
+                else if (g.loops) fold ? go(k_pairs<true, false, true>, grid, ph, cur) : go(k_pairs<false, false, true>, grid, ph, cur);
+                else fold ? go(k_pairs<true, false, false>, grid, ph, cur) : go(k_pairs<false, false, false>, grid, ph, cur);
             };
             phase(blocks, 1, cur1);
             CK(cudaGetLastError());
@@ -3273,12 +3286,11 @@ __global__ void k_materialize(const RunParams *__restrict__ rp, uint32_t first, 
 constexpr uint32_t kDumpRows = 1u << 22;  // rows materialised per piece
 
 // True when the fused count of levels p and p + 1 runs in k_pairs: a symmetric
-// graph without self-loops (its pairs are unordered) with membership tables,
-// no list of level p + 1 on p itself beyond the pair's, and no plain fold
+// graph (its pairs are unordered) with membership tables, no list of level p + 1 on p itself beyond the pair's, and no plain fold
 // whose list or window moves with the vertex at p.  Everything else keeps
 // k_fused.  CUTS_FUSE_WALK=0 keeps k_fused always (A/B comparisons).
 bool pairs_plan(const DeviceGraph &g, const Plan &plan, uint32_t p) {
-    if (!g.symmetric || g.loops || !g.tab || g.max_deg >= (1u << 31)) return false;
+    if (!g.symmetric || !g.tab || g.max_deg >= (1u << 31)) return false;
     const LevelPlan &Lc = plan.lv[p + 1];
     const LevelPlan &Lf = plan.lv[p + 2 < plan.k ? p + 2 : p + 1];
     for (uint32_t t = 0; t < Lc.nj; ++t)
@@ -3385,7 +3397,7 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
         if (fuse && i >= stored) break;
         tests = tests || L.nj >= 2 || (counting && (L.fold || L.fold2 || L.closed_form));
     }
-    if ((tests || (fuse && g.symmetric && !g.loops)) && (rc = device_tables(g))) return rc;
+    if ((tests || (fuse && g.symmetric)) && (rc = device_tables(g))) return rc;
     hp->pairs = fuse && pairs_plan(g, hp->plan, cl - 1);
     hp->stored = stored;
     // before a fused count of levels p = cl - 1 and cl, the entries of

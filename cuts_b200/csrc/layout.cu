@@ -292,7 +292,8 @@ __global__ void k_bwd(uint32_t n, const uint2 *__restrict__ info, const uint32_t
 }
 
 // Dense core rows: one warp per core vertex d, its list entries u >= core0
-// set bit u - core0 of row d - core0 (rows are zeroed before).
+// other than d itself set bit u - core0 of row d - core0 (rows are zeroed
+// before).
 __global__ void k_core_bits(uint32_t n, uint32_t core0, const uint2 *__restrict__ info,
                             const uint32_t *__restrict__ adj, uint32_t *__restrict__ bits) {
     const uint32_t lane = threadIdx.x & 31;
@@ -303,7 +304,7 @@ __global__ void k_core_bits(uint32_t n, uint32_t core0, const uint2 *__restrict_
         const uint32_t *l = adj + inf.x;
         for (uint32_t i = lbound(l, inf.y, core0) + lane; i < inf.y; i += 32) {
             const uint32_t u = l[i] - core0;
-            atomicOr(bits + size_t(d - core0) * words + (u >> 5), 1u << (u & 31));
+            if (u != d - core0) atomicOr(bits + size_t(d - core0) * words + (u >> 5), 1u << (u & 31));
         }
     }
 }
