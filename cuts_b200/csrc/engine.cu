@@ -130,12 +130,18 @@ __device__ __forceinline__ uint32_t orbit_weight(const DevView &g, const LevelPl
 // position j <= k-3, the number of (t1, t2) with t1 in A's window of the
 // list, t2 in B's, both unmatched, t1 != t2, and -- kind 2 -- t2 above
 // (below) t1 on the same window.  O(log degree) per candidate.  Adds |A'|
-// (the level k-2 size) to lvl2.
+// (the level k-2 size) to lvl2.  The lists' own vertex is in them only where
+// there are self-loops, so a star tests nothing (3-star, 1M vertices / 10M
+// edges, plain / symmetry breaking 70 / 103 ms with its four table tests per
+// candidate, 40 / 71 without them).
 template <class M>
 __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const LevelPlan &B, uint32_t kind,
                                   uint32_t lvl, bool loops, M m, unsigned long long &lvl2) {
     const uint32_t pen = 1u << (lvl + 1);
     uint32_t lo[2], hi[2], s0[2], e0[2], off[2], len[2], cnt[2], u[2];
+    auto has = [&](int r, uint32_t guar, uint32_t j, uint32_t mj) {
+        return ((guar >> j) & 1u) || ((loops || mj != u[r]) && in_list(g, off[r], len[r], mj));
+    };
     for (int r = 0; r < 2; ++r) {
         const LevelPlan &L = r ? B : A;
         u[r] = m(L.jpos[0]);
@@ -155,7 +161,7 @@ __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const Le
         uint32_t sub = 0;
         for (uint32_t j = 0; j <= lvl; ++j) {
             const uint32_t mj = m(j);
-            if (mj >= lo[r] && mj < hi[r] && (((guar >> j) & 1u) || in_list(g, off[r], len[r], mj))) ++sub;
+            if (mj >= lo[r] && mj < hi[r] && has(r, guar, j, mj)) ++sub;
         }
         cnt[r] = e0[r] - s0[r] - sub;
     }
@@ -172,9 +178,7 @@ __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const Le
         for (uint32_t j = 0; j <= lvl; ++j) {
             const uint32_t mj = m(j);
             if (mj < wlo || mj >= whi) continue;
-            const bool in0 = ((A.guar1 >> j) & 1u) || in_list(g, off[0], len[0], mj);
-            const bool in1 = ((B.guar_mask >> j) & 1u) || in_list(g, off[1], len[1], mj);
-            if (in0 && in1) --both;
+            if (has(0, A.guar1, j, mj) && has(1, B.guar_mask, j, mj)) --both;
         }
     }
     return uint64_t(cnt[0]) * cnt[1] - both;
