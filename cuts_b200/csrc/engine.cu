@@ -132,8 +132,8 @@ __device__ __forceinline__ uint32_t orbit_weight(const DevView &g, const LevelPl
 // (below) t1 on the same window.  O(log degree) per candidate.  Adds |A'|
 // (the level k-2 size) to lvl2.  The lists' own vertex is in them only where
 // there are self-loops, so a star tests nothing (3-star, 1M vertices / 10M
-// edges, plain / symmetry breaking 70 / 103 ms with its four table tests per
-// candidate, 40 / 71 without them).
+// edges, plain / symmetry breaking 60 / 107 ms with its table tests per
+// candidate, 40 / 71 without; 21 / 38 in an instance of its own).
 template <class M>
 __device__ uint64_t pendant_pairs(const DevView &g, const LevelPlan &A, const LevelPlan &B, uint32_t kind,
                                   uint32_t lvl, bool loops, M m, unsigned long long &lvl2) {
@@ -530,11 +530,18 @@ __host__ __device__ inline uint32_t flat_words(uint32_t lvl, uint32_t nj, bool e
     return 32 * lvl + 64 * nj + 128 + 32 + (expand ? 3 * kOutBuf : 0);
 }
 
+// What a counted level counts with it, one instance each: nothing, the last
+// level by a plain or an orbit fold, both of a pendant pair, a twin.  One
+// instance with all of them behind branches in its inner loop issued three
+// times the instructions (3-path, 1M vertices / 10M edges, plain 28 -> 7.7 ms,
+// symmetry breaking 0.77 -> 0.28; 3-star above; a directed four-vertex query
+// with twins 2.8 -> 1.8).
+enum Folded { kNoFold = 0, kPlainFold, kOrbitFold, kPendants, kTwins, kFolds };
+
 // MODE kExpand writes L_lvl (adding its entries' child bounds to *acc where
 // acc is given), kCountMode counts, kBytesMode adds the bytes the
-// count reads.  FOLD: the level also counts the one or two after it (plain or
-// orbit fold, pendant pair, twins).
-template <int MODE, bool FOLD>
+// count reads (with any FOLD).
+template <int MODE, int FOLD>
 __global__ void __launch_bounds__(kFW * 32, FOLD ? 8 : 10)
 k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t turns, const Parents parents,
              uint32_t *__restrict__ cursor, uint32_t *__restrict__ out_n, uint32_t out_cap,
@@ -554,7 +561,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
         for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
             reinterpret_cast<uint32_t *>(&sL)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[lvl])[i];
             reinterpret_cast<uint32_t *>(&sN)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl])[i];
-            if (FOLD) reinterpret_cast<uint32_t *>(&sN2)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl2])[i];
+            if (FOLD == kPendants) reinterpret_cast<uint32_t *>(&sN2)[i] = reinterpret_cast<const uint32_t *>(&rp->plan.lv[nl2])[i];
         }
         if (threadIdx.x < kMaxK) {
             s_vert[threadIdx.x] = rp->vert[threadIdx.x];
@@ -576,10 +583,10 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     uint32_t *const ob_v = sm_m + 32 * lvl;                   // staged output (expand)
     uint32_t *const ob_p = ob_v + kOutBuf, *const ob_u = ob_p + kOutBuf;
     // pendant pair: this level (k-3) also counts levels k-2 and k-1
-    const uint32_t fold2 = FOLD && MODE != kExpand ? sL.fold2 : 0u;
+    const uint32_t fold2 = FOLD == kPendants ? sL.fold2 : 0u;
     // twins: this level (k-2) also counts level k-1, from each parent's number
     // of candidates (counted into `starts`' place by the parent's lane)
-    const uint32_t twin = FOLD && MODE != kExpand ? sL.twin : 0u;
+    const uint32_t twin = FOLD == kTwins ? sL.twin : 0u;
     unsigned long long local3 = 0;
     const bool store_pos = MODE == kExpand && lvl == rp->pos_lvl;
     const bool need_ub = (MODE == kExpand && lvl + 1 < rp->stored) || store_pos;
@@ -596,7 +603,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     // level k-2 counting level k-1 too: each candidate c adds the last
     // level's closed form, |window of L| - matched vertices in it, where L
     // is an earlier vertex's list and c itself is one of the matched
-    const bool fold = FOLD && MODE != kExpand && sL.fold;
+    const bool fold = MODE == kBytesMode ? sL.fold != 0 : FOLD == kPlainFold || FOLD == kOrbitFold;
     const bool fold_guar_c = fold && ((sN.guar_mask >> lvl) & 1u);
     const bool loops = rp->plan.data_loops != 0;
     // parents per warp and turn: fewer than 32 where that would leave a warp
@@ -669,7 +676,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                         const uint32_t u = sm_m[32 * sN.jpos[t] + lane];
                         ubp = min(ubp, (sN.jdir[t] ? g.in_info[u] : g.out_info[u]).y);
                     }
-            if (fold && sN.ofold) {
+            if (MODE == kBytesMode ? fold && sN.ofold : FOLD == kOrbitFold) {
                 fbase = orbit_base(g, sN, lvl, [&](uint32_t j) { return sm_m[32 * j + lane]; });
             } else if (fold) {
                 const uint32_t u = sm_m[32 * sN.jpos[0] + lane];
@@ -742,7 +749,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
         }
         __syncwarp();
         const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(live)) ? starts[lane] : kFullMask;
-        if (FOLD && twin) {
+        if (FOLD == kTwins) {
             __syncwarp();
             starts[lane] = 0;  // from here on: candidates of the lane's parent
             __syncwarp();
@@ -806,7 +813,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                     if (check_sig) ok = ci.y >= sL.qin && co.y >= sL.qout;
                 }
                 if constexpr (MODE == kCountMode) {
-                    if (twin) {
+                    if constexpr (FOLD == kTwins) {
                         // lanes of one parent are neighbours: the first of them adds
                         const unsigned m = __ballot_sync(kFullMask, ok);
                         const uint32_t up = __shfl_up_sync(kFullMask, owner, 1);
@@ -816,23 +823,26 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                         const unsigned seg = (next ? (1u << (__ffs(next) - 1)) - 1u : kFullMask) & ~lanemask_lt;
                         if (head) starts[owner] += __popc(m & seg);
                         __syncwarp();
-                    } else if (fold2) {
+                    } else if constexpr (FOLD == kPendants) {
                         if (ok) {
                             const uint64_t p2 = pendant_pairs(g, sN, sN2, fold2, lvl, loops,
                                 [&](uint32_t j) { return j == lvl ? c : sm_m[32 * j + owner]; }, local3);
                             local += p2;
                             ++local2;
                         }
-                    } else if (fold) {
+                    } else if constexpr (FOLD == kOrbitFold) {
+                        const uint32_t o_fbase = __shfl_sync(kFullMask, fbase, int(owner));
+                        if (ok) {
+                            local += orbit_weight(g, sN, lvl, o_fbase, c, loops);
+                            ++local2;
+                        }
+                    } else if constexpr (FOLD == kPlainFold) {
                         const uint32_t o_fbase = __shfl_sync(kFullMask, fbase, int(owner));
                         const uint32_t o_foff = __shfl_sync(kFullMask, f_off, int(owner));
                         const uint32_t o_fdeg = __shfl_sync(kFullMask, f_deg, int(owner));
                         const uint32_t o_flo = __shfl_sync(kFullMask, f_lo, int(owner));
                         const uint32_t o_fhi = __shfl_sync(kFullMask, f_hi, int(owner));
-                        if (ok && sN.ofold) {
-                            local += orbit_weight(g, sN, lvl, o_fbase, c, loops);
-                            ++local2;
-                        } else if (ok) {
+                        if (ok) {
                             const bool hit = c >= o_flo && c < o_fhi &&
                                              (fold_guar_c || in_list(g, o_foff, o_fdeg, c));
                             local += o_fbase - (hit ? 1u : 0u);
@@ -862,7 +872,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
             }
         }
         __syncwarp();
-        if (FOLD && twin && have && len) {
+        if (FOLD == kTwins && have && len) {
             const unsigned long long n = starts[lane], pr = n ? n * (n - 1) : 0;
             local2 += n;
             local += twin == 2 ? pr / 2 : pr;
@@ -2705,7 +2715,7 @@ k_plan(const uint64_t *__restrict__ tsum, uint32_t ntiles, unsigned long long ca
 
 int g_num_sms = 0;
 int g_level_blocks[3] = {0, 0, 0};
-int g_flat_blocks[3][2] = {};  // blocks of k_level_flat<mode, fold> per SM by registers and threads
+int g_flat_blocks[3][kFolds] = {};  // blocks of k_level_flat<mode, fold> per SM by registers and threads
 int g_fused_blocks[3] = {0, 0, 0};
 int g_edge_blocks = 0;  // blocks of k_edges per SM by registers and threads
 int g_pair_blocks[2] = {0, 0};  // blocks of k_pairs<fold> per SM by registers and threads
@@ -2724,14 +2734,19 @@ int launch_geometry() {
     g_level_blocks[kCountMode] = std::max(1, b) * g_num_sms;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level<kBytesMode>, kWarps * 32, 0));
     g_level_blocks[kBytesMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kExpand, false>, kFW * 32, 0));
-    g_flat_blocks[kExpand][0] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kCountMode, false>, kFW * 32, 0));
-    g_flat_blocks[kCountMode][0] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kCountMode, true>, kFW * 32, 0));
-    g_flat_blocks[kCountMode][1] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_flat<kBytesMode, true>, kFW * 32, 0));
-    g_flat_blocks[kBytesMode][1] = std::max(1, b);
+    auto flat = [&](auto *kernel, int mode, int fold) -> int {
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kFW * 32, 0));
+        g_flat_blocks[mode][fold] = std::max(1, b);
+        return CUTS_OK;
+    };
+    int rc = flat(k_level_flat<kExpand, kNoFold>, kExpand, kNoFold);
+    if (!rc) rc = flat(k_level_flat<kCountMode, kNoFold>, kCountMode, kNoFold);
+    if (!rc) rc = flat(k_level_flat<kCountMode, kPlainFold>, kCountMode, kPlainFold);
+    if (!rc) rc = flat(k_level_flat<kCountMode, kOrbitFold>, kCountMode, kOrbitFold);
+    if (!rc) rc = flat(k_level_flat<kCountMode, kPendants>, kCountMode, kPendants);
+    if (!rc) rc = flat(k_level_flat<kCountMode, kTwins>, kCountMode, kTwins);
+    if (!rc) rc = flat(k_level_flat<kBytesMode, kPlainFold>, kBytesMode, kPlainFold);
+    if (rc) return rc;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kCountMode>, kZW * 32, 0));
     g_fused_blocks[kCountMode] = std::max(1, b) * g_num_sms;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kBytesMode>, kZW * 32, 0));
@@ -2752,7 +2767,7 @@ int launch_geometry() {
 uint32_t flat_smem(int mode, uint32_t lvl, uint32_t nj) {
     return 4 * kFW * flat_words(lvl, nj, mode == kExpand);
 }
-uint32_t flat_grid(int mode, bool fold, uint32_t smem) {
+uint32_t flat_grid(int mode, int fold, uint32_t smem) {
     const uint32_t fixed = 3 * uint32_t(sizeof(LevelPlan)) + 16 * kMaxK + 1024;
     const uint32_t by_smem = 227u * 1024u / (smem + fixed);
     return std::max(1u, std::min(uint32_t(g_flat_blocks[mode][fold]), by_smem)) * uint32_t(g_num_sms);
@@ -2974,7 +2989,13 @@ struct Run {
         const uint32_t pa = par.a, pb = par.b;  // the warp-per-parent form: host-known ranges only
         const LevelPlan &L = hp->plan.lv[lvl];
         const bool flat = g_use_flat && L.nj <= uint32_t(kFJ);
-        const bool fold = mode == kBytesMode || (mode == kCountMode && (L.fold || L.fold2 || L.twin));
+        const int fold = mode == kBytesMode   ? kPlainFold
+                         : mode == kExpand    ? kNoFold
+                         : L.fold2            ? kPendants
+                         : L.twin             ? kTwins
+                         : !L.fold            ? kNoFold
+                         : hp->plan.lv[lvl + 1].ofold ? kOrbitFold
+                                                      : kPlainFold;
         const uint32_t smem = flat ? flat_smem(mode, lvl, L.nj) : 0;
         // the flattened form deals out single parents when there are few
         const uint32_t warps_needed = flat ? work : (work + grain - 1) / grain;
@@ -2994,15 +3015,16 @@ struct Run {
                 kernel<<<blocks, kFW * 32, smem, g.stream>>>(view, dp, lvl, flat_turns(g.max_deg), par, cursor, out_n, ocap,
                                                            g.d_u32 + kSlotErr, a1, a2, a3);
             };
+            auto count = [&](auto *kernel) { go(kernel, 0, g.d_u64, g.d_u64 + 3, g.d_u64 + kU64Pair); };
             if (mode == kExpand)
-                go(k_level_flat<kExpand, false>, uint32_t(cap), cs && lvl + 1 < uint32_t(kMaxK) ? cs->bound + lvl + 1 : nullptr,
+                go(k_level_flat<kExpand, kNoFold>, uint32_t(cap), cs && lvl + 1 < uint32_t(kMaxK) ? cs->bound + lvl + 1 : nullptr,
                    nullptr, nullptr);
-            else if (mode == kCountMode && fold)
-                go(k_level_flat<kCountMode, true>, 0, g.d_u64, g.d_u64 + 3, g.d_u64 + kU64Pair);
-            else if (mode == kCountMode)
-                go(k_level_flat<kCountMode, false>, 0, g.d_u64, g.d_u64 + 3, g.d_u64 + kU64Pair);
-            else
-                go(k_level_flat<kBytesMode, true>, 0, g.d_u64 + 2, nullptr, nullptr);
+            else if (mode == kBytesMode) go(k_level_flat<kBytesMode, kPlainFold>, 0, g.d_u64 + 2, nullptr, nullptr);
+            else if (fold == kPlainFold) count(k_level_flat<kCountMode, kPlainFold>);
+            else if (fold == kOrbitFold) count(k_level_flat<kCountMode, kOrbitFold>);
+            else if (fold == kPendants) count(k_level_flat<kCountMode, kPendants>);
+            else if (fold == kTwins) count(k_level_flat<kCountMode, kTwins>);
+            else count(k_level_flat<kCountMode, kNoFold>);
         } else if (mode == kExpand)
             k_level<kExpand><<<blocks, kWarps * 32, 0, g.stream>>>(view, dp, lvl, pa, pb, grain,
                 cursor, out_n, uint32_t(cap), g.d_u32 + kSlotErr, g.d_u64);
