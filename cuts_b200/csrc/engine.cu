@@ -607,9 +607,11 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
     const bool fold_guar_c = fold && ((sN.guar_mask >> lvl) & 1u);
     const bool loops = rp->plan.data_loops != 0;
     // parents per warp and turn: fewer than 32 where that would leave a warp
-    // fewer than `turns` turns
+    // fewer than `turns` turns; 32 where no candidates are walked, so that every
+    // parent costs the same few loads (an edge, 1M vertices in 4 root slices:
+    // 0.22 ms with 8 turns, 0.14 this way; 200,000 in 16: 0.26 and 0.15)
     const uint32_t nturns = turns * gridDim.x * kFW;
-    const uint32_t grab = min(32u, (total + nturns - 1) / nturns);
+    const uint32_t grab = closed || MODE == kBytesMode ? 32u : min(32u, (total + nturns - 1) / nturns);
     const unsigned long long deadline = run_deadline(rp);
     unsigned long long local = 0, local2 = 0;
     uint32_t obn = 0;
@@ -2997,8 +2999,10 @@ struct Run {
                          : hp->plan.lv[lvl + 1].ofold ? kOrbitFold
                                                       : kPlainFold;
         const uint32_t smem = flat ? flat_smem(mode, lvl, L.nj) : 0;
-        // the flattened form deals out single parents when there are few
-        const uint32_t warps_needed = flat ? work : (work + grain - 1) / grain;
+        // the flattened form deals out single parents when there are few, but
+        // for a closed form, which walks no candidates
+        const bool closed = mode == kCountMode && L.closed_form;
+        const uint32_t warps_needed = !flat ? (work + grain - 1) / grain : closed ? (work - 1) / 32 + 1 : work;
         const uint32_t wpb = flat ? kFW : kWarps;
         uint32_t blocks = std::min<uint32_t>(flat ? flat_grid(mode, fold, smem) : uint32_t(g_level_blocks[mode]),
                                              (warps_needed + wpb - 1) / wpb);
