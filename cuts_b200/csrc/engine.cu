@@ -98,14 +98,14 @@ __device__ __forceinline__ bool past_deadline(const RunParams *rp, unsigned long
 //   sum_{x in O, x < upto} ( |L(m_x)| - #{j < upto : m_j in L(m_x)} ),
 // where m(j) gives the matched vertex of position j.
 template <class M>
-__device__ __forceinline__ uint32_t orbit_base(const DevView &g, const LevelPlan &F, uint32_t upto, M m) {
+__device__ __forceinline__ uint32_t orbit_base(const DevView &g, const LevelPlan &F, uint32_t upto, bool loops, M m) {
     uint32_t base = 0;
     for (uint32_t xm = F.ofold & ((1u << upto) - 1); xm; xm &= xm - 1) {
         const uint32_t x = __ffs(xm) - 1;
         const uint2 inf = F.jdir[0] ? g.in_info[m(x)] : g.out_info[m(x)];
         uint32_t sub = 0;
         for (uint32_t j = 0; j < upto; ++j)
-            if (((F.oguar[x] >> j) & 1u) || in_list(g, inf.x, inf.y, m(j))) ++sub;
+            if (((F.oguar[x] >> j) & 1u) || ((loops || j != x) && in_list(g, inf.x, inf.y, m(j)))) ++sub;
         base += inf.y - sub;
     }
     return base;
@@ -679,7 +679,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                         ubp = min(ubp, (sN.jdir[t] ? g.in_info[u] : g.out_info[u]).y);
                     }
             if (MODE == kBytesMode ? fold && sN.ofold : FOLD == kOrbitFold) {
-                fbase = orbit_base(g, sN, lvl, [&](uint32_t j) { return sm_m[32 * j + lane]; });
+                fbase = orbit_base(g, sN, lvl, loops, [&](uint32_t j) { return sm_m[32 * j + lane]; });
             } else if (fold) {
                 const uint32_t u = sm_m[32 * sN.jpos[0] + lane];
                 const uint2 inf = sN.jdir[0] ? g.in_info[u] : g.out_info[u];
@@ -693,6 +693,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                 uint32_t sub = 0;
                 for (uint32_t j = 0; j < lvl; ++j) {
                     const uint32_t mj = sm_m[32 * j + lane];
+                    if (j == sN.jpos[0] && !loops) continue;  // not in its own list
                     if (mj >= f_lo && mj < f_hi && (((sN.guar_mask >> j) & 1u) || in_list(g, f_off, f_deg, mj))) ++sub;
                 }
                 fbase = (we > ws ? we - ws : 0) - sub;
@@ -725,6 +726,7 @@ k_level_flat(DevView g, const RunParams *__restrict__ rp, uint32_t lvl, uint32_t
                 uint32_t sub = 0;
                 for (uint32_t j = 0; j < lvl; ++j) {
                     const uint32_t mj = sm_m[32 * j + lane];
+                    if (j == sL.jpos[0] && !loops) continue;  // not in its own list
                     if (mj >= lo && mj < hi && (((sL.guar_mask >> j) & 1u) || in_list(g, moff, mdeg, mj))) ++sub;
                 }
                 local += (e0 - s0) - sub;
@@ -1029,7 +1031,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                 ostart = iters ? ls0 : ts;
                 oend = iters ? ls1 : te;
                 if (cfold && sF.ofold) {
-                    fbase = orbit_base(g, sF, p + 1, [&](uint32_t j) { return j == p ? sv : my_m[j]; });
+                    fbase = orbit_base(g, sF, p + 1, loops, [&](uint32_t j) { return j == p ? sv : my_m[j]; });
                 } else if (cfold) {
                     // folded last level: f_base(s) = |window of L_F| - matched in it
                     const uint32_t jf = sF.jpos[0];
@@ -1165,7 +1167,7 @@ k_fused(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
             uint32_t fbase = 0, fdeg = 0, flo = 0, fhi = kFullMask;
             const uint32_t *fl = nullptr;
             if (cfold && sF.ofold) {
-                fbase = orbit_base(g, sF, p + 1, [&](uint32_t j) { return j == p ? sv : my_m[j]; });
+                fbase = orbit_base(g, sF, p + 1, loops, [&](uint32_t j) { return j == p ? sv : my_m[j]; });
             } else if (cfold) {
                 const uint32_t jf = sF.jpos[0];
                 const uint32_t u = jf == p ? sv : my_m[jf];
@@ -2855,6 +2857,9 @@ static int device_graph_build(uint32_t n, const uint64_t *out_off, const uint32_
     g->arena_bytes = size_t(want);
     g->arena_default = g->arena_bytes;
     g->tab_limit = (freeb - std::min(freeb, g->arena_bytes)) / 2;
+    // CUTS_TABLES=0 does without the tables' memory (lists are searched)
+    const char *tb = std::getenv("CUTS_TABLES");
+    if (tb && tb[0] == '0') g->tab_limit = 0;
     *out = g;
     return CUTS_OK;
 }
@@ -3330,6 +3335,16 @@ bool pairs_plan(const DeviceGraph &g, const Plan &plan, uint32_t p) {
     return !(w && w[0] == '0');
 }
 
+// True when an orbit fold's weights look a vertex below position `upto` up in
+// an orbit vertex's list (orbit_base, orbit_weight).
+bool orbit_tests(const LevelPlan &F, uint32_t upto, bool loops) {
+    if (loops) return true;
+    for (uint32_t x = 0; x < upto; ++x)
+        if ((F.ofold >> x) & 1u)
+            if (~(F.oguar[x] | (1u << x)) & ((1u << upto) - 1)) return true;
+    return false;
+}
+
 // CUTS_NO_FUSE=1: fusion off process-wide (A/B comparisons)
 bool no_fuse_env() {
     const char *nf = std::getenv("CUTS_NO_FUSE");
@@ -3420,12 +3435,25 @@ int prepare(DeviceGraph &g, const Query &q, uint32_t flags, uint32_t stored, Run
             L.check_sig = 0;
         }
     // membership tables, for the levels that test candidates in other lists
-    // or matched vertices in a folded one
+    // or matched vertices in a list that a closed form counts (a graph whose
+    // counts are edges and stars does without: their build is 0.3 ms for 20M
+    // arcs, an edge count 0.1)
     bool tests = false;
+    // positions below upto that L's list may hold for all the plan knows
+    auto unknown = [&](const LevelPlan &L, uint32_t guar, uint32_t upto) {
+        const uint32_t known = guar | (g.loops ? 0u : 1u << L.jpos[0]);
+        return (~known & ((1u << upto) - 1)) != 0;
+    };
     for (uint32_t i = 1; i < k && i <= stored; ++i) {
         const LevelPlan &L = hp->plan.lv[i];
         if (fuse && i >= stored) break;
-        tests = tests || L.nj >= 2 || (counting && (L.fold || L.fold2 || L.closed_form));
+        tests = tests || L.nj >= 2;
+        if (!counting) continue;
+        const LevelPlan &F = hp->plan.lv[k - 1];
+        if (i == k - 1 && L.closed_form) tests = tests || unknown(L, L.guar_mask, i);
+        else if (L.fold2) tests = tests || unknown(hp->plan.lv[i + 1], hp->plan.lv[i + 1].guar1, i + 1) || unknown(F, F.guar_mask, i + 1);
+        else if (L.fold && F.ofold) tests = tests || orbit_tests(F, i, g.loops);
+        else if (L.fold) tests = tests || unknown(F, F.guar_mask, i + 1);
     }
     if ((tests || (fuse && g.symmetric)) && (rc = device_tables(g))) return rc;
     hp->pairs = fuse && pairs_plan(g, hp->plan, cl - 1);
