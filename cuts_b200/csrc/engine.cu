@@ -3699,6 +3699,7 @@ int device_count(DeviceGraph &g, const Query &q, const CountOptions &opt, CountR
     const uint32_t k = q.k;
     RunParams *hp = nullptr, *dp = nullptr;
     uint64_t cap = 0;
+    const bool had_tables = g.tab != nullptr;
     rc = prepare(g, q, opt.flags, k - 1, hp, dp, cap);
     if (rc) return rc;
     Run run{g, graph_view(g), hp, dp, k, cap, 4, false, res};
@@ -3708,7 +3709,8 @@ int device_count(DeviceGraph &g, const Query &q, const CountOptions &opt, CountR
         hp->budget_ns = (unsigned long long)(opt.budget_ms * 1e6);
         CK(cudaMemcpyAsync(dp, hp, sizeof(RunParams), cudaMemcpyHostToDevice, g.stream));
     }
-    CK(cudaEventRecord(g.ev0, g.stream));
+    // the time starts here, or with the tables that this count had built
+    if (had_tables || !g.tab) CK(cudaEventRecord(g.ev0, g.stream));
     uint32_t n0 = 0;
     if (k >= 2 && g.n && run.can_chain()) {
         rc = run_roots(g, run, opt.shard, opt.nshards, n0, opt.chunks);

@@ -79,8 +79,8 @@ int device_graph_from_csr(uint32_t n, const uint64_t *out_off, const uint32_t *o
 // (in-lists given), -1 decide; validate checks offsets and list order.
 int device_layout(uint32_t n, const uint64_t *out_off, const uint32_t *out_adj, const uint64_t *in_off,
                   const uint32_t *in_adj, int sym_hint, bool validate, DeviceGraph &g);
-// Builds g.tab on g.stream, once; leaves it null (lists are searched
-// instead) when the device cannot hold it.
+// Builds g.tab on g.stream, once (recording g.ev0 where the build starts);
+// leaves it null (lists are searched instead) when the device cannot hold it.
 int device_tables(DeviceGraph &g);
 int host_degrees(DeviceGraph &g);
 int host_orig(DeviceGraph &g);

@@ -792,6 +792,7 @@ int device_tables(DeviceGraph &g) {
             if (tab) cudaFreeAsync(tab, g.stream);
         }
     } hold{g, tab};
+    LCK(cudaEventRecord(g.ev0, g.stream));  // the device time of the count that builds them includes the build
     const int rc = build_tables(g, tab);
     if (rc) return rc;
     hold.tab = nullptr;
