@@ -406,10 +406,13 @@ __device__ __forceinline__ bool counts_next(const BQuery &Q, uint32_t d) {
     return d + 2 == Q.k || (d + 3 == Q.k && (Q.lv[d + 1].fold || Q.lv[d + 1].twin));
 }
 
-// Single-range roots of one task: 32 where they are counted at once, fewer
-// where the warp goes through them one after another (a tail of 32 subtrees).
+// Single-range roots of one task: 32 where they are counted at once, 8 where
+// the warp goes through them one after another and a root is a frontier or two,
+// one where subtrees are deeper: finding the root is then little of the work,
+// and 8 subtrees in a row are the launch's tail (a 5-vertex query on 5,000
+// vertices / 15,000 edges alone 0.8 ms with one, 2.3 with 8).
 __host__ __device__ inline uint32_t roots_per_task(const BQuery &Q) {
-    return Q.k == 2 || (Q.k == 3 && Q.lv[1].fold) ? 32u : 8u;
+    return Q.k == 2 || (Q.k == 3 && Q.lv[1].fold) ? 32u : Q.k <= 4 ? 8u : 1u;
 }
 
 // One vertex of level d's frontier becomes matched; its children are next.
