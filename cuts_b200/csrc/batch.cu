@@ -976,6 +976,7 @@ struct NoAllocScratch {
     BQuery queries[kNoAllocMaxQueries];
     unsigned long long task_ctr;
     uint32_t stop;
+    uint32_t longest;  // list of the graph (or kSlices slices' worth)
     uint32_t aborted[kNoAllocMaxQueries];
 };
 
@@ -1006,30 +1007,64 @@ __global__ void k_noalloc_plans(const NoAllocPlans plans, uint32_t first, uint32
     if (first == 0 && threadIdx.x == 0) {
         sc->task_ctr = 0;
         sc->stop = 0;
+        sc->longest = 0;
     }
 }
 
-// Tasks are (slice, query, block of 32 roots): the lanes look at the block's
-// roots at once, and of each root that passes the level-0 signature the warp
-// runs the slice's part of its level-1 list depth first, with the same level
-// steps as k_batch.  Slice r of kSlices holds the blocks b of kSliceLen
-// level-1 candidates with b % kSlices == r, so a hub's work is spread over
-// kSlices warps; the slices above 0, empty for most roots, come first.  With
-// the whole list of a root as one task, hubs were the launch's tail: 16
-// queries of 2-4 vertices on 50,001 vertices / 300,000 edges took 67.5 ms,
-// 16.8 ms this way (frontiers counted at once included).  No budget: every
-// query runs to completion.
+// The longest list, for the number of slices (one launch more than the plans':
+// it saves the empty slices' tasks, an atomic each, on graphs without hubs).
+__global__ void __launch_bounds__(256)
+k_noalloc_longest(const uint2 *__restrict__ info_out, const uint2 *__restrict__ info_in, uint32_t n,
+                  NoAllocScratch *__restrict__ sc) {
+    uint32_t len = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        len = max(len, max(info_out[v].y, info_in[v].y));
+    len = __reduce_max_sync(kFullMask, len);
+    if ((threadIdx.x & 31) == 0) atomicMax(&sc->longest, len);
+}
+
+// Tasks are (slice, query, block of up to 32 roots): the lanes look at the
+// block's roots at once, and of each root that passes the level-0 signature the
+// warp runs the slice's part of its level-1 list depth first, with the same
+// level steps as k_batch.  Slice r of (up to) kSlices holds the blocks b of
+// kSliceLen level-1 candidates with b % slices == r, so a hub's work is spread
+// over as many warps; the slices above 0, empty for most roots, come first, and
+// there are only as many as the longest list has.  With the whole list of a root
+// as one task, hubs were the launch's tail: 16 queries of 2-4 vertices on 50,001
+// vertices / 300,000 edges took 67.5 ms, 3.7 ms this way (frontiers counted at
+// once and twins included).  Slice 0, where nearly all work is, has blocks of 32
+// in calls with roots enough; of fewer roots a block takes so many that every
+// warp gets several (na_block): 4 queries on 200 vertices 0.20 ms in blocks of
+// 32, 0.06 this way, one of 6 vertices on 3,000 vertices / 9,000 edges 0.91 and
+// 0.27 (0.08 and 0.47 with one root per task).  No budget: every query runs to
+// completion.
 constexpr uint32_t kSlices = 16;
 constexpr uint32_t kSliceLen = 32;
 
+// Roots per block of slice 0 for `roots` (query, root) pairs on `warps` warps: 4 blocks a
+// warp or more, 16 where subtrees are deep (5 vertices and more).
+uint32_t na_block(unsigned long long roots, uint32_t warps, bool deep) {
+    const unsigned long long per = roots / ((unsigned long long)warps * (deep ? 16 : 4));
+    return uint32_t(std::max<unsigned long long>(1, std::min<unsigned long long>(32, per)));
+}
+
 __global__ void __launch_bounds__(kBW * 32)
-k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq,
+k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq, uint32_t blk, uint32_t upblk,
                 unsigned long long *__restrict__ counts) {
     __shared__ BWarp ws[kBW];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Ctx c{g, nullptr, &ws[warp], lane};
-    const uint32_t nblk = (g.n + 31) / 32;
-    const unsigned long long per = (unsigned long long)nq * nblk, total = per * kSlices;
+    // the task space, in shared memory (registers are what this kernel is short of)
+    __shared__ unsigned long long upper, total;  // tasks of the slices above 0, and all
+    __shared__ uint32_t slices, nblk[2];
+    if (threadIdx.x == 0) {
+        slices = min(kSlices, (max(sc->longest, 1u) - 1) / kSliceLen + 1);
+        nblk[0] = (g.n - 1) / upblk + 1;
+        nblk[1] = (g.n - 1) / blk + 1;
+        upper = (unsigned long long)nq * nblk[0] * (slices - 1);
+        total = upper + (unsigned long long)nq * nblk[1];
+    }
+    __syncthreads();
     uint32_t cur = kFullMask;
     unsigned long long qcount = 0;
     while (true) {
@@ -1037,9 +1072,11 @@ k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq,
         if (lane == 0) t = atomicAdd(&sc->task_ctr, 1ull);
         t = __shfl_sync(kFullMask, t, 0);
         if (t >= total) break;
-        const uint32_t slice = kSlices - 1 - uint32_t(t / per);
-        const unsigned long long in = t % per;
-        const uint32_t q = uint32_t(in / nblk), u0 = uint32_t(in % nblk) * 32;
+        const bool first = t >= upper;  // slice 0
+        const uint32_t nb = nblk[first], roots = first ? blk : upblk;
+        const unsigned long long at = first ? t - upper : t;
+        const uint32_t run = uint32_t(at / nb), u0 = uint32_t(at - (unsigned long long)run * nb) * roots;
+        const uint32_t q = first ? run : run % nq, slice = first ? 0u : slices - 1 - run / nq;
         if (q != cur) {
             if (cur != kFullMask) add_count(&counts[cur], qcount, lane);
             qcount = 0;
@@ -1050,7 +1087,7 @@ k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq,
         if (Q.k < 2) continue;
         // the block's roots with level-1 candidates in this slice
         bool pass = false;
-        if (u0 + lane < g.n) {
+        if (uint32_t(lane) < roots && u0 + lane < g.n) {
             const uint2 uo = g.out_info[u0 + lane], ui = g.in_info[u0 + lane];
             uint32_t len = kFullMask;
             for (uint32_t j = 0; j < Q.lv[1].nj; ++j) len = min(len, Q.lv[1].jdir[j] ? ui.y : uo.y);
@@ -1061,7 +1098,7 @@ k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq,
             __syncwarp();
             enter_level(c, 1);  // the whole shortest level-1 list
             const uint32_t xend = c.S->xend[1];
-            for (uint32_t x0 = slice * kSliceLen; x0 < xend; x0 += kSlices * kSliceLen) {
+            for (uint32_t x0 = slice * kSliceLen; x0 < xend; x0 += slices * kSliceLen) {
                 __syncwarp();
                 if (lane == 0) {
                     c.S->x[1] = x0;
@@ -1114,6 +1151,7 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
     // the query plans, built on the stack (fixed size, no allocation)
     NoAllocPlans table[kNoAllocMaxQueries / kNoAllocPlansPerLaunch];
     const bool sym = symmetric != 0 || info_in == nullptr;
+    bool deep = false;
     for (uint32_t i = 0; i < nq; ++i) {
         if (!qs[i]) return set_error(CUTS_ERR_ARG, "cuts_count_noalloc: null query");
         const Query &q = *qs[i];
@@ -1125,6 +1163,7 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
         BQuery &b = table[i / kNoAllocPlansPerLaunch].q[i % kNoAllocPlansPerLaunch];
         std::memset(&b, 0, sizeof(b));
         b.k = q.k;
+        deep = deep || q.k >= 5;
         for (uint32_t d = 0; d < q.k; ++d) {
             const LevelPlan &L = plan.lv[d];
             if (L.nj > uint32_t(kBatchMaxJ))
@@ -1185,9 +1224,13 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
     const DevView view{reinterpret_cast<const uint2 *>(info_out),
                        reinterpret_cast<const uint2 *>(sym ? info_out : info_in), adj, n, nullptr, nullptr,
                        nullptr, 0, nullptr};
-    const unsigned long long total = (unsigned long long)nq * ((n + 31) / 32) * kSlices;
+    const uint32_t blk = na_block((unsigned long long)nq * n, blocks * kBW, deep);
+    const uint32_t upblk = std::max(blk, deep ? 8u : 32u);  // of the slices above 0: most such tasks find nothing
+    k_noalloc_longest<<<std::min<uint32_t>((n - 1) / 256 + 1, blocks), 256, 0, stream>>>(view.out_info, view.in_info, n, sc);
+    const unsigned long long total =
+        (unsigned long long)nq * ((n - 1) / blk + 1 + (unsigned long long)((n - 1) / upblk + 1) * (kSlices - 1));
     const uint32_t grid = uint32_t(std::min<unsigned long long>(blocks, (total + kBW - 1) / kBW));
-    k_batch_noalloc<<<std::max<uint32_t>(grid, 1), kBW * 32, 0, stream>>>(view, sc, nq, counts);
+    k_batch_noalloc<<<std::max<uint32_t>(grid, 1), kBW * 32, 0, stream>>>(view, sc, nq, blk, upblk, counts);
     if (cudaGetLastError() != cudaSuccess)
         return set_error(CUTS_ERR_CUDA, "cuts_count_noalloc: launch failed");
     return CUTS_OK;
