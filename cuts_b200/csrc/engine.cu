@@ -1838,6 +1838,13 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
         kconst = ((sF.guar_mask >> p) & 1u) == ((sF.guar_mask >> (p + 1)) & 1u);
     }
     const uint32_t orders = (o1 ? 1u : 0u) + (o2 ? 1u : 0u);
+    // with every member admissible, A(s) + B(t) is then the same for both orders
+    // of a pair (A is B plus a constant), so a hit costs one weight and no test:
+    // triangle + pendant, 60-regular graph of 700,003 vertices, plain 17.2 ->
+    // 12.1 ms, symmetry breaking 5.8 -> 5.0; 4-clique + pendant, 1M / 10M 8.1 ->
+    // 7.5.  degs: B is the degree less this
+    const bool even = FOLD && cfold && ts && kconst;
+    const uint32_t degs = FOLD && !LOOPS && sF.ofold && ((sF.ofold >> (p + 1)) & 1u) ? p + 1 : 0u;
     uint32_t free_pos = below;  // positions below p whose lists P does not join (all with self-loops)
     if (!LOOPS)
         for (uint32_t t = 0; t < njp; ++t) free_pos &= ~(1u << sP.jpos[t]);
@@ -2011,11 +2018,12 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                     const uint32_t r = __popc(ilive & lanemask_lt), excl = iincl - ilen;
                     rec[r] = make_uint4(ibase - excl, ow | (mode << 8) | (i << 16), ioff, ideg);
                     starts[r] = excl;
-                    if (FOLD) itemA[r] = o1 ? pair_a<LOOPS>(x, ow, a) : 0u;
+                    if (FOLD) itemA[r] = o1 || even ? pair_a<LOOPS>(x, ow, a) : 0u;
                 }
                 __syncwarp();
                 const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(ilive)) ? starts[lane] : kFullMask;
-                uint32_t started = 0, hits = 0;  // hits: of a batch without weights
+                uint32_t started = 0, hits = 0;   // hits: of a batch whose pairs weigh the same in both orders
+                unsigned long long weight = 0;    // their weights in one order
                 for (uint32_t fstep = 0; fstep < itotal; fstep += 64) {
                     uint4 rc[2];
                     uint32_t tv[2], rk[2];
@@ -2048,6 +2056,11 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                                       : pair_above_in_set(x, rc[h].y & 255u, free_pos, t);
                         if (!FOLD && ts) {
                             hits += ok;
+                        } else if (FOLD && even) {
+                            if (ok) {
+                                ++hits;
+                                weight += uint32_t(itemA[rk[h]] + (degs ? g.out_info[t].y - degs : pair_b<LOOPS>(x, rc[h].y & 255u, t)));
+                            }
                         } else if (ok) {
                             const uint32_t l = rc[h].y & 255u;
                             {
@@ -2064,7 +2077,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         }
                     }
                 }
-                local += uint64_t(hits) * orders;
+                local += (FOLD ? weight : uint64_t(hits)) * orders;
                 local_c += uint64_t(hits) * orders;
                 __syncwarp();
             }
