@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -327,13 +328,14 @@ __device__ __forceinline__ void tab_insert(uint32_t *base, uint32_t len, uint32_
 // tables of up to kTabWords list words at a time in shared memory and writes
 // them out whole -- 4 B read and 8 B written per entry, the atomics in shared
 // memory (built by compare-and-swap in global memory they took 2.3 ms for 20M
-// entries, 0.28 ms with the hub kernels below).  A list longer than that (ids not degree-ranked)
-// is built in place.
+// entries, 0.28 ms with the hub kernels below).  A longer list (ids not
+// degree-ranked) is queued for k_tables_queue.
 constexpr uint32_t kTabWords = 1024;
 constexpr int kTabWarps = 4;
 
 __global__ void __launch_bounds__(kTabWarps * 32)
-k_tables(uint32_t h0, const uint2 *__restrict__ info, const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab) {
+k_tables(uint32_t h0, const uint2 *__restrict__ info, const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab,
+         uint32_t *__restrict__ queue, uint32_t *__restrict__ queued) {
     __shared__ uint4 sh[kTabWarps][kTabWords / 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint4 *const t4 = sh[warp];
@@ -357,13 +359,10 @@ k_tables(uint32_t h0, const uint2 *__restrict__ info, const uint32_t *__restrict
             const uint32_t off0 = __shfl_sync(kFullMask, inf.x, first);
             const unsigned sel = __ballot_sync(kFullMask, left != 0 && incl <= kTabWords);
             if (!sel) {  // the first one alone is too long
-                const uint32_t len = __shfl_sync(kFullMask, inf.y, first);
-                uint32_t *const base = tab + 2 * size_t(off0);
-                for (uint32_t i = lane; i < 2 * padded(len); i += 32) base[i] = kTabEmpty;
-                __syncwarp();
-                for (uint32_t i = lane; i < len; i += 32) tab_insert(base, len, __ldg(adj + off0 + i));
-                __syncwarp();
-                if (lane == first) left = 0;
+                if (lane == first) {
+                    queue[atomicAdd(queued, 1u)] = v;
+                    left = 0;
+                }
                 continue;
             }
             const bool mine = (sel >> lane) & 1u;
@@ -411,6 +410,22 @@ k_tables_hub(uint32_t h0, uint32_t h1, const uint2 *__restrict__ info, const uin
         uint4 *const out = reinterpret_cast<uint4 *>(tab + 2 * size_t(inf.x));
         for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x) out[i] = t4[i];
         __syncthreads();
+    }
+}
+
+// The queued lists, one block each, in place (20M arcs in the host's order,
+// lists of up to 20,000: first count 4 ms over a later one with one warp per
+// such list, 1.3 this way; lists of up to 300,000: 12 and 0.7).
+__global__ void __launch_bounds__(1024)
+k_tables_queue(const uint2 *__restrict__ info, const uint32_t *__restrict__ adj, uint32_t *__restrict__ tab,
+               const uint32_t *__restrict__ queue, const uint32_t *__restrict__ queued) {
+    const uint32_t nq = *queued;
+    for (uint32_t i = blockIdx.x; i < nq; i += gridDim.x) {
+        const uint2 inf = info[queue[i]];
+        uint32_t *const base = tab + 2 * size_t(inf.x);
+        for (uint32_t j = threadIdx.x; j < 2 * padded(inf.y); j += blockDim.x) base[j] = kTabEmpty;
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < inf.y; j += blockDim.x) tab_insert(base, inf.y, __ldg(adj + inf.x + j));
     }
 }
 
@@ -732,7 +747,7 @@ static int build_tables(DeviceGraph &g, uint32_t *tab) {
     cudaStream_t s = g.stream;
     const int dirs = g.symmetric ? 1 : 2;
     // ids are degree ranks (unless relabelling is off: then every list goes
-    // to the first kernel), so no list of the vertices below n - c has more
+    // to the first kernel, which queues the long ones), so no list of the vertices below n - c has more
     // than L entries, c being at least the number of vertices of degree above
     // L; out- plus in-degree above L needs one of them above L / 2
     auto longer = [&](uint64_t L) {
@@ -749,10 +764,19 @@ static int build_tables(DeviceGraph &g, uint32_t *tab) {
     constexpr uint32_t kShort = 128, kMid = 4096, kBig = 24576;
     const uint32_t h0 = longer(kShort), hm = longer(kTabWords), h1 = longer(kMid), h2 = longer(kBig);
     LCK(cudaFuncSetAttribute(k_tables_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBig * 8)));
+    std::unique_ptr<Scratch> sc;  // (its end waits for the stream)
+    uint32_t *queued = nullptr, *queue = nullptr;  // lists too long for k_tables
+    if (!g.ranked && g.max_deg > kTabWords) {
+        sc = std::make_unique<Scratch>(s);
+        LCK(sc->get(&queued, size_t(g.n) + 1));
+        queue = queued + 1;
+    }
     for (int dir = 0; dir < dirs; ++dir) {
         const uint2 *info = dir ? g.in_info : g.out_info;
+        if (queue) LCK(cudaMemsetAsync(queued, 0, sizeof(uint32_t), s));
         k_tables<<<std::max<uint32_t>(1, std::min<uint32_t>((h0 + 127) / 128, 148u * 7)), kTabWarps * 32, 0, s>>>(
-            h0, info, g.adj, tab);
+            h0, info, g.adj, tab, queue, queued);
+        if (queue) k_tables_queue<<<148 * 2, 1024, 0, s>>>(info, g.adj, tab, queue, queued);
         if (hm > h0) k_tables_hub<<<std::min<uint32_t>(hm - h0, 148u * 16), 128, kTabWords * 8, s>>>(h0, hm, info, g.adj, tab);
         if (h1 > hm) k_tables_hub<<<std::min<uint32_t>(h1 - hm, 148u * 6), 256, kMid * 8, s>>>(hm, h1, info, g.adj, tab);
         if (h2 > h1) k_tables_hub<<<std::min<uint32_t>(h2 - h1, 148u), 1024, kBig * 8, s>>>(h1, h2, info, g.adj, tab);
