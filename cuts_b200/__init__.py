@@ -414,7 +414,7 @@ class Graph:
         _check(lib().cuts_graph_set_arena_bytes(self._h, nbytes))
 
     def set_fuse_split(self, split: int) -> None:
-        """|S| above which the fused count splits a parent over all warps (0 = default)."""
+        """Candidates above which the fused count splits a parent over all warps (0 = defaults)."""
         _check(lib().cuts_graph_set_fuse_split(self._h, split))
 
     def count(self, q: Query, chunks: int = 1, flags: int = 0, stats: bool = False,

@@ -25,7 +25,8 @@ import cuts_b200 as cb
 
 GRAINS = (16, 32, 64, 128, 256)
 CHUNKS = (1, 2, 4, 8)
-SPLITS = (64, 128, 256)
+# 0: the kernels' defaults (512 for the pair kernel, its most)
+SPLITS = (0, 64, 128, 256)
 LEVEL_CAPS = (0,)
 GRABS = (1, 4)
 BLOCKS = (0, 4)
