@@ -406,13 +406,20 @@ __device__ __forceinline__ bool counts_next(const BQuery &Q, uint32_t d) {
     return d + 2 == Q.k || (d + 3 == Q.k && (Q.lv[d + 1].fold || Q.lv[d + 1].twin));
 }
 
-// Single-range roots of one task: 32 where they are counted at once, 8 where
-// the warp goes through them one after another and a root is a frontier or two,
-// one where subtrees are deeper: finding the root is then little of the work,
-// and 8 subtrees in a row are the launch's tail (a 5-vertex query on 5,000
-// vertices / 15,000 edges alone 0.8 ms with one, 2.3 with 8).
-__host__ __device__ inline uint32_t roots_per_task(const BQuery &Q) {
-    return Q.k == 2 || (Q.k == 3 && Q.lv[1].fold) ? 32u : Q.k <= 4 ? 8u : 1u;
+// Single-range roots of one task, at most: 32 where they are counted at once, 8
+// where the warp goes through them one after another and a root is a frontier or
+// two, one where subtrees are deeper: finding the root is then little of the
+// work, and 8 subtrees in a row are the launch's tail (a 5-vertex query on 5,000
+// vertices / 15,000 edges alone 0.8 ms with one, 2.3 with 8).  Fewer in a launch
+// of so few roots that warps would get less than a task each, or 4 tasks of
+// 4-vertex queries (one on 1,500 vertices of a directed graph alone 3.7 ms in
+// bundles of 8, 1.3 with one root per task before the bundles, 0.55 now).
+// The warps are a number, not a device's: shards on several GPUs have to cut
+// the same tasks.
+constexpr unsigned long long kLaunchWarps = 148 * 4 * kBW;
+inline uint32_t roots_per_task(const BQuery &Q, unsigned long long roots) {
+    const unsigned long long most = Q.k == 2 || (Q.k == 3 && Q.lv[1].fold) ? 32 : Q.k <= 4 ? 8 : 1;
+    return uint32_t(std::max<unsigned long long>(1, std::min(most, roots / ((Q.k <= 3 ? 1 : 4) * kLaunchWarps))));
 }
 
 // One vertex of level d's frontier becomes matched; its children are next.
@@ -528,7 +535,7 @@ k_batch(DevView g, const BQuery *__restrict__ qs, uint32_t nq,
             if (local >= heavy) {
                 // roots of one range each: looked at together, and counted
                 // together where level 1 is the last one walked
-                const uint32_t per = roots_per_task(Q);
+                const uint32_t per = Q.per;
                 const uint32_t ri = Q.heavy_roots + uint32_t(local - heavy) * per + lane;
                 uint32_t u = 0;
                 bool pass = uint32_t(lane) < per && ri < Q.root_cnt;
@@ -719,6 +726,7 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
     aut.assign(nq, 1);
     eligible.assign(nq, 0);
     const uint32_t n = g->n;
+    unsigned long long light = 0;  // roots of one range, over all queries of the launch
     if ((rc = device_tables(*g))) return rc;
     for (uint32_t i = 0; i < nq; ++i) {
         const Query &q = *qs[i];
@@ -762,7 +770,6 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
         if (ok && q.k >= 4 && route_level && (route_all || level_engine_pays(q, g->symmetric, flags))) ok = false;
         const bool edges = ok && q.k >= 4 && route_level && level_engine_edges(q, *g, flags);
         if (edges) ok = false;
-        unsigned long long tasks = 0;
         if (ok) {
             b.k = q.k;
             bool has_out = false, has_in = false;
@@ -780,10 +787,8 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
                 const uint64_t longer = over < g->stats.out_ge.size() ? g->stats.out_ge[over] : 0;
                 b.heavy_roots = b.type == 0 ? uint32_t(std::min<uint64_t>(b.root_cnt, longer)) : b.root_cnt;
                 info_tasks += pref[b.root_cnt];
-                const uint32_t rpt = roots_per_task(b);
-                tasks = pref[b.heavy_roots] + (b.root_cnt - b.heavy_roots + rpt - 1) / rpt;
+                light += b.root_cnt - b.heavy_roots;
                 hq.push_back(b);
-                qbase.push_back(qbase.back() + tasks);
                 index.push_back(i);
             }
         }
@@ -792,6 +797,11 @@ int Batch::create(DeviceGraph &dg, const std::vector<const Query *> &qs, uint32_
     // eligible: 1 = in the launch, 2 = no root (count 0), 0 = counted by the
     // level engine, 3 = the same, within the launch's budget
     nb = uint32_t(hq.size());
+    for (BQuery &b : hq) {
+        b.per = roots_per_task(b, light);
+        const unsigned long long *pref = g->batch_pref_host.data() + size_t(b.type) * (n + 1);
+        qbase.push_back(qbase.back() + pref[b.heavy_roots] + (b.root_cnt - b.heavy_roots + b.per - 1) / b.per);
+    }
     total_tasks = qbase.back();
     BCK(cudaMalloc(&d_queries, sizeof(BQuery) * std::max<size_t>(hq.size(), 1)));
     BCK(cudaMalloc(&d_qbase, sizeof(unsigned long long) * qbase.size()));
@@ -992,7 +1002,7 @@ std::mutex g_noalloc_mutex;
 // The query plans travel as kernel parameters, copied into the scratch array
 // by a one-block kernel: the launch records them by value when it is queued,
 // so the call needs no host staging buffer and returns without waiting.
-constexpr uint32_t kNoAllocPlansPerLaunch = 16;  // 16 x 656 B of parameters
+constexpr uint32_t kNoAllocPlansPerLaunch = 16;  // 16 x 660 B of parameters
 struct NoAllocPlans {
     BQuery q[kNoAllocPlansPerLaunch];
 };

@@ -25,6 +25,7 @@ struct BQuery {
     uint32_t type;      // level-1 candidate list: 0 out, 1 in, 2 the shorter
     uint32_t root_cnt;  // roots = the first root_cnt vertices in out-degree order
     uint32_t heavy_roots;  // those with more than one level-1 range, a prefix
+    uint32_t per;          // of the others, roots per task
 };
 
 // Launch shape picked by the autotuner (0 = default).
