@@ -3105,8 +3105,14 @@ struct Run {
             // parents that are roots (p = 1) have their own list's window for S,
             // so dealing them out in pieces repeats no test, and it keeps a
             // hub's pairs from one warp: 64 there (triangle, 4M / 40M: 512 14.6 ms,
-            // 128 12.7 ms, 64 9.5 ms)
-            if (p == 1) split = std::min(split, kPK);
+            // 128 12.7 ms, 64 9.3 ms).  Not where the longest list is little more
+            // (3 of them; 4 with an order, whose windows are about half of the
+            // lists): the second launch and its bitmaps took 40 of 72 us of a root
+            // slice (triangle, symmetry breaking, 2,000 vertices / 80,000 edges in
+            // 17 slices 1.21 -> 0.60 ms, 5,000 / 250,000 at once 0.21 -> 0.14; 3,000
+            // / 300,000 plain, lists of 250, would lose 0.54 -> 0.60)
+            const uint32_t few = (hp->plan.lv[p].gt_mask | hp->plan.lv[p].lt_mask ? 4 : 3) * kPK;
+            if (p == 1 && (es || g.fuse_split || g.max_deg > few)) split = std::min(split, kPK);
             const bool fold = hp->plan.lv[p + 1].fold != 0;
             const uint32_t smem = 4 * kPW * pair_words(p, hp->plan.lv[p].nj);
             const uint32_t fixed = 3 * uint32_t(sizeof(LevelPlan)) + 16 * kMaxK + 1024;
@@ -3126,7 +3132,9 @@ struct Run {
             phase(blocks, 1, cur1);
             CK(cudaGetLastError());
             res.launches++;
-            if (pair_defers(p, split, g.max_deg, 32ull * g.max_deg)) {
+            // (a turn is of `most` parents dealt out as in the kernel, at most)
+            const uint32_t turn = std::min(32u, std::max(1u, most / (4 * blocks * kPW)));
+            if (pair_defers(p, split, g.max_deg, uint64_t(turn) * g.max_deg)) {
                 k_fused_scan<<<1, 1024, 0, g.stream>>>(pb.n, pb.cap, pb.len, kPK, pb.pref);
                 k_pair_bits<false><<<full, kPW * 32, smem, g.stream>>>(view, dp, p, pb);
                 phase(full, 2, cur2);
