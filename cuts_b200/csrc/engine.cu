@@ -1562,6 +1562,30 @@ __host__ __device__ inline uint32_t pair_words(uint32_t p, uint32_t njp) {
     return kPS + kPS / 4 + 128 + 4 * 32 + 2 * (kCore / 32) + 32 * (kPairRows + p + 2 * njp);
 }
 
+// The pair kernel's weights: none, a fold in general, and a fold under which
+// every member of S is admissible as t and A(v) - B(v) is the same for all v of
+// one parent, so that a pair weighs the same in both orders.
+enum PairFold { kNoWeights = 0, kWeights, kEvenWeights };
+
+// Every member of S is admissible as t: C tests nothing beyond P.
+__host__ __device__ inline bool pair_same_set(const LevelPlan &P, const LevelPlan &C, uint32_t p) {
+    const uint32_t below = (1u << p) - 1;
+    const bool sig = C.sig_lo <= P.sig_lo && (!C.check_sig || (P.check_sig && C.qin <= P.qin && C.qout <= P.qout));
+    return !C.fuse_extra && sig && (C.gt_mask & below) == (P.gt_mask & below) && (C.lt_mask & below) == (P.lt_mask & below);
+}
+
+// A(v) - B(v) is the same for every v of one parent: both or neither of p and
+// c in the orbit and every membership given by the query's arcs, or a plain fold
+// that treats both alike.
+__host__ __device__ inline bool pair_even(const LevelPlan &F, uint32_t p) {
+    const uint32_t c = p + 1, below = (1u << p) - 1;
+    if (!F.ofold) return ((F.guar_mask >> p) & 1u) == ((F.guar_mask >> c) & 1u);
+    if (((F.ofold >> p) & 1u) != ((F.ofold >> c) & 1u)) return false;
+    for (uint32_t x = 0; x < p; ++x)
+        if (((F.ofold >> x) & 1u) && !((F.oguar[x] >> p) & 1u)) return false;
+    return !((F.ofold >> p) & 1u) || (F.oguar[p] & below) == below;
+}
+
 // What the level-p and level-c tests of one warp's parents need.
 struct PairCtx {
     const DevView &g;
@@ -1792,16 +1816,13 @@ __device__ __forceinline__ PairParent pair_parent(const DevView &g, const RunPar
     uint32_t *const col_off = row + 32 * kPairRows, *const col_deg = col_off + 32 * njp;                      \
     uint32_t *const col_m = col_deg + 32 * njp;                                                               \
     const uint32_t below = (1u << p) - 1;                                                                     \
-    const bool cfold = FOLD && sC.fold != 0;                                                                  \
+    const bool cfold = FOLD != 0;                                                                             \
     const uint32_t extra = sC.fuse_extra;                                                                     \
-    const bool sig_same = sC.sig_lo <= sP.sig_lo && (!sC.check_sig || (sP.check_sig && sC.qin <= sP.qin &&    \
-                                                                       sC.qout <= sP.qout));                  \
-    const bool ts = !extra && sig_same && (sC.gt_mask & below) == (sP.gt_mask & below) &&                     \
-                    (sC.lt_mask & below) == (sP.lt_mask & below);                                             \
+    const bool ts = FOLD == kEvenWeights || pair_same_set(sP, sC, p);                                         \
     const PairCtx x{g, sP, sC, sF, p, extra, cfold, ts, col_m, col_off, col_deg, row};
 
 // LOOPS: the graph has self-loops.
-template <bool FOLD, bool TALLY, bool LOOPS>
+template <int FOLD, bool TALLY, bool LOOPS>
 __global__ void __launch_bounds__(kPW * 32, 8)
 k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents parents, uint32_t phase, uint32_t split,
         uint32_t *__restrict__ cursor, PairBig big, unsigned long long *__restrict__ acc,
@@ -1813,7 +1834,10 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
     PAIR_PROLOGUE()
     const uint32_t lanemask_lt = (1u << lane) - 1, lanemask_le = lanemask_lt | (1u << lane);
     // t above s only, below s only, or both
-    const bool o1 = !((sC.lt_mask >> p) & 1u), o2 = !((sC.gt_mask >> p) & 1u);
+    const bool t_up = !((sC.lt_mask >> p) & 1u), t_down = !((sC.gt_mask >> p) & 1u);
+    // even weights: counted in one order, times the number of orders at the end
+    constexpr bool once = FOLD == kEvenWeights;
+    const bool o1 = once || t_up, o2 = !once && t_down;
     const bool phase2 = phase == 2;
     uint32_t nbig = 0;
     if (phase2) {
@@ -1826,25 +1850,16 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
     const uint32_t grab = min(phase2 ? 1u : 32u, max(1u, total / (4 * nwarps)));
     const unsigned long long deadline = run_deadline(rp);
     unsigned long long local = 0, local_c = 0, local_p = 0, tb = 0;
-    // A(v) - B(v) is the same for every v of one parent: both or neither of p
-    // and c in the orbit and every membership given by the query's arcs, or a
-    // plain fold that treats both alike
-    bool kconst = !cfold;
-    if (cfold && sF.ofold) {
-        kconst = ((sF.ofold >> p) & 1u) == ((sF.ofold >> (p + 1)) & 1u);
-        for (uint32_t xm = sF.ofold & below; xm; xm &= xm - 1) kconst = kconst && ((sF.oguar[__ffs(xm) - 1] >> p) & 1u);
-        if ((sF.ofold >> p) & 1u) kconst = kconst && (sF.oguar[p] & below) == below;
-    } else if (cfold) {
-        kconst = ((sF.guar_mask >> p) & 1u) == ((sF.guar_mask >> (p + 1)) & 1u);
-    }
+    const bool kconst = FOLD != kWeights || pair_even(sF, p);
     const uint32_t orders = (o1 ? 1u : 0u) + (o2 ? 1u : 0u);
-    // with every member admissible, A(s) + B(t) is then the same for both orders
-    // of a pair (A is B plus a constant), so a hit costs one weight and no test:
-    // triangle + pendant, 60-regular graph of 700,003 vertices, plain 17.2 ->
-    // 12.1 ms, symmetry breaking 5.8 -> 5.0; 4-clique + pendant, 1M / 10M 8.1 ->
-    // 7.5.  degs: B is the degree less this
-    const bool even = FOLD && cfold && ts && kconst;
-    const uint32_t degs = FOLD && !LOOPS && sF.ofold && ((sF.ofold >> (p + 1)) & 1u) ? p + 1 : 0u;
+    const uint32_t times = once && t_up && t_down ? 2u : 1u;
+    // even weights: a hit costs one of them and no test, in an instance without
+    // the code of the others, for the fold's inner loop is bound by the
+    // instruction cache.  Triangle + pendant, 60-regular graph of 700,003
+    // vertices, plain 17.2 -> 11.9 ms; 50,000, symmetry breaking 0.50 -> 0.37;
+    // power law, 1M / 10M, 2.93 -> 2.59; 4-clique + pendant there 7.8 -> 6.3.
+    // degs: B is the degree less this
+    const uint32_t degs = once && !LOOPS && ((sF.ofold >> (p + 1)) & 1u) ? p + 1 : 0u;
     uint32_t free_pos = below;  // positions below p whose lists P does not join (all with self-loops)
     if (!LOOPS)
         for (uint32_t t = 0; t < njp; ++t) free_pos &= ~(1u << sP.jpos[t]);
@@ -2018,12 +2033,11 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                     const uint32_t r = __popc(ilive & lanemask_lt), excl = iincl - ilen;
                     rec[r] = make_uint4(ibase - excl, ow | (mode << 8) | (i << 16), ioff, ideg);
                     starts[r] = excl;
-                    if (FOLD) itemA[r] = o1 || even ? pair_a<LOOPS>(x, ow, a) : 0u;
+                    if (FOLD) itemA[r] = o1 ? pair_a<LOOPS>(x, ow, a) : 0u;
                 }
                 __syncwarp();
                 const uint32_t my_start = uint32_t(lane) < uint32_t(__popc(ilive)) ? starts[lane] : kFullMask;
-                uint32_t started = 0, hits = 0;   // hits: of a batch whose pairs weigh the same in both orders
-                unsigned long long weight = 0;    // their weights in one order
+                uint32_t started = 0, hits = 0;  // hits: of a batch without weights
                 for (uint32_t fstep = 0; fstep < itotal; fstep += 64) {
                     uint4 rc[2];
                     uint32_t tv[2], rk[2];
@@ -2056,10 +2070,10 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                                       : pair_above_in_set(x, rc[h].y & 255u, free_pos, t);
                         if (!FOLD && ts) {
                             hits += ok;
-                        } else if (FOLD && even) {
+                        } else if (once) {
                             if (ok) {
-                                ++hits;
-                                weight += uint32_t(itemA[rk[h]] + (degs ? g.out_info[t].y - degs : pair_b<LOOPS>(x, rc[h].y & 255u, t)));
+                                ++local_c;
+                                local += uint32_t(itemA[rk[h]] + (degs ? g.out_info[t].y - degs : pair_b<LOOPS>(x, rc[h].y & 255u, t)));
                             }
                         } else if (ok) {
                             const uint32_t l = rc[h].y & 255u;
@@ -2077,7 +2091,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
                         }
                     }
                 }
-                local += (FOLD ? weight : uint64_t(hits)) * orders;
+                local += uint64_t(hits) * orders;
                 local_c += uint64_t(hits) * orders;
                 __syncwarp();
             }
@@ -2194,6 +2208,8 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
         }
         __syncwarp();
     }
+    local *= times;
+    local_c *= times;
     #pragma unroll
     for (int o = 16; o; o >>= 1) {
         local += __shfl_xor_sync(kFullMask, local, o);
@@ -2209,7 +2225,7 @@ k_pairs(DevView g, const RunParams *__restrict__ rp, uint32_t p, const Parents p
 }
 
 // Core members of the deferred parents' sets, one warp per parent.
-template <bool FOLD>
+template <int FOLD>
 __global__ void __launch_bounds__(kPW * 32)
 k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big) {
     const unsigned long long n0 = big.n[0];
@@ -2735,7 +2751,7 @@ int g_level_blocks[3] = {0, 0, 0};
 int g_flat_blocks[3][kFolds] = {};  // blocks of k_level_flat<mode, fold> per SM by registers and threads
 int g_fused_blocks[3] = {0, 0, 0};
 int g_edge_blocks = 0;  // blocks of k_edges per SM by registers and threads
-int g_pair_blocks[2] = {0, 0};  // blocks of k_pairs<fold> per SM by registers and threads
+int g_pair_blocks[3] = {0, 0, 0};  // blocks of k_pairs<fold> per SM by registers and threads
 // CUTS_LEVEL_KERNEL=warp selects the warp-per-parent form (A/B comparisons)
 bool g_use_flat = true;
 
@@ -2768,10 +2784,12 @@ int launch_geometry() {
     g_fused_blocks[kCountMode] = std::max(1, b) * g_num_sms;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused<kBytesMode>, kZW * 32, 0));
     g_fused_blocks[kBytesMode] = std::max(1, b) * g_num_sms;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<false, false, false>, kPW * 32, 0));
-    g_pair_blocks[0] = std::max(1, b);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<true, false, false>, kPW * 32, 0));
-    g_pair_blocks[1] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<kNoWeights, false, false>, kPW * 32, 0));
+    g_pair_blocks[kNoWeights] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<kWeights, false, false>, kPW * 32, 0));
+    g_pair_blocks[kWeights] = std::max(1, b);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs<kEvenWeights, false, false>, kPW * 32, 0));
+    g_pair_blocks[kEvenWeights] = std::max(1, b);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edges<true, false>, kPW * 32, 0));
     g_edge_blocks = std::max(1, b);
     const char *kv = std::getenv("CUTS_LEVEL_KERNEL");
@@ -3113,7 +3131,10 @@ struct Run {
             // / 300,000 plain, lists of 250, would lose 0.54 -> 0.60)
             const uint32_t few = (hp->plan.lv[p].gt_mask | hp->plan.lv[p].lt_mask ? 4 : 3) * kPK;
             if (p == 1 && (es || g.fuse_split || g.max_deg > few)) split = std::min(split, kPK);
-            const bool fold = hp->plan.lv[p + 1].fold != 0;
+            const LevelPlan &LP = hp->plan.lv[p], &LC = hp->plan.lv[p + 1];
+            const int fold = !LC.fold ? kNoWeights
+                             : pair_same_set(LP, LC, p) && pair_even(hp->plan.lv[p + 2], p) ? kEvenWeights
+                                                                                          : kWeights;
             const uint32_t smem = 4 * kPW * pair_words(p, hp->plan.lv[p].nj);
             const uint32_t fixed = 3 * uint32_t(sizeof(LevelPlan)) + 16 * kMaxK + 1024;
             const uint32_t full = std::max(1u, std::min(uint32_t(g_pair_blocks[fold]), 227u * 1024u / (smem + fixed))) *
@@ -3125,9 +3146,14 @@ struct Run {
             };
             auto phase = [&](uint32_t grid, uint32_t ph, uint32_t *cur) {
                 // (the byte tally is not timed: one instance, for graphs with and without loops)
-                if (tal) fold ? go(k_pairs<true, true, true>, grid, ph, cur) : go(k_pairs<false, true, true>, grid, ph, cur);
-                else if (g.loops) fold ? go(k_pairs<true, false, true>, grid, ph, cur) : go(k_pairs<false, false, true>, grid, ph, cur);
-                else fold ? go(k_pairs<true, false, false>, grid, ph, cur) : go(k_pairs<false, false, false>, grid, ph, cur);
+                auto pick = [&](auto *none, auto *any, auto *even) {
+                    go(fold == kNoWeights ? none : fold == kWeights ? any : even, grid, ph, cur);
+                };
+                if (tal) pick(k_pairs<kNoWeights, true, true>, k_pairs<kWeights, true, true>, k_pairs<kWeights, true, true>);
+                else if (g.loops)
+                    pick(k_pairs<kNoWeights, false, true>, k_pairs<kWeights, false, true>, k_pairs<kEvenWeights, false, true>);
+                else
+                    pick(k_pairs<kNoWeights, false, false>, k_pairs<kWeights, false, false>, k_pairs<kEvenWeights, false, false>);
             };
             phase(blocks, 1, cur1);
             CK(cudaGetLastError());
@@ -3136,7 +3162,7 @@ struct Run {
             const uint32_t turn = std::min(32u, std::max(1u, most / (4 * blocks * kPW)));
             if (pair_defers(p, split, g.max_deg, uint64_t(turn) * g.max_deg)) {
                 k_fused_scan<<<1, 1024, 0, g.stream>>>(pb.n, pb.cap, pb.len, kPK, pb.pref);
-                k_pair_bits<false><<<full, kPW * 32, smem, g.stream>>>(view, dp, p, pb);
+                k_pair_bits<kNoWeights><<<full, kPW * 32, smem, g.stream>>>(view, dp, p, pb);
                 phase(full, 2, cur2);
                 CK(cudaGetLastError());
                 res.launches += 3;
