@@ -1,7 +1,8 @@
 """Fused pairs on graphs of bounded degree with enough roots that a warp takes
 up to 32 of them a turn: the parents that its first launch leaves to the second
-are counted there whatever the largest degree (40, 60, 64 and 65: below, at and
-above the length from which a single window is dealt out in pieces).
+are counted there whatever the largest degree (40, 60, 64 and 65), and so are
+windows dealt out in pieces because the longest list is long enough for it (192
+and 193 entries, 256 and 257 with an order).
 
 The graphs are circulants, vertex i joined to i +- 1 .. i +- r, whose counts
 are known: r (r - 1) / 2 triangles per vertex.  Labels are permuted, so the
@@ -37,7 +38,8 @@ def _circulant(n, r, extra=False):
     return off, out
 
 
-@pytest.mark.parametrize("n,r,extra", [(700003, 20, False), (700003, 30, False), (400009, 32, False), (400009, 32, True)])
+@pytest.mark.parametrize("n,r,extra", [(700003, 20, False), (700003, 30, False), (400009, 32, False), (400009, 32, True)] +
+                         [(20011, 96, x) for x in (False, True)] + [(9001, 128, x) for x in (False, True)])
 def test_all_deferred_parents_counted(n, r, extra):
     off, adj = _circulant(n, r, extra)
     g = cb.Graph.from_csr(n, off, adj)
