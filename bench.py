@@ -559,7 +559,8 @@ def main():
                 ex_ms += r.expand_ms
                 lv, _ = q.plan_levels(sym, args.flags)
                 fused = any(x["fuse"] for x in lv) and os.environ.get("CUTS_NO_FUSE") != "1"
-                kinds.append(f"{'k_pairs' if fused else 'counting kernel'} ({name})")
+                pairs = not any(os.environ.get(v, "")[:1] == "0" for v in ("CUTS_FUSE_WALK", "CUTS_TABLES"))
+                kinds.append(f"{('k_pairs' if pairs else 'k_fused') if fused else 'counting kernel'} ({name})")
             achieved = (ll_bytes / max(ll_n, 1)) / ((ll_ms / max(ll_n, 1)) / 1e3) / 1e9 if ll_ms else None
             roofline.update({
                 "kernel": "last counted level: " + ", ".join(kinds),
@@ -571,10 +572,11 @@ def main():
                 "l2_hit_rate_ncu": ncu.get("l2_hit_rate"),
                 "l2_throughput_frac_ncu": ncu.get("l2_throughput_frac"),
                 "note": "achieved = the bytes the counting launch's algorithm reads from global memory "
-                        "(tallied by the same kernel in an untimed pass) / its CUDA-event time; the 90 MB "
-                        "graph and the 128 KB core bitmap are served from L2 (l2_hit_rate_ncu), DRAM is "
-                        "nearly idle (dram_frac_ncu), so the kernel is bound by L2 latency and issue; frac "
-                        "is against the measured HBM copy bandwidth as the measurement asks",
+                        "(tallied by the same kernel in an untimed pass) / its CUDA-event time; of the 270 MB "
+                        "of graph and membership tables, what the hub slice reads and the 128 KB core bitmap "
+                        "are served from L2 (l2_hit_rate_ncu), DRAM is nearly idle there (dram_frac_ncu), so "
+                        "the kernel is bound by L2 latency, issue and the instruction cache; frac is against "
+                        "the measured HBM copy bandwidth as the measurement asks",
             })
 
         cpu = None

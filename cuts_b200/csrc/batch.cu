@@ -12,10 +12,10 @@
 // Warps take tasks from one global counter (work stealing across all SMs)
 // and run the query's levels depth-first from the task's level-1 range,
 // with a 32-candidate frontier per level in shared memory: the trie is
-// walked, never stored, so a batch needs no trie arena.  Each level step is
-// the same warp-cooperative join as the level kernels: candidates from the
-// shortest joined list, one per lane, lower-bound membership in the other
-// lists, ballot/popc compaction.  Counts accumulate per warp and are added
+// walked, never stored, so a batch needs no trie arena.  A level step takes 32
+// candidates of the shortest joined list, one per lane, tests them in the other
+// lists' tables (by search without tables) and compacts them with a ballot; the
+// last level is counted for a whole frontier at once (count_frontier).  Counts accumulate per warp and are added
 // to the query's counter when the warp moves on.  A device-clock budget
 // stops the launch cleanly: tasks not finished mark their query incomplete.
 #include <cuda_runtime.h>
@@ -205,8 +205,8 @@ __device__ unsigned long long count_level_fold(const Ctx &c, uint32_t d) {
 // walked 64 candidates a step, as in k_level_flat (engine.cu).  Counting one
 // frontier vertex after another left most lanes idle on short lists: 64 mixed
 // queries of 3 and 4 vertices on 200,000 vertices / 1.6M edges took 480 ms,
-// 207 ms this way.  With a fold at e, each candidate adds the closed form
-// of level e + 1.  Returns the lane's part of the count.
+// 207 ms this way (60 ms since, with twins and edge counts).  With a fold at e,
+// each candidate adds the closed form of level e + 1.  Returns the lane's part of the count.
 __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
     const uint32_t e = d + 1, nj = c.Q->lv[e].nj;
     const BLevel &L = c.Q->lv[e];

@@ -8,10 +8,14 @@
 // signature.  The last level is counted, not stored.
 //
 // B200 layout of the work:
-//   * one warp per parent entry, parents handed out by a global work cursor
-//     in grains (work stealing across all SMs of a persistent grid);
-//   * the smallest joined list supplies the candidates (32 per step, one
-//     per lane); membership in the other lists is a lower-bound search;
+//   * a warp takes up to 32 parent entries, one per lane, handed out by a global
+//     work cursor in turns (work stealing across all SMs of a persistent grid);
+//   * each parent's smallest joined list supplies its candidates, the windows of
+//     all lanes one sequence walked 64 a step; membership in the other lists is
+//     one table read (in_list), a search of the list without tables;
+//   * the last two or three levels are counted together where the plan allows:
+//     closed forms and folds (k_level_flat), pairs of one candidate set (k_pairs,
+//     k_fused), edges between two (k_edges);
 //   * survivors are placed with a warp ballot/popc into a per-warp shared
 //     staging buffer and flushed with one global atomic per buffer, so the
 //     next level is written in coalesced runs;
@@ -1502,13 +1506,13 @@ k_fused_scan(const unsigned long long *__restrict__ nb, uint32_t cap, const uint
 // deals them out in pieces of kPK candidates (their core members as bitmaps
 // from k_pair_bits); a piece pairs its vertices with neighbours above only.
 //
-// Bound: L2 latency and instruction issue (46 % of issue slots in the 4-clique
-// + pendant's hub slice).  Whole counts against the form with one parent per
+// Bound: L2 latency, instruction issue and the instruction cache (46 % of issue
+// slots in the 4-clique + pendant's hub slice).  Whole counts against the form with one parent per
 // warp, a hash table of S in shared memory and a degree gather per pair (and,
 // without an order between p and c, galloping intersections): 4-clique +
-// pendant, 1M vertices / 10M edges, symmetry breaking 33.4 -> 8.2 ms; triangle
+// pendant, 1M vertices / 10M edges, symmetry breaking 33.4 -> 6.6 ms; triangle
 // there, plain 75.5 -> 6.2 ms; triangle, 4M / 40M, symmetry breaking 20.2 ->
-// 9.2 ms.
+// 9.1 to 10.3 ms.
 constexpr int kPW = 4;            // warps per block
 constexpr uint32_t kPS = 512;     // candidates of one round, shared memory words per warp
 constexpr uint32_t kPC = 32;      // core members from which a set's core part is counted by rows
@@ -2285,8 +2289,8 @@ k_pair_bits(DevView g, const RunParams *__restrict__ rp, uint32_t p, PairBig big
 // vertices / 1M edges has 6.9e9 of them with 1.5 last-level candidates each.
 // Whole counts against expanding L_d and counting its entries: that 5-cycle
 // 273 -> 45 ms, the house on 100,000 / 500,000 22 -> 18.4 ms, the 4-cycle on
-// 10,000 / 40,000 117 -> 101 us.  Bound: instruction issue (55 % of slots) and
-// L2 latency.
+// 10,000 / 40,000 117 -> 101 us.  Bound: instruction issue (45 % of slots), L1
+// (79 % of its throughput) and L2 latency.
 constexpr uint32_t kECore = 8;    // core members of each set from which they are counted by rows
 enum EdgeRow : int { kECOff = 0, kECDeg, kETOff, kETDeg, kEOLo, kEOHi, kEOBase, kEOLen, kESide, kEMatched, kEONear, kECut, kEdgeRows };
 

@@ -268,6 +268,8 @@ int cuts_search(const char *query_file, const char *data_file, int write_to_disk
 typedef struct cuts_mlp_s *cuts_mlp;
 int cuts_mlp_create(uint32_t in_dim, uint64_t seed, int device, cuts_mlp *out);
 int cuts_mlp_param_count(cuts_mlp m, uint32_t *n);
+/* The weights rounded to FP32 (they are kept in FP64): a model given them by
+ * cuts_mlp_set_params predicts the same to FP32 rounding of the weights. */
 int cuts_mlp_get_params(cuts_mlp m, float *params);
 int cuts_mlp_set_params(cuts_mlp m, const float *params);
 /* Mean squared error over n rows and its gradient (n_params floats). */
