@@ -1059,16 +1059,19 @@ uint32_t na_block(unsigned long long roots, uint32_t warps, bool deep) {
 }
 
 __global__ void __launch_bounds__(kBW * 32)
-k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq, uint32_t blk, uint32_t upblk,
+k_batch_noalloc(DevView g, NoAllocScratch *__restrict__ sc, uint32_t nq, uint32_t blk, uint32_t deep,
                 unsigned long long *__restrict__ counts) {
     __shared__ BWarp ws[kBW];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Ctx c{g, nullptr, &ws[warp], lane};
     // the task space, in shared memory (registers are what this kernel is short of)
     __shared__ unsigned long long upper, total;  // tasks of the slices above 0, and all
-    __shared__ uint32_t slices, nblk[2];
+    __shared__ uint32_t slices, nblk[2], upblk;
     if (threadIdx.x == 0) {
         slices = min(kSlices, (max(sc->longest, 1u) - 1) / kSliceLen + 1);
+        // blocks of the slices above 0: most such tasks find nothing, but a few
+        // roots of deep queries in one are a tail where there are few slices
+        upblk = max(blk, deep ? min(8u, slices) : 32u);
         nblk[0] = (g.n - 1) / upblk + 1;
         nblk[1] = (g.n - 1) / blk + 1;
         upper = (unsigned long long)nq * nblk[0] * (slices - 1);
@@ -1235,12 +1238,11 @@ int count_noalloc(const uint32_t *info_out, const uint32_t *info_in, const uint3
                        reinterpret_cast<const uint2 *>(sym ? info_out : info_in), adj, n, nullptr, nullptr,
                        nullptr, 0, nullptr};
     const uint32_t blk = na_block((unsigned long long)nq * n, blocks * kBW, deep);
-    const uint32_t upblk = std::max(blk, deep ? 8u : 32u);  // of the slices above 0: most such tasks find nothing
     k_noalloc_longest<<<std::min<uint32_t>((n - 1) / 256 + 1, blocks), 256, 0, stream>>>(view.out_info, view.in_info, n, sc);
     const unsigned long long total =
-        (unsigned long long)nq * ((n - 1) / blk + 1 + (unsigned long long)((n - 1) / upblk + 1) * (kSlices - 1));
+        (unsigned long long)nq * ((n - 1) / blk + 1) * kSlices;  // at most
     const uint32_t grid = uint32_t(std::min<unsigned long long>(blocks, (total + kBW - 1) / kBW));
-    k_batch_noalloc<<<std::max<uint32_t>(grid, 1), kBW * 32, 0, stream>>>(view, sc, nq, blk, upblk, counts);
+    k_batch_noalloc<<<std::max<uint32_t>(grid, 1), kBW * 32, 0, stream>>>(view, sc, nq, blk, deep ? 1 : 0, counts);
     if (cudaGetLastError() != cudaSuccess)
         return set_error(CUTS_ERR_CUDA, "cuts_count_noalloc: launch failed");
     return CUTS_OK;
