@@ -15,9 +15,10 @@
 // walked, never stored, so a batch needs no trie arena.  A level step takes 32
 // candidates of the shortest joined list, one per lane, tests them in the other
 // lists' tables (by search without tables) and compacts them with a ballot; the
-// last level is counted for a whole frontier at once (count_frontier).  Counts accumulate per warp and are added
-// to the query's counter when the warp moves on.  A device-clock budget
-// stops the launch cleanly: tasks not finished mark their query incomplete.
+// last level is counted for a whole frontier at once (count_frontier).  Counts
+// accumulate per warp and are added to the query's counter when the warp moves
+// on.  A device-clock budget stops the launch cleanly: tasks not finished mark
+// their query incomplete.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -206,7 +207,8 @@ __device__ unsigned long long count_level_fold(const Ctx &c, uint32_t d) {
 // frontier vertex after another left most lanes idle on short lists: 64 mixed
 // queries of 3 and 4 vertices on 200,000 vertices / 1.6M edges took 480 ms,
 // 207 ms this way (60 ms since, with twins and edge counts).  With a fold at e,
-// each candidate adds the closed form of level e + 1.  Returns the lane's part of the count.
+// each candidate adds the closed form of level e + 1.  Returns the lane's part of
+// the count.
 __device__ unsigned long long count_frontier(const Ctx &c, uint32_t d) {
     const uint32_t e = d + 1, nj = c.Q->lv[e].nj;
     const BLevel &L = c.Q->lv[e];
@@ -926,17 +928,18 @@ int Batch::run(double budget_ms, std::vector<uint64_t> &counts, std::vector<int>
         counts[i] = r.count;
         t += r.ms;
     }
-    if (!again.empty() && (rc = run_spare(again, budget_ms > 0 ? left : 0, counts, status, t))) return rc;
+    if (!again.empty()) {
+        rc = budget_ms > 0 && left <= 0 ? CUTS_ERR_BUDGET
+                                        : run_spare(again, budget_ms > 0 ? left : 0, counts, status, t);
+        if (rc)
+            for (uint32_t i : again) status[i] = rc;
+    }
     if (ms) *ms = t;
     return CUTS_OK;
 }
 
 int Batch::run_spare(const std::vector<uint32_t> &which, double budget_ms, std::vector<uint64_t> &counts,
                      std::vector<int> &status, float &ms) {
-    if (budget_ms < 0) {
-        for (uint32_t i : which) status[i] = CUTS_ERR_BUDGET;
-        return CUTS_OK;
-    }
     if (!spare || spare_of != which) {
         if (spare) spare->destroy();
         spare = std::make_unique<Batch>();
@@ -986,7 +989,7 @@ struct NoAllocScratch {
     BQuery queries[kNoAllocMaxQueries];
     unsigned long long task_ctr;
     uint32_t stop;
-    uint32_t longest;  // list of the graph (or kSlices slices' worth)
+    uint32_t longest;  // the graph's longest list
     uint32_t aborted[kNoAllocMaxQueries];
 };
 
@@ -1051,8 +1054,8 @@ k_noalloc_longest(const uint2 *__restrict__ info_out, const uint2 *__restrict__ 
 constexpr uint32_t kSlices = 16;
 constexpr uint32_t kSliceLen = 32;
 
-// Roots per block of slice 0 for `roots` (query, root) pairs on `warps` warps: 4 blocks a
-// warp or more, 16 where subtrees are deep (5 vertices and more).
+// Roots per block of slice 0 for `roots` (query, root) pairs on `warps` warps: 4
+// blocks a warp or more, 16 where subtrees are deep (5 vertices and more).
 uint32_t na_block(unsigned long long roots, uint32_t warps, bool deep) {
     const unsigned long long per = roots / ((unsigned long long)warps * (deep ? 16 : 4));
     return uint32_t(std::max<unsigned long long>(1, std::min<unsigned long long>(32, per)));
