@@ -351,33 +351,61 @@ void Mlp::destroy() {
     d_grad = nullptr;
 }
 
+int Mlp::Room::alloc(size_t bytes) {
+    pooled = bytes >= (size_t(2) << 20);
+    if (pooled) MCK(cudaMallocAsync(&p, bytes, cudaStreamLegacy));
+    else MCK(cudaMalloc(&p, bytes));
+    return CUTS_OK;
+}
+
+void Mlp::Room::free() {
+    if (!p) return;
+    if (pooled) cudaFreeAsync(p, cudaStreamLegacy);
+    else cudaFree(p);
+    p = nullptr;
+}
+
 void Mlp::release() {
-    if (d_part && pooled) cudaFreeAsync(d_part, cudaStreamLegacy);
-    else cudaFree(d_part);
+    part.free();
+    samples.free();
     d_part = nullptr;
     d_X = nullptr;
     cap_rows = part_blocks = 0;
 }
 
 // Room for the partial gradients of `blocks` blocks and for `rows` staged
-// samples, kept for later calls: one allocation for both, for a model's first
-// fit is usually its only one.  Below 2 MB from the runtime's allocator, which
-// has such blocks at hand (first fit of 500 rows x 2 epochs 0.13 ms, from the
-// pool 0.37), larger ones from the device's pool: there a program that has
-// loaded a graph has the memory already (4,096 rows, one step: 0.42 ms from
-// the runtime, 0.32 to 0.35 from the pool, 0.10 after a graph; the form with
-// shared-memory atomics, which had no partials, 0.38).
+// samples, kept for later calls: one allocation where both have to grow, for a
+// model's first fit is usually its only one.  Below 2 MB from the runtime's
+// allocator, which has such blocks at hand (first fit of 500 rows x 2 epochs
+// 0.13 ms, from the pool 0.37), larger ones from the device's pool: there a
+// program that has loaded a graph has the memory already (4,096 rows, one
+// step: 0.42 ms from the runtime, 0.32 to 0.35 from the pool, 0.10 after a
+// graph; the form with shared-memory atomics, which had no partials, 0.38).
+// Where one of the two outgrows its room the other stays: a fit of 672 rows,
+// then a prediction of 937, gives the samples a small block of their own
+// (0.05 ms; with the partials allocated anew 0.75).
 int Mlp::reserve(int rows, int blocks) {
-    if (rows <= cap_rows && blocks <= part_blocks) return CUTS_OK;
+    const bool more_part = blocks > part_blocks, more_rows = rows > cap_rows;
+    if (!more_part && !more_rows) return CUTS_OK;
+    const bool inside = d_X && !samples.p;  // the samples lie behind the partials
+    const size_t part_bytes = sizeof(double) * size_t(n_params(in)) * size_t(std::max(blocks, part_blocks));
+    const size_t x_bytes = sizeof(float) * size_t(std::max(rows, cap_rows)) * (in + 2);
+    int rc;
+    if (!more_part || (!more_rows && !inside)) {
+        Room &r = more_part ? part : samples;
+        if (more_part) d_part = nullptr, part_blocks = 0;
+        else d_X = nullptr, cap_rows = 0;
+        r.free();
+        if ((rc = r.alloc(more_part ? part_bytes : x_bytes))) return rc;
+        if (more_part) d_part = static_cast<double *>(part.p), part_blocks = blocks;
+        else d_X = static_cast<float *>(samples.p), cap_rows = rows;
+        return CUTS_OK;
+    }
     rows = std::max(rows, cap_rows);
-    blocks = std::max(blocks, part_blocks);
     release();
-    const size_t part = size_t(n_params(in)) * size_t(blocks);
-    const size_t bytes = sizeof(double) * part + sizeof(float) * size_t(rows) * (in + 2);
-    pooled = bytes >= (size_t(2) << 20);
-    if (pooled) MCK(cudaMallocAsync(reinterpret_cast<void **>(&d_part), bytes, cudaStreamLegacy));
-    else MCK(cudaMalloc(&d_part, bytes));
-    d_X = reinterpret_cast<float *>(d_part + part);
+    if ((rc = part.alloc(part_bytes + x_bytes))) return rc;
+    d_part = static_cast<double *>(part.p);
+    d_X = reinterpret_cast<float *>(static_cast<char *>(part.p) + part_bytes);
     cap_rows = rows;
     part_blocks = blocks;
     return CUTS_OK;

@@ -1,5 +1,6 @@
 // mlp.hpp -- MLP cost model for the learned matching order.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 
 #include "host.hpp"
@@ -18,9 +19,8 @@ struct Mlp {
     // weights and Adam's moments in FP64 (FP32 at the interface)
     double *d_params = nullptr, *d_m = nullptr, *d_v = nullptr;
     float *d_grad = nullptr;
-    double *d_part = nullptr;   // [part_blocks][params]: partial gradients of one step; d_X lies behind it
+    double *d_part = nullptr;   // [part_blocks][params]: partial gradients of one step
     int part_blocks = 0;
-    bool pooled = false;        // d_part comes from the device's memory pool
     double *d_loss = nullptr;   // [max_blocks]: partial sums of squared errors
     int max_blocks = 1;
     float *d_X = nullptr;  // staged samples: X rows, then targets / outputs
@@ -39,6 +39,14 @@ struct Mlp {
     int set_params(const float *p);
 
   private:
+    // device memory from the runtime's allocator, or from the pool where large
+    struct Room {
+        void *p = nullptr;
+        bool pooled = false;
+        int alloc(size_t bytes);
+        void free();
+    };
+    Room part, samples;  // samples: unused while d_X lies behind the partials
     int upload(const float *X, const float *T, int n, int blocks);
     int grid_for(int n) const;
     int reserve(int rows, int blocks);
