@@ -351,8 +351,22 @@ void Mlp::destroy() {
     d_grad = nullptr;
 }
 
-int Mlp::Room::alloc(size_t bytes) {
-    pooled = bytes >= (size_t(2) << 20);
+// Below 2 MB from the runtime's allocator, which has such blocks at hand (first
+// fit of 500 rows x 2 epochs 0.13 ms, from the pool 0.37).  Larger ones from
+// the device's pool where it holds that much unused, as after a graph (4,096
+// rows, one step: 0.10 ms, from the runtime 0.42 to 0.5; the form with
+// shared-memory atomics, which had no partials, 0.38 to 0.42); a pool that has
+// to grow is not asked, for its first growth in a process takes 6 ms.
+int Mlp::Room::alloc(int device, size_t bytes) {
+    pooled = false;
+    cudaMemPool_t pool = nullptr;
+    uint64_t held = 0, used = 0;
+    if (bytes >= (size_t(2) << 20)) {
+        MCK(cudaDeviceGetDefaultMemPool(&pool, device));
+        MCK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+        MCK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+        pooled = held >= used + bytes;
+    }
     if (pooled) MCK(cudaMallocAsync(&p, bytes, cudaStreamLegacy));
     else MCK(cudaMalloc(&p, bytes));
     return CUTS_OK;
@@ -375,15 +389,10 @@ void Mlp::release() {
 
 // Room for the partial gradients of `blocks` blocks and for `rows` staged
 // samples, kept for later calls: one allocation where both have to grow, for a
-// model's first fit is usually its only one.  Below 2 MB from the runtime's
-// allocator, which has such blocks at hand (first fit of 500 rows x 2 epochs
-// 0.13 ms, from the pool 0.37), larger ones from the device's pool: there a
-// program that has loaded a graph has the memory already (4,096 rows, one
-// step: 0.42 ms from the runtime, 0.32 to 0.35 from the pool, 0.10 after a
-// graph; the form with shared-memory atomics, which had no partials, 0.38).
-// Where one of the two outgrows its room the other stays: a fit of 672 rows,
-// then a prediction of 937, gives the samples a small block of their own
-// (0.05 ms; with the partials allocated anew 0.75).
+// model's first fit is usually its only one.  Where one of the two outgrows its
+// room the other stays: a fit of 672 rows, then a prediction of 937, gives the
+// samples a small block of their own (0.05 ms; with the partials allocated anew
+// 0.75).
 int Mlp::reserve(int rows, int blocks) {
     const bool more_part = blocks > part_blocks, more_rows = rows > cap_rows;
     if (!more_part && !more_rows) return CUTS_OK;
@@ -396,14 +405,14 @@ int Mlp::reserve(int rows, int blocks) {
         if (more_part) d_part = nullptr, part_blocks = 0;
         else d_X = nullptr, cap_rows = 0;
         r.free();
-        if ((rc = r.alloc(more_part ? part_bytes : x_bytes))) return rc;
+        if ((rc = r.alloc(device, more_part ? part_bytes : x_bytes))) return rc;
         if (more_part) d_part = static_cast<double *>(part.p), part_blocks = blocks;
         else d_X = static_cast<float *>(samples.p), cap_rows = rows;
         return CUTS_OK;
     }
     rows = std::max(rows, cap_rows);
     release();
-    if ((rc = part.alloc(part_bytes + x_bytes))) return rc;
+    if ((rc = part.alloc(device, part_bytes + x_bytes))) return rc;
     d_part = static_cast<double *>(part.p);
     d_X = reinterpret_cast<float *>(static_cast<char *>(part.p) + part_bytes);
     cap_rows = rows;

@@ -43,7 +43,7 @@ struct Mlp {
     struct Room {
         void *p = nullptr;
         bool pooled = false;
-        int alloc(size_t bytes);
+        int alloc(int device, size_t bytes);
         void free();
     };
     Room part, samples;  // samples: unused while d_X lies behind the partials
